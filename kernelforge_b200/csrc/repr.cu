@@ -58,29 +58,40 @@ __device__ inline double half_cos_decay(double r, double cut) {
     return 0.5 * (cos(M_PI * r / cut) + 1.0);
 }
 
-// Two-body radial value and d/dr for basis function k.
-__device__ inline void two_body(const ReprParams &P, double r, int k, double &v, double &dv) {
+// Two-body terms of a distance that do not depend on the basis function, with
+// their derivatives: mu, sig^2 and the prefactor.
+struct TwoBody {
+    double mu, s2, pref, dpref, dmu, ds2;
+};
+__device__ inline TwoBody two_body_terms(const ReprParams &P, double r) {
     const double t = P.eta2 / fmax(r * r, REPR_EPS);
     const double s2 = log1p(t);
     const double sig = sqrt(fmax(s2, 0.0));
-    v = dv = 0.0;
-    if (sig < REPR_EPS) return;
-    const double mu = log(r) - 0.5 * s2;
-    const double ds2 = -2.0 * t / (r * (1.0 + t));
-    const double dsig = ds2 / (2.0 * sig);
-    const double dmu = 1.0 / r - 0.5 * ds2;
+    if (sig < REPR_EPS) return {0.0, 1.0, 0.0, 0.0, 0.0, 0.0};
+    TwoBody b;
+    b.s2 = s2;
+    b.mu = log(r) - 0.5 * s2;
+    b.ds2 = -2.0 * t / (r * (1.0 + t));
+    const double dsig = b.ds2 / (2.0 * sig);
+    b.dmu = 1.0 / r - 0.5 * b.ds2;
     const double dec = half_cos_decay(r, P.rcut);
     const double ddec = -0.5 * M_PI / P.rcut * sin(M_PI * r / P.rcut);
     const double rp = pow(r, -P.p2);
     const double c = 1.0 / (sqrt(2.0 * M_PI) * sig);
-    const double pref = dec * rp * c;
-    const double dpref = (ddec * rp - dec * P.p2 * rp / r) * c - pref * dsig / sig;
+    b.pref = dec * rp * c;
+    b.dpref = (ddec * rp - dec * P.p2 * rp / r) * c - b.pref * dsig / sig;
+    return b;
+}
+
+// Two-body radial value and d/dr for basis function k.
+__device__ inline void two_body(const ReprParams &P, const TwoBody &b, int k, double &v,
+                                double &dv) {
     const double Rs = P.rcut * (k + 1) / P.nRs2;
-    const double L = log(Rs) - mu;
-    const double g = exp(-0.5 * L * L / s2);
-    const double dg = g * (L * dmu / s2 + 0.5 * L * L * ds2 / (s2 * s2));
-    v = pref * g / Rs;
-    dv = (dpref * g + pref * dg) / Rs;
+    const double L = log(Rs) - b.mu;
+    const double g = exp(-0.5 * L * L / b.s2);
+    const double dg = g * (L * b.dmu / b.s2 + 0.5 * L * L * b.ds2 / (b.s2 * b.s2));
+    v = b.pref * g / Rs;
+    dv = (b.dpref * g + b.pref * dg) / Rs;
 }
 
 // Angular basis of the centre angle: cos(o theta), sin(o theta) times the
@@ -220,7 +231,8 @@ __global__ void __launch_bounds__(REPR_WARPS * 32) fchl19_kernel(
             for (int e = lane; e < P.three_off; e += 32) {
                 const int k = e - eo * P.nRs2;
                 double v = 0.0, dv = 0.0;
-                if (k >= 0 && k < P.nRs2 && r_io <= P.rcut) two_body(P, r_io, k, v, dv);
+                if (k >= 0 && k < P.nRs2 && r_io <= P.rcut)
+                    two_body(P, two_body_terms(P, r_io), k, v, dv);
                 const double g[3] = {dv * dio.x / r_io, dv * dio.y / r_io, dv * dio.z / r_io};
 #pragma unroll
                 for (int t = 0; t < 3; ++t) {
@@ -232,7 +244,7 @@ __global__ void __launch_bounds__(REPR_WARPS * 32) fchl19_kernel(
         } else if (r_io <= P.rcut) {
             for (int k = lane; k < P.nRs2; k += 32) {
                 double v, dv;
-                two_body(P, r_io, k, v, dv);
+                two_body(P, two_body_terms(P, r_io), k, v, dv);
                 if (v != 0.0) atomicAdd(&xs[eo * P.nRs2 + k], v);
             }
         }
@@ -346,6 +358,251 @@ __global__ void __launch_bounds__(REPR_WARPS * 32) fchl19_kernel(
             go[(size_t)(e / 3) * ld + 3 * i + e % 3] = (TO)gc[e];
 }
 
+// ------------------------------------------------------ values and gradients
+// The gradients of one centre i are made row by row: a warp takes a few
+// consecutive rows of one channel (a two-body element or a pair of elements),
+// computes the columns of the atoms that the channel involves, adds up the
+// centre's own columns (minus their sum) and writes the rows whole, zeros
+// included.  No atomics, and every store is coalesced along the row.
+//
+// Three-body rows of channel (p, e), radial index l, from atom o of element p
+// and partners q of element e (or the other way round):
+//   V_a   = sum_q rad_l S_a,            S_a = ang_a atm dec_o dec_q
+//   dV_a  = sum_q rad_l A_a + drad_l S_a e_io,   drad_l = -eta3 (rbar - Rs3_l) rad_l,
+//   A_a   = dec_o dec_q (ang_a datm + dang_a atm dcos) + ang_a atm dec_q dec'_o e_io,
+// with the 8 numbers (A_0, A_1, S_0, S_1) of every ordered pair (o, q) formed
+// once per centre in shared memory: a radial index costs one exp and 14 other
+// FP64 operations per partner.  What bounds the kernel is FP64 latency (the
+// chain of a term's exp), so the rows of a centre are small work items that
+// the block's warps draw from a counter.
+constexpr int RG_WARPS = 8;
+constexpr int RG_ROWS = 8;         // rows of an item at most (four radial indices, or eight two-body rows)
+constexpr int RG_PAIR = 8;         // doubles per ordered pair
+constexpr int RG_ATOM = 12;        // doubles per atom: r, e (3), dec3, dec3', and the two-body terms
+
+__host__ __device__ inline size_t rg_smem(int ma) {
+    return ((size_t)ma * (ma | 1) * RG_PAIR + (size_t)ma * RG_ATOM + (size_t)RG_WARPS * RG_ROWS * 3 * ma) *
+               sizeof(double) +
+           (size_t)RG_WARPS * RG_ROWS * ma * sizeof(double) +
+           (size_t)(2 * ma + REPR_MAX_ELEM + 4 + REPR_MAX_ELEM + REPR_MAX_ELEM * (REPR_MAX_ELEM + 1) / 2) *
+               sizeof(int);
+}
+
+template <class TO>
+__global__ void __launch_bounds__(RG_WARPS * 32, 3) fchl19_grad_kernel(
+    const TO *__restrict__ coords, const int *__restrict__ elem, const int *__restrict__ natoms,
+    int ma, ReprParams P, TO *__restrict__ rep_out, TO *__restrict__ grad_out) {
+    extern __shared__ __align__(16) unsigned char rp_raw[];
+    double *pairs = reinterpret_cast<double *>(rp_raw);                  // [RG_PAIR][n][n | 1]
+    double *atoms = pairs + (size_t)ma * (ma | 1) * RG_PAIR;             // [n][RG_ATOM]
+    double *stage = atoms + (size_t)ma * RG_ATOM;                        // [warps][RG_ROWS][3 ma]
+    double *values = stage + (size_t)RG_WARPS * RG_ROWS * 3 * ma;        // [warps][RG_ROWS][ma]
+    int *el = reinterpret_cast<int *>(values + (size_t)RG_WARPS * RG_ROWS * ma);      // [ma]
+    int *order = el + ma;                          // partner atoms sorted by element
+    int *estart = order + ma;                      // [nelem + 1] runs of `order`
+    int *next_item = estart + REPR_MAX_ELEM + 1;   // item counter, number of items
+    int *cend = next_item + 2;                     // items up to and including each channel
+    const int m = blockIdx.y, i = blockIdx.x;
+    const int n = min(max(natoms[m], 0), ma);
+    // an odd row length: lanes of different atoms o read different banks
+    const int ns = n | 1, plane = n * ns;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int rep = P.rep, ld = 3 * ma, nelem = P.nelem;
+    TO *xo = rep_out + ((size_t)m * ma + i) * rep;
+    TO *go = grad_out + ((size_t)m * ma + i) * rep * (size_t)ld;
+    if (i >= n) {  // padded centre: zeros
+        for (int e = threadIdx.x; e < rep; e += blockDim.x) xo[e] = TO(0);
+        for (size_t e = threadIdx.x; e < (size_t)rep * ld; e += blockDim.x) go[e] = TO(0);
+        return;
+    }
+    const TO *cm = coords + (size_t)m * ma * 3;
+    auto position = [&](int a) {
+        return Vec3{(double)cm[3 * a], (double)cm[3 * a + 1], (double)cm[3 * a + 2]};
+    };
+    const Vec3 Ri = position(i);
+    // ---- per atom: distance, direction, decays and two-body terms
+    for (int o = threadIdx.x; o < n; o += blockDim.x) {
+        el[o] = elem[(size_t)m * ma + o];
+        if (o == i) continue;
+        double *A = atoms + o * RG_ATOM;
+        const Vec3 d = sub(position(o), Ri);
+        const double r = sqrt(dot(d, d));
+        A[0] = r;
+        A[1] = d.x / r;
+        A[2] = d.y / r;
+        A[3] = d.z / r;
+        A[4] = half_cos_decay(r, P.acut);
+        A[5] = -0.5 * M_PI / P.acut * sin(M_PI * r / P.acut);
+        const TwoBody tb = two_body_terms(P, r);
+        A[6] = tb.mu;
+        A[7] = tb.s2;
+        A[8] = tb.pref;
+        A[9] = tb.dpref;
+        A[10] = tb.dmu;
+        A[11] = tb.ds2;
+    }
+    __syncthreads();
+    // ---- partners by element (stable), items per channel
+    const int npair = nelem * (nelem + 1) / 2;
+    if (warp == 0) {
+        int at = 0;
+        for (int e = 0; e < nelem; ++e) {
+            if (lane == 0) estart[e] = at;
+            for (int a0 = 0; a0 < n; a0 += 32) {
+                const int a = a0 + lane;
+                const bool in = a < n && a != i && el[a] == e;
+                const unsigned b = __ballot_sync(0xffffffffu, in);
+                if (in) order[at + __popc(b & ((1u << lane) - 1u))] = a;
+                at += __popc(b);
+            }
+        }
+        if (lane == 0) estart[nelem] = at;
+        __syncwarp();
+        // two-body: RG_ROWS rows an item; three-body: RG_ROWS / 2 radial indices
+        const int it2 = (P.nRs2 + RG_ROWS - 1) / RG_ROWS;
+        const int it3 = (P.nRs3 + RG_ROWS / 2 - 1) / (RG_ROWS / 2);
+        if (lane == 0) {
+            next_item[0] = 0;
+            for (int c = 0; c < nelem + npair; ++c)
+                cend[c] = (c ? cend[c - 1] : 0) + (c < npair ? it3 : it2);
+            next_item[1] = cend[nelem + npair - 1];
+        }
+    }
+    // ---- ordered pairs (o, q)
+    for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
+        const int o = e / n, q = e - o * n;
+        if (o == i || q == i || o == q) continue;
+        double *S = pairs + o * ns + q;
+        const double r_o = atoms[o * RG_ATOM], r_q = atoms[q * RG_ATOM];
+        if (!(r_o <= P.acut && r_q <= P.acut)) {
+#pragma unroll
+            for (int k = 0; k < RG_PAIR; ++k) S[k * plane] = 0.0;
+            continue;
+        }
+        const Triple T = make_triple(P, Ri, position(o), position(q), r_o, r_q);
+        const double wv = P.ang_w[0];
+        const double ang[2] = {wv * T.cos_i, wv * T.sin_i};
+        const double dang[2] = {wv * T.sin_i, -wv * T.cos_i};
+#pragma unroll
+        for (int a = 0; a < 2; ++a) {
+            const Vec3 g = axpby(1.0, axpby(ang[a] * T.dec, T.datm, dang[a] * T.dec * T.atm, T.dcos),
+                                 ang[a] * T.atm, T.ddec);
+            S[3 * a * plane] = g.x;
+            S[(3 * a + 1) * plane] = g.y;
+            S[(3 * a + 2) * plane] = g.z;
+            S[(6 + a) * plane] = ang[a] * T.atm * T.dec;
+        }
+    }
+    __syncthreads();
+    const int nitems = next_item[1];
+    double *st = stage + (size_t)warp * RG_ROWS * ld, *vb = values + (size_t)warp * RG_ROWS * ma;
+    while (true) {
+        int it = 0;
+        if (lane == 0) it = atomicAdd(next_item, 1);
+        it = __shfl_sync(0xffffffffu, it, 0);
+        if (it >= nitems) break;
+        int ch = 0;   // three-body channels first (the heavier items)
+        while (it >= cend[ch]) ++ch;
+        const int local = it - (ch ? cend[ch - 1] : 0);
+        int row0, nrow, p, e;
+        const bool three = ch < npair;
+        if (three) {
+            p = 0;
+            e = ch;
+            while (e >= nelem - p) {
+                e -= nelem - p;
+                ++p;
+            }
+            e += p;
+            const int l0 = local * (RG_ROWS / 2);
+            nrow = 2 * min(RG_ROWS / 2, P.nRs3 - l0);
+            row0 = P.three_off + (ch * P.nRs3 + l0) * 2;
+        } else {
+            p = e = ch - npair;
+            nrow = min(RG_ROWS, P.nRs2 - local * RG_ROWS);
+            row0 = p * P.nRs2 + local * RG_ROWS;
+        }
+        const int np = estart[p + 1] - estart[p], ne = estart[e + 1] - estart[e];
+        // atoms that the channel's rows depend on
+        const int nact = !three ? np : np == 0 || ne == 0 ? 0 : p == e ? (np > 1 ? np : 0) : np + ne;
+        TO *gr = go + (size_t)row0 * ld;
+        if (nact == 0) {
+            for (int k = lane; k < nrow; k += 32) xo[row0 + k] = TO(0);
+            for (int k = lane; k < nrow * ld; k += 32) gr[k] = TO(0);
+            continue;
+        }
+        for (int k = lane; k < nrow * ld; k += 32) st[k] = 0.0;
+        __syncwarp();
+        const int groups = three ? nrow / 2 : nrow;   // radial indices of the item
+        for (int w = lane; w < nact * groups; w += 32) {
+            const int lg = w / nact, k = w - lg * nact;
+            const int o = k < np ? order[estart[p] + k] : order[estart[e] + k - np];
+            const double *A = atoms + o * RG_ATOM;
+            if (three) {
+                const int qe = k < np ? e : p;   // element of the partners
+                const int l = (row0 - P.three_off) / 2 - ch * P.nRs3 + lg;
+                double g[6] = {0, 0, 0, 0, 0, 0}, s0 = 0, s1 = 0, v0 = 0, v1 = 0;
+                if (A[0] <= P.acut) {
+                    const double shift = 0.5 * A[0] - P.acut * (l + 1) / P.nRs3;
+                    for (int z = estart[qe]; z < estart[qe + 1]; ++z) {
+                        const int q = order[z];
+                        if (q == o) continue;
+                        const double *S = pairs + o * ns + q;
+                        const double dr = fma(0.5, atoms[q * RG_ATOM], shift);
+                        const double rad = exp(-P.eta3 * dr * dr);
+                        const double drad = -P.eta3 * dr * rad;
+                        const double S0 = S[6 * plane], S1 = S[7 * plane];
+#pragma unroll
+                        for (int t = 0; t < 6; ++t) g[t] = fma(rad, S[t * plane], g[t]);
+                        s0 = fma(drad, S0, s0);
+                        s1 = fma(drad, S1, s1);
+                        // the value of an unordered pair comes from its atom of
+                        // element p, or from the lower atom
+                        if (p != e ? k < np : o < q) {
+                            v0 = fma(rad, S0, v0);
+                            v1 = fma(rad, S1, v1);
+                        }
+                    }
+                    double *r0 = st + (size_t)(2 * lg) * ld + 3 * o, *r1 = r0 + ld;
+#pragma unroll
+                    for (int t = 0; t < 3; ++t) {
+                        r0[t] = fma(s0, A[1 + t], g[t]);
+                        r1[t] = fma(s1, A[1 + t], g[3 + t]);
+                    }
+                }
+                vb[(2 * lg) * ma + k] = v0;
+                vb[(2 * lg + 1) * ma + k] = v1;
+            } else {
+                double v = 0.0, dv = 0.0;
+                if (A[0] <= P.rcut) {
+                    const TwoBody tb{A[6], A[7], A[8], A[9], A[10], A[11]};
+                    two_body(P, tb, row0 - p * P.nRs2 + lg, v, dv);
+                }
+                double *r0 = st + (size_t)lg * ld + 3 * o;
+#pragma unroll
+                for (int t = 0; t < 3; ++t) r0[t] = dv * A[1 + t];
+                vb[lg * ma + k] = v;
+            }
+        }
+        __syncwarp();
+        // lane (row, 0..2): the centre's column, minus the sum of the atoms'
+        // (translation invariance); lane (row, 3): the row's value
+        if ((lane >> 2) < nrow) {
+            const int r = lane >> 2, t = lane & 3;
+            double sum = 0.0;
+            for (int k = 0; k < nact; ++k) {
+                const int o = k < np ? order[estart[p] + k] : order[estart[e] + k - np];
+                sum += t < 3 ? st[(size_t)r * ld + 3 * o + t] : vb[r * ma + k];
+            }
+            if (t < 3) st[(size_t)r * ld + 3 * i + t] = -sum;
+            else xo[row0 + r] = (TO)sum;
+        }
+        __syncwarp();
+        for (int k = lane; k < nrow * ld; k += 32) gr[k] = (TO)st[k];
+        __syncwarp();
+    }
+}
+
 }  // namespace
 
 }  // namespace kfb
@@ -422,6 +679,23 @@ kfb_status kfb_fchl19_repr(const void *coords, const int32_t *elem, const int32_
                                               (int)smem));
         return KFB_OK;
     };
+    // the row-wise gradient kernel holds a centre's pairs in shared memory (40
+    // atoms); larger molecules take the kernel that forms them as it goes
+    const size_t rg = rg_smem(ma);
+    if (g && rg <= 200 * 1024) {
+        auto run = [&](auto kern, auto *c, auto *r, auto *d) -> kfb_status {
+            KFB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              (int)rg));
+            kern<<<grid, RG_WARPS * 32, rg, s>>>(c, de, dn, ma, P, r, d);
+            KFB_CUDA_TRY(cudaGetLastError());
+            return KFB_OK;
+        };
+        if (dt == KFB_F64)
+            return run(fchl19_grad_kernel<double>, static_cast<const double *>(coords),
+                       static_cast<double *>(rep), static_cast<double *>(grad));
+        return run(fchl19_grad_kernel<float>, static_cast<const float *>(coords),
+                   static_cast<float *>(rep), static_cast<float *>(grad));
+    }
     if (dt == KFB_F64) {
         if (g) {
             KFB_TRY(launch(fchl19_kernel<double, true>));

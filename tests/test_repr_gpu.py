@@ -119,6 +119,34 @@ def test_against_restatement_and_finite_differences():
                                    atol=1e-6 * np.abs(J).max())
 
 
+@pytest.mark.parametrize("n", [1, 2, 9, 20, 33, 40])
+@pytest.mark.parametrize("hyper", [{}, dict(nRs2=7, nRs3=5, rcut=3.0, acut=2.5)])
+def test_row_wise_gradients_match_large_molecule_kernel(n, hyper):
+    """Up to 40 padded atoms the Jacobian rows come from shared-memory pair terms, above from the
+    kernel that forms them as it goes: the same molecules padded to 40 and to 41 atoms.  Both sum
+    the same FP64 terms in another order (1e-13 of the largest entry); atoms beyond the cutoffs,
+    elements that one or no atom has, partial row groups."""
+    import torch
+    from kernelforge_b200 import fchl19_repr as fr
+    rng = np.random.default_rng(n)
+    nm = 3
+    C = np.zeros((nm, 41, 3))
+    Z = np.zeros((nm, 41), np.int32)
+    grid = np.stack(np.meshgrid(*[np.arange(4)] * 3), -1).reshape(-1, 3) * 1.3
+    for m in range(nm):
+        C[m, :n] = grid[rng.permutation(64)[:n]] + rng.uniform(-0.2, 0.2, (n, 3))
+        Z[m, :n] = rng.choice([[1], [1, 6], [1, 6, 8, 16]][m], n)
+    N = np.array([n, n, max(n - 1, 0)], np.int32)
+    out = []
+    for ma in (40, 41):
+        X, dX = fr.generate_batched(C[:, :ma], Z[:, :ma], N, gradients=True, dtype="float64",
+                                    **hyper)
+        assert not dX[:, :, :, 3 * n:].any() and not X[2, N[2]:].any()
+        out.append((X[:, :40].cpu().numpy(), dX[:, :40, :, :120].cpu().numpy()))
+    for a, b in zip(*out):
+        np.testing.assert_allclose(a, b, rtol=0, atol=1e-13 * max(1e-3, np.abs(b).max()))
+
+
 def test_edge_cases_and_errors():
     from kernelforge_b200 import fchl19_repr as fr
     X, J = fr.generate_fchl_acsf_and_gradients(np.zeros((1, 3)), [6])
