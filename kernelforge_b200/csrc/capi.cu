@@ -103,22 +103,27 @@ bool use_tc(kfb_precision prec, int rep) {
     return prec == KFB_PREC_SPLIT_F16 && rep % 16 == 0 && device_is_sm100();
 }
 
-kfb_status jac_any(kfb_dtype dt, kfb_precision prec, const DerivSet &outer,
-                   const DerivSet &inner, int rep, double sigma, double alpha,
-                   const ElemSink &sink, cudaStream_t s) {
+// tc: use_tc of the call's own rep (the widths that compact() leaves are
+// multiples of 16 as well).
+kfb_status jac_any(kfb_dtype dt, bool tc, const DerivSet &outer, const DerivSet &inner, int rep,
+                   double sigma, double alpha, const ElemSink &sink, cudaStream_t s) {
     if (rep <= 0) return KFB_OK;
-    const bool tc = use_tc(prec, rep);
     if (dt == KFB_F64) return jacobian_core<double>(outer, inner, rep, sigma, alpha, tc, sink, s);
     return jacobian_core<float>(outer, inner, rep, sigma, alpha, tc, sink, s);
 }
 
-kfb_status hess_any(kfb_dtype dt, kfb_precision prec, const DerivSet &s1, const DerivSet &s2,
-                    int rep, double sigma, bool symmetric, const ElemSink &sink,
-                    cudaStream_t s) {
+kfb_status hess_any(kfb_dtype dt, bool tc, const DerivSet &s1, const DerivSet &s2, int rep,
+                    double sigma, bool symmetric, const ElemSink &sink, cudaStream_t s) {
     if (rep <= 0) return KFB_OK;
-    const bool tc = use_tc(prec, rep);
     if (dt == KFB_F64) return hessian_core<double>(s1, s2, rep, sigma, symmetric, tc, sink, s);
     return hessian_core<float>(s1, s2, rep, sigma, symmetric, tc, sink, s);
+}
+
+// The two sets of a derivative kernel without the columns that neither uses.
+kfb_status compact(kfb_dtype dt, DerivSet &s1, DerivSet &s2, int &rep, CompactSets &keep,
+                   cudaStream_t s) {
+    if (dt == KFB_F64) return compact_columns<double>(s1, s2, rep, keep, s);
+    return compact_columns<float>(s1, s2, rep, keep, s);
 }
 
 DerivSet dset(const void *x, const void *dx, const int32_t *q, const int32_t *n, int nm, int ma) {
@@ -281,8 +286,11 @@ kfb_status kfb_kernel_gaussian_jacobian(const void *x1, const void *x2, const vo
     sink.f64 = dt == KFB_F64;
     sink.mode = EM_RECT;
     sink.ld = naq2;
-    return jac_any(dt, prec, dset(x1, nullptr, q1, n1, nm1, ma1), dset(x2, dx2, q2, n2, nm2, ma2), rep,
-                   sigma, 1.0, sink, s);
+    DerivSet d1 = dset(x1, nullptr, q1, n1, nm1, ma1), d2 = dset(x2, dx2, q2, n2, nm2, ma2);
+    const bool tc = use_tc(prec, rep);
+    CompactSets keep;
+    KFB_TRY(compact(dt, d1, d2, rep, keep, s));
+    return jac_any(dt, tc, d1, d2, rep, sigma, 1.0, sink, s);
 }
 
 kfb_status kfb_kernel_gaussian_jacobian_t(const void *x1, const void *dx1, const void *x2,
@@ -311,8 +319,11 @@ kfb_status kfb_kernel_gaussian_jacobian_t(const void *x1, const void *dx1, const
     sink.f64 = dt == KFB_F64;
     sink.mode = EM_RECT_T;
     sink.ld = nm2;
-    return jac_any(dt, prec, dset(x2, nullptr, q2, n2, nm2, ma2), dset(x1, dx1, q1, n1, nm1, ma1), rep,
-                   sigma, -1.0, sink, s);
+    DerivSet d1 = dset(x1, dx1, q1, n1, nm1, ma1), d2 = dset(x2, nullptr, q2, n2, nm2, ma2);
+    const bool tc = use_tc(prec, rep);
+    CompactSets keep;
+    KFB_TRY(compact(dt, d1, d2, rep, keep, s));
+    return jac_any(dt, tc, d2, d1, rep, sigma, -1.0, sink, s);
 }
 
 kfb_status kfb_kernel_gaussian_hessian(const void *x1, const void *dx1, const void *x2,
@@ -340,8 +351,11 @@ kfb_status kfb_kernel_gaussian_hessian(const void *x1, const void *dx1, const vo
     sink.f64 = dt == KFB_F64;
     sink.mode = EM_RECT;
     sink.ld = naq2;
-    return hess_any(dt, prec, dset(x1, dx1, q1, n1, nm1, ma1), dset(x2, dx2, q2, n2, nm2, ma2), rep,
-                    sigma, false, sink, s);
+    DerivSet d1 = dset(x1, dx1, q1, n1, nm1, ma1), d2 = dset(x2, dx2, q2, n2, nm2, ma2);
+    const bool tc = use_tc(prec, rep);
+    CompactSets keep;
+    KFB_TRY(compact(dt, d1, d2, rep, keep, s));
+    return hess_any(dt, tc, d1, d2, rep, sigma, false, sink, s);
 }
 
 kfb_status kfb_kernel_gaussian_hessian_symm(const void *x, const void *dx, const int32_t *q,
@@ -367,8 +381,11 @@ kfb_status kfb_kernel_gaussian_hessian_symm(const void *x, const void *dx, const
     sink.mode = EM_SYM;
     sink.layout = layout == KFB_DENSE ? LAYOUT_DENSE_LOWER : layout;
     sink.ld = naq;
-    DerivSet d = dset(x, dx, q, n, nm, ma);
-    return hess_any(dt, prec, d, d, rep, sigma, true, sink, s);
+    DerivSet d1 = dset(x, dx, q, n, nm, ma), d2 = d1;
+    const bool tc = use_tc(prec, rep);
+    CompactSets keep;
+    KFB_TRY(compact(dt, d1, d2, rep, keep, s));
+    return hess_any(dt, tc, d1, d2, rep, sigma, true, sink, s);
 }
 
 kfb_status kfb_kernel_gaussian_full(const void *x1, const void *dx1, const void *x2,
@@ -404,7 +421,10 @@ kfb_status kfb_kernel_gaussian_full(const void *x1, const void *dx1, const void 
     ps.mode = OUT_RECT;
     ps.n = C;
     KFB_TRY(scalar_dispatch(p, prec, ps, s));
-    const DerivSet d1 = dset(x1, dx1, q1, n1, nm1, ma1), d2 = dset(x2, dx2, q2, n2, nm2, ma2);
+    DerivSet d1 = dset(x1, dx1, q1, n1, nm1, ma1), d2 = dset(x2, dx2, q2, n2, nm2, ma2);
+    const bool tc = use_tc(prec, rep);
+    CompactSets keep;
+    KFB_TRY(compact(dt, d1, d2, rep, keep, s));
     // [0:nm1, nm2:] = +jacobian(X1, X2, dX2)
     ElemSink sj;
     sj.out = out;
@@ -412,7 +432,7 @@ kfb_status kfb_kernel_gaussian_full(const void *x1, const void *dx1, const void 
     sj.mode = EM_RECT;
     sj.ld = C;
     sj.col_base = nm2;
-    KFB_TRY(jac_any(dt, prec, d1, d2, rep, sigma, 1.0, sj, s));
+    KFB_TRY(jac_any(dt, tc, d1, d2, rep, sigma, 1.0, sj, s));
     // [nm1:, 0:nm2] = -jacobian_t(X1, dX1, X2) = G^T with G from (outer 2, inner 1)
     ElemSink st;
     st.out = out;
@@ -420,7 +440,7 @@ kfb_status kfb_kernel_gaussian_full(const void *x1, const void *dx1, const void 
     st.mode = EM_RECT_T;
     st.ld = C;
     st.col_base = nm1;
-    KFB_TRY(jac_any(dt, prec, d2, d1, rep, sigma, 1.0, st, s));
+    KFB_TRY(jac_any(dt, tc, d2, d1, rep, sigma, 1.0, st, s));
     // [nm1:, nm2:] = hessian
     ElemSink sh;
     sh.out = out;
@@ -429,7 +449,7 @@ kfb_status kfb_kernel_gaussian_full(const void *x1, const void *dx1, const void 
     sh.ld = C;
     sh.row_base = nm1;
     sh.col_base = nm2;
-    return hess_any(dt, prec, d1, d2, rep, sigma, false, sh, s);
+    return hess_any(dt, tc, d1, d2, rep, sigma, false, sh, s);
 }
 
 kfb_status kfb_kernel_gaussian_full_symm(const void *x, const void *dx, const int32_t *q,
@@ -466,7 +486,10 @@ kfb_status kfb_kernel_gaussian_full_symm(const void *x, const void *dx, const in
         TraceScope tr("full_symm:scalar", s);
         KFB_TRY(scalar_dispatch(p, prec, ps, s));
     }
-    const DerivSet d = dset(x, dx, q, n, nm, ma);
+    DerivSet d = dset(x, dx, q, n, nm, ma), d2 = d;
+    const bool tc = use_tc(prec, rep);
+    CompactSets keep;
+    KFB_TRY(compact(dt, d, d2, rep, keep, s));
     // jacobian block at rows [0, nm), columns [nm, big) and its mirror
     ElemSink sj;
     sj.out = out;
@@ -477,7 +500,7 @@ kfb_status kfb_kernel_gaussian_full_symm(const void *x, const void *dx, const in
     sj.col_base = nm;
     {
         TraceScope tr("full_symm:jacobian", s);
-        KFB_TRY(jac_any(dt, prec, d, d, rep, sigma, 1.0, sj, s));
+        KFB_TRY(jac_any(dt, tc, d, d2, rep, sigma, 1.0, sj, s));
     }
     ElemSink sh;
     sh.out = out;
@@ -488,7 +511,7 @@ kfb_status kfb_kernel_gaussian_full_symm(const void *x, const void *dx, const in
     sh.row_base = nm;
     sh.col_base = nm;
     TraceScope tr("full_symm:hessian", s);
-    return hess_any(dt, prec, d, d, rep, sigma, true, sh, s);
+    return hess_any(dt, tc, d, d2, rep, sigma, true, sh, s);
 }
 
 kfb_status kfb_full_to_rfp(const void *a, int n, kfb_layout uplo, kfb_dtype dt, void *arf,

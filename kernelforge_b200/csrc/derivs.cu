@@ -31,6 +31,7 @@
 #include <climits>
 #include <cmath>
 #include <cstdlib>
+#include <cstring>
 #include <memory>
 #include <numeric>
 #include <string>
@@ -310,6 +311,97 @@ __global__ void __launch_bounds__(JV_THREADS, sizeof(T) == 4 ? 3 : 2) jac_v_kern
                 }
             }
         }
+    }
+}
+
+// -------------------------------------------------------- unused columns
+// used[k] = 1 where column k of any real atom (j < nat[m]) is not zero, in x
+// (nm, ma, rep) and, with dx, in its Jacobian's columns c < 3 nat[m] (NaN is
+// not zero); amax (optional): [0] max |x|, [1] max |dx| of the same entries.
+// Block per atom; the Jacobian is read along its rows, 16 bytes a lane (VEC,
+// rep a multiple of 4): the pass is bound by HBM.
+template <class T, bool VEC>
+__global__ void __launch_bounds__(256) used_columns_kernel(const T *__restrict__ x,
+                                                           const T *__restrict__ dx, int ma,
+                                                           int rep, const int *__restrict__ nat,
+                                                           int *__restrict__ used, int staged,
+                                                           float *__restrict__ amax) {
+    // the block's flags; rows too long for 48 KB raise the call's own
+    extern __shared__ int uc_s[];   // [rep]
+    int *uc = staged ? uc_s : used;
+    const int m = blockIdx.x / ma, j = blockIdx.x - m * ma;
+    const int na = min(max(nat[m], 0), ma);
+    if (j >= na) return;
+    float mx = 0.f, md = 0.f;
+    for (int k = threadIdx.x; k < rep; k += blockDim.x) {
+        const T v = x[(size_t)blockIdx.x * rep + k];
+        if (staged) uc[k] = 0;
+        if (!(v == T(0))) uc[k] = 1;
+        mx = fmaxf(mx, fabsf((float)v));
+    }
+    __syncthreads();
+    if (dx) {
+        const unsigned ld = 3 * ma, nc = 3 * na;
+        const T *J = dx + (size_t)blockIdx.x * rep * ld;
+        if constexpr (VEC) {
+            constexpr int PER = 16 / sizeof(T);
+            const unsigned n = (unsigned)rep * ld / PER;
+#pragma unroll 4
+            for (unsigned e = threadIdx.x; e < n; e += blockDim.x) {
+                const uint4 w = reinterpret_cast<const uint4 *>(J)[e];
+                const T *v = reinterpret_cast<const T *>(&w);
+                unsigned k = e * PER / ld, c = e * PER - k * ld;
+#pragma unroll
+                for (int u = 0; u < PER; ++u) {
+                    if (c < nc && !(v[u] == T(0))) {
+                        uc[k] = 1;
+                        md = fmaxf(md, fabsf((float)v[u]));
+                    }
+                    if (++c == ld) {
+                        c = 0;
+                        ++k;
+                    }
+                }
+            }
+        } else {
+            for (int k = threadIdx.x >> 5; k < rep; k += blockDim.x >> 5)
+                for (unsigned c = threadIdx.x & 31; c < nc; c += 32) {
+                    const T v = J[(size_t)k * ld + c];
+                    if (!(v == T(0))) uc[k] = 1;
+                    md = fmaxf(md, fabsf((float)v));
+                }
+        }
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; staged && k < rep; k += blockDim.x)
+        if (uc[k] && !used[k]) used[k] = 1;
+    if (!amax) return;
+    for (int o = 16; o; o >>= 1) {
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        md = fmaxf(md, __shfl_xor_sync(0xffffffffu, md, o));
+    }
+    // non-negative floats order like their bit patterns
+    if ((threadIdx.x & 31) == 0) {
+        if (mx > 0.f) atomicMax(reinterpret_cast<int *>(amax), __float_as_int(mx));
+        if (md > 0.f) atomicMax(reinterpret_cast<int *>(amax + 1), __float_as_int(md));
+    }
+}
+
+// dst[r][k][:] = src[r][cols[k]][:] for k < n, zero for n <= k < np (rows of w
+// values); block per r.
+template <class T>
+__global__ void __launch_bounds__(256) compact_columns_kernel(const T *__restrict__ src,
+                                                              const int *__restrict__ cols, int n,
+                                                              int np, int rep, int w,
+                                                              T *__restrict__ dst) {
+    extern __shared__ int uc[];   // [n]
+    for (int k = threadIdx.x; k < n; k += blockDim.x) uc[k] = cols[k];
+    __syncthreads();
+    const T *s = src + (size_t)blockIdx.x * rep * w;
+    T *d = dst + (size_t)blockIdx.x * np * w;
+    for (unsigned e = threadIdx.x; e < (unsigned)(np * w); e += blockDim.x) {
+        const unsigned k = e / (unsigned)w, c = e - k * (unsigned)w;
+        d[e] = k < (unsigned)n ? s[(size_t)uc[k] * w + c] : T(0);
     }
 }
 
@@ -716,24 +808,38 @@ __global__ void __launch_bounds__(256) centred_split_kernel(
     }
 }
 
-// PB[(m, j)][c] = (x_j - mu_l) . J_j[:, c] (FP64 sums), block per atom (m, j)
+// PB[(m, j)][c] = (x_j - mu_l) . J_j[:, c] (FP64 sums), block per atom (m, j):
+// 64 columns c by 4 slices of rep (a thread per column alone walked rep in one
+// latency-bound chain: 0.57 ms for 6,300 atoms of 21 at rep 720).
 template <class T>
-__global__ void pb_kernel(const T *__restrict__ x2, const T *__restrict__ dx2,
-                          const int *__restrict__ lidx2, int ma2, int rep,
-                          const double *__restrict__ sums, const double *__restrict__ inv_count,
-                          float *__restrict__ PB) {
+__global__ void __launch_bounds__(256) pb_kernel(const T *__restrict__ x2,
+                                                 const T *__restrict__ dx2,
+                                                 const int *__restrict__ lidx2, int ma2, int rep,
+                                                 const double *__restrict__ sums,
+                                                 const double *__restrict__ inv_count,
+                                                 float *__restrict__ PB) {
+    __shared__ double part[4][64];
     const size_t mj = blockIdx.x;
     const int ld2 = 3 * ma2;
     const int l = lidx2[mj];
     const T *xj = x2 + mj * rep;
     const T *J = dx2 + mj * rep * ld2;
-    for (int c = threadIdx.x; c < ld2; c += blockDim.x) {
+    const int cl = threadIdx.x & 63, q = threadIdx.x >> 6;
+    for (int c0 = 0; c0 < ld2; c0 += 64) {
+        const int c = c0 + cl;
         double acc = 0.0;
-        if (l >= 0)
-            for (int k = 0; k < rep; ++k)
-                acc = fma((double)xj[k] - sums[(size_t)l * rep + k] * inv_count[l],
+        if (l >= 0 && c < ld2) {
+            const double ic = inv_count[l];
+#pragma unroll 8
+            for (int k = q; k < rep; k += 4)
+                acc = fma((double)xj[k] - sums[(size_t)l * rep + k] * ic,
                           (double)J[(size_t)k * ld2 + c], acc);
-        PB[mj * ld2 + c] = (float)acc;
+        }
+        part[q][cl] = acc;
+        __syncthreads();
+        if (q == 0 && c < ld2)
+            PB[mj * ld2 + c] = (float)(part[0][cl] + part[1][cl] + part[2][cl] + part[3][cl]);
+        __syncthreads();
     }
 }
 
@@ -1275,15 +1381,18 @@ __global__ void __launch_bounds__(128) jk_split_kernel(const T *__restrict__ dx,
 }
 
 // Ws[r kj + j] = scale * W[border[q]][i][j] (r = q ma1 + i) as an fp16 pair,
-// zero for j >= ma2; a thread per (row, eight columns).
+// zero for j >= ma2, and the Y GEMM's column map: ymap[r] = (pair, i), pair -1
+// for padding atoms i; a thread per (row, eight columns).
 __global__ void w_split_kernel(const float *__restrict__ W, const int *__restrict__ border,
-                               int nrows, int ma1, int ma2, int kj, float scale,
-                               __half *__restrict__ hi, __half *__restrict__ lo) {
+                               const HessPair *__restrict__ pairs, int nrows, int ma1, int ma2,
+                               int kj, float scale, __half *__restrict__ hi,
+                               __half *__restrict__ lo, int2 *__restrict__ ymap) {
     const int ng = kj / 8;
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= (long long)nrows * ng) return;
     const int r = (int)(e / ng), j0 = (int)(e - (long long)r * ng) * 8;
     const int q = r / ma1, i = r - q * ma1;
+    if (j0 == 0) ymap[r] = make_int2(i < pairs[border[q]].na ? border[q] : -1, i);
     const float *w = W + ((size_t)border[q] * ma1 + i) * ma2;
     unsigned hw[4], lw[4];
 #pragma unroll
@@ -1449,6 +1558,112 @@ size_t budget_bytes() {
 
 }  // namespace
 
+template <class T>
+kfb_status scan_columns(const DerivSet &d, int rep, const int *nat, int *used, float *amax,
+                        cudaStream_t s) {
+    const T *x = static_cast<const T *>(d.x), *dx = static_cast<const T *>(d.dx);
+    const long long atoms = (long long)d.v.nm * d.v.ma;
+    if (atoms == 0) return KFB_OK;
+    const bool staged = (size_t)rep * sizeof(int) <= 48 * 1024;
+    const bool vec = rep % 4 == 0 && (reinterpret_cast<size_t>(dx) & 15) == 0 &&
+                     (long long)rep * 3 * d.v.ma < (1LL << 31);
+    auto kern = vec ? used_columns_kernel<T, true> : used_columns_kernel<T, false>;
+    kern<<<(unsigned)atoms, 256, staged ? rep * sizeof(int) : 0, s>>>(x, dx, d.v.ma, rep, nat,
+                                                                      used, staged ? 1 : 0, amax);
+    KFB_CUDA_TRY(cudaGetLastError());
+    return KFB_OK;
+}
+template kfb_status scan_columns<float>(const DerivSet &, int, const int *, int *, float *,
+                                        cudaStream_t);
+template kfb_status scan_columns<double>(const DerivSet &, int, const int *, int *, float *,
+                                         cudaStream_t);
+
+template <class T>
+kfb_status compact_columns(DerivSet &s1, DerivSet &s2, int &rep, CompactSets &keep,
+                           cudaStream_t s) {
+    // one array for both sets is scanned once (where the atom counts agree too) and copied once
+    const bool shape = s1.v.nm == s2.v.nm && s1.v.ma == s2.v.ma;
+    const bool same_x = shape && s1.x == s2.x, same_dx = shape && s1.dx == s2.dx;
+    bool same_n = shape;
+    for (int m = 0; same_n && m < s1.v.nm; ++m) same_n = s1.v.natoms(m) == s2.v.natoms(m);
+    // flags of the columns, then max |x|, |dx| of set 1 and of set 2
+    DevBuf used, dn;
+    KFB_TRY(used.alloc((size_t)(rep + 4) * sizeof(int), s));
+    KFB_TRY(zero(used.ptr, (size_t)(rep + 4) * sizeof(int), s));
+    float *amax = reinterpret_cast<float *>(used.as<int>() + rep);
+    std::vector<int> nat;
+    for (const DerivSet *d : {&s1, &s2})
+        for (int m = 0; m < d->v.nm; ++m) nat.push_back(d->v.natoms(m));
+    KFB_TRY(upload(dn, nat, s));
+    KFB_TRY(scan_columns<T>(s1, rep, dn.as<int>(), used.as<int>(), amax, s));
+    const bool once = same_x && same_dx && same_n;
+    if (!once)
+        KFB_TRY(scan_columns<T>(s2, rep, dn.as<int>() + s1.v.nm, used.as<int>(), amax + 2, s));
+    std::vector<int> u(rep + 4), cols;
+    KFB_CUDA_TRY(cudaMemcpyAsync(u.data(), used.ptr, u.size() * sizeof(int),
+                                 cudaMemcpyDeviceToHost, s));
+    KFB_CUDA_TRY(cudaStreamSynchronize(s));
+    float mx[4];
+    std::memcpy(mx, u.data() + rep, sizeof(mx));
+    s1.dx_max = mx[1];
+    s2.dx_max = once ? mx[1] : mx[3];
+    for (int k = 0; k < rep; ++k)
+        if (u[k]) cols.push_back(k);
+    const int n = (int)cols.size(), np = std::max(16, (n + 15) / 16 * 16);
+    if (np > rep - rep / 8) return KFB_OK;
+    auto width = [](const DerivSet &d) { return 3LL * d.v.ma; };
+    auto bytes = [&](const DerivSet &d, bool jac) {
+        return (size_t)d.v.nm * d.v.ma * np * (jac ? width(d) : 1) * sizeof(T);
+    };
+    size_t need = bytes(s1, false) + (same_x ? 0 : bytes(s2, false));
+    if (s1.dx) need += bytes(s1, true);
+    if (s2.dx && !same_dx) need += bytes(s2, true);
+    size_t fr = 0, tot = 0;
+    KFB_CUDA_TRY(cudaMemGetInfo(&fr, &tot));
+    if (need > fr / 4) return KFB_OK;
+    DevBuf dcols;
+    cols.resize(std::max(n, 1));
+    KFB_TRY(upload(dcols, cols, s));
+    auto copy = [&](const void *&src, const DerivSet &d, int w, DevBuf &buf) -> kfb_status {
+        const long long atoms = (long long)d.v.nm * d.v.ma;
+        KFB_TRY(buf.alloc(std::max<size_t>(1, (size_t)atoms * np * w * sizeof(T)), s));
+        if (atoms > 0) {
+            compact_columns_kernel<T><<<(unsigned)atoms, 256, std::max(n, 1) * sizeof(int), s>>>(
+                static_cast<const T *>(src), dcols.as<int>(), n, np, rep, w, buf.as<T>());
+            KFB_CUDA_TRY(cudaGetLastError());
+        }
+        src = buf.ptr;
+        return KFB_OK;
+    };
+    KFB_TRY(copy(s1.x, s1, 1, keep.x1));
+    if (s1.dx) KFB_TRY(copy(s1.dx, s1, (int)width(s1), keep.dx1));
+    if (same_x) s2.x = s1.x;
+    else KFB_TRY(copy(s2.x, s2, 1, keep.x2));
+    if (s2.dx && same_dx) s2.dx = s1.dx;
+    else if (s2.dx) KFB_TRY(copy(s2.dx, s2, (int)width(s2), keep.dx2));
+    rep = np;
+    return KFB_OK;
+}
+
+// Pipeline-timeout flag shared by the tensor-core products of a call, read
+// once at its end: a read after every product (six per batch of the Hessian)
+// left the GPU idle for a tenth of the energy + force kernel.
+struct TcErr {
+    DevBuf buf;
+    kfb_status init(cudaStream_t s) {
+        KFB_TRY(buf.alloc(sizeof(int), s));
+        return zero(buf.ptr, sizeof(int), s);
+    }
+    int *flag() const { return buf.as<int>(); }
+    kfb_status check(cudaStream_t s) const {
+        int herr = 0;
+        KFB_CUDA_TRY(cudaMemcpyAsync(&herr, buf.ptr, sizeof(int), cudaMemcpyDeviceToHost, s));
+        KFB_CUDA_TRY(cudaStreamSynchronize(s));
+        if (herr) return set_error(KFB_ERR_TIMEOUT, "tensor-core GEMM: a pipeline wait timed out");
+        return KFB_OK;
+    }
+};
+
 // ---------------------------------------------------------------------------
 // Jacobian core: G[o, off_in[m] + c] (through `sink`, scaled by alpha) for all
 // outer molecules o and inner molecules m.
@@ -1602,7 +1817,7 @@ kfb_status jacobian_core(const DerivSet &outer, const DerivSet &inner, int rep, 
         TraceScope tr("jacobian:split_dx", s);
         KFB_TRY(transpose_split_dx<T>(static_cast<const T *>(inner.dx), inner.v.nm, ma_in, rep,
                                       d_nin.as<int>(), jth.as<__half>(), jtl.as<__half>(),
-                                      &jt_scale, s));
+                                      &jt_scale, s, inner.dx_max));
         KFB_TRY(vh.alloc((size_t)chunk * NU * rep * sizeof(__half), s));
         KFB_TRY(vl.alloc((size_t)chunk * NU * rep * sizeof(__half), s));
         // |v| <= (sum_i w_iu) (max|x_out| + max|x_in|) <= ns_max / sigma^2 (...)
@@ -1636,6 +1851,8 @@ kfb_status jacobian_core(const DerivSet &outer, const DerivSet &inner, int rep, 
     cublasHandle_t h = nullptr;
     KFB_TRY(blas_for_stream(s, &h));
     const int ld_in = 3 * inner.v.ma;
+    TcErr err;   // one pipeline-timeout flag for the call's tensor-core products
+    if (tc) KFB_TRY(err.init(s));
     std::vector<long long> cinfo(2 * nlab);
     for (int o0 = 0; o0 < nmo; o0 += chunk) {
         const int nout = std::min(chunk, nmo - o0);
@@ -1690,7 +1907,7 @@ kfb_status jacobian_core(const DerivSet &outer, const DerivSet &inner, int rep, 
                 epi.mode = EPI_DENSE;
                 epi.zf32 = reinterpret_cast<float *>(Dd.ptr);
                 epi.ld = NU;
-                KFB_TRY(tc_gemm_grouped(A, B, 3, false, dprobs, ElemSink(), s, epi));
+                KFB_TRY(tc_gemm_grouped(A, B, 3, false, dprobs, ElemSink(), s, epi, err.flag()));
             }
             KFB_TRY(upload(d_cinfo, cinfo, s));
         }
@@ -1744,7 +1961,7 @@ kfb_status jacobian_core(const DerivSet &outer, const DerivSet &inner, int rep, 
             // order, so the ragged ends of the K loops fall in the last wave
             std::stable_sort(tprobs.begin(), tprobs.end(),
                              [](const TcProb &x, const TcProb &y) { return x.K > y.K; });
-            KFB_TRY(tc_gemm_grouped(A, B, 3, false, tprobs, sink, s));
+            KFB_TRY(tc_gemm_grouped(A, B, 3, false, tprobs, sink, s, TcEpi(), err.flag()));
             continue;
         }
         std::vector<GemmProb> probs;
@@ -1768,7 +1985,7 @@ kfb_status jacobian_core(const DerivSet &outer, const DerivSet &inner, int rep, 
         }
         KFB_TRY(launch_gemm<T>(probs, sink, s));
     }
-    return KFB_OK;
+    return tc ? err.check(s) : KFB_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -1898,23 +2115,18 @@ long long label_problems(const LabelMajor &R, int r0, int r1, int mar, const Lab
 kfb_status hess_y_gemm(const HessPair *pairs, int np, int ma1, int ma2, int rep, int kj,
                        const float *W, const DevBuf &jkh, const DevBuf &jkl, float jk_scale,
                        float w_scale, float y_scale, DevBuf &wsh, DevBuf &wsl, DevBuf &d_ymap,
-                       DevBuf &d_border, long long jk_rows, __half *yhi, __half *ylo,
-                       cudaStream_t s) {
+                       DevBuf &d_border, long long jk_rows, const HessPair *dpairs, __half *yhi,
+                       __half *ylo, int *err, cudaStream_t s) {
     const int ld2 = 3 * ma2;
     std::vector<int> border(np);
     for (int p = 0; p < np; ++p) border[p] = p;
     std::stable_sort(border.begin(), border.end(),
                      [&](int x, int y) { return pairs[x].b < pairs[y].b; });
-    std::vector<int2> ymap((size_t)np * ma1);
     std::vector<TcProb> probs;
     for (int q = 0; q < np;) {
         const HessPair &pr = pairs[border[q]];
         int q1 = q;
-        for (; q1 < np && pairs[border[q1]].b == pr.b; ++q1) {
-            const int p = border[q1];
-            for (int i = 0; i < ma1; ++i)
-                ymap[(size_t)q1 * ma1 + i] = make_int2(i < pairs[p].na ? p : -1, i);
-        }
+        while (q1 < np && pairs[border[q1]].b == pr.b) ++q1;
         TcProb pb{};
         pb.a_row0 = (int)((long long)pr.b * ld2 * rep);
         pb.b_row0 = q * ma1;
@@ -1927,12 +2139,11 @@ kfb_status hess_y_gemm(const HessPair *pairs, int np, int ma1, int ma2, int rep,
     }
     KFB_CUDA_TRY(cudaMemcpyAsync(d_border.ptr, border.data(), (size_t)np * sizeof(int),
                                  cudaMemcpyHostToDevice, s));
-    KFB_CUDA_TRY(cudaMemcpyAsync(d_ymap.ptr, ymap.data(), ymap.size() * sizeof(int2),
-                                 cudaMemcpyHostToDevice, s));
     const int nrows = np * ma1;
     const long long nthr = (long long)nrows * (kj / 8);
     w_split_kernel<<<(unsigned)((nthr + 255) / 256), 256, 0, s>>>(
-        W, d_border.as<int>(), nrows, ma1, ma2, kj, w_scale, wsh.as<__half>(), wsl.as<__half>());
+        W, d_border.as<int>(), dpairs, nrows, ma1, ma2, kj, w_scale, wsh.as<__half>(),
+        wsl.as<__half>(), d_ymap.as<int2>());
     KFB_CUDA_TRY(cudaGetLastError());
     TcOperand A, B;
     A.hi = jkh.ptr;
@@ -1951,7 +2162,7 @@ kfb_status hess_y_gemm(const HessPair *pairs, int np, int ma1, int ma2, int rep,
     epi.y_rep = rep;
     epi.y_ma1 = ma1;
     epi.y_ld2 = ld2;
-    return tc_gemm_grouped(A, B, 3, false, probs, ElemSink(), s, epi);
+    return tc_gemm_grouped(A, B, 3, false, probs, ElemSink(), s, epi, err);
 }
 
 template <class T>
@@ -2006,7 +2217,7 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
         KFB_TRY(upload(d_n1, n1, s));
         KFB_TRY(transpose_split_dx<T>(static_cast<const T *>(s1.dx), s1.v.nm, ma1, rep,
                                       d_n1.as<int>(), jth.as<__half>(), jtl.as<__half>(),
-                                      &jt_scale, s));
+                                      &jt_scale, s, s1.dx_max));
         KFB_TRY(yamax.alloc(sizeof(float), s));
         KFB_TRY(yth.alloc((size_t)batch * ld2 * ma1 * rep * sizeof(__half), s));
         KFB_TRY(ytl.alloc((size_t)batch * ld2 * ma1 * rep * sizeof(__half), s));
@@ -2037,7 +2248,9 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
     // (b, c, k) with kj atom columns, resident for the call
     bool ygemm = false;
     int kj = 0;
-    float w_scale = 1.f;
+    float w_scale = 1.f, yg_scale = 1.f;
+    TcErr err;
+    if (tc) KFB_TRY(err.init(s));
     DevBuf jkh, jkl, wsh, wsl, d_ymap, d_border;
     if constexpr (std::is_same<T, float>::value) {
         const std::vector<int> labs1 = collect_labels(s1.v, nullptr);
@@ -2142,16 +2355,12 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
             KFB_TRY(jrl.alloc(jr_elems * sizeof(__half), s));
             KFB_TRY(transpose_split_dx_rows<float>(dx2f, s2.v.nm, ma2, rep, d_nat2.as<int>(),
                                                    jrh.as<__half>(), jrl.as<__half>(),
-                                                   &jr_scale, s, d_rank2.as<int>()));
+                                                   &jr_scale, s, d_rank2.as<int>(),
+                                                   s2.dx_max));
             KFB_TRY(d_pb.alloc((size_t)s2.v.nm * bcols * sizeof(float), s));
-            pb_kernel<float><<<(unsigned)(s2.v.nm * ma2), 128, 0, s>>>(
+            pb_kernel<float><<<(unsigned)(s2.v.nm * ma2), 256, 0, s>>>(
                 x2f, dx2f, d_l2.as<int>(), ma2, rep, d_sums.as<double>(), d_invc.as<double>(),
                 d_pb.as<float>());
-            KFB_CUDA_TRY(cudaGetLastError());
-            KFB_TRY(d_jbm.alloc((size_t)s2.v.nm * sizeof(float), s));
-            KFB_TRY(zero(d_jbm.ptr, (size_t)s2.v.nm * sizeof(float), s));
-            jmax_per_mol_kernel<float><<<dim3((unsigned)s2.v.nm, 32), 256, 0, s>>>(
-                dx2f, ma2, rep, d_nat2.as<int>(), d_jbm.as<float>());
             KFB_CUDA_TRY(cudaGetLastError());
             if (hrank) {
                 // set-1 Jacobian rows and PB1 (the set-2 ones for a symmetric call)
@@ -2167,9 +2376,9 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
                     KFB_TRY(jr1l.alloc(jr1_elems * sizeof(__half), s));
                     KFB_TRY(transpose_split_dx_rows<float>(
                         dx1f, s1.v.nm, ma1, rep, d_nat1.as<int>(), jr1h.as<__half>(),
-                        jr1l.as<__half>(), &jr1_scale, s, d_rank1.as<int>()));
+                        jr1l.as<__half>(), &jr1_scale, s, d_rank1.as<int>(), s1.dx_max));
                     KFB_TRY(d_pb1.alloc((size_t)Mq * sizeof(float), s));
-                    pb_kernel<float><<<(unsigned)Mrows, 128, 0, s>>>(
+                    pb_kernel<float><<<(unsigned)Mrows, 256, 0, s>>>(
                         x1f, dx1f, d_l1.as<int>(), ma1, rep, d_sums.as<double>(),
                         d_invc.as<double>(), d_pb1.as<float>());
                     KFB_CUDA_TRY(cudaGetLastError());
@@ -2208,6 +2417,13 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
                         (long long)batch * ma1 < INT_MAX &&
                         jk_bytes + (long long)budget_bytes() <= (long long)free_b;
             }
+            if (!ygemm) {   // per-molecule max |J| for the bound of |Y|
+                KFB_TRY(d_jbm.alloc((size_t)s2.v.nm * sizeof(float), s));
+                KFB_TRY(zero(d_jbm.ptr, (size_t)s2.v.nm * sizeof(float), s));
+                jmax_per_mol_kernel<float><<<dim3((unsigned)s2.v.nm, 32), 256, 0, s>>>(
+                    dx2f, ma2, rep, d_nat2.as<int>(), d_jbm.as<float>());
+                KFB_CUDA_TRY(cudaGetLastError());
+            }
             if (ygemm) {
                 TraceScope tr_j("hessian:jk-split", s);
                 const size_t jk_elems = (size_t)s2.v.nm * ld2 * rep * kj;
@@ -2228,6 +2444,15 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
                 KFB_TRY(d_border.alloc((size_t)batch * sizeof(int), s));
                 // 0 < w <= 1 / sigma^2: a fixed power of two brings it under 2^14
                 w_scale = std::exp2(std::floor(std::log2(16384.0 * sigma * sigma)));
+                // |Y| <= max|J| sum_j w_ij <= (2^14 / jr_scale) n / sigma^2 for at most n
+                // atoms of one label in a molecule b: one scale for every batch, so
+                // that no batch waits for its own maximum
+                int ns = 1;
+                for (int m = 0; m < s2.v.nm; ++m)
+                    for (int l = 0; l < L; ++l) ns = std::max(ns, lm2.count(l, m, m));
+                const double yb = 16384.0 / (double)jr_scale * ns / (sigma * sigma);
+                yg_scale = (float)std::exp2(14.0 - std::ceil(std::log2(yb)));
+                if (!(yg_scale > 0.f) || !std::isfinite(yg_scale)) yg_scale = 1.f;
             }
             note_path(ygemm ? "hessian:y-gemm" : "hessian:y-cuda-core");
         }
@@ -2256,7 +2481,7 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
         auto tr_t = std::make_unique<TraceScope>("hessian:t", s);
         // with tensor cores kernel 1 also bounds |Y| for the power-of-two
         // scale of the fp16 split that kernel 2 writes
-        if (tc) KFB_TRY(zero(yamax.ptr, sizeof(float), s));
+        if (tc && !ygemm) KFB_TRY(zero(yamax.ptr, sizeof(float), s));
         if constexpr (std::is_same<T, float>::value) {
             if (pform) {
                 // rows of the batch's molecules a only (pairs sorted by a):
@@ -2286,7 +2511,7 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
                 epi.mode = EPI_DENSE;
                 epi.zf32 = d_P.as<float>();
                 epi.ld = ldp;
-                KFB_TRY(tc_gemm_grouped(A, B, 3, false, pps, ElemSink(), s, epi));
+                KFB_TRY(tc_gemm_grouped(A, B, 3, false, pps, ElemSink(), s, epi, err.flag()));
                 TcOperand A1;  // centred set-1 rows in atom order
                 A1.hi = xh1.ptr;
                 A1.lo = xl1.ptr;
@@ -2310,7 +2535,7 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
                 eg.mode = EPI_DENSE;
                 eg.zf32 = d_G.as<float>();
                 eg.ld = pg.N;
-                KFB_TRY(tc_gemm_grouped(A1, B2, 3, false, {pg}, ElemSink(), s, eg));
+                KFB_TRY(tc_gemm_grouped(A1, B2, 3, false, {pg}, ElemSink(), s, eg, err.flag()));
                 // the Y GEMM reads every weight: those of other-label pairs are 0
                 if (ygemm) KFB_TRY(zero(W.ptr, (size_t)np * ma1 * ma2 * sizeof(float), s));
                 hess_t_p_kernel<<<np, 256, smem_p, s>>>(
@@ -2319,7 +2544,7 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
                     d_lab1.as<int>(), d_perm2.as<int>(), d_lab2.as<int>(), ma1, ma2, c2, is2, is4,
                     d_P.as<float>(), ldp, d_prow.as<int>(), d_pcol.as<int>(), amin, bmin,
                     d_pb.as<float>(), d_jbm.as<float>(),
-                    hrank ? 0 : 1, W.as<T>(), Tt.as<T>(), yamax.as<float>());
+                    hrank ? 0 : 1, W.as<T>(), Tt.as<T>(), ygemm ? nullptr : yamax.as<float>());
                 KFB_CUDA_TRY(cudaGetLastError());
             }
         }
@@ -2332,12 +2557,14 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
         auto tr_y = std::make_unique<TraceScope>("hessian:y", s);
         float y_scale = 1.f;
         if (tc) {
-            KFB_TRY(pow2_from_device(yamax.as<float>(), s, &y_scale));
+            y_scale = yg_scale;
+            if (!ygemm) KFB_TRY(pow2_from_device(yamax.as<float>(), s, &y_scale));
             if (ygemm)
                 KFB_TRY(hess_y_gemm(pairs.data() + p0, np, ma1, ma2, rep, kj, W.as<float>(),
                                     jkh, jkl, jr_scale, w_scale, y_scale, wsh, wsl, d_ymap,
-                                    d_border, (long long)s2.v.nm * ld2 * rep, yth.as<__half>(),
-                                    ytl.as<__half>(), s));
+                                    d_border, (long long)s2.v.nm * ld2 * rep,
+                                    dpairs.as<HessPair>(), yth.as<__half>(), ytl.as<__half>(),
+                                    err.flag(), s));
             else if (hrank)
                 KFB_TRY((launch_hess_y<T, 3>(dpairs.as<HessPair>(), np, x1p, x2p, dx2p,
                                              d_perm1.as<int>(), d_lab1.as<int>(),
@@ -2408,7 +2635,7 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
             ec.tile_n64 = narrow ? 1 : 0;
             ec.sink_t = narrow ? 1 : 0;
             KFB_TRY(tc_gemm_grouped(narrow ? Yo : J, narrow ? J : Yo, 3, false, tprobs, sink, s,
-                                    ec));
+                                    ec, err.flag()));
             tr_g.reset();
             if constexpr (std::is_same<T, float>::value) {
                 if (hrank) {
@@ -2441,7 +2668,7 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
                     eq.mode = EPI_DENSE;
                     eq.zf32 = d_Q.as<float>();
                     eq.ld = ldq;
-                    KFB_TRY(tc_gemm_grouped(Aq, Bq, 3, false, pqs, ElemSink(), s, eq));
+                    KFB_TRY(tc_gemm_grouped(Aq, Bq, 3, false, pqs, ElemSink(), s, eq, err.flag()));
                     const unsigned tiles =
                         (unsigned)(((ld1 + HR_T - 1) / HR_T) * ((ld2 + HR_T - 1) / HR_T));
                     hess_rank_kernel<<<dim3(tiles, (unsigned)np), 256, 0, s>>>(
@@ -2476,9 +2703,13 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
         }
         KFB_TRY(launch_gemm<T>(probs, sink, s));
     }
-    return KFB_OK;
+    return tc ? err.check(s) : KFB_OK;
 }
 
+template kfb_status compact_columns<double>(DerivSet &, DerivSet &, int &, CompactSets &,
+                                            cudaStream_t);
+template kfb_status compact_columns<float>(DerivSet &, DerivSet &, int &, CompactSets &,
+                                           cudaStream_t);
 template kfb_status jacobian_core<double>(const DerivSet &, const DerivSet &, int, double,
                                           double, bool, ElemSink, cudaStream_t);
 template kfb_status jacobian_core<float>(const DerivSet &, const DerivSet &, int, double, double,

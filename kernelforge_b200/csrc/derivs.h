@@ -38,6 +38,7 @@ struct DerivSet {
     const void *x = nullptr;   // device (nm, ma, rep)
     const void *dx = nullptr;  // device (nm, ma, rep, 3 ma) or null
     SetView v;
+    float dx_max = -1.f;       // max |dx| over the real atoms (< 0: not known)
 };
 
 __device__ __forceinline__ void sink_put(const ElemSink &s, long long idx, double v) {
@@ -100,6 +101,27 @@ __device__ __forceinline__ void sink_positions(const ElemSink &s, long long R, l
         }
     }
 }
+
+// Columns of the descriptors that no real atom of either set uses (x and dx
+// zero everywhere) contribute nothing to any derivative kernel.  When they are
+// at least an eighth of the columns and the copies fit in a quarter of the
+// free memory, s1 and s2 are replaced by copies without them (held by `keep`,
+// padded with zero columns to a multiple of 16) and rep by their width.  Either
+// way dx_max of the sets is filled in.  Synchronises the stream (the width is
+// needed on the host).
+// used[k] = 1 (device, rep ints, cleared by the caller) where a real atom of d
+// uses column k in x or dx (null: x alone); amax (optional, device, cleared):
+// [0] max |x|, [1] max |dx| over the real atoms; nat: their counts (device).
+template <class T>
+kfb_status scan_columns(const DerivSet &d, int rep, const int *nat, int *used, float *amax,
+                        cudaStream_t s);
+
+struct CompactSets {
+    DevBuf x1, dx1, x2, dx2;
+};
+template <class T>
+kfb_status compact_columns(DerivSet &s1, DerivSet &s2, int &rep, CompactSets &keep,
+                           cudaStream_t s);
 
 // tc: run the contraction GEMMs on the tensor cores (split fp16, three
 // products); needs rep % 16 == 0 and an sm_100 device.

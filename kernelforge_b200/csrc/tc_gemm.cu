@@ -896,12 +896,15 @@ kfb_status tc_gemm_grouped(const TcOperand &A, const TcOperand &B, int nprod, bo
 // Power of two that brings the largest |value| to about 2^14: keeps the hi/lo
 // fp16 pair out of fp16's subnormal range for the small entries (the pair
 // then carries ~22 significant bits over ~28 binades below the maximum).
+float pow2_for(float m) {
+    return (m > 0.f && std::isfinite(m)) ? std::ldexp(1.f, 14 - (int)std::ceil(std::log2(m))) : 1.f;
+}
+
 kfb_status pow2_from_device(const float *dmax, cudaStream_t s, float *scale) {
     float m = 0.f;
     KFB_CUDA_TRY(cudaMemcpyAsync(&m, dmax, sizeof(float), cudaMemcpyDeviceToHost, s));
     KFB_CUDA_TRY(cudaStreamSynchronize(s));
-    *scale = 1.f;
-    if (m > 0.f && std::isfinite(m)) *scale = std::ldexp(1.f, 14 - (int)std::ceil(std::log2(m)));
+    *scale = pow2_for(m);
     return KFB_OK;
 }
 
@@ -931,11 +934,13 @@ kfb_status split_rows(const T *src, long long n, __half *hi, __half *lo, float *
 
 template <class T>
 kfb_status transpose_split_dx(const T *dx, int nm, int ma, int rep, const int *nat, __half *hi,
-                              __half *lo, float *scale, cudaStream_t s) {
+                              __half *lo, float *scale, cudaStream_t s, float dx_max) {
     const long long kk = (long long)ma * rep;
     *scale = 1.f;
     if (nm <= 0) return KFB_OK;
-    {
+    if (dx_max >= 0.f) {
+        *scale = pow2_for(dx_max);
+    } else {
         DevBuf d;
         KFB_TRY(d.alloc(sizeof(float), s));
         KFB_TRY(zero(d.ptr, sizeof(float), s));
@@ -955,10 +960,12 @@ kfb_status transpose_split_dx(const T *dx, int nm, int ma, int rep, const int *n
 template <class T>
 kfb_status transpose_split_dx_rows(const T *dx, int nm, int ma, int rep, const int *nat,
                                    __half *hi, __half *lo, float *scale, cudaStream_t s,
-                                   const int *blockmap) {
+                                   const int *blockmap, float dx_max) {
     *scale = 1.f;
     if (nm <= 0) return KFB_OK;
-    {
+    if (dx_max >= 0.f) {
+        *scale = pow2_for(dx_max);
+    } else {
         DevBuf d;
         KFB_TRY(d.alloc(sizeof(float), s));
         KFB_TRY(zero(d.ptr, sizeof(float), s));
@@ -993,11 +1000,11 @@ template kfb_status split_rows<double>(const double *, long long, __half *, __ha
                                        cudaStream_t);
 template kfb_status transpose_split_dx_rows<float>(const float *, int, int, int, const int *,
                                                    __half *, __half *, float *, cudaStream_t,
-                                                   const int *);
+                                                   const int *, float);
 template kfb_status transpose_split_dx<float>(const float *, int, int, int, const int *, __half *,
-                                              __half *, float *, cudaStream_t);
+                                              __half *, float *, cudaStream_t, float);
 template kfb_status transpose_split_dx<double>(const double *, int, int, int, const int *,
-                                               __half *, __half *, float *, cudaStream_t);
+                                               __half *, __half *, float *, cudaStream_t, float);
 template kfb_status transpose_split_y<float>(const float *, int, int, int, int, const float *,
                                              __half *, __half *, float *, cudaStream_t);
 template kfb_status transpose_split_y<double>(const double *, int, int, int, int, const float *,

@@ -97,6 +97,8 @@ kfb_status tc_gemm_grouped(const TcOperand &A, const TcOperand &B, int nprod, bo
 //   transpose_split_dx: nat (device int32, per molecule) limits the scale to
 //                       the real atoms, padding may hold anything; 32 x 32
 //                       tiles wholly beyond the real atoms stay unwritten;
+//                       dx_max >= 0 is that largest magnitude when the caller
+//                       knows it (else a pass and a synchronisation find it);
 //   transpose_split_y:  amax (device float) is the largest |entry| the
 //                       producer wrote (the rest of Y is never read).
 template <class T>
@@ -109,10 +111,12 @@ kfb_status split_rows(const T *src, long long n, __half *hi, __half *lo, float *
 template <class T>
 kfb_status transpose_split_dx_rows(const T *dx, int nm, int ma, int rep, const int *nat,
                                    __half *hi, __half *lo, float *scale, cudaStream_t s,
-                                   const int *blockmap = nullptr);
+                                   const int *blockmap = nullptr, float dx_max = -1.f);
 template <class T>
 kfb_status transpose_split_dx(const T *dx, int nm, int ma, int rep, const int *nat, __half *hi,
-                              __half *lo, float *scale, cudaStream_t s);
+                              __half *lo, float *scale, cudaStream_t s, float dx_max = -1.f);
+// Power of two that brings m to about 2^14 (1 for 0 and what is not finite).
+float pow2_for(float m);
 // Host copy of a power of two that brings the device float *dmax to about
 // 2^14 (synchronises the stream).
 kfb_status pow2_from_device(const float *dmax, cudaStream_t s, float *scale);

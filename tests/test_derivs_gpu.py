@@ -115,6 +115,44 @@ def test_tensor_core_contractions_match_oracle(rep):
           o.kernel_gaussian_full(X1, dX1, X2, dX2, Q1, Q2, N1, N2, s), p)
 
 
+@pytest.mark.parametrize("precision", ["fp64", "fp32", "split_f16"])
+@pytest.mark.parametrize("rep,used", [(48, 0), (48, 5), (48, 30), (48, 31), (96, 17), (50, 20)])
+def test_unused_columns(rep, used, precision):
+    """Columns that no real atom of either set uses are left out (when they are an eighth of the
+    columns or more after rounding up to 16, 32 and 33 of 48): padding holds values there, one column is used by a single
+    Jacobian entry of set 2 alone, another by a descriptor of set 1 alone."""
+    from kernelforge_b200 import local_kernels as lk
+    X1, dX1, Q1, N1 = make_set(7, 6, rep, 3, 31 + used)
+    X2, dX2, Q2, N2 = make_set(5, 5, rep, 3, 32 + used)
+    sc = 1.0 / np.sqrt(max(used, 1))
+    rng = np.random.default_rng(used)
+    off = rng.permutation(rep)[used:]
+    for X, dX in ((X1, dX1), (X2, dX2)):
+        X *= 2 * sc
+        dX *= sc
+        X[:, :, off] = 0.0
+        dX[:, :, off] = 0.0
+    for m in range(len(N1)):     # padding is not read
+        X1[m, N1[m]:] = 7.0
+        dX1[m, N1[m]:] = 7.0
+        dX1[m, :, :, 3 * N1[m]:] = 7.0
+    dX2[1, 0, off[0], 1] = 0.5
+    X1[2, 0, off[-1]] = 0.5
+    s, p = 2.0, precision
+    close(lk.kernel_gaussian_jacobian(X1, X2, dX2, Q1, Q2, N1, N2, s, precision=p),
+          o.kernel_gaussian_jacobian(X1, X2, dX2, Q1, Q2, N1, N2, s), p)
+    close(lk.kernel_gaussian_jacobian_t(X1, dX1, X2, Q1, Q2, N1, N2, s, precision=p),
+          o.kernel_gaussian_jacobian_t(X1, dX1, X2, Q1, Q2, N1, N2, s), p)
+    close(lk.kernel_gaussian_full(X1, dX1, X2, dX2, Q1, Q2, N1, N2, s, precision=p),
+          o.kernel_gaussian_full(X1, dX1, X2, dX2, Q1, Q2, N1, N2, s), p)
+    close(lk.kernel_gaussian_full_symm_rfp(X1, dX1, Q1, N1, s, precision=p),
+          o.kernel_gaussian_full_symm_rfp(X1, dX1, Q1, N1, s), p)
+    # one array, two sets of atom counts
+    N3 = np.maximum(N1 - 1, 0).astype(np.int32)
+    close(lk.kernel_gaussian_hessian(X1, dX1, X1, dX1, Q1, Q1, N3, N1, s, precision=p),
+          o.kernel_gaussian_hessian(X1, dX1, X1, dX1, Q1, Q1, N3, N1, s), p)
+
+
 @pytest.mark.parametrize("precision,rep", [("fp64", 33), ("fp32", 33), ("split_f16", 48)])
 def test_jacobian_chunked_outer_molecules(precision, rep, monkeypatch):
     """A workspace of a few kB splits the outer molecules into chunks (each with
