@@ -20,11 +20,12 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
+#include <cstring>
 #include <exception>
 #include <mutex>
 #include <vector>
 
-#include "kfb_internal.h"
+#include "derivs.h"
 #include "tc_gemm.h"
 
 using bf16 = __nv_bfloat16;
@@ -367,46 +368,199 @@ size_t feature_budget() {
     return b;
 }
 
-// ---------------------------------------------------------------- RFF forces
-// K-padded operands for the force path (the tensor-core GEMM needs K % 16 == 0):
-// dst (rows, kpad) with dst[r][k] = src row r (stride src_ld) for k < rep, else 0.
+// ---------------------------------------------------------------- RFF
+// Operands of the RFF products (x W_e and dX^T W_e): fp16 pairs with K along
+// the descriptor columns that the atoms use (cols, n of them; W's rows that
+// meet only zeros are left out), K padded with zeros to a multiple of 16, and
+// one power-of-two scale for all of x, of dX and of W.
+
+// *amax = max |w|; a column with a value that is not finite counts as used
+// (its products with zeros are not zero).  Rows of d values, row r is column
+// r % rep.
+__global__ void __launch_bounds__(256) rff_weight_scan_kernel(const float *__restrict__ w, int rep,
+                                                              int d, float *__restrict__ amax,
+                                                              int *__restrict__ used) {
+    const float *row = w + (size_t)blockIdx.x * d;
+    float m = 0.f;
+    bool bad = false;
+    for (int c = threadIdx.x; c < d; c += blockDim.x) {
+        const float v = fabsf(row[c]);
+        m = fmaxf(m, v);
+        bad |= !(v <= 3.402823466e38f);
+    }
+    if (bad) used[blockIdx.x % rep] = 1;
+    for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<int *>(amax), __float_as_int(m));
+}
+
+__device__ __forceinline__ void split_fp16(float v, __half &h, __half &l) {
+    h = __float2half_rn(v);
+    l = __float2half_rn(v - __half2float(h));
+}
+
+// out[r][p] = pair of scale x[idx[r]][cols[p]] (p < n), zero for n <= p < kpad
 template <class T>
-__global__ void gather_pad_rows_kernel(const T *__restrict__ x, const int *__restrict__ idx,
-                                       int nrows, int rep, int kpad, float *__restrict__ out) {
-    const long long n = (long long)nrows * kpad;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
+__global__ void rff_x_rows_kernel(const T *__restrict__ x, const int *__restrict__ idx, int nrows,
+                                  int rep, const int *__restrict__ cols, int n, int kpad,
+                                  float scale, __half *__restrict__ hi, __half *__restrict__ lo) {
+    const long long total = (long long)nrows * kpad;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
          i += (long long)gridDim.x * blockDim.x) {
-        const int r = (int)(i / kpad), k = (int)(i % kpad);
-        out[i] = k < rep ? (float)x[(size_t)idx[r] * rep + k] : 0.f;
+        const int r = (int)(i / kpad), p = (int)(i - (long long)r * kpad);
+        const float v = p < n ? (float)x[(size_t)idx[r] * rep + cols[p]] * scale : 0.f;
+        split_fp16(v, hi[i], lo[i]);
     }
 }
 
-// wt (d, kpad) = W_e^T, zero beyond rep
-__global__ void transpose_pad_kernel(const float *__restrict__ w, int rep, int d, int kpad,
-                                     float *__restrict__ wt) {
+// wt[c][p] = pair of scale w[cols[p]][c] (w: rep rows of d), zero for n <= p < kpad
+__global__ void rff_w_rows_kernel(const float *__restrict__ w, int d, const int *__restrict__ cols,
+                                  int n, int kpad, float scale, __half *__restrict__ hi,
+                                  __half *__restrict__ lo) {
     __shared__ float tile[32][33];
-    const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
+    const int p0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
     for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-        const int rr = r0 + r, cc = c0 + threadIdx.x;
-        tile[r][threadIdx.x] = (rr < rep && cc < d) ? w[(size_t)rr * d + cc] : 0.f;
+        const int p = p0 + r, c = c0 + threadIdx.x;
+        tile[r][threadIdx.x] = (p < n && c < d) ? w[(size_t)cols[p] * d + c] * scale : 0.f;
     }
     __syncthreads();
     for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-        const int cc = c0 + r, rr = r0 + threadIdx.x;  // output row cc (feature), column rr
-        if (cc < d && rr < kpad) wt[(size_t)cc * kpad + rr] = tile[threadIdx.x][r];
+        const int c = c0 + r, p = p0 + threadIdx.x;
+        if (c < d && p < kpad) {
+            const size_t o = (size_t)c * kpad + p;
+            split_fp16(tile[threadIdx.x][r], hi[o], lo[o]);
+        }
     }
 }
 
-// Jacobian rows: out[r][k] = dx[(src[r] * rep + k) * ld + col[r]] (k < rep), 0 beyond
+// Jacobian rows of a chunk's atoms: row + c step = pair of scale
+// dx[atom][cols[.]][c] for c < ncol; with them the destination row dst + c and
+// the atom's number in the chunk (its row of sines).  Tiles of 64 columns x 32
+// coordinates through shared memory: dX is read along its rows, the pairs are
+// written 128 bytes a warp (a row per thread block read dX 4 bytes per 32-byte
+// sector: 0.59 ms for 3,150 atoms of 21).
+struct RffAtom {
+    int atom, row, step, ncol, dst;
+};
 template <class T>
-__global__ void jacobian_rows_kernel(const T *__restrict__ dx, const int *__restrict__ src,
-                                     const int *__restrict__ col, int nrows, int rep, int ld,
-                                     int kpad, float *__restrict__ out) {
-    const int r = blockIdx.x;
-    if (r >= nrows) return;
-    const T *base = dx + (size_t)src[r] * rep * ld + col[r];
-    for (int k = threadIdx.x; k < kpad; k += blockDim.x)
-        out[(size_t)r * kpad + k] = k < rep ? (float)base[(size_t)k * ld] : 0.f;
+__global__ void __launch_bounds__(256) rff_jacobian_rows_kernel(
+    const T *__restrict__ dx, const RffAtom *__restrict__ atoms, int rep, int ld,
+    const int *__restrict__ cols, int n, int kpad, float scale, __half *__restrict__ hi,
+    __half *__restrict__ lo, int *__restrict__ dst, int *__restrict__ aux) {
+    __shared__ float tile[64][33];
+    const RffAtom a = atoms[blockIdx.x];
+    const int p0 = blockIdx.y * 64, c0 = blockIdx.z * 32;
+    if (c0 >= a.ncol) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const T *base = dx + (size_t)a.atom * rep * ld;
+    for (int r = warp; r < 64; r += 8) {
+        const int p = p0 + r, c = c0 + lane;
+        tile[r][lane] = (p < n && c < a.ncol) ? (float)base[(size_t)cols[p] * ld + c] * scale : 0.f;
+    }
+    __syncthreads();
+    const int p = p0 + 2 * lane;
+    for (int r = warp; r < 32; r += 8) {
+        const int c = c0 + r;
+        if (c >= a.ncol) break;
+        const long long row = a.row + (long long)c * a.step;
+        if (p < kpad) {   // kpad is a multiple of 16
+            __half2 h, l;
+            split_fp16(tile[2 * lane][r], h.x, l.x);
+            split_fp16(tile[2 * lane + 1][r], h.y, l.y);
+            *reinterpret_cast<__half2 *>(hi + row * kpad + p) = h;
+            *reinterpret_cast<__half2 *>(lo + row * kpad + p) = l;
+        }
+        if (p0 == 0 && lane == 0) {
+            dst[row] = a.dst + c;
+            aux[row] = (int)blockIdx.x;
+        }
+    }
+}
+
+// What both RFF maps prepare: used columns, scales, element rows.
+struct RffPlan {
+    ElemRows er;
+    DevBuf cols, err, wh, wl, xh, xl;
+    int n = 0, kpad = 0;
+    float x_scale = 1.f, dx_scale = 1.f, w_scale = 1.f;
+};
+
+template <class T>
+kfb_status rff_plan(const T *x, const T *dx, const int *q, const int *n, int nm, int ma, int rep,
+                    const float *w, int nelem, int d, RffPlan &pl, cudaStream_t s) {
+    KFB_TRY(elem_rows(q, n, nm, ma, nelem, pl.er));
+    // used columns (rep ints), then max |x|, |dx|, |w|
+    DevBuf scan, dn;
+    KFB_TRY(scan.alloc((size_t)rep * sizeof(int) + 3 * sizeof(float), s));
+    KFB_TRY(zero(scan.ptr, (size_t)rep * sizeof(int) + 3 * sizeof(float), s));
+    float *amax = reinterpret_cast<float *>(scan.as<int>() + rep);
+    std::vector<int> nat(n, n + nm);
+    KFB_TRY(upload(dn, nat, s));
+    DerivSet ds;
+    ds.x = x;
+    ds.dx = dx;
+    ds.v.n = nat.data();
+    ds.v.nm = nm;
+    ds.v.ma = ma;
+    KFB_TRY(scan_columns<T>(ds, rep, dn.as<int>(), scan.as<int>(), amax, s));
+    rff_weight_scan_kernel<<<(unsigned)(nelem * rep), 256, 0, s>>>(w, rep, d, amax + 2,
+                                                                  scan.as<int>());
+    KFB_CUDA_TRY(cudaGetLastError());
+    std::vector<int> host(rep + 3), cols;
+    KFB_CUDA_TRY(cudaMemcpyAsync(host.data(), scan.ptr, host.size() * sizeof(int),
+                                 cudaMemcpyDeviceToHost, s));
+    KFB_CUDA_TRY(cudaStreamSynchronize(s));
+    float mx[3];
+    std::memcpy(mx, host.data() + rep, sizeof(mx));
+    pl.x_scale = pow2_for(mx[0]);
+    pl.dx_scale = pow2_for(mx[1]);
+    pl.w_scale = pow2_for(mx[2]);
+    for (int k = 0; k < rep; ++k)
+        if (host[k]) cols.push_back(k);
+    pl.n = (int)cols.size();
+    pl.kpad = std::max(16, (pl.n + 15) / 16 * 16);
+    cols.resize(std::max<size_t>(cols.size(), 1));
+    KFB_TRY(upload(pl.cols, cols, s));
+    KFB_TRY(pl.err.alloc(sizeof(int), s));
+    KFB_TRY(zero(pl.err.ptr, sizeof(int), s));
+    KFB_TRY(pl.wh.alloc((size_t)d * pl.kpad * sizeof(__half), s));
+    KFB_TRY(pl.wl.alloc((size_t)d * pl.kpad * sizeof(__half), s));
+    return KFB_OK;
+}
+
+// W_e as rows of features (B operand of the products)
+kfb_status rff_weights(const RffPlan &pl, const float *w, int d, TcOperand &B, cudaStream_t s) {
+    rff_w_rows_kernel<<<dim3(nblk(d, 32), nblk(pl.kpad, 32)), dim3(32, 8), 0, s>>>(
+        w, d, pl.cols.as<int>(), pl.n, pl.kpad, pl.w_scale, pl.wh.as<__half>(),
+        pl.wl.as<__half>());
+    KFB_CUDA_TRY(cudaGetLastError());
+    B.hi = pl.wh.ptr;
+    B.lo = pl.wl.ptr;
+    B.rows = d;
+    B.cols = pl.kpad;
+    return KFB_OK;
+}
+
+// Descriptor rows idx[0 .. nr) (device) as the A operand
+template <class T>
+kfb_status rff_rows(RffPlan &pl, const T *x, const int *idx, int nr, int rep, TcOperand &A,
+                    cudaStream_t s) {
+    rff_x_rows_kernel<T><<<nblk((long long)nr * pl.kpad, 256 * 8), 256, 0, s>>>(
+        x, idx, nr, rep, pl.cols.as<int>(), pl.n, pl.kpad, pl.x_scale, pl.xh.as<__half>(),
+        pl.xl.as<__half>());
+    KFB_CUDA_TRY(cudaGetLastError());
+    A.hi = pl.xh.ptr;
+    A.lo = pl.xl.ptr;
+    A.rows = nr;
+    A.cols = pl.kpad;
+    return KFB_OK;
+}
+
+kfb_status rff_done(const RffPlan &pl, cudaStream_t s) {
+    int herr = 0;
+    KFB_CUDA_TRY(cudaMemcpyAsync(&herr, pl.err.ptr, sizeof(int), cudaMemcpyDeviceToHost, s));
+    KFB_CUDA_TRY(cudaStreamSynchronize(s));
+    if (herr) return set_error(KFB_ERR_TIMEOUT, "RFF features: a tensor-core pipeline wait timed out");
+    return KFB_OK;
 }
 
 template <class T>
@@ -414,67 +568,50 @@ kfb_status rff_features_t(const T *x, const int *q, const int *n, int nm, int ma
                           const float *w, const float *b, int nelem, int d, float *z,
                           cudaStream_t s) {
     KFB_TRY(zero(z, (size_t)nm * d * sizeof(float), s));
-    ElemRows er;
-    KFB_TRY(elem_rows(q, n, nm, ma, nelem, er));
-    // W_e^T (d, kpad) split once per element; K padded with zeros to a multiple of 16
-    const int kpad = (rep + 15) / 16 * 16;
-    DevBuf wt, wh, wl;
-    KFB_TRY(wt.alloc((size_t)d * kpad * sizeof(float), s));
-    KFB_TRY(wh.alloc((size_t)d * kpad * sizeof(__half), s));
-    KFB_TRY(wl.alloc((size_t)d * kpad * sizeof(__half), s));
-    const size_t row_bytes = (size_t)kpad * (sizeof(float) + 2 * sizeof(__half));
-    const int chunk = (int)std::max<size_t>(128, feature_budget() / row_bytes);
-    DevBuf xr, xh, xl, didx, dmol;
-    const float sc = std::sqrt(2.f / (float)d);
+    RffPlan pl;
+    KFB_TRY(rff_plan<T>(x, nullptr, q, n, nm, ma, rep, w, nelem, d, pl, s));
+    const size_t row_bytes = (size_t)pl.kpad * 2 * sizeof(__half);
+    const int chunk = (int)std::min<size_t>(1 << 30, std::max<size_t>(128, feature_budget() / row_bytes));
+    // rows and molecules of every element, one upload
+    std::vector<int> rows;
+    int most = 1;
     for (int e = 0; e < nelem; ++e) {
-        const int ne = (int)er.idx[e].size();
+        rows.insert(rows.end(), pl.er.idx[e].begin(), pl.er.idx[e].end());
+        rows.insert(rows.end(), pl.er.mol[e].begin(), pl.er.mol[e].end());
+        most = std::max(most, std::min(chunk, (int)pl.er.idx[e].size()));
+    }
+    if (rows.empty()) return KFB_OK;
+    DevBuf drows;
+    KFB_TRY(upload(drows, rows, s));
+    KFB_TRY(pl.xh.alloc((size_t)most * pl.kpad * sizeof(__half), s));
+    KFB_TRY(pl.xl.alloc((size_t)most * pl.kpad * sizeof(__half), s));
+    const float sc = std::sqrt(2.f / (float)d);
+    const int *idx = drows.as<int>();
+    for (int e = 0; e < nelem; ++e) {
+        const int ne = (int)pl.er.idx[e].size();
         if (ne == 0) continue;
-        transpose_pad_kernel<<<dim3(nblk(d, 32), nblk(kpad, 32)), dim3(32, 8), 0, s>>>(
-            w + (size_t)e * rep * d, rep, d, kpad, wt.as<float>());
-        KFB_CUDA_TRY(cudaGetLastError());
-        float w_scale = 1.f;
-        KFB_TRY(split_rows<float>(wt.as<float>(), (long long)d * kpad, wh.as<__half>(),
-                                  wl.as<__half>(), &w_scale, s));
-        KFB_TRY(upload(didx, er.idx[e], s));
-        KFB_TRY(upload(dmol, er.mol[e], s));
-        const int rows_max = std::min(ne, chunk);
-        KFB_TRY(xr.alloc((size_t)rows_max * kpad * sizeof(float), s));
-        KFB_TRY(xh.alloc((size_t)rows_max * kpad * sizeof(__half), s));
-        KFB_TRY(xl.alloc((size_t)rows_max * kpad * sizeof(__half), s));
+        TcOperand A, B;
+        KFB_TRY(rff_weights(pl, w + (size_t)e * rep * d, d, B, s));
         for (int r0 = 0; r0 < ne; r0 += chunk) {
             const int nr = std::min(chunk, ne - r0);
-            gather_pad_rows_kernel<T><<<nblk((long long)nr * kpad, 256 * 8), 256, 0, s>>>(
-                x, didx.as<int>() + r0, nr, rep, kpad, xr.as<float>());
-            KFB_CUDA_TRY(cudaGetLastError());
-            float x_scale = 1.f;
-            KFB_TRY(split_rows<float>(xr.as<float>(), (long long)nr * kpad, xh.as<__half>(),
-                                      xl.as<__half>(), &x_scale, s));
-            TcOperand A, B;
-            A.hi = xh.ptr;
-            A.lo = xl.ptr;
-            A.rows = nr;
-            A.cols = kpad;
-            B.hi = wh.ptr;
-            B.lo = wl.ptr;
-            B.rows = d;
-            B.cols = kpad;
+            KFB_TRY(rff_rows<T>(pl, x, idx + r0, nr, rep, A, s));
             TcProb p{};
             p.M = nr;
             p.N = d;
-            p.K = kpad;
-            p.row_off = 0;
-            p.alpha = 1.0 / ((double)x_scale * (double)w_scale);
+            p.K = pl.kpad;
+            p.alpha = 1.0 / ((double)pl.x_scale * (double)pl.w_scale);
             TcEpi epi;
             epi.mode = EPI_COS_MOLSUM;
             epi.bias = b + (size_t)e * d;
-            epi.mol = dmol.as<int>() + r0;
+            epi.mol = idx + ne + r0;
             epi.molsum = z;
             epi.ld = d;
             epi.scale = sc;
-            KFB_TRY(tc_gemm_grouped(A, B, 3, false, {p}, ElemSink(), s, epi));
+            KFB_TRY(tc_gemm_grouped(A, B, 3, false, {p}, ElemSink(), s, epi, pl.err.as<int>()));
         }
+        idx += 2 * (size_t)ne;
     }
-    return KFB_OK;
+    return rff_done(pl, s);
 }
 
 // G (naq, d) += rows 3 off_m + c: sqrt(2/d) sum_j sin(z_j) (W_e^T dX[m, j, :, c]), z_j the
@@ -486,121 +623,107 @@ kfb_status rff_gradient_t(const T *x, const T *dx, const int *q, const int *n, i
     std::vector<int> offs(nm + 1, 0);
     for (int m = 0; m < nm; ++m) offs[m + 1] = offs[m] + 3 * std::min(std::max(n[m], 0), ma);
     KFB_TRY(zero(g, (size_t)std::max(offs[nm], 1) * d * sizeof(float), s));
-    ElemRows er;
-    KFB_TRY(elem_rows(q, n, nm, ma, nelem, er));
-    const int kpad = (rep + 15) / 16 * 16, ld = 3 * ma;
-    DevBuf wt, wh, wl;
-    KFB_TRY(wt.alloc((size_t)d * kpad * sizeof(float), s));
-    KFB_TRY(wh.alloc((size_t)d * kpad * sizeof(__half), s));
-    KFB_TRY(wl.alloc((size_t)d * kpad * sizeof(__half), s));
-    // per atom: one Z row (d floats) and up to 3 ma Jacobian rows (kpad wide, FP32 + pair)
+    RffPlan pl;
+    KFB_TRY(rff_plan<T>(x, dx, q, n, nm, ma, rep, w, nelem, d, pl, s));
+    const int kpad = pl.kpad, ld = 3 * ma;
+    // per atom: one row of d sines, one descriptor and up to 3 ma Jacobian rows
     const size_t atom_bytes = (size_t)d * sizeof(float) +
-                              (size_t)(1 + ld) * kpad * (sizeof(float) + 2 * sizeof(__half));
-    const int chunk = (int)std::max<size_t>(1, feature_budget() / atom_bytes);
-    const float sc = std::sqrt(2.f / (float)d);
-    DevBuf zpre, xr, xh, xl, jr, jh, jl, didx, dsrc, dcol, ddst, daux;
+                              (size_t)(1 + ld) * kpad * 2 * sizeof(__half) +
+                              (size_t)ld * 2 * sizeof(int);
+    const int chunk = (int)std::min<size_t>((size_t)(1 << 30) / ld,
+                                            std::max<size_t>(1, feature_budget() / atom_bytes));
+    // every element's atoms: descriptor row, then its Jacobian rows, ordered
+    // (molecule, c, atom) inside a chunk so that one destination is one run
+    std::vector<RffAtom> atoms;
+    std::vector<int> idx;
+    struct Chunk {
+        int e, a0, na, nr;
+    };
+    std::vector<Chunk> chunks;
+    int most_a = 1, most_r = 1;
     for (int e = 0; e < nelem; ++e) {
-        const int ne = (int)er.idx[e].size();
-        if (ne == 0) continue;
-        transpose_pad_kernel<<<dim3(nblk(d, 32), nblk(kpad, 32)), dim3(32, 8), 0, s>>>(
-            w + (size_t)e * rep * d, rep, d, kpad, wt.as<float>());
-        KFB_CUDA_TRY(cudaGetLastError());
-        float w_scale = 1.f;
-        KFB_TRY(split_rows<float>(wt.as<float>(), (long long)d * kpad, wh.as<__half>(),
-                                  wl.as<__half>(), &w_scale, s));
-        TcOperand B;
-        B.hi = wh.ptr;
-        B.lo = wl.ptr;
-        B.rows = d;
-        B.cols = kpad;
-        for (int a0 = 0; a0 < ne; a0 += chunk) {
-            const int na = std::min(chunk, ne - a0);
-            // rows of the chunk, ordered (molecule, c, atom): one destination per run
-            std::vector<int> src, col, dst, aux;
+        const std::vector<int> &ai = pl.er.idx[e], &am = pl.er.mol[e];
+        for (int a0 = 0; a0 < (int)ai.size(); a0 += chunk) {
+            const int na = std::min<int>(chunk, (int)ai.size() - a0);
+            Chunk ck{e, (int)atoms.size(), na, 0};
+            int row = 0;
             for (int t = 0; t < na;) {
-                const int m = er.mol[e][a0 + t];
+                const int m = am[a0 + t];
                 int t1 = t;
-                while (t1 < na && er.mol[e][a0 + t1] == m) ++t1;
+                while (t1 < na && am[a0 + t1] == m) ++t1;
                 const int nc = offs[m + 1] - offs[m];
-                for (int c = 0; c < nc; ++c)
-                    for (int u = t; u < t1; ++u) {
-                        src.push_back(er.idx[e][a0 + u]);
-                        col.push_back(c);
-                        dst.push_back(offs[m] + c);
-                        aux.push_back(u);
-                    }
+                for (int u = t; u < t1; ++u) {
+                    atoms.push_back({ai[a0 + u], row + (u - t), t1 - t, nc, offs[m]});
+                    idx.push_back(ai[a0 + u]);
+                }
+                row += nc * (t1 - t);
                 t = t1;
             }
-            const int nr = (int)src.size();
-            std::vector<int> aidx(er.idx[e].begin() + a0, er.idx[e].begin() + a0 + na);
-            KFB_TRY(upload(didx, aidx, s));
-            KFB_TRY(upload(dsrc, src, s));
-            KFB_TRY(upload(dcol, col, s));
-            KFB_TRY(upload(ddst, dst, s));
-            KFB_TRY(upload(daux, aux, s));
-            // pre-activations Z = X_e W_e + b_e (na, d), FP32
-            KFB_TRY(zpre.alloc((size_t)na * d * sizeof(float), s));
-            KFB_TRY(xr.alloc((size_t)na * kpad * sizeof(float), s));
-            KFB_TRY(xh.alloc((size_t)na * kpad * sizeof(__half), s));
-            KFB_TRY(xl.alloc((size_t)na * kpad * sizeof(__half), s));
-            gather_pad_rows_kernel<T><<<nblk((long long)na * kpad, 256 * 8), 256, 0, s>>>(
-                x, didx.as<int>(), na, rep, kpad, xr.as<float>());
-            KFB_CUDA_TRY(cudaGetLastError());
-            float x_scale = 1.f;
-            KFB_TRY(split_rows<float>(xr.as<float>(), (long long)na * kpad, xh.as<__half>(),
-                                      xl.as<__half>(), &x_scale, s));
-            {
-                TcOperand A;
-                A.hi = xh.ptr;
-                A.lo = xl.ptr;
-                A.rows = na;
-                A.cols = kpad;
-                TcProb p{};
-                p.M = na;
-                p.N = d;
-                p.K = kpad;
-                p.alpha = 1.0 / ((double)x_scale * (double)w_scale);
-                TcEpi epi;
-                epi.mode = EPI_DENSE;
-                epi.zf32 = zpre.as<float>();
-                epi.bias = b + (size_t)e * d;
-                epi.ld = d;
-                KFB_TRY(tc_gemm_grouped(A, B, 3, false, {p}, ElemSink(), s, epi));
-            }
-            // Jacobian rows (nr, kpad) times W_e, weighted by sqrt(2/d) sin(Z) and
-            // summed into G per destination row
-            KFB_TRY(jr.alloc((size_t)nr * kpad * sizeof(float), s));
-            KFB_TRY(jh.alloc((size_t)nr * kpad * sizeof(__half), s));
-            KFB_TRY(jl.alloc((size_t)nr * kpad * sizeof(__half), s));
-            jacobian_rows_kernel<T><<<nr, 128, 0, s>>>(dx, dsrc.as<int>(), dcol.as<int>(), nr, rep,
-                                                       ld, kpad, jr.as<float>());
-            KFB_CUDA_TRY(cudaGetLastError());
-            float j_scale = 1.f;
-            KFB_TRY(split_rows<float>(jr.as<float>(), (long long)nr * kpad, jh.as<__half>(),
-                                      jl.as<__half>(), &j_scale, s));
-            TcOperand A;
-            A.hi = jh.ptr;
-            A.lo = jl.ptr;
-            A.rows = nr;
-            A.cols = kpad;
-            TcProb p{};
-            p.M = nr;
-            p.N = d;
-            p.K = kpad;
-            p.alpha = 1.0 / ((double)j_scale * (double)w_scale);
-            TcEpi epi;
-            epi.mode = EPI_SIN_RUNSUM;
-            epi.mol = ddst.as<int>();
-            epi.atom = daux.as<int>();
-            epi.aux = zpre.as<float>();
-            epi.ld_aux = d;
-            epi.molsum = g;
-            epi.ld = d;
-            epi.scale = sc;
-            KFB_TRY(tc_gemm_grouped(A, B, 3, false, {p}, ElemSink(), s, epi));
+            ck.nr = row;
+            chunks.push_back(ck);
+            most_a = std::max(most_a, na);
+            most_r = std::max(most_r, row);
         }
     }
-    return KFB_OK;
+    if (atoms.empty()) return KFB_OK;
+    DevBuf datoms, didx, sines, jh, jl, ddst, daux;
+    KFB_TRY(upload(datoms, atoms, s));
+    KFB_TRY(upload(didx, idx, s));
+    KFB_TRY(pl.xh.alloc((size_t)most_a * kpad * sizeof(__half), s));
+    KFB_TRY(pl.xl.alloc((size_t)most_a * kpad * sizeof(__half), s));
+    KFB_TRY(sines.alloc((size_t)most_a * d * sizeof(float), s));
+    KFB_TRY(jh.alloc((size_t)most_r * kpad * sizeof(__half), s));
+    KFB_TRY(jl.alloc((size_t)most_r * kpad * sizeof(__half), s));
+    KFB_TRY(ddst.alloc((size_t)most_r * sizeof(int), s));
+    KFB_TRY(daux.alloc((size_t)most_r * sizeof(int), s));
+    const float sc = std::sqrt(2.f / (float)d);
+    int elem = -1;
+    TcOperand A, B;
+    for (const Chunk &ck : chunks) {
+        if (ck.e != elem) KFB_TRY(rff_weights(pl, w + (size_t)ck.e * rep * d, d, B, s));
+        elem = ck.e;
+        // sqrt(2/d) sin(x W_e + b_e) of the chunk's atoms: once per atom and
+        // feature, not once per Jacobian row (63 of a 21-atom molecule)
+        KFB_TRY(rff_rows<T>(pl, x, didx.as<int>() + ck.a0, ck.na, rep, A, s));
+        TcProb p{};
+        p.M = ck.na;
+        p.N = d;
+        p.K = kpad;
+        p.alpha = 1.0 / ((double)pl.x_scale * (double)pl.w_scale);
+        TcEpi epi;
+        epi.mode = EPI_DENSE;
+        epi.zf32 = sines.as<float>();
+        epi.zsin = 1;
+        epi.scale = sc;
+        epi.bias = b + (size_t)ck.e * d;
+        epi.ld = d;
+        KFB_TRY(tc_gemm_grouped(A, B, 3, false, {p}, ElemSink(), s, epi, pl.err.as<int>()));
+        // Jacobian rows times W_e, weighted by the sines and summed into G per
+        // destination row
+        rff_jacobian_rows_kernel<T><<<dim3(ck.na, nblk(kpad, 64), nblk(ld, 32)), 256, 0, s>>>(
+            dx, datoms.as<RffAtom>() + ck.a0, rep, ld, pl.cols.as<int>(), pl.n, kpad,
+            pl.dx_scale, jh.as<__half>(), jl.as<__half>(), ddst.as<int>(), daux.as<int>());
+        KFB_CUDA_TRY(cudaGetLastError());
+        A.hi = jh.ptr;
+        A.lo = jl.ptr;
+        A.rows = ck.nr;
+        A.cols = kpad;
+        TcProb pj{};
+        pj.M = ck.nr;
+        pj.N = d;
+        pj.K = kpad;
+        pj.alpha = 1.0 / ((double)pl.dx_scale * (double)pl.w_scale);
+        TcEpi ej;
+        ej.mode = EPI_ROW_RUNSUM;
+        ej.mol = ddst.as<int>();
+        ej.atom = daux.as<int>();
+        ej.aux = sines.as<float>();
+        ej.ld_aux = d;
+        ej.molsum = g;
+        ej.ld = d;
+        KFB_TRY(tc_gemm_grouped(A, B, 3, false, {pj}, ElemSink(), s, ej, pl.err.as<int>()));
+    }
+    return rff_done(pl, s);
 }
 
 kfb_status check_cosmlp(const kfb_cosmlp *h) {

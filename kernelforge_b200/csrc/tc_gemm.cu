@@ -420,6 +420,10 @@ __global__ void __launch_bounds__(Cfg<NPROD, NEPI, BNT>::THREADS, 1)
 #pragma unroll
                     for (int j = 0; j < 32; ++j)
                         z[j] = v[j] * alpha + __shfl_sync(0xffffffffu, bl, j);
+                    if (epi.zsin) {
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) z[j] = epi.scale * sinf(z[j]);
+                    }
                     float(*scr)[33] = molsum_scr[warp - EPI_WARP0];
                     const long long grow0 = (long long)pb.row_off + tl.m0 + q * 32;
                     const int mrows = min(32, pb.M - (tl.m0 + q * 32));  // valid rows of the chunk
@@ -516,13 +520,13 @@ __global__ void __launch_bounds__(Cfg<NPROD, NEPI, BNT>::THREADS, 1)
                         if (j < nvalid)
                             epi.act_t[(gcol0 + j) * epi.ld_t + grow] =
                                 __float2bfloat16_rn(-v[j] * alpha * sinf(g[j]));
-                } else {  // EPI_COS_MOLSUM, EPI_SIN_RUNSUM
+                } else {  // EPI_COS_MOLSUM, EPI_ROW_RUNSUM
                     // rows with one destination are consecutive: sum each run of rows
                     // per column through shared memory, one atomic add per (run, column)
                     float(*scr)[33] = molsum_scr[warp - EPI_WARP0];
                     const int mol = mvalid ? epi.mol[grow] : -1;
-                    if (epi.mode == EPI_SIN_RUNSUM) {
-                        // scale sin(aux[atom row, col]) times the product
+                    if (epi.mode == EPI_ROW_RUNSUM) {
+                        // aux[atom row, col] times the product
                         const float *a =
                             epi.aux + (long long)(mvalid ? epi.atom[grow] : 0) * epi.ld_aux + gcol0;
                         float g[32];
@@ -542,7 +546,7 @@ __global__ void __launch_bounds__(Cfg<NPROD, NEPI, BNT>::THREADS, 1)
 #pragma unroll
                         for (int j = 0; j < 32; ++j) {
                             const bool ok = mvalid && j < nvalid;
-                            scr[j][lane] = ok ? epi.scale * sinf(g[j]) * (v[j] * alpha) : 0.f;
+                            scr[j][lane] = ok ? g[j] * (v[j] * alpha) : 0.f;
                         }
                     } else {
                         const float bl = (epi.bias && lane < nvalid && nvalid > 0)
@@ -671,7 +675,7 @@ kfb_status launch(const TcOperand &A, const TcOperand &B, bool bf16,
     if (e.mode != EPI_SINK) {
         auto al = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
         bool v = e.ld % 8 == 0 && al(e.zf32) && al(e.act) && al(e.aux);
-        if (e.mode == EPI_SIN_RUNSUM) v = v && e.ld_aux % 4 == 0;
+        if (e.mode == EPI_ROW_RUNSUM) v = v && e.ld_aux % 4 == 0;
         for (const TcProb &pb : probs) v = v && pb.col_off % 8 == 0;
         e.vec = v ? 1 : 0;
     }

@@ -36,15 +36,16 @@ struct TcTile {
 // ElemSink.  The other modes serve the feature-map kernels; (row, col) is the
 // global position (row_off + m, col_off + n) and z = alpha * acc + bias[col]
 // (bias optional):
-//   EPI_DENSE      zf32[row * ld + col] = z  (or += z, atomically, with accumulate)
+//   EPI_DENSE      zf32[row * ld + col] = z  (or += z, atomically, with accumulate;
+//                  scale * sin z with zsin)
 //                  act[row * ld + col] = bf16(cos z)       (optional)
 //                  act_t[col * ld_t + row] = bf16(cos z)   (optional)
 //   EPI_DSIN_T     act_t[col * ld_t + row] = bf16(-alpha * acc * sin(aux[row * ld + col]))
 //                  (back-propagation through a cos activation)
 //   EPI_COS_MOLSUM molsum[mol[row] * ld + col] += scale * cos z, each run of
 //                  rows of one molecule summed before its atomic add
-//   EPI_SIN_RUNSUM molsum[mol[row] * ld + col] +=
-//                      scale * sin(aux[atom[row] * ld_aux + col]) * alpha * acc,
+//   EPI_ROW_RUNSUM molsum[mol[row] * ld + col] +=
+//                      aux[atom[row] * ld_aux + col] * alpha * acc,
 //                  runs of rows with one destination summed as above
 //   EPI_YSPLIT     the Hessian's Y in the layout its contraction reads: problem
 //                  row m = (c, k) = (m / y_rep, m % y_rep), column n ->
@@ -56,7 +57,7 @@ enum TcEpiMode : int {
     EPI_DENSE = 1,
     EPI_DSIN_T = 2,
     EPI_COS_MOLSUM = 3,
-    EPI_SIN_RUNSUM = 4,
+    EPI_ROW_RUNSUM = 4,
     EPI_YSPLIT = 5
 };
 
@@ -66,13 +67,14 @@ struct TcEpi {
     int sink_t = 0;    // EPI_SINK: alpha * acc stored at (col, row) instead of (row, col)
     int vec = 0;         // set by tc_gemm_grouped: 16-byte row stores allowed
     int accumulate = 0;  // EPI_DENSE: zf32 += z (atomic; split-K problems)
+    int zsin = 0;        // EPI_DENSE: zf32 = scale * sin z
     float *zf32 = nullptr;
     __nv_bfloat16 *act = nullptr;
     __nv_bfloat16 *act_t = nullptr;
     const float *aux = nullptr;
     const float *bias = nullptr;
     const int *mol = nullptr;
-    const int *atom = nullptr;  // EPI_SIN_RUNSUM: row of aux for each output row
+    const int *atom = nullptr;  // EPI_ROW_RUNSUM: row of aux for each output row
     float *molsum = nullptr;
     long long ld = 0, ld_t = 0, ld_aux = 0;
     float scale = 1.f;

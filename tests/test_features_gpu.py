@@ -346,3 +346,39 @@ def test_rff_force_features_match_reference(case, xdtype):
     Gt = crf.rff_gradient_elemental_col_major(X, dX, a["Q"], a["N"], W, b)
     np.testing.assert_allclose(Gt.cpu().numpy(), G.cpu().numpy().T, rtol=0,
                                atol=1e-6 * np.abs(Gd).max())
+
+
+@pytest.mark.parametrize("rep,used,ma,D", [(20, 0, 3, 8), (20, 3, 5, 40), (37, 16, 11, 72),
+                                           (64, 17, 21, 136), (70, 70, 13, 128)])
+def test_rff_unused_columns_and_ragged_sizes(rep, used, ma, D):
+    """Columns that are zero in every X and dX are left out of the products: none, one K step and
+    one more, all; molecules without an element, without atoms and with padding (-1, values that
+    are not read); rows, coordinates and features off the tile sizes.  Split-fp16 products with
+    FP32 sums: the tolerance of the golden cases."""
+    import torch
+    from kernelforge_b200 import cuda_rff_features as crf
+    rng = np.random.default_rng(rep + used)
+    nm, nelem = 6, 3
+    X = rng.standard_normal((nm, ma, rep)).astype(np.float32)
+    dX = rng.standard_normal((nm, ma, rep, 3 * ma)).astype(np.float32)
+    off = rng.permutation(rep)[used:]
+    X[:, :, off] = 0.0
+    dX[:, :, off] = 0.0
+    N = rng.integers(1, ma + 1, nm).astype(np.int32)
+    N[2], N[4] = 0, ma
+    Q = rng.integers(0, nelem - 1, (nm, ma)).astype(np.int32)
+    Q[0, 0] = nelem - 1
+    for m in range(nm):
+        Q[m, N[m]:] = -1
+        X[m, N[m]:] = 9.0
+        dX[m, N[m]:] = 9.0
+        dX[m, :, :, 3 * N[m]:] = 9.0
+    W = (rng.standard_normal((nelem, rep, D)) / 2).astype(np.float32)
+    b = rng.uniform(0, 6.28, (nelem, D)).astype(np.float32)
+    c = lambda a: cuda(a, torch.float32)
+    Z = crf.rff_features_elemental(c(X), Q, N, c(W), c(b))
+    G = crf.rff_gradient_elemental(c(X), c(dX), Q, N, c(W), c(b))
+    Zr = of.rff_features_elemental(X.astype(np.float64), Q, N, W, b)
+    Gr = of.rff_gradient_elemental(X.astype(np.float64), dX.astype(np.float64), Q, N, W, b)
+    assert rel(Z.cpu().numpy(), Zr) <= 2e-5
+    assert np.abs(G.cpu().numpy() - Gr).max() <= 2e-5 * max(1.0, np.abs(Gr).max())
