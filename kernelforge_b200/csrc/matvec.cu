@@ -25,10 +25,11 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
+#include <cstring>
 #include <memory>
 #include <vector>
 
-#include "kfb_internal.h"
+#include "kernels_common.cuh"
 #include "ozaki.h"
 
 namespace kfb {
@@ -82,10 +83,11 @@ __global__ void gather_f64_kernel(const Tin *__restrict__ src, const int *__rest
     }
 }
 
-// sc[r] = x_r . Ad_r and aE[r] = alpha_E[mol[r]] (0 without alpha_E)
+// sc[r] = x_r . Ad_r and aE[r] = alpha_E of atom idx[r]'s molecule (0 without
+// alpha_E)
 __global__ void train_scalars_kernel(const double *__restrict__ X, const double *__restrict__ Ad,
-                                     const int *__restrict__ mol, const double *__restrict__ alpha_e,
-                                     int nrows, int rep, double *__restrict__ sc,
+                                     const int *__restrict__ idx, int ma,
+                                     const double *__restrict__ alpha_e, int nrows, int rep, double *__restrict__ sc,
                                      double *__restrict__ ae) {
     const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
@@ -96,7 +98,7 @@ __global__ void train_scalars_kernel(const double *__restrict__ X, const double 
     for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (lane == 0) {
         sc[r] = s;
-        ae[r] = alpha_e ? alpha_e[mol[r]] : 0.0;
+        ae[r] = alpha_e ? alpha_e[idx[r] / ma] : 0.0;
     }
 }
 
@@ -107,8 +109,8 @@ __global__ void train_scalars_kernel(const double *__restrict__ X, const double 
 __global__ void pair_weights_kernel(double *__restrict__ G, double *__restrict__ P, int r2,
                                     const double *__restrict__ n1, const double *__restrict__ n2,
                                     const double *__restrict__ sc, const double *__restrict__ ae,
-                                    const int *__restrict__ mol1, int with_ad, int with_f,
-                                    double c, double is2, double is4, double *__restrict__ E,
+                                    const int *__restrict__ idx1, int ma1, int with_ad,
+                                    int with_f, double c, double is2, double is4, double *__restrict__ E,
                                     double *__restrict__ rowv) {
     const int i = blockIdx.x;
     double *Gi = G + (size_t)i * r2;
@@ -144,7 +146,7 @@ __global__ void pair_weights_kernel(double *__restrict__ G, double *__restrict__
             te += red[0][w];
             tv += red[1][w];
         }
-        if (E) atomicAdd(E + mol1[i], te);
+        if (E) atomicAdd(E + idx1[i] / ma1, te);
         if (rowv) rowv[i] = tv;
     }
 }
@@ -156,23 +158,313 @@ __global__ void add_row_scaled_kernel(const double *__restrict__ X1, const doubl
     if (e < (long long)rows * rep) g[e] += rowv[e / rep] * X1[e];
 }
 
-// F[off_a + c] += sum_k dX1[a, i, k, c] g[r, k] for the query rows r of the
-// chunk (molecule a, atom i); threads over c (coalesced along dX1 rows).
+// F[off_a + c] += sum_k dX1[a, i, k, c] (g[r, k] + rowv[r] x1[a, i, k]) for the
+// query rows r (molecule a, atom i) and the columns k of this block's slice
+// (blockIdx.y); rowv null: g alone.  Lanes over c (64 at a time, coalesced
+// along the Jacobian's rows), 4 columns k at once; the slices of a row fill
+// the SMs that one block per row left idle for a few molecules.
+constexpr int FC_K = 80;
+
 template <class Tin>
-__global__ void force_contract_kernel(const Tin *__restrict__ dx1, const int *__restrict__ idx1,
-                                      const int *__restrict__ mol1, const int *__restrict__ n1,
-                                      const int *__restrict__ off1, int ma1, int rep,
-                                      const double *__restrict__ g, double *__restrict__ F) {
-    const int r = blockIdx.x;
-    const int flat = idx1[r], a = mol1[r], i = flat - a * ma1;
+__global__ void __launch_bounds__(256) force_contract_kernel(
+    const Tin *__restrict__ x1, const Tin *__restrict__ dx1, const int *__restrict__ idx1,
+    const int *__restrict__ n1, const int *__restrict__ off1, int ma1, int rep,
+    const double *__restrict__ g, const double *__restrict__ rowv,
+    double *__restrict__ F) {
+    __shared__ double gs[FC_K], part[4][64];
+    const int r = blockIdx.x, k0 = blockIdx.y * FC_K, nk = min(FC_K, rep - k0);
+    const int flat = idx1[r], a = flat / ma1;
     const int na = min(max(n1[a], 0), ma1);
     const int ld = 3 * ma1, nc = 3 * na;
-    const Tin *J = dx1 + ((size_t)a * ma1 + i) * rep * (size_t)ld;
-    const double *gr = g + (size_t)r * rep;
-    for (int c = threadIdx.x; c < nc; c += blockDim.x) {
+    const double rv = rowv ? rowv[r] : 0.0;
+    for (int k = threadIdx.x; k < nk; k += 256) {
+        const double gk = g[(size_t)r * rep + k0 + k];
+        gs[k] = rowv ? fma(rv, (double)x1[(size_t)flat * rep + k0 + k], gk) : gk;
+    }
+    __syncthreads();
+    const Tin *J = dx1 + ((size_t)flat * rep + k0) * (size_t)ld;
+    const int cl = threadIdx.x & 63, kq = threadIdx.x >> 6;
+    for (int c0 = 0; c0 < nc; c0 += 64) {
+        const int cc = c0 + cl;
         double acc = 0.0;
-        for (int k = 0; k < rep; ++k) acc = fma((double)J[(size_t)k * ld + c], gr[k], acc);
-        atomicAdd(F + off1[a] + c, acc);
+        if (cc < nc) {
+#pragma unroll 10
+            for (int k = kq; k < nk; k += 4) acc = fma((double)J[(size_t)k * ld + cc], gs[k], acc);
+        }
+        part[kq][cl] = acc;
+        __syncthreads();
+        if (kq == 0 && cc < nc)
+            atomicAdd(F + off1[a] + cc, part[0][cl] + part[1][cl] + part[2][cl] + part[3][cl]);
+        __syncthreads();
+    }
+}
+
+// ----------------------------------------------------- direct FP64 products
+// Few (query, training) atom pairs: the digit planes of the training rows and
+// of their transposes cost more than the products themselves, and a launch per
+// label and product leaves most SMs idle.  Two kernels take every label at
+// once and form the same sums with FP64 mma.sync (37 TFLOP/s measured on B200,
+// the FP64 FMA rate, at a quarter of the shared-memory loads).
+//
+// Label l: query rows [sa, sa + ra), training rows [sb, sb + rb), W and V of
+// ra rows of ldw doubles from woff; blocks [tile1, next label's tile1) of the
+// weights kernel and [tile2, ...) of the gradient kernel.
+struct MvLabel {
+    int sa, ra, sb, rb;
+    int tile1, tile2, ldw, pad;
+    long long woff;
+};
+constexpr int MD_M = 32, MD_N = 64, MD_K = 32;
+constexpr int MD_LDK = MD_K + 4;   // row strides = 4 mod 16 doubles: the fragment
+constexpr int MD_LDN = MD_N + 4;   // loads of a half warp hit 16 different banks
+
+// v[u] = p[k + u] for k + u < n, else 0; vec: p + k is aligned to 16 bytes and
+// n a multiple of N.
+template <class Tin, int N>
+__device__ __forceinline__ void load_row(const Tin *p, int k, int n, bool vec, double (&v)[N]) {
+    if (vec && k < n) {
+        constexpr int PER = 16 / sizeof(Tin);
+#pragma unroll
+        for (int u = 0; u < N; u += PER) {
+            const uint4 w = *reinterpret_cast<const uint4 *>(p + k + u);
+            const Tin *e = reinterpret_cast<const Tin *>(&w);
+#pragma unroll
+            for (int r = 0; r < PER; ++r) v[u + r] = (double)e[r];
+        }
+    } else {
+#pragma unroll
+        for (int u = 0; u < N; ++u) v[u] = k + u < n ? (double)p[k + u] : 0.0;
+    }
+}
+
+// Tile of MD_M query rows x MD_N training rows of a label: G = x1 . x2 and
+// P = x1 . Ad over all columns, then e, w, v of every pair, the energy sums (E
+// of the query row's molecule), and with forces W = w, V = -v and rowsum(V).
+// The norms and x . Ad of the rows are summed while they are staged.  Warp
+// (wm, wn) holds 16 x 16 of both products.
+template <class Tin>
+__global__ void __launch_bounds__(256, 2) mv_weights_kernel(
+    const Tin *__restrict__ x1, const int *__restrict__ idx1, int ma1,
+    const Tin *__restrict__ x2, const int *__restrict__ idx2, int ma2,
+    const double *__restrict__ ad, const double *__restrict__ alpha_e,
+    const MvLabel *__restrict__ labels, int nlab, int rep, int vec, int with_f, double c,
+    double is2, double is4, double *__restrict__ W, double *__restrict__ V,
+    double *__restrict__ E, double *__restrict__ rowv) {
+    __shared__ double As[MD_M][MD_LDK], Xs[MD_N][MD_LDK], Ds[MD_N][MD_LDK];
+    __shared__ double n1s[MD_M], n2s[MD_N], scs[MD_N];
+    int l = 0;
+    while (l + 1 < nlab && (int)blockIdx.x >= labels[l + 1].tile1) ++l;
+    const MvLabel lb = labels[l];
+    const int mt = (lb.ra + MD_M - 1) / MD_M;
+    const int local = blockIdx.x - lb.tile1;
+    const int i0 = (local % mt) * MD_M, j0 = (local / mt) * MD_N;
+    const int na = min(MD_M, lb.ra - i0), nb = min(MD_N, lb.rb - j0);
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    // staging: 4 columns of row t / 8 of the queries, 8 columns of training row t / 4
+    const int ar = t >> 3, ak = (t & 7) * 4, br = t >> 2, bk = (t & 3) * 8;
+    const bool av = ar < na, bv = br < nb;
+    const Tin *pa = x1 + (size_t)(av ? idx1[lb.sa + i0 + ar] : 0) * rep;
+    const int jrow = bv ? idx2[lb.sb + j0 + br] : 0;
+    const Tin *pb = x2 + (size_t)jrow * rep;
+    const double *pd = ad ? ad + (size_t)jrow * rep : nullptr;
+    double ra[4], rb[8], rd[8], n1 = 0.0, n2 = 0.0, sc = 0.0;
+    auto fetch = [&](int k0) {
+        load_row<Tin, 4>(pa, k0 + ak, av ? rep : 0, vec, ra);
+        load_row<Tin, 8>(pb, k0 + bk, bv ? rep : 0, vec, rb);
+        if (pd) load_row<double, 8>(pd, k0 + bk, bv ? rep : 0, vec, rd);
+    };
+    const int wm = warp & 1, wn = warp >> 1;
+    const bool active = 16 * wm < na;
+    double g[2][2][2] = {}, p[2][2][2] = {};
+    fetch(0);
+    for (int k0 = 0; k0 < rep; k0 += MD_K) {
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            As[ar][ak + u] = ra[u];
+            n1 = fma(ra[u], ra[u], n1);
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            Xs[br][bk + u] = rb[u];
+            n2 = fma(rb[u], rb[u], n2);
+            if (pd) {
+                Ds[br][bk + u] = rd[u];
+                sc = fma(rb[u], rd[u], sc);
+            }
+        }
+        __syncthreads();
+        if (k0 + MD_K < rep) fetch(k0 + MD_K);
+        if (!active) continue;
+#pragma unroll
+        for (int kk = 0; kk < MD_K; kk += 4) {
+            const int r = lane >> 2, k = kk + (lane & 3);
+            const double a0 = As[16 * wm + r][k], a1 = As[16 * wm + 8 + r][k];
+#pragma unroll
+            for (int nj = 0; nj < 2; ++nj) {
+                const double x = Xs[16 * wn + 8 * nj + r][k];
+                dmma(g[0][nj], a0, x);
+                dmma(g[1][nj], a1, x);
+                if (pd) {
+                    const double d = Ds[16 * wn + 8 * nj + r][k];
+                    dmma(p[0][nj], a0, d);
+                    dmma(p[1][nj], a1, d);
+                }
+            }
+        }
+    }
+    // row sums of the staged values: 8 threads of a query row, 4 of a training row
+    for (int o = 4; o; o >>= 1) n1 += __shfl_xor_sync(0xffffffffu, n1, o);
+    for (int o = 2; o; o >>= 1) {
+        n2 += __shfl_xor_sync(0xffffffffu, n2, o);
+        sc += __shfl_xor_sync(0xffffffffu, sc, o);
+    }
+    if ((t & 7) == 0) n1s[ar] = n1;
+    if ((t & 3) == 0) {
+        n2s[br] = n2;
+        scs[br] = sc;
+    }
+    __syncthreads();   // (also: every warp is past its fragment loads)
+    double *es = &As[0][0], *vs = es + 4 * MD_M;   // [wn][row] partial sums
+    if (active) {
+#pragma unroll
+        for (int mi = 0; mi < 2; ++mi) {
+            const int i = 16 * wm + 8 * mi + (lane >> 2);
+            double esum = 0.0, vsum = 0.0;
+#pragma unroll
+            for (int nj = 0; nj < 2; ++nj) {
+                const int j = 16 * wn + 8 * nj + 2 * (lane & 3);
+                double w[2] = {0.0, 0.0}, v[2] = {0.0, 0.0};
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    if (i >= na || j + u >= nb) continue;
+                    const double d2 = fmax(n1s[i] + n2s[j + u] - 2.0 * g[mi][nj][u], 0.0);
+                    const double e = exp(c * d2);
+                    const double dad = pd ? p[mi][nj][u] - scs[j + u] : 0.0;
+                    const double ae = alpha_e ? alpha_e[idx2[lb.sb + j0 + j + u] / ma2] : 0.0;
+                    w[u] = e * is2;
+                    v[u] = w[u] * ae + e * is4 * dad;
+                    esum += ae * e + w[u] * dad;
+                    vsum += v[u];
+                }
+                if (with_f && i < na && j < nb) {
+                    // ldw is even and j too: 16-byte stores, the second value in the row's padding
+                    const long long at = lb.woff + (long long)(i0 + i) * lb.ldw + j0 + j;
+                    *reinterpret_cast<double2 *>(W + at) = make_double2(w[0], w[1]);
+                    *reinterpret_cast<double2 *>(V + at) = make_double2(v[0], v[1]);
+                }
+            }
+            for (int o = 2; o; o >>= 1) {
+                esum += __shfl_xor_sync(0xffffffffu, esum, o);
+                vsum += __shfl_xor_sync(0xffffffffu, vsum, o);
+            }
+            if ((lane & 3) == 0) {
+                es[wn * MD_M + i] = esum;
+                vs[wn * MD_M + i] = vsum;
+            }
+        }
+    }
+    __syncthreads();
+    if (t < na) {
+        double te = 0.0, tv = 0.0;
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            te += es[w * MD_M + t];
+            tv += vs[w * MD_M + t];
+        }
+        if (E) atomicAdd(E + idx1[lb.sa + i0 + t] / ma1, te);
+        if (with_f) atomicAdd(rowv + lb.sa + i0 + t, -tv);
+    }
+}
+
+// g[i, k] += sum_j W_ij Ad_jk + (-v)_ij x2_jk over the training rows
+// [split jlen, ...) of a label: MD_M query rows x MD_N columns per block, the
+// split-K sums combined by atomics.
+constexpr int MD_GRAD_SMEM = (2 * MD_M * MD_LDK + 2 * MD_K * MD_LDN) * (int)sizeof(double);
+
+template <class Tin>
+__global__ void __launch_bounds__(256, 2) mv_grad_kernel(
+    const Tin *__restrict__ x2, const int *__restrict__ idx2, const double *__restrict__ ad,
+    const MvLabel *__restrict__ labels, int nlab, int rep, int jlen, int vec,
+    const double *__restrict__ W, const double *__restrict__ V, double *__restrict__ g) {
+    extern __shared__ __align__(16) double md_raw[];
+    double (*Ws)[MD_LDK] = reinterpret_cast<double (*)[MD_LDK]>(md_raw);
+    double (*Vs)[MD_LDK] = Ws + MD_M;
+    double (*Xs)[MD_LDN] = reinterpret_cast<double (*)[MD_LDN]>(md_raw + 2 * MD_M * MD_LDK);
+    double (*Ds)[MD_LDN] = Xs + MD_K;
+    int l = 0;
+    while (l + 1 < nlab && (int)blockIdx.x >= labels[l + 1].tile2) ++l;
+    const MvLabel lb = labels[l];
+    const int mt = (lb.ra + MD_M - 1) / MD_M, nt = (rep + MD_N - 1) / MD_N;
+    const int local = blockIdx.x - lb.tile2;
+    const int i0 = (local % mt) * MD_M, n0 = (local / mt % nt) * MD_N;
+    const int jb = local / (mt * nt) * jlen, je = min(lb.rb, jb + jlen);
+    const int na = min(MD_M, lb.ra - i0);
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    // staging: 4 partners of query row t / 8; 8 columns of training row t / 8
+    const int ar = t >> 3, aj = (t & 7) * 4, bk = (t & 7) * 8;
+    const long long wrow = lb.woff + (long long)(i0 + (ar < na ? ar : 0)) * lb.ldw;
+    double rw[4], rv[4], rx[8], rd[8];
+    auto fetch = [&](int j0) {
+        const int n = ar < na ? je : 0;
+        load_row<double, 4>(W + wrow, j0 + aj, n, false, rw);
+        load_row<double, 4>(V + wrow, j0 + aj, n, false, rv);
+        const int j = j0 + ar;
+        const bool jv = j < je;
+        const size_t row = (size_t)(jv ? idx2[lb.sb + j] : 0) * rep;
+        load_row<Tin, 8>(x2 + row, n0 + bk, jv ? rep : 0, vec, rx);
+        if (ad) load_row<double, 8>(ad + row, n0 + bk, jv ? rep : 0, vec, rd);
+    };
+    const int wm = warp & 1, wn = warp >> 1;
+    const bool active = 16 * wm < na;
+    double acc[2][2][2] = {};
+    fetch(jb);
+    for (int j0 = jb; j0 < je; j0 += MD_K) {
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            Ws[ar][aj + u] = rw[u];
+            Vs[ar][aj + u] = rv[u];
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            Xs[ar][bk + u] = rx[u];
+            if (ad) Ds[ar][bk + u] = rd[u];
+        }
+        __syncthreads();
+        if (j0 + MD_K < je) fetch(j0 + MD_K);
+        if (!active) continue;
+#pragma unroll
+        for (int kk = 0; kk < MD_K; kk += 4) {
+            const int r = lane >> 2, k = kk + (lane & 3);
+            const double v0 = Vs[16 * wm + r][k], v1 = Vs[16 * wm + 8 + r][k];
+            const double w0 = Ws[16 * wm + r][k], w1 = Ws[16 * wm + 8 + r][k];
+#pragma unroll
+            for (int nj = 0; nj < 2; ++nj) {
+                const double x = Xs[k][16 * wn + 8 * nj + r];
+                dmma(acc[0][nj], v0, x);
+                dmma(acc[1][nj], v1, x);
+                if (ad) {
+                    const double d = Ds[k][16 * wn + 8 * nj + r];
+                    dmma(acc[0][nj], w0, d);
+                    dmma(acc[1][nj], w1, d);
+                }
+            }
+        }
+    }
+    if (!active) return;
+#pragma unroll
+    for (int mi = 0; mi < 2; ++mi) {
+        const int i = 16 * wm + 8 * mi + (lane >> 2);
+        if (i >= na) continue;
+        double *row = g + (size_t)(lb.sa + i0 + i) * rep + n0;
+#pragma unroll
+        for (int nj = 0; nj < 2; ++nj) {
+            const int n = 16 * wn + 8 * nj + 2 * (lane & 3);
+#pragma unroll
+            for (int u = 0; u < 2; ++u)
+                if (n0 + n + u < rep) atomicAdd(row + n + u, acc[mi][nj][u]);
+        }
     }
 }
 
@@ -246,6 +538,94 @@ kfb_status mv_gemm(const OzSlices &A, const OzSlices &B, int M, int N, double *C
     return oz_gemm_gen(A, B, g, epi, err, s);
 }
 
+// Same-label (query atom, training atom) pairs up to which the direct FP64
+// kernels are used.
+constexpr long long MD_MAX_PAIRS = 6LL << 20;
+
+template <class Tin>
+kfb_status matvec_direct(const Tin *x1, const Tin *dx1, const Tin *x2, const double *ad,
+                         const double *alpha_e, const SetView &s1, const std::vector<int> &off1,
+                         int s2_ma, const Buckets &b1, const Buckets &b2, int rep, double sigma,
+                         double *E, double *F, cudaStream_t s) {
+    const int L = (int)b1.labels.size();
+    std::vector<MvLabel> labs;
+    std::vector<int> src1, src2;   // rows of the labels that both sets have
+    long long words = 0, blocks = 0;
+    int tiles1 = 0;
+    const int nt = (rep + MD_N - 1) / MD_N;
+    for (int l = 0; l < L; ++l) {
+        const int a0 = b1.lab_start[l], a1 = b1.lab_start[l + 1];
+        const int c0 = b2.lab_start[l], c1 = b2.lab_start[l + 1];
+        if (a1 == a0 || c1 == c0) continue;
+        MvLabel m{};
+        m.sa = (int)src1.size();
+        m.ra = a1 - a0;
+        m.sb = (int)src2.size();
+        m.rb = c1 - c0;
+        src1.insert(src1.end(), b1.src.begin() + a0, b1.src.begin() + a1);
+        src2.insert(src2.end(), b2.src.begin() + c0, b2.src.begin() + c1);
+        m.tile1 = tiles1;
+        tiles1 += (m.ra + MD_M - 1) / MD_M * ((m.rb + MD_N - 1) / MD_N);
+        m.ldw = (m.rb + 1) / 2 * 2;
+        m.woff = words;
+        words += (long long)m.ra * m.ldw;
+        blocks += (long long)((m.ra + MD_M - 1) / MD_M) * nt * ((m.rb + MD_K - 1) / MD_K);
+        labs.push_back(m);
+    }
+    if (labs.empty()) return KFB_OK;
+    // training rows per gradient block: enough blocks for four per SM, but not
+    // so few rows that the atomics of the split outweigh them
+    const long long per = std::max<long long>(4, blocks / (4LL * device_sm_count()));
+    const int jlen = (int)std::min<long long>(per, 1 << 20) * MD_K;
+    int tiles2 = 0;
+    for (MvLabel &m : labs) {
+        m.tile2 = tiles2;
+        tiles2 += (m.ra + MD_M - 1) / MD_M * nt * ((m.rb + jlen - 1) / jlen);
+    }
+    // one upload: label table, then the rows of both sets, offsets, atom counts
+    std::vector<int> blob(labs.size() * sizeof(MvLabel) / sizeof(int));
+    std::memcpy(blob.data(), labs.data(), labs.size() * sizeof(MvLabel));
+    auto append = [&](const std::vector<int> &v) {
+        const size_t at = blob.size();
+        blob.insert(blob.end(), v.begin(), v.end());
+        return at;
+    };
+    const int R1 = (int)src1.size();
+    const size_t o_src1 = append(src1), o_src2 = append(src2), o_off1 = append(off1);
+    const size_t o_n1 = blob.size();
+    for (int m = 0; m < s1.nm; ++m) blob.push_back(s1.natoms(m));
+    DevBuf plan, wv, gr;
+    KFB_TRY(upload(plan, blob, s));
+    const int *dp = plan.as<int>();
+    const bool with_f = F != nullptr;
+    if (with_f) {
+        KFB_TRY(wv.alloc((size_t)words * 2 * sizeof(double), s));
+        KFB_TRY(gr.alloc((size_t)R1 * (rep + 1) * sizeof(double), s));
+        KFB_TRY(zero(gr.ptr, (size_t)R1 * (rep + 1) * sizeof(double), s));
+    }
+    double *W = wv.as<double>(), *V = W + words;
+    double *g = gr.as<double>(), *rowv = g + (size_t)R1 * rep;
+    auto aligned = [](const void *p) { return (reinterpret_cast<size_t>(p) & 15) == 0; };
+    const int vec = rep % 8 == 0 && aligned(x1) && aligned(x2) && aligned(ad);
+    const double c = -1.0 / (2.0 * sigma * sigma), is2 = 1.0 / (sigma * sigma), is4 = is2 * is2;
+    const int nlab = (int)labs.size();
+    const MvLabel *dl = reinterpret_cast<const MvLabel *>(dp);
+    mv_weights_kernel<Tin><<<tiles1, 256, 0, s>>>(
+        x1, dp + o_src1, s1.ma, x2, dp + o_src2, s2_ma, ad, alpha_e, dl, nlab, rep, vec,
+        with_f ? 1 : 0, c, is2, is4, W, V, E, rowv);
+    KFB_CUDA_TRY(cudaGetLastError());
+    if (!with_f) return KFB_OK;
+    KFB_CUDA_TRY(cudaFuncSetAttribute(mv_grad_kernel<Tin>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, MD_GRAD_SMEM));
+    mv_grad_kernel<Tin><<<tiles2, 256, MD_GRAD_SMEM, s>>>(x2, dp + o_src2, ad, dl, nlab, rep, jlen,
+                                                          vec, W, V, g);
+    KFB_CUDA_TRY(cudaGetLastError());
+    force_contract_kernel<Tin><<<dim3(R1, (rep + FC_K - 1) / FC_K), 256, 0, s>>>(
+        x1, dx1, dp + o_src1, dp + o_n1, dp + o_off1, s1.ma, rep, g, rowv, F);
+    KFB_CUDA_TRY(cudaGetLastError());
+    return KFB_OK;
+}
+
 template <class Tin>
 kfb_status matvec_t(const Tin *x1, const Tin *dx1, const Tin *x2, const double *ad,
                     const double *alpha_e, const SetView &s1, const SetView &s2, int rep,
@@ -259,15 +639,20 @@ kfb_status matvec_t(const Tin *x1, const Tin *dx1, const Tin *x2, const double *
     if (!device_is_sm100())
         return set_error(KFB_ERR_UNSUPPORTED, "the contracted prediction needs an sm_100 (B200) device");
     const Buckets b1 = make_buckets(s1, labels), b2 = make_buckets(s2, labels);
+    long long pairs = 0;
+    for (size_t l = 0; l < labels.size(); ++l)
+        pairs += (long long)(b1.lab_start[l + 1] - b1.lab_start[l]) *
+                 (b2.lab_start[l + 1] - b2.lab_start[l]);
+    if (pairs <= MD_MAX_PAIRS && (size_t)pairs * 2 * sizeof(double) <= workspace_budget())
+        return matvec_direct<Tin>(x1, dx1, x2, ad, alpha_e, s1, off1, s2.ma, b1, b2, rep, sigma, E, F,
+                                  s);
     std::vector<int> n1v(s1.nm);
     for (int m = 0; m < s1.nm; ++m) n1v[m] = s1.natoms(m);
-    DevBuf dn1, doff1, didx1, dmol1, didx2, dmol2, derr, mx;
+    DevBuf dn1, doff1, didx1, didx2, derr, mx;
     KFB_TRY(upload(dn1, n1v, s));
     KFB_TRY(upload(doff1, off1, s));
     KFB_TRY(upload(didx1, b1.src, s));
-    KFB_TRY(upload(dmol1, b1.mol, s));
     KFB_TRY(upload(didx2, b2.src, s));
-    KFB_TRY(upload(dmol2, b2.mol, s));
     // one pipeline-timeout flag for every tensor-core product of the call
     KFB_TRY(derr.alloc(sizeof(int), s));
     KFB_TRY(zero(derr.ptr, sizeof(int), s));
@@ -293,8 +678,8 @@ kfb_status matvec_t(const Tin *x1, const Tin *dx1, const Tin *x2, const double *
                                                          Adl.as<double>(), nullptr);
         }
         train_scalars_kernel<<<nblk(r2, 8), 256, 0, s>>>(
-            X2l.as<double>(), with_ad ? Adl.as<double>() : nullptr, dmol2.as<int>() + sb,
-            alpha_e, r2, rep, scl.as<double>(), ael.as<double>());
+            X2l.as<double>(), with_ad ? Adl.as<double>() : nullptr, didx2.as<int>() + sb,
+            s2.ma, alpha_e, r2, rep, scl.as<double>(), ael.as<double>());
         KFB_CUDA_TRY(cudaGetLastError());
         // digit planes of the training rows (K = rep) and, for the force
         // products g = W Ad - V X2 (K = r2, in chunks of MV_KMAX), of their
@@ -340,7 +725,7 @@ kfb_status matvec_t(const Tin *x1, const Tin *dx1, const Tin *x2, const double *
                 KFB_TRY(mv_gemm(Ads.sl, X1s.sl, r2, rc, Pm.as<double>(), r2, 1.0, false, err, s));
             pair_weights_kernel<<<rc, 256, 0, s>>>(
                 Gm.as<double>(), Pm.as<double>(), r2, n1c.as<double>(), n2l.as<double>(),
-                scl.as<double>(), ael.as<double>(), dmol1.as<int>() + sa + q0, with_ad ? 1 : 0,
+                scl.as<double>(), ael.as<double>(), didx1.as<int>() + sa + q0, s1.ma, with_ad ? 1 : 0,
                 with_f ? 1 : 0, c, is2, is4, E, with_f ? rowv.as<double>() : nullptr);
             KFB_CUDA_TRY(cudaGetLastError());
             if (!with_f) continue;
@@ -364,9 +749,8 @@ kfb_status matvec_t(const Tin *x1, const Tin *dx1, const Tin *x2, const double *
                 KFB_TRY(mv_gemm(X2t[kc]->sl, Ms.sl, rep, rc, gm.as<double>(), rep, -1.0, true,
                                 err, s));
             }
-            force_contract_kernel<Tin><<<rc, 128, 0, s>>>(
-                dx1, didx1.as<int>() + sa + q0, dmol1.as<int>() + sa + q0, dn1.as<int>(),
-                doff1.as<int>(), s1.ma, rep, gm.as<double>(), F);
+            force_contract_kernel<Tin><<<dim3(rc, (rep + FC_K - 1) / FC_K), 256, 0, s>>>(
+                x1, dx1, didx1.as<int>() + sa + q0, dn1.as<int>(), doff1.as<int>(), s1.ma, rep, gm.as<double>(), nullptr, F);
             KFB_CUDA_TRY(cudaGetLastError());
         }
     }

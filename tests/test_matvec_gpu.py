@@ -98,6 +98,32 @@ def test_chunked_query_rows(monkeypatch):
     close(F, Fr)
 
 
+@pytest.mark.parametrize("nm1,nm2,ma,rep", [(1, 1, 1, 7), (1, 5, 7, 8), (2, 9, 8, 31),
+                                            (3, 11, 11, 32), (4, 13, 16, 33), (5, 17, 16, 64),
+                                            (7, 19, 13, 65), (9, 33, 12, 72)])
+def test_direct_products_tile_edges(nm1, nm2, ma, rep, monkeypatch):
+    """Few atom pairs take the FP64 mma kernels, more than the workspace holds the digit planes:
+    both against the oracle with one label (rows at and around the 16-, 32- and 64-row tiles and
+    the 32- and 64-column slices) and three, with and without alpha_E, energies or forces alone.
+    The error of either is a few hundred roundings of sums of a few thousand terms."""
+    from kernelforge_b200 import local_kernels as lk
+    for species in (1, 3):
+        X1, dX1, Q1, N1, X2, dX2, Q2, N2, aE, aF = _problem(81 + rep, nm1=nm1, nm2=nm2, ma1=ma,
+                                                            ma2=ma, rep=rep, species=species)
+        N1[0] = ma
+        ad = om.alpha_desc(dX2, Q2, N2, np.resize(aF, int(3 * N2.sum())))
+        tail = (Q1, Q2, N1, N2, 0.9)
+        Er, Fr = om.matvec(X1, dX1, X2, ad, aE, *tail)
+        Er0, Fr0 = om.matvec(X1, dX1, X2, ad, 0 * aE, *tail)
+        for budget, tol in (("4", 1e-11), ("0.0000001", 1e-10)):
+            monkeypatch.setenv("KFB_WORKSPACE_GB", budget)
+            E, F = lk.kernel_gaussian_local_full_matvec(X1, dX1, X2, ad, aE, *tail)
+            close(E, Er, tol)
+            close(F, Fr, tol)
+            close(lk.kernel_gaussian_local_jacobian_t_matvec(X1, X2, ad, *tail), Er0, tol)
+            close(lk.kernel_gaussian_local_hessian_matvec(X1, dX1, X2, ad, *tail), Fr0, tol)
+
+
 def test_edge_cases():
     from kernelforge_b200 import local_kernels as lk
     X1, dX1, Q1, N1, X2, dX2, Q2, N2, aE, aF = _problem(41)
