@@ -10,9 +10,9 @@ namespace kfb {
 
 // Tile of two label buckets: packed rows [a0, a_end) x [b0, b_end), at most
 // the kernel's tile height each; `diag` marks a diagonal tile of a symmetric
-// problem (both operands the same rows).
+// problem (both operands the same rows); `lab` is the index of its label.
 struct PairTile {
-    int a0, a_end, b0, b_end, diag, pad0, pad1, pad2;
+    int a0, a_end, b0, b_end, diag, lab, pad1, pad2;
 };
 
 __device__ __forceinline__ void atomic_add_out(const PairSink &s, long long idx, double v) {

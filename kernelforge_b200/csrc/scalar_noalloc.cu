@@ -1,4 +1,4 @@
-// Allocation-free variant of the symmetric scalar kernel (FP64 CUDA cores).
+// Allocation-free variant of the symmetric scalar kernel (FP64).
 //
 // Some callers cannot allocate device memory during a call: a host framework
 // that reserves the whole device-memory budget up front and hands the library
@@ -92,17 +92,17 @@ kfb_status run(const ScalarProblem &p, const PairSink &sink, cudaStream_t s) {
     int *mol = reinterpret_cast<int *>(b + off_mol);
     int *src = reinterpret_cast<int *>(b + off_src);
     PairTile *dtiles = reinterpret_cast<PairTile *>(b + off_tiles);
-    KFB_CUDA_TRY(cudaMemcpyAsync(mol, bk.mol.data(), R * sizeof(int), cudaMemcpyHostToDevice, s));
     KFB_CUDA_TRY(cudaMemcpyAsync(src, bk.src.data(), R * sizeof(int), cudaMemcpyHostToDevice, s));
     KFB_CUDA_TRY(cudaMemcpyAsync(dtiles, tiles.data(), tiles.size() * sizeof(PairTile),
                                  cudaMemcpyHostToDevice, s));
     const int rows_per_block = 8;
     simt::pack_rows_kernel<Tin, T><<<(R + rows_per_block - 1) / rows_per_block, 256, 0, s>>>(
-        static_cast<const Tin *>(p.x1), src, R, p.rep, Dp, packed, norm);
+        static_cast<const Tin *>(p.x1), src, R, p.rep, Dp, nullptr, 0, nullptr, nullptr,
+        p.s1.ma, packed, norm, mol);
     KFB_CUDA_TRY(cudaGetLastError());
     const T coef = T(-1.0 / (2.0 * p.sigma * p.sigma));
-    simt::scalar_tile_kernel<T><<<(unsigned)tiles.size(), simt::SIMT_THREADS, 0, s>>>(
-        packed, packed, Dp, norm, norm, mol, mol, dtiles, coef, sink);
+    simt::scalar_dmma_kernel<<<(unsigned)tiles.size(), simt::SIMT_THREADS, 0, s>>>(
+        packed, packed, Dp, nullptr, norm, norm, mol, mol, dtiles, coef, sink);
     KFB_CUDA_TRY(cudaGetLastError());
     // the host vectors above are read by the copies before cudaMemcpyAsync
     // returns (pageable memory), so nothing here outlives the call

@@ -32,6 +32,7 @@ struct SuperBlock {
     int nti, ntj;        // tiles of the label
     int symmetric;
     long long offset;    // index of the super-block's first tile in the list
+    int lab;             // label index
 };
 std::vector<SuperBlock> make_super_blocks(const Buckets &a, const Buckets &b, bool symmetric,
                                           int tm, int tn, size_t row_bytes, long long &ntiles);

@@ -9,6 +9,7 @@
 // Mathematics: kernel_gaussian / _symm / _symm_rfp, src/local_kernels.cpp:155-758.
 #include <algorithm>
 
+#include "columns.cuh"
 #include "kernels_common.cuh"
 #include "scalar_plan.h"
 #include "scalar_simt_kernels.cuh"
@@ -22,19 +23,31 @@ using simt::scalar_tile_kernel;
 using simt::SK;
 using simt::ST;
 
+// Packed rows of a set.  `map` (L x rep column places, then L counts): made
+// here from the set's rows when `first`, else the one set 1 left.
 template <class Tin, class T>
-kfb_status pack_set(const Tin *x, const Buckets &bk, int rep, int Dp, DevBuf &packed,
-                    DevBuf &norms, DevBuf &mol, cudaStream_t s) {
-    const int R = bk.rows();
-    DevBuf src;
+kfb_status pack_set(const Tin *x, const Buckets &bk, int ma, int rep, int Dp, DevBuf &map, bool first,
+                    DevBuf &packed, DevBuf &norms, DevBuf &mol, cudaStream_t s) {
+    const int R = bk.rows(), L = (int)bk.labels.size();
+    DevBuf src, lab;
     KFB_TRY(upload(src, bk.src, s));
-    KFB_TRY(upload(mol, bk.mol, s));
+    KFB_TRY(mol.alloc((size_t)std::max(R, 1) * sizeof(int), s));
+    KFB_TRY(upload(lab, bk.lab_start, s));
+    int *pos = map.as<int>(), *ncols = pos + (size_t)L * rep;
+    if (first) {
+        KFB_TRY(zero(map.ptr, (size_t)L * rep * sizeof(int), s));
+        label_columns_kernel<Tin><<<dim3((rep + 31) / 32, 16, L), 256, 0, s>>>(
+            x, src.as<int>(), lab.as<int>(), rep, pos);
+        pack_columns_kernel<<<L, 256, 0, s>>>(rep, pos, ncols);
+        KFB_CUDA_TRY(cudaGetLastError());
+    }
     KFB_TRY(packed.alloc((size_t)std::max(R, 1) * Dp * sizeof(T), s));
     KFB_TRY(norms.alloc((size_t)std::max(R, 1) * sizeof(T), s));
     if (R > 0) {
         const int threads = 256, rows_per_block = threads / 32;
         pack_rows_kernel<Tin, T><<<(R + rows_per_block - 1) / rows_per_block, threads, 0, s>>>(
-            x, src.as<int>(), R, rep, Dp, packed.as<T>(), norms.as<T>());
+            x, src.as<int>(), R, rep, Dp, lab.as<int>(), L, pos, ncols, ma, packed.as<T>(),
+            norms.as<T>(), mol.as<int>());
         KFB_CUDA_TRY(cudaGetLastError());
     }
     return KFB_OK;
@@ -53,10 +66,15 @@ kfb_status run_simt(const ScalarProblem &p, const PairSink &sink, cudaStream_t s
         make_super_blocks(b1, bb, p.symmetric, ST, ST, (size_t)Dp_ * sizeof(T), ntiles_ll);
     if (ntiles_ll == 0) return KFB_OK;
     const int Dp = (p.rep + SK - 1) / SK * SK;
-    DevBuf pa, na, ma, pb, nb, mb, dt;
-    KFB_TRY((pack_set<Tin, T>(static_cast<const Tin *>(p.x1), b1, p.rep, Dp, pa, na, ma, s)));
+    DevBuf pa, na, ma, pb, nb, mb, dt, map;
+    const size_t L = labels.size();
+    KFB_TRY(map.alloc(L * (p.rep + 1) * sizeof(int), s));
+    KFB_TRY((pack_set<Tin, T>(static_cast<const Tin *>(p.x1), b1, p.s1.ma, p.rep, Dp, map, true,
+                              pa, na, ma, s)));
     if (!p.symmetric)
-        KFB_TRY((pack_set<Tin, T>(static_cast<const Tin *>(p.x2), b2, p.rep, Dp, pb, nb, mb, s)));
+        KFB_TRY((pack_set<Tin, T>(static_cast<const Tin *>(p.x2), b2, p.s2.ma, p.rep, Dp, map, false,
+                                  pb, nb, mb, s)));
+    const int *ncols = map.as<int>() + L * p.rep;
     KFB_TRY(expand_tiles(sbs, ntiles_ll, ST, ST, dt, s));
     const T coef = T(-1.0 / (2.0 * p.sigma * p.sigma));
     const DevBuf &PB = p.symmetric ? pa : pb, &NB = p.symmetric ? na : nb,
@@ -67,9 +85,14 @@ kfb_status run_simt(const ScalarProblem &p, const PairSink &sink, cudaStream_t s
     timer.start();
     for (size_t off = 0; off < ntiles; off += (size_t)1 << 30) {
         const unsigned nb_ = (unsigned)std::min<size_t>(ntiles - off, (size_t)1 << 30);
-        scalar_tile_kernel<T><<<nb_, simt::SIMT_THREADS, 0, s>>>(
-            pa.as<T>(), PB.as<T>(), Dp, na.as<T>(), NB.as<T>(), ma.as<int>(), MB.as<int>(),
-            dt.as<PairTile>() + off, coef, sink);
+        if constexpr (sizeof(T) == 8)
+            simt::scalar_dmma_kernel<<<nb_, simt::SIMT_THREADS, 0, s>>>(
+                pa.as<T>(), PB.as<T>(), Dp, ncols, na.as<T>(), NB.as<T>(), ma.as<int>(),
+                MB.as<int>(), dt.as<PairTile>() + off, coef, sink);
+        else
+            scalar_tile_kernel<T><<<nb_, simt::SIMT_THREADS, 0, s>>>(
+                pa.as<T>(), PB.as<T>(), Dp, ncols, na.as<T>(), NB.as<T>(), ma.as<int>(),
+                MB.as<int>(), dt.as<PairTile>() + off, coef, sink);
         KFB_CUDA_TRY(cudaGetLastError());
     }
     timer.stop();
@@ -108,7 +131,7 @@ std::vector<SuperBlock> make_super_blocks(const Buckets &a, const Buckets &b, bo
         const int nti = (ea - sa + tm - 1) / tm, ntj = (eb - sb + tn - 1) / tn;
         for (int bi = 0; bi < nti; bi += group)
             for (int bj = symmetric ? bi : 0; bj < ntj; bj += group) {
-                SuperBlock s{sa, ea, sb, eb, bi, bj, group, nti, ntj, symmetric ? 1 : 0, ntiles};
+                SuperBlock s{sa, ea, sb, eb, bi, bj, group, nti, ntj, symmetric ? 1 : 0, ntiles, l};
                 long long cnt = 0;
                 for (int ti = bi; ti < std::min(nti, bi + group); ++ti) {
                     int f, e;
@@ -154,6 +177,7 @@ __global__ void expand_tiles_kernel(const SuperBlock *__restrict__ sbs, int nsb,
             pt.b_end = min(sb.eb, sb.sb + (tj + ncol) * tn);
             if (merge == 1) pt.b_end = sb.eb;
             pt.diag = (sb.symmetric && ti == tj) ? 1 : 0;
+            pt.lab = sb.lab;
             out[t] = pt;
             return;
         }
@@ -206,6 +230,7 @@ std::vector<PairTile> make_pair_tiles(const Buckets &a, const Buckets &b, bool s
                 t.b0 = sb.sb + tj * tn;
                 t.b_end = merge == 1 ? sb.eb : std::min(sb.eb, sb.sb + (tj + ncol) * tn);
                 t.diag = (sb.symmetric && ti == tj) ? 1 : 0;
+                t.lab = sb.lab;
                 out.push_back(t);
             }
         }

@@ -85,6 +85,37 @@ def test_multi_tile_ragged(rep, precision):
         close32(rect, rref)
 
 
+@pytest.mark.parametrize("precision", ["fp64", "split_f16"])
+@pytest.mark.parametrize("rep,used", [(70, 0), (70, 1), (130, 16), (130, 17), (200, 64), (200, 65),
+                                      (201, 200), (720, 496)])
+def test_unused_columns(rep, used, precision):
+    """Columns that are zero in every row of a label (a different set for each label) are left
+    out of the products: one MMA step and one K slice, at and around their edges, none and all of
+    the columns used.  Set 2 of the rectangular kernel is non-zero in columns that set 1 does not
+    use, and the other way round."""
+    from kernelforge_b200 import local_kernels as lk
+    X, _, Q, N = make_set(40, 9, rep, 2, rep + used, species=[1, 6])
+    X2, _, Q2, N2 = make_set(25, 7, rep, 2, rep + used + 1, species=[6, 1])
+    X, X2 = X * 0.3, X2 * 0.3
+    rng = np.random.default_rng(used)
+    for q in (1, 6):
+        off = rng.permutation(rep)[used:]
+        off2 = rng.permutation(rep)[used:]
+        m, i = np.nonzero(Q == q)
+        X[m[:, None], i[:, None], off[None, :]] = 0.0
+        m, i = np.nonzero(Q2 == q)
+        X2[m[:, None], i[:, None], off2[None, :]] = 0.0
+    got = lk.kernel_gaussian_symm(X, Q, N, 2.0, precision=precision)
+    rect = lk.kernel_gaussian(X, X2, Q, Q2, N, N2, 2.0, precision=precision)
+    ref, rref = o.kernel_gaussian_symm(X, Q, N, 2.0), o.kernel_gaussian(X, X2, Q, Q2, N, N2, 2.0)
+    if precision == "fp64":
+        np.testing.assert_allclose(got, ref, rtol=1e-12, atol=1e-12)
+        np.testing.assert_allclose(rect, rref, rtol=1e-12, atol=1e-12)
+    else:
+        close32(got, ref)
+        close32(rect, rref)
+
+
 def test_no_shared_labels_gives_zero():
     from kernelforge_b200 import local_kernels as lk
     X1, _, Q1, N1 = make_set(3, 4, 6, 1, 0, species=[1])
