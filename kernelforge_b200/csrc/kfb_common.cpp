@@ -4,8 +4,8 @@
 #include <chrono>
 #include <cstdlib>
 #include <cstring>
+#include <map>
 #include <mutex>
-#include <set>
 
 #include "kfb_internal.h"
 
@@ -73,75 +73,115 @@ void DevBuf::release() {
 }
 
 // Labels are nuclear charges or element indices: small non-negative integers
-// take a direct table, anything else a sorted set.
-static constexpr int LABEL_TABLE = 4096;
+// take a direct table, anything else a map.  Labels are numbered in the order
+// they are met and sorted at the end.
+namespace {
 
-std::vector<int> collect_labels(const SetView &a, const SetView *b) {
-    std::vector<unsigned char> seen(LABEL_TABLE, 0);
-    std::set<int> other;
-    auto scan = [&](const SetView &v) {
-        for (int m = 0; m < v.nm; ++m) {
-            const int32_t *q = v.q + (size_t)m * v.ma;
-            const int na = v.natoms(m);
-            for (int i = 0; i < na; ++i) {
-                const int l = q[i];
-                if (l >= 0 && l < LABEL_TABLE) seen[l] = 1;
-                else other.insert(l);
-            }
+class LabelIndex {
+public:
+    LabelIndex() { std::fill(table_, table_ + TABLE, -1); }
+    // number of label q, given a new one when it has none
+    int number(int q) {
+        const int l = (unsigned)q < (unsigned)TABLE ? table_[q] : -1;
+        return l >= 0 ? l : find(q);
+    }
+    const std::vector<int> &labels() const { return labels_; }
+
+private:
+    int find(int q) {
+        if (q < 0 || q >= TABLE) {
+            const auto it = other_.find(q);
+            if (it != other_.end()) return it->second;
+            other_[q] = (int)labels_.size();
+        } else {
+            table_[q] = (int)labels_.size();
         }
-    };
-    scan(a);
-    if (b) scan(*b);
-    std::vector<int> out;
-    for (int l : other)
-        if (l < 0) out.push_back(l);
-    for (int l = 0; l < LABEL_TABLE; ++l)
-        if (seen[l]) out.push_back(l);
-    for (int l : other)
-        if (l >= LABEL_TABLE) out.push_back(l);
-    return out;  // ascending
+        labels_.push_back(q);
+        return (int)labels_.size() - 1;
+    }
+    static constexpr int TABLE = 512;
+    int table_[TABLE];
+    std::map<int, int> other_;
+    std::vector<int> labels_;
+};
+
+// Scratch of a plan, kept per thread while it is small: a fresh array of this
+// size is mapped and faulted in page by page on every call (0.4 ms of the
+// 1.2 ms that 150,000 atoms took).
+constexpr size_t PLAN_KEEP = (size_t)1 << 22;   // bytes
+
+// Label number of every active atom of a set, in order, and the label counts.
+void number_atoms(const SetView &v, LabelIndex &ix, std::vector<int> &num,
+                  std::vector<int> &count) {
+    num.resize((size_t)v.nm * v.ma);
+    int *out = num.data();
+    count.assign(ix.labels().size() + 1, 0);
+    int *cnt = count.data();
+    for (int m = 0; m < v.nm; ++m) {
+        const int32_t *q = v.q + (size_t)m * v.ma;
+        const int na = v.natoms(m);
+        for (int i = 0; i < na; ++i) {
+            const int l = ix.number(q[i]);
+            if (l + 1 >= (int)count.size()) {
+                count.resize(2 * (l + 2), 0);
+                cnt = count.data();
+            }
+            ++cnt[l];
+            *out++ = l;
+        }
+    }
 }
 
-Buckets make_buckets(const SetView &s, const std::vector<int> &labels) {
-    Buckets bk;
-    bk.labels = labels;
+void fill_buckets(const SetView &v, const std::vector<int> &labels, const std::vector<int> &order,
+                  const std::vector<int> &num, std::vector<int> &count, Buckets &bk) {
     const int L = (int)labels.size();
-    std::vector<int> table(LABEL_TABLE, -1);
-    for (int l = 0; l < L; ++l)
-        if (labels[l] >= 0 && labels[l] < LABEL_TABLE) table[labels[l]] = l;
-    auto lidx = [&](int lbl) -> int {
-        if (lbl >= 0 && lbl < LABEL_TABLE) return table[lbl];
-        const auto it = std::lower_bound(labels.begin(), labels.end(), lbl);
-        return (it != labels.end() && *it == lbl) ? (int)(it - labels.begin()) : -1;
-    };
-    // label of each active atom, counted in one pass
-    std::vector<int> count(L + 1, 0);
-    for (int m = 0; m < s.nm; ++m) {
-        const int32_t *q = s.q + (size_t)m * s.ma;
-        const int na = s.natoms(m);
-        for (int i = 0; i < na; ++i) {
-            const int l = lidx(q[i]);
-            if (l >= 0) count[l + 1]++;
-        }
-    }
+    count.resize(std::max<size_t>(count.size(), L), 0);
+    bk.labels.resize(L);
     bk.lab_start.assign(L + 1, 0);
-    for (int l = 0; l < L; ++l) bk.lab_start[l + 1] = bk.lab_start[l] + count[l + 1];
-    const int R = bk.lab_start[L];
-    bk.src.resize(R);
-    bk.mol.resize(R);
-    std::vector<int> fill(bk.lab_start.begin(), bk.lab_start.end() - 1);
-    for (int m = 0; m < s.nm; ++m) {
-        const int32_t *q = s.q + (size_t)m * s.ma;
-        const int na = s.natoms(m);
-        for (int i = 0; i < na; ++i) {
-            const int l = lidx(q[i]);
-            if (l < 0) continue;
-            const int r = fill[l]++;
-            bk.src[r] = m * s.ma + i;
-            bk.mol[r] = m;
-        }
+    std::vector<int> fill(L);
+    for (int s = 0; s < L; ++s) {
+        bk.labels[s] = labels[order[s]];
+        fill[order[s]] = bk.lab_start[s];
+        bk.lab_start[s + 1] = bk.lab_start[s] + count[order[s]];
     }
-    return bk;
+    bk.src.resize(bk.lab_start[L]);
+    int *src = bk.src.data(), *f = fill.data();
+    const int *l = num.data();
+    for (int m = 0; m < v.nm; ++m) {
+        const int na = v.natoms(m), base = m * v.ma;
+        for (int i = 0; i < na; ++i) src[f[*l++]++] = base + i;
+    }
+}
+
+}  // namespace
+
+std::vector<int> collect_labels(const SetView &a, const SetView *b) {
+    LabelIndex ix;
+    for (const SetView *v : {&a, b})
+        for (int m = 0; v && m < v->nm; ++m) {
+            const int32_t *q = v->q + (size_t)m * v->ma;
+            const int na = v->natoms(m);
+            for (int i = 0; i < na; ++i) ix.number(q[i]);
+        }
+    std::vector<int> out = ix.labels();
+    std::sort(out.begin(), out.end());
+    return out;
+}
+
+void plan_buckets(const SetView &a, const SetView *b, Buckets &ba, Buckets *bb) {
+    static thread_local std::vector<int> num_a, num_b;
+    LabelIndex ix;
+    std::vector<int> count_a, count_b;
+    number_atoms(a, ix, num_a, count_a);
+    if (b) number_atoms(*b, ix, num_b, count_b);
+    const std::vector<int> &labels = ix.labels();
+    std::vector<int> order(labels.size());
+    for (size_t i = 0; i < order.size(); ++i) order[i] = (int)i;
+    std::sort(order.begin(), order.end(), [&](int x, int y) { return labels[x] < labels[y]; });
+    fill_buckets(a, labels, order, num_a, count_a, ba);
+    if (b) fill_buckets(*b, labels, order, num_b, count_b, *bb);
+    for (std::vector<int> *n : {&num_a, &num_b})
+        if (n->capacity() * sizeof(int) > PLAN_KEEP) std::vector<int>().swap(*n);
 }
 
 long long deriv_offsets(const SetView &s, std::vector<int> &offs) {

@@ -79,16 +79,16 @@ struct SetView {
 struct Buckets {
     std::vector<int> labels;     // distinct labels, ascending
     std::vector<int> lab_start;  // packed row range of label l: [lab_start[l], lab_start[l+1])
-    std::vector<int> src;        // packed row -> padded row index (m * ma + atom)
-    std::vector<int> mol;        // packed row -> molecule index
+    std::vector<int> src;        // packed row -> padded row index (m * ma + atom); src / ma is
+                                 // its molecule
     int rows() const { return (int)src.size(); }
 };
 
 // Distinct labels present in the active atoms of one or two sets
 // (collect_distinct_labels_T, src/local_kernels.cpp:31-58).
 std::vector<int> collect_labels(const SetView &a, const SetView *b);
-// Bucket one set by the given label list.
-Buckets make_buckets(const SetView &s, const std::vector<int> &labels);
+// Both sets bucketed by the labels that either has (b null: one set).
+void plan_buckets(const SetView &a, const SetView *b, Buckets &ba, Buckets *bb);
 // Derivative-axis offsets: offs[m] = 3 * sum_{m' < m} n[m'], returns naq.
 long long deriv_offsets(const SetView &s, std::vector<int> &offs);
 

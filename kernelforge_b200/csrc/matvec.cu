@@ -634,11 +634,12 @@ kfb_status matvec_t(const Tin *x1, const Tin *dx1, const Tin *x2, const double *
     std::vector<int> off1;
     const long long naq1 = deriv_offsets(s1, off1);
     if (F) KFB_TRY(zero(F, (size_t)std::max<long long>(naq1, 1) * sizeof(double), s));
-    const std::vector<int> labels = collect_labels(s1, &s2);
+    Buckets b1, b2;
+    plan_buckets(s1, &s2, b1, &b2);
+    const std::vector<int> &labels = b1.labels;
     if (labels.empty()) return KFB_OK;
     if (!device_is_sm100())
         return set_error(KFB_ERR_UNSUPPORTED, "the contracted prediction needs an sm_100 (B200) device");
-    const Buckets b1 = make_buckets(s1, labels), b2 = make_buckets(s2, labels);
     long long pairs = 0;
     for (size_t l = 0; l < labels.size(); ++l)
         pairs += (long long)(b1.lab_start[l + 1] - b1.lab_start[l]) *

@@ -64,8 +64,8 @@ inline size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 template <class Tin>
 kfb_status run(const ScalarProblem &p, const PairSink &sink, cudaStream_t s) {
     using T = double;
-    std::vector<int> labels = collect_labels(p.s1, nullptr);
-    Buckets bk = make_buckets(p.s1, labels);
+    Buckets bk;
+    plan_buckets(p.s1, nullptr, bk, nullptr);
     std::vector<PairTile> tiles = make_pair_tiles(bk, bk, true, simt::ST, simt::ST);
     const int R = bk.rows();
     const int Dp = (p.rep + simt::SK - 1) / simt::SK * simt::SK;

@@ -38,6 +38,9 @@ std::vector<SuperBlock> make_super_blocks(const Buckets &a, const Buckets &b, bo
                                           int tm, int tn, size_t row_bytes, long long &ntiles);
 kfb_status expand_tiles(const std::vector<SuperBlock> &sbs, long long ntiles, int tm, int tn,
                         DevBuf &tiles, cudaStream_t s, int merge = 1);
+// The same from super-blocks that are on the device already.
+kfb_status expand_tiles(const SuperBlock *dsbs, int nsb, long long ntiles, int tm, int tn,
+                        DevBuf &tiles, cudaStream_t s, int merge = 1);
 // Rewrite the offsets of sbs for tiles of `merge` column tiles; returns the
 // number of merged tiles.
 long long merge_offsets(std::vector<SuperBlock> &sbs, int merge);

@@ -55,10 +55,10 @@ kfb_status pack_set(const Tin *x, const Buckets &bk, int ma, int rep, int Dp, De
 
 template <class Tin, class T>
 kfb_status run_simt(const ScalarProblem &p, const PairSink &sink, cudaStream_t s) {
-    std::vector<int> labels = collect_labels(p.s1, p.symmetric ? nullptr : &p.s2);
+    Buckets b1, b2;
+    plan_buckets(p.s1, p.symmetric ? nullptr : &p.s2, b1, &b2);
+    const std::vector<int> &labels = b1.labels;
     if (labels.empty()) return KFB_OK;
-    Buckets b1 = make_buckets(p.s1, labels);
-    Buckets b2 = p.symmetric ? Buckets() : make_buckets(p.s2, labels);
     const Buckets &bb = p.symmetric ? b1 : b2;
     const int Dp_ = (p.rep + SK - 1) / SK * SK;
     long long ntiles_ll = 0;
@@ -199,16 +199,21 @@ long long merge_offsets(std::vector<SuperBlock> &sbs, int merge) {
     return n;
 }
 
-kfb_status expand_tiles(const std::vector<SuperBlock> &sbs, long long ntiles, int tm, int tn,
+kfb_status expand_tiles(const SuperBlock *dsbs, int nsb, long long ntiles, int tm, int tn,
                         DevBuf &tiles, cudaStream_t s, int merge) {
     KFB_TRY(tiles.alloc((size_t)std::max<long long>(ntiles, 1) * sizeof(PairTile), s));
     if (ntiles == 0) return KFB_OK;
-    DevBuf dsb;
-    KFB_TRY(upload(dsb, sbs, s));
     expand_tiles_kernel<<<(unsigned)((ntiles + 255) / 256), 256, 0, s>>>(
-        dsb.as<SuperBlock>(), (int)sbs.size(), ntiles, tm, tn, merge, tiles.as<PairTile>());
+        dsbs, nsb, ntiles, tm, tn, merge, tiles.as<PairTile>());
     KFB_CUDA_TRY(cudaGetLastError());
     return KFB_OK;
+}
+
+kfb_status expand_tiles(const std::vector<SuperBlock> &sbs, long long ntiles, int tm, int tn,
+                        DevBuf &tiles, cudaStream_t s, int merge) {
+    DevBuf dsb;
+    KFB_TRY(upload(dsb, sbs, s));
+    return expand_tiles(dsb.as<SuperBlock>(), (int)sbs.size(), ntiles, tm, tn, tiles, s, merge);
 }
 
 std::vector<PairTile> make_pair_tiles(const Buckets &a, const Buckets &b, bool symmetric,
