@@ -202,9 +202,11 @@ __global__ void __launch_bounds__(256) force_contract_kernel(
 // ----------------------------------------------------- direct FP64 products
 // Few (query, training) atom pairs: the digit planes of the training rows and
 // of their transposes cost more than the products themselves, and a launch per
-// label and product leaves most SMs idle.  Two kernels take every label at
-// once and form the same sums with FP64 mma.sync (37 TFLOP/s measured on B200,
-// the FP64 FMA rate, at a quarter of the shared-memory loads).
+// label and product leaves most SMs idle.  Three kernels take every label at
+// once: row sums, weights, gradient rows; the products are FP64 mma.sync.
+// Columns are taken in groups of 8, and groups in which the training rows and
+// their coefficients are all zero (the sulphur channels of molecules without
+// sulphur: 28 of 90) add nothing to any product and are skipped.
 //
 // Label l: query rows [sa, sa + ra), training rows [sb, sb + rb), W and V of
 // ra rows of ldw doubles from woff; blocks [tile1, next label's tile1) of the
@@ -215,43 +217,143 @@ struct MvLabel {
     long long woff;
 };
 constexpr int MD_M = 32, MD_N = 64, MD_K = 32;
-constexpr int MD_LDK = MD_K + 4;   // row strides = 4 mod 16 doubles: the fragment
-constexpr int MD_LDN = MD_N + 4;   // loads of a half warp hit 16 different banks
+constexpr int MD_LDK = MD_K + 4;   // row strides (elements): the fragment loads of a warp
+                                   // (floats) or half warp (doubles) hit different banks
+template <class Tin> constexpr int md_ldn() { return MD_N + (sizeof(Tin) == 4 ? 8 : 4); }
 
-// v[u] = p[k + u] for k + u < n, else 0; vec: p + k is aligned to 16 bytes and
-// n a multiple of N.
-template <class Tin, int N>
-__device__ __forceinline__ void load_row(const Tin *p, int k, int n, bool vec, double (&v)[N]) {
-    if (vec && k < n) {
-        constexpr int PER = 16 / sizeof(Tin);
-#pragma unroll
-        for (int u = 0; u < N; u += PER) {
-            const uint4 w = *reinterpret_cast<const uint4 *>(p + k + u);
-            const Tin *e = reinterpret_cast<const Tin *>(&w);
-#pragma unroll
-            for (int r = 0; r < PER; ++r) v[u + r] = (double)e[r];
-        }
+__device__ __forceinline__ void md_cp16(void *dst, const void *src, bool ok) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                     static_cast<unsigned>(__cvta_generic_to_shared(dst))),
+                 "l"(src), "r"(ok ? 16 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void md_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void md_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// dst[0 .. 16 / sizeof(T)) = src[0 ..] (with vec 16-byte aligned, and an address of the array
+// where !ok too), zeros where !ok and for columns from `left` on.
+template <class T>
+__device__ __forceinline__ void md_piece(T *dst, const T *src, bool ok, int left, bool vec) {
+    if (vec) {
+        md_cp16(dst, src, ok);
     } else {
 #pragma unroll
-        for (int u = 0; u < N; ++u) v[u] = k + u < n ? (double)p[k + u] : 0.0;
+        for (int u = 0; u < 16 / (int)sizeof(T); ++u) dst[u] = ok && u < left ? src[u] : T(0);
     }
 }
 
+// Warp per row.  Query rows r < R1: n1[r] = |x|^2.  Training rows: n2 = |x|^2,
+// sc = x . Ad, and used[g] = 1 for the column groups with a value that is not
+// zero.  Four columns a lane (vec: 16-byte loads, 128 columns of the warp in
+// flight per step), so a group of 8 is two neighbouring lanes.
+template <class Tin>
+__global__ void __launch_bounds__(256) mv_rows_kernel(
+    const Tin *__restrict__ x1, const int *__restrict__ idx1, int R1, const Tin *__restrict__ x2,
+    const int *__restrict__ idx2, int R2, const double *__restrict__ ad, int rep, int vec,
+    double *__restrict__ n1, double *__restrict__ n2, double *__restrict__ sc,
+    int *__restrict__ used) {
+    const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (r >= R1 + R2) return;
+    const bool train = r >= R1;
+    const size_t at = (size_t)(train ? idx2[r - R1] : idx1[r]) * rep;
+    const Tin *x = (train ? x2 : x1) + at;
+    const double *a = train && ad ? ad + at : nullptr;
+    double n = 0.0, s = 0.0;
+#pragma unroll 3
+    for (int k0 = 0; k0 < rep; k0 += 128) {
+        const int k = k0 + 4 * lane;
+        double v[4] = {0.0, 0.0, 0.0, 0.0}, w[4] = {0.0, 0.0, 0.0, 0.0};
+        if (vec && k < rep) {
+            if constexpr (sizeof(Tin) == 4) {
+                const float4 f = *reinterpret_cast<const float4 *>(x + k);
+                v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+            } else {
+                const double2 f = *reinterpret_cast<const double2 *>(x + k);
+                const double2 h = *reinterpret_cast<const double2 *>(x + k + 2);
+                v[0] = f.x; v[1] = f.y; v[2] = h.x; v[3] = h.y;
+            }
+            if (a) {
+                const double2 f = *reinterpret_cast<const double2 *>(a + k);
+                const double2 h = *reinterpret_cast<const double2 *>(a + k + 2);
+                w[0] = f.x; w[1] = f.y; w[2] = h.x; w[3] = h.y;
+            }
+        } else {
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (k + u < rep) {
+                    v[u] = (double)x[k + u];
+                    if (a) w[u] = a[k + u];
+                }
+        }
+        bool on = false;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            n = fma(v[u], v[u], n);
+            s = fma(v[u], w[u], s);
+            on |= !(v[u] == 0.0) || !(w[u] == 0.0);
+        }
+        if (train && on && !used[k >> 3]) used[k >> 3] = 1;
+    }
+    for (int o = 16; o; o >>= 1) {
+        n += __shfl_xor_sync(0xffffffffu, n, o);
+        s += __shfl_xor_sync(0xffffffffu, s, o);
+    }
+    if (lane == 0) {
+        if (train) {
+            n2[r - R1] = n;
+            sc[r - R1] = s;
+        } else {
+            n1[r] = n;
+        }
+    }
+}
+
+// list = the used groups in order; returns their number (whole block; warp 0 works).
+__device__ __forceinline__ int md_groups(const int *__restrict__ used, int ng, int *list,
+                                         int *count) {
+    if (threadIdx.x < 32) {
+        int n = 0;
+        for (int g0 = 0; g0 < ng; g0 += 32) {
+            const int g = g0 + threadIdx.x;
+            const bool on = g < ng && used[g] != 0;
+            const unsigned m = __ballot_sync(0xffffffffu, on);
+            if (on) list[n + __popc(m & ((1u << threadIdx.x) - 1u))] = g;
+            n += __popc(m);
+        }
+        if (threadIdx.x == 0) *count = n;
+    }
+    __syncthreads();
+    return *count;
+}
+
+// Stages of the weights kernel: x1 (MD_M rows), x2 (MD_N) and Ad (MD_N) of MD_K columns.
+template <class Tin> struct MvW {
+    static constexpr int NST = sizeof(Tin) == 4 ? 3 : 2;
+    static constexpr int A = 0, X = MD_M * MD_LDK * (int)sizeof(Tin);
+    static constexpr int D = X + MD_N * MD_LDK * (int)sizeof(Tin);
+    static constexpr int STAGE = D + MD_N * MD_LDK * (int)sizeof(double);
+};
+
 // Tile of MD_M query rows x MD_N training rows of a label: G = x1 . x2 and
-// P = x1 . Ad over all columns, then e, w, v of every pair, the energy sums (E
-// of the query row's molecule), and with forces W = w, V = -v and rowsum(V).
-// The norms and x . Ad of the rows are summed while they are staged.  Warp
-// (wm, wn) holds 16 x 16 of both products.
+// P = x1 . Ad over the used columns, then e, w, v of every pair, the energy
+// sums (E of the query row's molecule), and with forces W = w, V = -v and
+// rowsum(V).  Warp (wm, wn) holds 16 x 16 of both products.
 template <class Tin>
 __global__ void __launch_bounds__(256, 2) mv_weights_kernel(
     const Tin *__restrict__ x1, const int *__restrict__ idx1, int ma1,
     const Tin *__restrict__ x2, const int *__restrict__ idx2, int ma2,
     const double *__restrict__ ad, const double *__restrict__ alpha_e,
     const MvLabel *__restrict__ labels, int nlab, int rep, int vec, int with_f, double c,
-    double is2, double is4, double *__restrict__ W, double *__restrict__ V,
-    double *__restrict__ E, double *__restrict__ rowv) {
-    __shared__ double As[MD_M][MD_LDK], Xs[MD_N][MD_LDK], Ds[MD_N][MD_LDK];
-    __shared__ double n1s[MD_M], n2s[MD_N], scs[MD_N];
+    double is2, double is4, const double *__restrict__ n1, const double *__restrict__ n2,
+    const double *__restrict__ sc, const int *__restrict__ used, double *__restrict__ W,
+    double *__restrict__ V, double *__restrict__ E, double *__restrict__ rowv) {
+    using S = MvW<Tin>;
+    extern __shared__ __align__(16) unsigned char md_raw[];
+    int *list = reinterpret_cast<int *>(md_raw + S::NST * S::STAGE);   // [ng], then the count
+    const int ng = (rep + 7) / 8;
+    const int nused = md_groups(used, ng, list, list + ng);
     int l = 0;
     while (l + 1 < nlab && (int)blockIdx.x >= labels[l + 1].tile1) ++l;
     const MvLabel lb = labels[l];
@@ -260,76 +362,91 @@ __global__ void __launch_bounds__(256, 2) mv_weights_kernel(
     const int i0 = (local % mt) * MD_M, j0 = (local / mt) * MD_N;
     const int na = min(MD_M, lb.ra - i0), nb = min(MD_N, lb.rb - j0);
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    // staging: 4 columns of row t / 8 of the queries, 8 columns of training row t / 4
-    const int ar = t >> 3, ak = (t & 7) * 4, br = t >> 2, bk = (t & 3) * 8;
-    const bool av = ar < na, bv = br < nb;
-    const Tin *pa = x1 + (size_t)(av ? idx1[lb.sa + i0 + ar] : 0) * rep;
-    const int jrow = bv ? idx2[lb.sb + j0 + br] : 0;
-    const Tin *pb = x2 + (size_t)jrow * rep;
-    const double *pd = ad ? ad + (size_t)jrow * rep : nullptr;
-    double ra[4], rb[8], rd[8], n1 = 0.0, n2 = 0.0, sc = 0.0;
-    auto fetch = [&](int k0) {
-        load_row<Tin, 4>(pa, k0 + ak, av ? rep : 0, vec, ra);
-        load_row<Tin, 8>(pb, k0 + bk, bv ? rep : 0, vec, rb);
-        if (pd) load_row<double, 8>(pd, k0 + bk, bv ? rep : 0, vec, rd);
+    // staging, in 16-byte pieces: PT of a row of Tin, PD of a row of Ad
+    constexpr int ET = 16 / sizeof(Tin), PT = MD_K / ET, PD = MD_K / 2;
+    auto stage = [&](int s, int chunk) {
+        unsigned char *base = md_raw + s * S::STAGE;
+        Tin *As = reinterpret_cast<Tin *>(base + S::A), *Xs = reinterpret_cast<Tin *>(base + S::X);
+        double *Ds = reinterpret_cast<double *>(base + S::D);
+        auto column = [&](int at, bool &ok) {   // of column `at` of the chunk
+            const int g = chunk * (MD_K / 8) + at / 8;
+            ok = ok && g < nused;
+            return g < nused ? list[g] * 8 + at % 8 : 0;
+        };
+        for (int e = t; e < MD_M * PT; e += 256) {
+            const int r = e / PT, at = (e - r * PT) * ET;
+            bool ok = r < na;
+            const int k = column(at, ok);
+            const Tin *row = x1 + (size_t)(r < na ? idx1[lb.sa + i0 + r] : 0) * rep;
+            md_piece<Tin>(As + r * MD_LDK + at, row + k, ok, rep - k, vec);
+        }
+#pragma unroll
+        for (int e = t; e < MD_N * PT; e += 256) {
+            const int r = e / PT, at = (e - r * PT) * ET;
+            bool ok = r < nb;
+            const int k = column(at, ok);
+            const Tin *row = x2 + (size_t)(r < nb ? idx2[lb.sb + j0 + r] : 0) * rep;
+            md_piece<Tin>(Xs + r * MD_LDK + at, row + k, ok, rep - k, vec);
+        }
+        if (ad) {
+#pragma unroll
+            for (int e = t; e < MD_N * PD; e += 256) {
+                const int r = e / PD, at = (e - r * PD) * 2;
+                bool ok = r < nb;
+                const int k = column(at, ok);
+                const double *row = ad + (size_t)(r < nb ? idx2[lb.sb + j0 + r] : 0) * rep;
+                md_piece<double>(Ds + r * MD_LDK + at, row + k, ok, rep - k, vec);
+            }
+        }
+        md_commit();
     };
     const int wm = warp & 1, wn = warp >> 1;
     const bool active = 16 * wm < na;
     double g[2][2][2] = {}, p[2][2][2] = {};
-    fetch(0);
-    for (int k0 = 0; k0 < rep; k0 += MD_K) {
-        __syncthreads();
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            As[ar][ak + u] = ra[u];
-            n1 = fma(ra[u], ra[u], n1);
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            Xs[br][bk + u] = rb[u];
-            n2 = fma(rb[u], rb[u], n2);
-            if (pd) {
-                Ds[br][bk + u] = rd[u];
-                sc = fma(rb[u], rd[u], sc);
-            }
-        }
-        __syncthreads();
-        if (k0 + MD_K < rep) fetch(k0 + MD_K);
+    const int nch = (nused + MD_K / 8 - 1) / (MD_K / 8);
+    for (int s = 0; s < S::NST - 1; ++s) {
+        if (s < nch) stage(s, s);
+        else md_commit();
+    }
+    for (int ch = 0; ch < nch; ++ch) {
+        md_wait<S::NST - 2>();
+        __syncthreads();   // the slice has landed, and the one before is read
+        if (ch + S::NST - 1 < nch) stage((ch + S::NST - 1) % S::NST, ch + S::NST - 1);
+        else md_commit();
         if (!active) continue;
+        const unsigned char *base = md_raw + (ch % S::NST) * S::STAGE;
+        const Tin *As = reinterpret_cast<const Tin *>(base + S::A);
+        const Tin *Xs = reinterpret_cast<const Tin *>(base + S::X);
+        const double *Ds = reinterpret_cast<const double *>(base + S::D);
+        const int r = lane >> 2, kl = lane & 3;
 #pragma unroll
         for (int kk = 0; kk < MD_K; kk += 4) {
-            const int r = lane >> 2, k = kk + (lane & 3);
-            const double a0 = As[16 * wm + r][k], a1 = As[16 * wm + 8 + r][k];
+            const int k = kk + kl;
+            const double a0 = (double)As[(16 * wm + r) * MD_LDK + k];
+            const double a1 = (double)As[(16 * wm + 8 + r) * MD_LDK + k];
 #pragma unroll
             for (int nj = 0; nj < 2; ++nj) {
-                const double x = Xs[16 * wn + 8 * nj + r][k];
+                const int row = (16 * wn + 8 * nj + r) * MD_LDK + k;
+                const double x = (double)Xs[row];
                 dmma(g[0][nj], a0, x);
                 dmma(g[1][nj], a1, x);
-                if (pd) {
-                    const double d = Ds[16 * wn + 8 * nj + r][k];
+                if (ad) {
+                    const double d = Ds[row];
                     dmma(p[0][nj], a0, d);
                     dmma(p[1][nj], a1, d);
                 }
             }
         }
     }
-    // row sums of the staged values: 8 threads of a query row, 4 of a training row
-    for (int o = 4; o; o >>= 1) n1 += __shfl_xor_sync(0xffffffffu, n1, o);
-    for (int o = 2; o; o >>= 1) {
-        n2 += __shfl_xor_sync(0xffffffffu, n2, o);
-        sc += __shfl_xor_sync(0xffffffffu, sc, o);
-    }
-    if ((t & 7) == 0) n1s[ar] = n1;
-    if ((t & 3) == 0) {
-        n2s[br] = n2;
-        scs[br] = sc;
-    }
-    __syncthreads();   // (also: every warp is past its fragment loads)
-    double *es = &As[0][0], *vs = es + 4 * MD_M;   // [wn][row] partial sums
+    md_wait<0>();
+    __syncthreads();   // every warp is past its fragment loads
+    double *es = reinterpret_cast<double *>(md_raw), *vs = es + 4 * MD_M;   // [wn][row] sums
     if (active) {
 #pragma unroll
         for (int mi = 0; mi < 2; ++mi) {
             const int i = 16 * wm + 8 * mi + (lane >> 2);
+            const double ni = i < na ? n1[lb.sa + i0 + i] : 0.0;
+            const double bad = ni - ni;   // 0, or NaN for a row that is not finite
             double esum = 0.0, vsum = 0.0;
 #pragma unroll
             for (int nj = 0; nj < 2; ++nj) {
@@ -338,10 +455,11 @@ __global__ void __launch_bounds__(256, 2) mv_weights_kernel(
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
                     if (i >= na || j + u >= nb) continue;
-                    const double d2 = fmax(n1s[i] + n2s[j + u] - 2.0 * g[mi][nj][u], 0.0);
+                    const int jr = lb.sb + j0 + j + u;
+                    const double d2 = fmax(ni + n2[jr] - 2.0 * g[mi][nj][u], 0.0);
                     const double e = exp(c * d2);
-                    const double dad = pd ? p[mi][nj][u] - scs[j + u] : 0.0;
-                    const double ae = alpha_e ? alpha_e[idx2[lb.sb + j0 + j + u] / ma2] : 0.0;
+                    const double dad = ad ? p[mi][nj][u] - sc[jr] + bad : 0.0;
+                    const double ae = alpha_e ? alpha_e[idx2[jr] / ma2] : 0.0;
                     w[u] = e * is2;
                     v[u] = w[u] * ae + e * is4 * dad;
                     esum += ae * e + w[u] * dad;
@@ -377,75 +495,108 @@ __global__ void __launch_bounds__(256, 2) mv_weights_kernel(
     }
 }
 
-// g[i, k] += sum_j W_ij Ad_jk + (-v)_ij x2_jk over the training rows
-// [split jlen, ...) of a label: MD_M query rows x MD_N columns per block, the
-// split-K sums combined by atomics.
-constexpr int MD_GRAD_SMEM = (2 * MD_M * MD_LDK + 2 * MD_K * MD_LDN) * (int)sizeof(double);
+// Stages of the gradient kernel: W and V (MD_M rows of MD_K partners), x2 and
+// Ad (MD_K rows of MD_N columns).
+template <class Tin> struct MvG {
+    static constexpr int NST = 2, LDN = md_ldn<Tin>(), LDD = md_ldn<double>();
+    static constexpr int W = 0, V = MD_M * MD_LDK * (int)sizeof(double);
+    static constexpr int X = 2 * V, D = X + MD_K * LDN * (int)sizeof(Tin);
+    static constexpr int STAGE = D + MD_K * LDD * (int)sizeof(double);
+};
 
+// g[i, k] += sum_j W_ij Ad_jk + (-v)_ij x2_jk over the training rows
+// [split jlen, ...) of a label: MD_M query rows x MD_N used columns per block,
+// the split-K sums combined by atomics.
 template <class Tin>
 __global__ void __launch_bounds__(256, 2) mv_grad_kernel(
     const Tin *__restrict__ x2, const int *__restrict__ idx2, const double *__restrict__ ad,
     const MvLabel *__restrict__ labels, int nlab, int rep, int jlen, int vec,
-    const double *__restrict__ W, const double *__restrict__ V, double *__restrict__ g) {
-    extern __shared__ __align__(16) double md_raw[];
-    double (*Ws)[MD_LDK] = reinterpret_cast<double (*)[MD_LDK]>(md_raw);
-    double (*Vs)[MD_LDK] = Ws + MD_M;
-    double (*Xs)[MD_LDN] = reinterpret_cast<double (*)[MD_LDN]>(md_raw + 2 * MD_M * MD_LDK);
-    double (*Ds)[MD_LDN] = Xs + MD_K;
+    const int *__restrict__ used, const double *__restrict__ W, const double *__restrict__ V,
+    double *__restrict__ g) {
+    using S = MvG<Tin>;
+    extern __shared__ __align__(16) unsigned char md_raw[];
+    int *list = reinterpret_cast<int *>(md_raw + S::NST * S::STAGE);
+    const int ng = (rep + 7) / 8;
+    const int nused = md_groups(used, ng, list, list + ng);
     int l = 0;
     while (l + 1 < nlab && (int)blockIdx.x >= labels[l + 1].tile2) ++l;
     const MvLabel lb = labels[l];
     const int mt = (lb.ra + MD_M - 1) / MD_M, nt = (rep + MD_N - 1) / MD_N;
     const int local = blockIdx.x - lb.tile2;
-    const int i0 = (local % mt) * MD_M, n0 = (local / mt % nt) * MD_N;
+    const int i0 = (local % mt) * MD_M, g0 = (local / mt % nt) * (MD_N / 8);
+    if (g0 >= nused) return;   // block-uniform
     const int jb = local / (mt * nt) * jlen, je = min(lb.rb, jb + jlen);
     const int na = min(MD_M, lb.ra - i0);
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    // staging: 4 partners of query row t / 8; 8 columns of training row t / 8
-    const int ar = t >> 3, aj = (t & 7) * 4, bk = (t & 7) * 8;
-    const long long wrow = lb.woff + (long long)(i0 + (ar < na ? ar : 0)) * lb.ldw;
-    double rw[4], rv[4], rx[8], rd[8];
-    auto fetch = [&](int j0) {
-        const int n = ar < na ? je : 0;
-        load_row<double, 4>(W + wrow, j0 + aj, n, false, rw);
-        load_row<double, 4>(V + wrow, j0 + aj, n, false, rv);
-        const int j = j0 + ar;
-        const bool jv = j < je;
-        const size_t row = (size_t)(jv ? idx2[lb.sb + j] : 0) * rep;
-        load_row<Tin, 8>(x2 + row, n0 + bk, jv ? rep : 0, vec, rx);
-        if (ad) load_row<double, 8>(ad + row, n0 + bk, jv ? rep : 0, vec, rd);
+    constexpr int ET = 16 / sizeof(Tin), PT = MD_N / ET, PD = MD_N / 2, PW = MD_K / 2;
+    auto stage = [&](int s, int j0) {
+        unsigned char *base = md_raw + s * S::STAGE;
+        double *Ws = reinterpret_cast<double *>(base + S::W);
+        double *Vs = reinterpret_cast<double *>(base + S::V);
+        Tin *Xs = reinterpret_cast<Tin *>(base + S::X);
+        double *Ds = reinterpret_cast<double *>(base + S::D);
+        // W, V rows: an odd last partner has a zero in the row's padding
+#pragma unroll
+        for (int e = t; e < MD_M * PW; e += 256) {
+            const int r = e / PW, at = (e - r * PW) * 2;
+            const bool ok = r < na && j0 + at < je;
+            const long long row = lb.woff + (long long)(i0 + (r < na ? r : 0)) * lb.ldw;
+            md_cp16(Ws + r * MD_LDK + at, ok ? W + row + j0 + at : W, ok);
+            md_cp16(Vs + r * MD_LDK + at, ok ? V + row + j0 + at : V, ok);
+        }
+        auto column = [&](int at, bool &ok) {
+            const int gi = g0 + at / 8;
+            ok = ok && gi < nused;
+            return gi < nused ? list[gi] * 8 + at % 8 : 0;
+        };
+#pragma unroll
+        for (int e = t; e < MD_K * PT; e += 256) {
+            const int r = e / PT, at = (e - r * PT) * ET, j = j0 + r;
+            bool ok = j < je;
+            const int k = column(at, ok);
+            const Tin *row = x2 + (size_t)(j < je ? idx2[lb.sb + j] : 0) * rep;
+            md_piece<Tin>(Xs + r * S::LDN + at, row + k, ok, rep - k, vec);
+        }
+        if (ad) {
+#pragma unroll
+            for (int e = t; e < MD_K * PD; e += 256) {
+                const int r = e / PD, at = (e - r * PD) * 2, j = j0 + r;
+                bool ok = j < je;
+                const int k = column(at, ok);
+                const double *row = ad + (size_t)(j < je ? idx2[lb.sb + j] : 0) * rep;
+                md_piece<double>(Ds + r * S::LDD + at, row + k, ok, rep - k, vec);
+            }
+        }
+        md_commit();
     };
     const int wm = warp & 1, wn = warp >> 1;
     const bool active = 16 * wm < na;
     double acc[2][2][2] = {};
-    fetch(jb);
-    for (int j0 = jb; j0 < je; j0 += MD_K) {
-        __syncthreads();
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            Ws[ar][aj + u] = rw[u];
-            Vs[ar][aj + u] = rv[u];
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            Xs[ar][bk + u] = rx[u];
-            if (ad) Ds[ar][bk + u] = rd[u];
-        }
-        __syncthreads();
-        if (j0 + MD_K < je) fetch(j0 + MD_K);
+    stage(0, jb);
+    int s = 0;
+    for (int j0 = jb; j0 < je; j0 += MD_K, s ^= 1) {
+        md_wait<0>();
+        __syncthreads();   // the slice has landed, and the other buffer is read
+        if (j0 + MD_K < je) stage(s ^ 1, j0 + MD_K);
         if (!active) continue;
+        const unsigned char *base = md_raw + s * S::STAGE;
+        const double *Ws = reinterpret_cast<const double *>(base + S::W);
+        const double *Vs = reinterpret_cast<const double *>(base + S::V);
+        const Tin *Xs = reinterpret_cast<const Tin *>(base + S::X);
+        const double *Ds = reinterpret_cast<const double *>(base + S::D);
+        const int r = lane >> 2, kl = lane & 3;
 #pragma unroll
         for (int kk = 0; kk < MD_K; kk += 4) {
-            const int r = lane >> 2, k = kk + (lane & 3);
-            const double v0 = Vs[16 * wm + r][k], v1 = Vs[16 * wm + 8 + r][k];
-            const double w0 = Ws[16 * wm + r][k], w1 = Ws[16 * wm + 8 + r][k];
+            const int k = kk + kl, r0 = (16 * wm + r) * MD_LDK + k, r1 = r0 + 8 * MD_LDK;
+            const double v0 = Vs[r0], v1 = Vs[r1], w0 = Ws[r0], w1 = Ws[r1];
 #pragma unroll
             for (int nj = 0; nj < 2; ++nj) {
-                const double x = Xs[k][16 * wn + 8 * nj + r];
+                const int col = 16 * wn + 8 * nj + r;
+                const double x = (double)Xs[k * S::LDN + col];
                 dmma(acc[0][nj], v0, x);
                 dmma(acc[1][nj], v1, x);
                 if (ad) {
-                    const double d = Ds[k][16 * wn + 8 * nj + r];
+                    const double d = Ds[k * S::LDD + col];
                     dmma(acc[0][nj], w0, d);
                     dmma(acc[1][nj], w1, d);
                 }
@@ -457,13 +608,15 @@ __global__ void __launch_bounds__(256, 2) mv_grad_kernel(
     for (int mi = 0; mi < 2; ++mi) {
         const int i = 16 * wm + 8 * mi + (lane >> 2);
         if (i >= na) continue;
-        double *row = g + (size_t)(lb.sa + i0 + i) * rep + n0;
+        double *row = g + (size_t)(lb.sa + i0 + i) * rep;
 #pragma unroll
         for (int nj = 0; nj < 2; ++nj) {
-            const int n = 16 * wn + 8 * nj + 2 * (lane & 3);
+            const int gi = g0 + 2 * wn + nj;
+            if (gi >= nused) continue;
+            const int k = list[gi] * 8 + 2 * (lane & 3);
 #pragma unroll
             for (int u = 0; u < 2; ++u)
-                if (n0 + n + u < rep) atomicAdd(row + n + u, acc[mi][nj][u]);
+                if (k + u < rep) atomicAdd(row + k + u, acc[mi][nj][u]);
         }
     }
 }
@@ -541,6 +694,7 @@ kfb_status mv_gemm(const OzSlices &A, const OzSlices &B, int M, int N, double *C
 // Same-label (query atom, training atom) pairs up to which the direct FP64
 // kernels are used.
 constexpr long long MD_MAX_PAIRS = 6LL << 20;
+constexpr int MD_MAX_REP = 1 << 16;   // (a list of column groups in shared memory)
 
 template <class Tin>
 kfb_status matvec_direct(const Tin *x1, const Tin *dx1, const Tin *x2, const double *ad,
@@ -594,31 +748,42 @@ kfb_status matvec_direct(const Tin *x1, const Tin *dx1, const Tin *x2, const dou
     const size_t o_src1 = append(src1), o_src2 = append(src2), o_off1 = append(off1);
     const size_t o_n1 = blob.size();
     for (int m = 0; m < s1.nm; ++m) blob.push_back(s1.natoms(m));
+    const int R2 = (int)src2.size(), ng = (rep + 7) / 8;
     DevBuf plan, wv, gr;
     KFB_TRY(upload(plan, blob, s));
     const int *dp = plan.as<int>();
     const bool with_f = F != nullptr;
-    if (with_f) {
-        KFB_TRY(wv.alloc((size_t)words * 2 * sizeof(double), s));
-        KFB_TRY(gr.alloc((size_t)R1 * (rep + 1) * sizeof(double), s));
-        KFB_TRY(zero(gr.ptr, (size_t)R1 * (rep + 1) * sizeof(double), s));
-    }
+    // cleared: gradient rows and rowsum(V) (with forces), then the group flags; then the row sums
+    const size_t gwords = with_f ? (size_t)R1 * (rep + 1) : 0;
+    const size_t clear = gwords * sizeof(double) + (size_t)(ng + 1) / 2 * sizeof(double);
+    if (with_f) KFB_TRY(wv.alloc((size_t)words * 2 * sizeof(double), s));
+    KFB_TRY(gr.alloc(clear + ((size_t)R1 + 2 * (size_t)R2) * sizeof(double), s));
+    KFB_TRY(zero(gr.ptr, clear, s));
     double *W = wv.as<double>(), *V = W + words;
     double *g = gr.as<double>(), *rowv = g + (size_t)R1 * rep;
+    int *used = reinterpret_cast<int *>(g + gwords);
+    double *n1 = reinterpret_cast<double *>(gr.as<char>() + clear), *n2 = n1 + R1, *sc = n2 + R2;
     auto aligned = [](const void *p) { return (reinterpret_cast<size_t>(p) & 15) == 0; };
     const int vec = rep % 8 == 0 && aligned(x1) && aligned(x2) && aligned(ad);
     const double c = -1.0 / (2.0 * sigma * sigma), is2 = 1.0 / (sigma * sigma), is4 = is2 * is2;
     const int nlab = (int)labs.size();
     const MvLabel *dl = reinterpret_cast<const MvLabel *>(dp);
-    mv_weights_kernel<Tin><<<tiles1, 256, 0, s>>>(
+    const size_t lbytes = (size_t)(ng + 1) * sizeof(int);
+    const size_t sm_w = (size_t)MvW<Tin>::NST * MvW<Tin>::STAGE + lbytes;
+    const size_t sm_g = (size_t)MvG<Tin>::NST * MvG<Tin>::STAGE + lbytes;
+    KFB_CUDA_TRY(cudaFuncSetAttribute(mv_weights_kernel<Tin>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_w));
+    KFB_CUDA_TRY(cudaFuncSetAttribute(mv_grad_kernel<Tin>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_g));
+    mv_rows_kernel<Tin><<<nblk((long long)R1 + R2, 8), 256, 0, s>>>(
+        x1, dp + o_src1, R1, x2, dp + o_src2, R2, ad, rep, vec, n1, n2, sc, used);
+    mv_weights_kernel<Tin><<<tiles1, 256, sm_w, s>>>(
         x1, dp + o_src1, s1.ma, x2, dp + o_src2, s2_ma, ad, alpha_e, dl, nlab, rep, vec,
-        with_f ? 1 : 0, c, is2, is4, W, V, E, rowv);
+        with_f ? 1 : 0, c, is2, is4, n1, n2, sc, used, W, V, E, rowv);
     KFB_CUDA_TRY(cudaGetLastError());
     if (!with_f) return KFB_OK;
-    KFB_CUDA_TRY(cudaFuncSetAttribute(mv_grad_kernel<Tin>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, MD_GRAD_SMEM));
-    mv_grad_kernel<Tin><<<tiles2, 256, MD_GRAD_SMEM, s>>>(x2, dp + o_src2, ad, dl, nlab, rep, jlen,
-                                                          vec, W, V, g);
+    mv_grad_kernel<Tin><<<tiles2, 256, sm_g, s>>>(x2, dp + o_src2, ad, dl, nlab, rep, jlen, vec,
+                                                  used, W, V, g);
     KFB_CUDA_TRY(cudaGetLastError());
     force_contract_kernel<Tin><<<dim3(R1, (rep + FC_K - 1) / FC_K), 256, 0, s>>>(
         x1, dx1, dp + o_src1, dp + o_n1, dp + o_off1, s1.ma, rep, g, rowv, F);
@@ -644,7 +809,8 @@ kfb_status matvec_t(const Tin *x1, const Tin *dx1, const Tin *x2, const double *
     for (size_t l = 0; l < labels.size(); ++l)
         pairs += (long long)(b1.lab_start[l + 1] - b1.lab_start[l]) *
                  (b2.lab_start[l + 1] - b2.lab_start[l]);
-    if (pairs <= MD_MAX_PAIRS && (size_t)pairs * 2 * sizeof(double) <= workspace_budget())
+    if (pairs <= MD_MAX_PAIRS && rep <= MD_MAX_REP &&
+        (size_t)pairs * 2 * sizeof(double) <= workspace_budget())
         return matvec_direct<Tin>(x1, dx1, x2, ad, alpha_e, s1, off1, s2.ma, b1, b2, rep, sigma, E, F,
                                   s);
     std::vector<int> n1v(s1.nm);

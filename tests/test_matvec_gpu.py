@@ -124,6 +124,30 @@ def test_direct_products_tile_edges(nm1, nm2, ma, rep, monkeypatch):
             close(lk.kernel_gaussian_local_hessian_matvec(X1, dX1, X2, ad, *tail), Fr0, tol)
 
 
+@pytest.mark.parametrize("rep", [24, 40, 720, 43])
+def test_direct_products_unused_groups(rep):
+    """Groups of 8 columns that are zero in the training rows and their coefficients are skipped:
+    the query rows are not zero there (their norms count), one group holds a single coefficient
+    and one a single descriptor value; no group at all is used with zero training data."""
+    from kernelforge_b200 import local_kernels as lk
+    X1, dX1, Q1, N1, X2, dX2, Q2, N2, aE, aF = _problem(91 + rep, nm1=5, nm2=9, ma1=7, ma2=7,
+                                                        rep=rep, scale=0.35 * (24 / rep) ** 0.5)
+    ad = om.alpha_desc(dX2, Q2, N2, np.resize(aF, int(3 * N2.sum())))
+    groups = np.arange(rep) // 8
+    off = np.isin(groups, np.unique(groups)[::2])
+    X2[:, :, off] = 0.0
+    ad[:, :, off] = 0.0
+    ad[1, 0, 3] = 0.7
+    X2[2, 0, min(19, rep - 1)] = 0.4
+    tail = (Q1, Q2, N1, N2, 0.9)
+    for scale in (1.0, 0.0):
+        X2s, ads = X2 * scale, ad * scale
+        Er, Fr = om.matvec(X1, dX1, X2s, ads, aE, *tail)
+        E, F = lk.kernel_gaussian_local_full_matvec(X1, dX1, X2s, ads, aE, *tail)
+        close(E, Er, 1e-11)
+        close(F, Fr, 1e-11)
+
+
 def test_edge_cases():
     from kernelforge_b200 import local_kernels as lk
     X1, dX1, Q1, N1, X2, dX2, Q2, N2, aE, aF = _problem(41)
