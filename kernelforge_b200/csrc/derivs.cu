@@ -319,7 +319,8 @@ __global__ void __launch_bounds__(JV_THREADS, sizeof(T) == 4 ? 3 : 2) jac_v_kern
 // (nm, ma, rep) and, with dx, in its Jacobian's columns c < 3 nat[m] (NaN is
 // not zero); amax (optional): [0] max |x|, [1] max |dx| of the same entries.
 // Block per atom; the Jacobian is read along its rows, 16 bytes a lane (VEC,
-// rep a multiple of 4): the pass is bound by HBM.
+// rep a multiple of 4), pieces of padding left out: 1.1 GB in 0.2 ms, which is
+// HBM (4 bytes a lane: 0.33 ms).
 template <class T, bool VEC>
 __global__ void __launch_bounds__(256) used_columns_kernel(const T *__restrict__ x,
                                                            const T *__restrict__ dx, int ma,
@@ -344,15 +345,16 @@ __global__ void __launch_bounds__(256) used_columns_kernel(const T *__restrict__
         const unsigned ld = 3 * ma, nc = 3 * na;
         const T *J = dx + (size_t)blockIdx.x * rep * ld;
         if constexpr (VEC) {
-            constexpr int PER = 16 / sizeof(T);
+            constexpr unsigned PER = 16 / sizeof(T);
             const unsigned n = (unsigned)rep * ld / PER;
 #pragma unroll 4
-            for (unsigned e = threadIdx.x; e < n; e += blockDim.x) {
-                const uint4 w = reinterpret_cast<const uint4 *>(J)[e];
-                const T *v = reinterpret_cast<const T *>(&w);
+            for (unsigned e = threadIdx.x; e < n; e += 256) {
                 unsigned k = e * PER / ld, c = e * PER - k * ld;
+                uint4 w = make_uint4(0u, 0u, 0u, 0u);   // (pieces of padding stay unread)
+                if (c < nc || c + PER > ld) w = reinterpret_cast<const uint4 *>(J)[e];
+                const T *v = reinterpret_cast<const T *>(&w);
 #pragma unroll
-                for (int u = 0; u < PER; ++u) {
+                for (unsigned u = 0; u < PER; ++u) {
                     if (c < nc && !(v[u] == T(0))) {
                         uc[k] = 1;
                         md = fmaxf(md, fabsf((float)v[u]));
@@ -387,21 +389,62 @@ __global__ void __launch_bounds__(256) used_columns_kernel(const T *__restrict__
     }
 }
 
-// dst[r][k][:] = src[r][cols[k]][:] for k < n, zero for n <= k < np (rows of w
-// values); block per r.
-template <class T>
-__global__ void __launch_bounds__(256) compact_columns_kernel(const T *__restrict__ src,
-                                                              const int *__restrict__ cols, int n,
-                                                              int np, int rep, int w,
-                                                              T *__restrict__ dst) {
-    extern __shared__ int uc[];   // [n]
-    for (int k = threadIdx.x; k < n; k += blockDim.x) uc[k] = cols[k];
-    __syncthreads();
+// dst[r][k][:] = src[r][cols[k]][:] for k < n, zero for n <= k < np (a multiple
+// of 16), for the real atoms r and at least the first 3 nat[m] of the w values
+// of a Jacobian row (w = 1: the descriptor).  What is padding in src may stay
+// unwritten: the derivative kernels do not read it.  Block per atom, a warp per
+// four rows; four rows that are neighbours in src too are one aligned run of w
+// 16-byte pieces (VEC; columns are unused by whole channels).
+template <class T, bool VEC>
+__global__ void __launch_bounds__(256) compact_columns_kernel(
+    const T *__restrict__ src, const int *__restrict__ cols, int n, int np, int rep, int w, int ma,
+    const int *__restrict__ nat, T *__restrict__ dst) {
+    const int m = blockIdx.x / ma, j = blockIdx.x - m * ma;
+    const int na = min(max(nat[m], 0), ma);
     const T *s = src + (size_t)blockIdx.x * rep * w;
     T *d = dst + (size_t)blockIdx.x * np * w;
-    for (unsigned e = threadIdx.x; e < (unsigned)(np * w); e += blockDim.x) {
-        const unsigned k = e / (unsigned)w, c = e - k * (unsigned)w;
-        d[e] = k < (unsigned)n ? s[(size_t)uc[k] * w + c] : T(0);
+    if (w == 1) {   // descriptors of padding atoms too: zeros
+        for (int k = threadIdx.x; k < np; k += blockDim.x)
+            d[k] = k < n && j < na ? s[cols[k]] : T(0);
+        return;
+    }
+    if (j >= na) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int nc = 3 * na;
+    constexpr int PER = 16 / sizeof(T);
+    for (int k0 = 4 * warp; k0 < np; k0 += 4 * nw) {
+        int at[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) at[u] = k0 + u < n ? cols[k0 + u] : -1;
+        if (VEC && at[0] >= 0 && at[0] % 4 == 0 && at[1] == at[0] + 1 && at[2] == at[0] + 2 &&
+            at[3] == at[0] + 3) {
+            const uint4 *sv = reinterpret_cast<const uint4 *>(s + (size_t)at[0] * w);
+            uint4 *dv = reinterpret_cast<uint4 *>(d + (size_t)k0 * w);
+            const int pieces = 4 * w / PER;
+            // (pieces of padding are left out)
+            for (int e0 = lane; e0 < pieces; e0 += 128) {
+                uint4 v[4];
+                bool in[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int e = e0 + 32 * u, c = e * PER % w;
+                    in[u] = e < pieces && (c < nc || c + PER > w);
+                    if (in[u]) v[u] = sv[e];
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (in[u]) dv[e0 + 32 * u] = v[u];
+            }
+            continue;
+        }
+#pragma unroll 2
+        for (int c = lane; c < nc; c += 32) {
+            T v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) v[u] = at[u] >= 0 ? s[(size_t)at[u] * w + c] : T(0);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) d[(size_t)(k0 + u) * w + c] = v[u];
+        }
     }
 }
 
@@ -1568,8 +1611,8 @@ kfb_status scan_columns(const DerivSet &d, int rep, const int *nat, int *used, f
     const bool vec = rep % 4 == 0 && (reinterpret_cast<size_t>(dx) & 15) == 0 &&
                      (long long)rep * 3 * d.v.ma < (1LL << 31);
     auto kern = vec ? used_columns_kernel<T, true> : used_columns_kernel<T, false>;
-    kern<<<(unsigned)atoms, 256, staged ? rep * sizeof(int) : 0, s>>>(x, dx, d.v.ma, rep, nat,
-                                                                      used, staged ? 1 : 0, amax);
+    kern<<<(unsigned)atoms, 256, staged ? rep * sizeof(int) : 0, s>>>(x, dx, d.v.ma, rep, nat, used,
+                                                                      staged ? 1 : 0, amax);
     KFB_CUDA_TRY(cudaGetLastError());
     return KFB_OK;
 }
@@ -1615,32 +1658,53 @@ kfb_status compact_columns(DerivSet &s1, DerivSet &s2, int &rep, CompactSets &ke
     auto bytes = [&](const DerivSet &d, bool jac) {
         return (size_t)d.v.nm * d.v.ma * np * (jac ? width(d) : 1) * sizeof(T);
     };
-    size_t need = bytes(s1, false) + (same_x ? 0 : bytes(s2, false));
+    const bool share_x = same_x && same_n, share_dx = same_dx && same_n;
+    size_t need = bytes(s1, false) + (share_x ? 0 : bytes(s2, false));
     if (s1.dx) need += bytes(s1, true);
-    if (s2.dx && !same_dx) need += bytes(s2, true);
-    size_t fr = 0, tot = 0;
-    KFB_CUDA_TRY(cudaMemGetInfo(&fr, &tot));
-    if (need > fr / 4) return KFB_OK;
+    if (s2.dx && !share_dx) need += bytes(s2, true);
+    // copies within the workspace budget are simply tried; larger ones must fit
+    // in a quarter of the free memory (the query can take milliseconds)
+    if (need > budget_bytes()) {
+        size_t fr = 0, tot = 0;
+        KFB_CUDA_TRY(cudaMemGetInfo(&fr, &tot));
+        if (need > fr / 4) return KFB_OK;
+    }
+    {
+        auto reserve = [&](const DerivSet &d, bool jac, DevBuf &buf) {
+            return buf.alloc(std::max<size_t>(1, bytes(d, jac)), s) == KFB_OK;
+        };
+        const bool got = reserve(s1, false, keep.x1) && (!s1.dx || reserve(s1, true, keep.dx1)) &&
+                         (share_x || reserve(s2, false, keep.x2)) &&
+                         (!s2.dx || share_dx || reserve(s2, true, keep.dx2));
+        if (!got) {
+            for (DevBuf *b : {&keep.x1, &keep.dx1, &keep.x2, &keep.dx2}) b->release();
+            return KFB_OK;
+        }
+    }
     DevBuf dcols;
     cols.resize(std::max(n, 1));
     KFB_TRY(upload(dcols, cols, s));
-    auto copy = [&](const void *&src, const DerivSet &d, int w, DevBuf &buf) -> kfb_status {
+    auto copy = [&](const void *&src, const DerivSet &d, const int *n_dev, int w,
+                    DevBuf &buf) -> kfb_status {
         const long long atoms = (long long)d.v.nm * d.v.ma;
-        KFB_TRY(buf.alloc(std::max<size_t>(1, (size_t)atoms * np * w * sizeof(T)), s));
         if (atoms > 0) {
-            compact_columns_kernel<T><<<(unsigned)atoms, 256, std::max(n, 1) * sizeof(int), s>>>(
-                static_cast<const T *>(src), dcols.as<int>(), n, np, rep, w, buf.as<T>());
+            const bool vec = rep % 4 == 0 && (reinterpret_cast<size_t>(src) & 15) == 0;
+            auto kern = vec ? compact_columns_kernel<T, true> : compact_columns_kernel<T, false>;
+            kern<<<(unsigned)atoms, 256, 0, s>>>(static_cast<const T *>(src), dcols.as<int>(), n,
+                                                 np, rep, w, d.v.ma, n_dev, buf.as<T>());
             KFB_CUDA_TRY(cudaGetLastError());
         }
         src = buf.ptr;
         return KFB_OK;
     };
-    KFB_TRY(copy(s1.x, s1, 1, keep.x1));
-    if (s1.dx) KFB_TRY(copy(s1.dx, s1, (int)width(s1), keep.dx1));
-    if (same_x) s2.x = s1.x;
-    else KFB_TRY(copy(s2.x, s2, 1, keep.x2));
-    if (s2.dx && same_dx) s2.dx = s1.dx;
-    else if (s2.dx) KFB_TRY(copy(s2.dx, s2, (int)width(s2), keep.dx2));
+    // (one array with two sets of atom counts is two copies: each holds its own atoms)
+    const int *dn1 = dn.as<int>(), *dn2 = dn1 + s1.v.nm;
+    KFB_TRY(copy(s1.x, s1, dn1, 1, keep.x1));
+    if (s1.dx) KFB_TRY(copy(s1.dx, s1, dn1, (int)width(s1), keep.dx1));
+    if (share_x) s2.x = s1.x;
+    else KFB_TRY(copy(s2.x, s2, dn2, 1, keep.x2));
+    if (s2.dx && share_dx) s2.dx = s1.dx;
+    else if (s2.dx) KFB_TRY(copy(s2.dx, s2, dn2, (int)width(s2), keep.dx2));
     rep = np;
     return KFB_OK;
 }
@@ -1774,14 +1838,17 @@ kfb_status jacobian_core(const DerivSet &outer, const DerivSet &inner, int rep, 
     // stay resident for its contraction
     const size_t row_bytes = (size_t)NU * rep * (tc ? 2 * sizeof(__half) : sizeof(T));
     size_t budget = budget_bytes();
-    if (!getenv("KFB_WORKSPACE_GB")) {
+    // more than the default budget only where it holds less than two M tiles of
+    // rows (a call of cudaMemGetInfo has taken from 0.1 to 6 ms)
+    if (!getenv("KFB_WORKSPACE_GB") && budget / std::max<size_t>(row_bytes, 1) < 256 &&
+        (size_t)nmo * row_bytes > budget) {
         size_t fr = 0, tot = 0;
         if (cudaMemGetInfo(&fr, &tot) == cudaSuccess)
             budget = std::max(budget, std::min<size_t>(fr / 4, (size_t)16 << 30));
     }
     int chunk = (int)std::max<size_t>(1, budget / std::max<size_t>(row_bytes, 1));
     chunk = std::min(chunk, nmo);
-    if (tc && chunk > 128) chunk -= chunk % 128;   // whole 128-row MMA tiles
+    if (tc && chunk > 128 && chunk < nmo) chunk -= chunk % 128;   // whole 128-row MMA tiles
     // dot products of a chunk: a row per matched outer atom (label blocks one
     // after the other), a column per sorted inner atom; only the label-diagonal
     // blocks are formed and read
@@ -2409,13 +2476,23 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
                 kj = (ma2 + 15) / 16 * 16;
                 const long long jk_rows = (long long)s2.v.nm * ld2 * rep;
                 const long long jk_bytes = jk_rows * kj * 2 * (long long)sizeof(__half);
-                size_t free_b = 0, total_b = 0;
-                KFB_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
                 const char *ye = std::getenv("KFB_HESSIAN_Y");
                 ygemm = !(ye && std::string(ye) == "cuda-core") && rep % 8 == 0 &&
                         jk_rows < INT_MAX &&
-                        (long long)batch * ma1 < INT_MAX &&
-                        jk_bytes + (long long)budget_bytes() <= (long long)free_b;
+                        (long long)batch * ma1 < INT_MAX;
+                // the workspace is allocated by now: up to its size this is simply
+                // tried, more must leave as much free (the query can take milliseconds)
+                if (ygemm && jk_bytes > (long long)budget_bytes()) {
+                    size_t free_b = 0, total_b = 0;
+                    KFB_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
+                    ygemm = jk_bytes + (long long)budget_bytes() <= (long long)free_b;
+                }
+                if (ygemm && (jkh.alloc((size_t)jk_bytes / 2, s) != KFB_OK ||
+                              jkl.alloc((size_t)jk_bytes / 2, s) != KFB_OK)) {
+                    jkh.release();
+                    jkl.release();
+                    ygemm = false;
+                }
             }
             if (!ygemm) {   // per-molecule max |J| for the bound of |Y|
                 KFB_TRY(d_jbm.alloc((size_t)s2.v.nm * sizeof(float), s));
@@ -2426,9 +2503,6 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
             }
             if (ygemm) {
                 TraceScope tr_j("hessian:jk-split", s);
-                const size_t jk_elems = (size_t)s2.v.nm * ld2 * rep * kj;
-                KFB_TRY(jkh.alloc(jk_elems * sizeof(__half), s));
-                KFB_TRY(jkl.alloc(jk_elems * sizeof(__half), s));
                 const size_t jsm = (size_t)8 * (ld2 + 1) * sizeof(float);
                 if (jsm > 48 * 1024)
                     KFB_CUDA_TRY(cudaFuncSetAttribute(jk_split_kernel<float>,
@@ -2451,7 +2525,8 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
                 for (int m = 0; m < s2.v.nm; ++m)
                     for (int l = 0; l < L; ++l) ns = std::max(ns, lm2.count(l, m, m));
                 const double yb = 16384.0 / (double)jr_scale * ns / (sigma * sigma);
-                yg_scale = (float)std::exp2(14.0 - std::ceil(std::log2(yb)));
+                // (a bound, not a maximum: 2^15 still leaves half of fp16's range)
+                yg_scale = (float)std::exp2(15.0 - std::ceil(std::log2(yb)));
                 if (!(yg_scale > 0.f) || !std::isfinite(yg_scale)) yg_scale = 1.f;
             }
             note_path(ygemm ? "hessian:y-gemm" : "hessian:y-cuda-core");
