@@ -4,19 +4,18 @@
 //
 // Two levels of blocking.  Outer panels of 512 columns; inside one, per
 // 128-column block j (c0 = 128 j, rows r0 = c0 + w .. n-1 below it):
-//   1. chol_block_kernel  one CTA factors the w x w diagonal block in shared
-//                         memory in 32-column sub-blocks (a warp factors each
-//                         32 x 32 diagonal sub-block in registers, then inverts
-//                         it; the CTA solves the rows below and updates the
-//                         rest of the block), then forms W = L_jj^{-1} by
-//                         block substitution; the first non-positive pivot is
+//   1. chol_block64_kernel (FP32-class factor: chol_block_kernel) one CTA
+//                         factors the w x w diagonal block in shared memory and
+//                         forms W = L_jj^{-1}; the first non-positive pivot is
 //                         recorded (LAPACK potrf's info);
 //   2. chol_panel_kernel  L_21 = A_21 W^T in FP64 (64 rows per CTA, W and the
 //                         rows staged in shared memory by cp.async), written
 //                         over A_21, together with the digit planes and row
 //                         exponents of L_21;
 //   3. inner update       the outer panel's remaining columns (all rows below
-//                         them) -= L_21 L_21^T, K = 128 (tensor cores);
+//                         them) -= L_21 L_21^T, K = 128 (tensor cores): the next
+//                         diagonal block on the critical stream, the rest on a
+//                         stream of its own beside that block's factorisation;
 // then, once per outer panel, the panel is sliced again (one row scale over
 // its 512 columns) and everything right of it is updated by tensor-core
 // products with K = 512 on the lower triangle only: the next outer panel's
@@ -35,6 +34,7 @@
 #include <cmath>
 
 #include "chol.h"
+#include "kernels_common.cuh"
 #include "ozaki.h"
 
 namespace kfb {
@@ -56,11 +56,10 @@ static_assert(NB == 4 * SB, "the block kernel assumes four sub-blocks");
 
 __host__ __device__ constexpr int wblk(int i, int j) { return i * (i + 1) / 2 + j; }
 
-template <class F>
-constexpr size_t blk_smem() {
-    return ((size_t)NB * LDT + (size_t)NWB * SB * LDW + SB) * sizeof(F) + 16;
-}
-constexpr size_t PANEL_SMEM = ((size_t)NB * NB + (size_t)NB * (PR + 1)) * sizeof(double);
+using F = float;   // arithmetic of the FP32-class diagonal block
+constexpr size_t BLK_SMEM = ((size_t)NB * LDT + (size_t)NWB * SB * LDW + SB) * sizeof(F) + 16;
+constexpr int LDP = NB + 4, LDX = PR + 4;   // panel kernel: strides of W and of the rows (4 mod 16)
+constexpr size_t PANEL_SMEM = (size_t)NB * (LDP + LDX) * sizeof(double);
 
 // Asynchronous global -> shared copies (cp.async): `bytes` of 8 or 16, with
 // the shared destination zero-filled instead when `valid` is false (the
@@ -96,25 +95,19 @@ __device__ __forceinline__ double pivot_rsqrt(double d) {
 }
 __device__ __forceinline__ float pivot_rsqrt(float d) { return rsqrtf(d); }
 
-template <class F> struct Vec2;
-template <> struct Vec2<double> { using type = double2; };
-template <> struct Vec2<float> { using type = float2; };
-
 // Factor the w x w block at (c0, c0) of the column-major matrix A in place
 // (lower triangle) and write W = L^{-1} column-major into Wout (NB x NB, zero
-// above the diagonal and beyond w), with the arithmetic in F: double for an
-// FP64-class factor, float for an FP32-class one (the FP32 pivot chain is
-// several times shorter: one-instruction shuffles, rsqrt, FMAs).
+// above the diagonal and beyond w), with FP32 arithmetic (an FP32-class
+// factor; chol_block64_kernel is the FP64 one).
 //
 // Shared memory: T[k * LDT + r] = A[c0 + r][c0 + k] (zero outside the lower
 // w x w triangle); WB holds the lower 32 x 32 blocks of W, block (i, j) at
 // WB + wblk(i, j) * SB * LDW, element (r, c) at [c * LDW + r]; rd[r] = 1 /
 // L[o + r][o + r] of the current sub-block.
-template <class F>
 __global__ void __launch_bounds__(BLK_THREADS, 1)
     chol_block_kernel(double *__restrict__ A, long long ld, int c0, int w,
                       double *__restrict__ Wout, int *info, int *skip) {
-    using F2 = typename Vec2<F>::type;
+    using F2 = float2;
     if (*(volatile int *)skip) return;
     extern __shared__ __align__(16) unsigned char sm_raw[];
     F *T = reinterpret_cast<F *>(sm_raw);
@@ -123,25 +116,7 @@ __global__ void __launch_bounds__(BLK_THREADS, 1)
     int *flag = reinterpret_cast<int *>(rd + SB);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const double *blk = A + (long long)c0 * ld + c0;
-    if constexpr (sizeof(F) == 8) {
-        if (w == NB && (ld & 1) == 0 && (c0 & 1) == 0) {
-            // a full block, 16-byte aligned rows: pairs of rows per copy (the
-            // strict upper triangle comes along and is never read)
-#pragma unroll 4
-            for (int idx = tid; idx < NB * NB / 2; idx += BLK_THREADS) {
-                const int k = idx / (NB / 2), r = 2 * (idx - k * (NB / 2));
-                cp_async(T + k * LDT + r, blk + (long long)k * ld + r, 16, true);
-            }
-        } else {
-#pragma unroll 4
-            for (int idx = tid; idx < NB * NB; idx += BLK_THREADS) {
-                const int k = idx / NB, r = idx - k * NB;
-                const bool v = r < w && k < w && r >= k;
-                cp_async(T + k * LDT + r, v ? blk + (long long)k * ld + r : blk, 8, v);
-            }
-        }
-        cp_async_wait_all();
-    } else {
+    {
         // eight independent loads in flight per thread, then the conversions
         constexpr int PER = NB * NB / BLK_THREADS;
         static_assert(PER % 8 == 0, "load batches");
@@ -183,21 +158,16 @@ __global__ void __launch_bounds__(BLK_THREADS, 1)
                     a[c] = l;
                     // the scaled column is final: write it, then read it back as
                     // a broadcast (faster than 31 shuffles on the pivot chain:
-                    // 164 vs 247 cycles per column in FP32, 420 vs 523 in FP64)
+                    // 164 vs 247 cycles per column)
                     if (lane >= c && lane < wp) T[(o + c) * LDT + o + lane] = l;
                     __syncwarp();
 #pragma unroll
                     for (int k = c + 1; k < SB; ++k) {
                         const F lk = T[(o + c) * LDT + o + k];   // L[k][c] (0 beyond wp)
-                        if constexpr (sizeof(F) == 4) {
-                            // FP32: a select and an unconditional FMA (no
-                            // divergent branch per k: 71 -> 60 us per block)
-                            const F m = (k <= lane) ? l : F(0);
-                            a[k] = fma(-m, lk, a[k]);
-                        } else {
-                            // FP64: the masked FMAs would cost more than the branch
-                            if (k <= lane) a[k] = fma(-l, lk, a[k]);
-                        }
+                        // a select and an unconditional FMA (no divergent
+                        // branch per k: 71 -> 60 us per block)
+                        const F m = (k <= lane) ? l : F(0);
+                        a[k] = fma(-m, lk, a[k]);
                     }
                 }
             }
@@ -358,12 +328,243 @@ __global__ void __launch_bounds__(BLK_THREADS, 1)
     }
 }
 
+// FP64 diagonal block on mma.sync: the w x w block at (c0, c0) factored in
+// place and W = L^{-1} written to Wout, as chol_block_kernel does in FP32.
+//
+// 16 micro-panels of 8 columns over the whole block, two barriers each:
+//   A  the 8 x 8 diagonal block of panel p, in one thread's registers (every
+//      lane of warp 0 the same: no exchange on the pivot chain);
+//   B  a thread per row below solves its 8 entries; another warp inverts the
+//      8 x 8 block;
+//   C  warp 0 updates the next diagonal block alone and goes on with its A,
+//      while warps 1..15 update the rest of the trailing triangle (8 x 8 tiles,
+//      K = 8) and form row block p of W, -W_pp sum_{k<p} L_pk W_kj, block by
+//      block.
+// What bounds it is the chain A-B over the panels; the rest hides behind A.
+// (32-column sub-blocks factored by one warp with a lane per row, then
+// inverted and applied in phases of their own, took 75-83 us a block.)
+//
+// Shared memory: T[k * DLT + r] holds the lower triangle in column k, row r;
+// its strict upper triangle takes W's blocks off the diagonal transposed into
+// the same index pattern, W[r][c] at T[r * DLT + c] (c < r); Wp[p] is W_pp by
+// rows.  Row strides of 4 and 12 mod 16 doubles keep the fragment loads of a
+// half warp on different banks.  Beyond w the block is the identity.
+constexpr int DB = 8, DP = NB / DB;      // micro-panel width, their number
+constexpr int DLT = NB + 4;              // shared column stride (4 mod 16)
+constexpr int DLW = DB + 4;              // row stride of an inverted 8 x 8 block
+constexpr size_t DBLK_SMEM =
+    ((size_t)NB * DLT + (size_t)DP * DB * DLW + DB * DB + DB) * sizeof(double) + 16;
+
+// a (lower triangle) -> its Cholesky factor, rinv = 1 / diagonal; returns the
+// first column with a non-positive pivot (DB: none).
+__device__ __forceinline__ int chol8(double (&a)[DB][DB], double (&rinv)[DB]) {
+    int bad = DB;
+#pragma unroll
+    for (int c = 0; c < DB; ++c) {
+        const double d = a[c][c];
+        if (!(d > 0.0) || !isfinite(d)) bad = min(bad, c);
+        rinv[c] = pivot_rsqrt(d);
+        a[c][c] = d * rinv[c];
+#pragma unroll
+        for (int r = c + 1; r < DB; ++r) a[r][c] *= rinv[c];
+#pragma unroll
+        for (int k = c + 1; k < DB; ++k)
+#pragma unroll
+            for (int r = k; r < DB; ++r) a[r][k] = fma(-a[r][c], a[k][c], a[r][k]);
+    }
+    return bad;
+}
+
+// Tile (kb, rb) of the trailing triangle -= X_rb X_kb^T for panel columns
+// o .. o + 7: D's rows are the tile's columns k, so that a lane's two values
+// are neighbours in memory.
+__device__ __forceinline__ void chol_tile(double *T, int o, int kb, int rb, int lane) {
+    const int i = lane >> 2, j = lane & 3;
+    double2 *c = reinterpret_cast<double2 *>(T + (DB * kb + i) * DLT + DB * rb + 2 * j);
+    const double *x0 = T + (o + j) * DLT, *x1 = x0 + 4 * DLT;
+    const double a0 = -x0[DB * kb + i], a1 = -x1[DB * kb + i];
+    const double b0 = x0[DB * rb + i], b1 = x1[DB * rb + i];
+    const double2 v = *c;
+    double d[2] = {v.x, v.y};
+    dmma(d, a0, b0);
+    dmma(d, a1, b1);
+    *c = make_double2(d[0], d[1]);
+}
+
+__global__ void __launch_bounds__(BLK_THREADS, 1)
+    chol_block64_kernel(double *__restrict__ A, long long ld, int c0, int w,
+                        double *__restrict__ Wout, int *info, int *skip) {
+    if (*(volatile int *)skip) return;
+    extern __shared__ __align__(16) unsigned char sm_raw[];
+    double *T = reinterpret_cast<double *>(sm_raw);
+    double *Wp = T + NB * DLT;            // [DP][DB][DLW]
+    double *Ls = Wp + DP * DB * DLW;      // [DB][DB] factor of the current 8 x 8 block, by rows
+    double *rd = Ls + DB * DB;            // [DB] 1 / its diagonal
+    int *flag = reinterpret_cast<int *>(rd + DB);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const double *blk = A + (long long)c0 * ld + c0;
+    if (w == NB && (ld & 1) == 0 && (c0 & 1) == 0) {
+        // 16-byte copies (the strict upper triangle comes along and is overwritten before it
+        // is read)
+#pragma unroll 4
+        for (int idx = tid; idx < NB * NB / 2; idx += BLK_THREADS) {
+            const int k = idx / (NB / 2), r = 2 * (idx - k * (NB / 2));
+            cp_async(T + k * DLT + r, blk + (long long)k * ld + r, 16, true);
+        }
+        cp_async_wait_all();
+    } else {
+#pragma unroll 4
+        for (int idx = tid; idx < NB * NB; idx += BLK_THREADS) {
+            const int k = idx / NB, r = idx - k * NB;
+            const bool v = r < w && k < w && r >= k;
+            cp_async(T + k * DLT + r, v ? blk + (long long)k * ld + r : blk, 8, v);
+        }
+        cp_async_wait_all();
+        __syncthreads();
+        for (int k = w + tid; k < NB; k += BLK_THREADS) T[k * DLT + k] = 1.0;
+    }
+    if (tid == 0) *flag = 0;
+    __syncthreads();
+
+    // phase A of panel p (warp 0)
+    auto factor = [&](int p) {
+        const int o = DB * p;
+        double a[DB][DB], rinv[DB];
+#pragma unroll
+        for (int c = 0; c < DB; ++c)
+#pragma unroll
+            for (int r = c; r < DB; ++r) a[r][c] = T[(o + c) * DLT + o + r];
+        const int bad = chol8(a, rinv);
+        if (o + bad < w && bad < DB) {
+            if (lane == 0) {
+                *info = c0 + o + bad + 1;
+                atomicExch(skip, 1);
+                *flag = 1;
+            }
+            return;
+        }
+        if (lane == 0) {
+#pragma unroll
+            for (int c = 0; c < DB; ++c) {
+                rd[c] = rinv[c];
+#pragma unroll
+                for (int r = c; r < DB; ++r) {
+                    Ls[r * DB + c] = a[r][c];
+                    T[(o + c) * DLT + o + r] = a[r][c];
+                }
+            }
+        }
+    };
+    if (warp == 0) factor(0);
+    for (int p = 0; p < DP; ++p) {
+        const int o = DB * p, below = NB - o - DB;
+        __syncthreads();
+        if (*flag) return;   // block-uniform after the barrier
+        // ---- B: rows below the panel's diagonal block, and its inverse
+        if (tid < below) {
+            double *x = T + o * DLT + o + DB + tid;
+            double v[DB];
+#pragma unroll
+            for (int c = 0; c < DB; ++c) v[c] = x[c * DLT];
+#pragma unroll
+            for (int c = 0; c < DB; ++c) {
+                v[c] *= rd[c];
+#pragma unroll
+                for (int k = c + 1; k < DB; ++k) v[k] = fma(-v[c], Ls[k * DB + c], v[k]);
+            }
+#pragma unroll
+            for (int c = 0; c < DB; ++c) x[c * DLT] = v[c];
+        } else if (warp == BLK_WARPS - 1 && lane < DB) {
+            // column `lane` of W_pp
+            double s[DB];
+#pragma unroll
+            for (int r = 0; r < DB; ++r) s[r] = r == lane ? 1.0 : 0.0;
+#pragma unroll
+            for (int r = 0; r < DB; ++r) {
+                s[r] *= rd[r];
+#pragma unroll
+                for (int k = r + 1; k < DB; ++k) s[k] = fma(-Ls[k * DB + r], s[r], s[k]);
+            }
+#pragma unroll
+            for (int r = 0; r < DB; ++r) Wp[(p * DB + r) * DLW + lane] = s[r];
+        }
+        __syncthreads();
+        // ---- C
+        if (warp == 0) {
+            if (p + 1 < DP) {
+                chol_tile(T, o, p + 1, p + 1, lane);
+                __syncwarp();
+                factor(p + 1);
+            }
+            continue;
+        }
+        // W row block p first (the longer chains): block column j to warp 1 + j
+        if (warp - 1 < p) {
+            const int j = warp - 1, i4 = lane >> 2, k4 = lane & 3;
+            double m0[2] = {0.0, 0.0}, m1[2] = {0.0, 0.0};
+            for (int k = j; k < p; ++k) {
+                // A = L_pk, B = W_kj, K = 8 in two steps
+                const double *l = T + (DB * k + k4) * DLT + o + i4;
+                const double *wk = k == j ? Wp + (DB * j + k4) * DLW + i4
+                                          : T + (DB * k + k4) * DLT + DB * j + i4;
+                const int ws = k == j ? DLW : DLT;
+                dmma(m0, l[0], wk[0]);
+                dmma(m1, l[4 * DLT], wk[4 * ws]);
+            }
+            m0[0] += m1[0];
+            m0[1] += m1[1];
+            // W_pj = -W_pp M: M from its accumulator lanes into B fragments
+            double d[2] = {0.0, 0.0};
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int src = (k4 + 4 * h) * 4 + (i4 >> 1);
+                const double e0 = __shfl_sync(FULL, m0[0], src), e1 = __shfl_sync(FULL, m0[1], src);
+                dmma(d, -Wp[(o + i4) * DLW + k4 + 4 * h], (i4 & 1) ? e1 : e0);
+            }
+            *reinterpret_cast<double2 *>(T + (o + i4) * DLT + DB * j + 2 * k4) =
+                make_double2(d[0], d[1]);
+        }
+        // trailing tiles but the next diagonal one, column by column
+        const int m = DP - 1 - p, ntile = m * (m + 1) / 2 - 1;
+        for (int t = BLK_WARPS - 1 - warp; t < ntile; t += BLK_WARPS - 1) {
+            // tile t + 1 of the triangle: columns q = 0 .. m - 1 of m - q tiles
+            int q = 0, left = t + 1;
+            while (left >= m - q) left -= m - q++;
+            chol_tile(T, o, p + 1 + q, p + 1 + q + left, lane);
+        }
+    }
+    __syncthreads();
+    double *ablk = A + (long long)c0 * ld + c0;
+    for (int idx = tid; idx < w * NB; idx += BLK_THREADS) {
+        const int k = idx / NB, r = idx - k * NB;
+        if (r < w && r >= k) ablk[(long long)k * ld + r] = T[k * DLT + r];
+    }
+    // W column-major, two rows per 16-byte store
+    for (int idx = tid; idx < NB * NB / 2; idx += BLK_THREADS) {
+        const int c = idx / (NB / 2), r = 2 * (idx - c * (NB / 2));
+        double v[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int rr = r + u;
+            v[u] = 0.0;
+            if (rr < w && c < w && rr >= c)
+                v[u] = rr / DB == c / DB ? Wp[rr * DLW + c % DB] : T[rr * DLT + c];
+        }
+        reinterpret_cast<double2 *>(Wout)[idx] = make_double2(v[0], v[1]);
+    }
+}
+
 // L_21 = A_21 W^T for rows r0 + 64 blockIdx.x ... of the panel (column c0 ..
 // c0 + 127), written over A_21, plus the S digit planes d[s][row][k] (kp =
 // NB) and row exponents of L_21 for the tensor-core trailing update.
 //
-// Shared memory: Ws[k * NB + c] = W[c][k] (= Wout, column-major W); Xs[k *
-// (PR + 1) + r] = A[row r][c0 + k], then the rows of L_21.
+// Products by FP64 mma.sync: warp v holds columns 8 v .. and 8 (15 - v) .. of
+// all 64 rows, so that every warp walks 17 blocks of W's triangle (on the FP64
+// units with 4 x 8 register tiles the kernel took 31 us for 5,000 rows, most of
+// it in shared-memory loads).
+//
+// Shared memory: Ws[k * LDP + c] = W[c][k] (= Wout, column-major W); Xs[k *
+// LDX + r] = A[row r][c0 + k], then the rows of L_21.
 template <int S>
 __global__ void __launch_bounds__(PANEL_THREADS)
     chol_panel_kernel(double *__restrict__ A, long long ld, int c0, int r0, int m,
@@ -372,13 +573,14 @@ __global__ void __launch_bounds__(PANEL_THREADS)
     if (*(volatile const int *)skip) return;
     extern __shared__ __align__(16) double sm[];
     double *Ws = sm;
-    double *Xs = sm + NB * NB;
-    constexpr int LDX = PR + 1;
-    const int tid = threadIdx.x;
+    double *Xs = sm + NB * LDP;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int rbase = blockIdx.x * PR;
 #pragma unroll 8
-    for (int idx = tid; idx < NB * NB / 2; idx += PANEL_THREADS)
-        cp_async(Ws + 2 * idx, Wout + 2 * idx, 16, true);
+    for (int idx = tid; idx < NB * NB / 2; idx += PANEL_THREADS) {
+        const int k = idx / (NB / 2), c = 2 * (idx - k * (NB / 2));
+        cp_async(Ws + k * LDP + c, Wout + 2 * idx, 16, true);
+    }
     const double *arows = A + (long long)c0 * ld + r0 + rbase;
 #pragma unroll 8
     for (int idx = tid; idx < NB * PR; idx += PANEL_THREADS) {
@@ -388,42 +590,45 @@ __global__ void __launch_bounds__(PANEL_THREADS)
     }
     cp_async_wait_all();
     __syncthreads();
-    // thread tile: rows 4 rg .. 4 rg + 3, columns 8 cg .. 8 cg + 7
-    const int rg = tid & 15, cg = tid >> 4;
-    double acc[4][8];
+    static_assert(PANEL_THREADS / 32 == NB / 16 && PR == 64, "two column tiles a warp");
+    const int t0 = warp, t1 = NB / 8 - 1 - warp;   // column tiles, t0 < t1
+    double acc[2][PR / 8][2];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int h = 0; h < 2; ++h)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = 0.0;
-    const int kmax = 8 * cg + 8;   // W[c][k] = 0 for k > c
-    for (int k = 0; k < kmax; ++k) {
-        double a[4], b[8];
+        for (int i = 0; i < PR / 8; ++i) acc[h][i][0] = acc[h][i][1] = 0.0;
+    {
+        const int i4 = lane >> 2, k4 = lane & 3;
+        const double *xk = Xs + k4 * LDX + i4, *wk = Ws + k4 * LDP + i4;
+        // W[c][k] = 0 for k > c
+        for (int k = 0; k < 8 * (t1 + 1); k += 4, xk += 4 * LDX, wk += 4 * LDP) {
+            const double b1 = wk[8 * t1];
+            double x[PR / 8];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) a[i] = Xs[k * LDX + 4 * rg + i];
-        const double2 *wv = reinterpret_cast<const double2 *>(Ws + k * NB + 8 * cg);
+            for (int i = 0; i < PR / 8; ++i) x[i] = xk[8 * i];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const double2 t = wv[j];
-            b[2 * j] = t.x;
-            b[2 * j + 1] = t.y;
+            for (int i = 0; i < PR / 8; ++i) dmma(acc[1][i], x[i], b1);
+            if (k < 8 * (t0 + 1)) {
+                const double b0 = wk[8 * t0];
+#pragma unroll
+                for (int i = 0; i < PR / 8; ++i) dmma(acc[0][i], x[i], b0);
+            }
         }
+        __syncthreads();   // every warp is past its loads of the rows
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int h = 0; h < 2; ++h)
 #pragma unroll
-            for (int j = 0; j < 8; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
+            for (int i = 0; i < PR / 8; ++i)
+#pragma unroll
+                for (int u = 0; u < 2; ++u)
+                    Xs[(8 * (h ? t1 : t0) + 2 * k4 + u) * LDX + 8 * i + i4] = acc[h][i][u];
     }
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) Xs[(8 * cg + j) * LDX + 4 * rg + i] = acc[i][j];
     __syncthreads();
     for (int idx = tid; idx < NB * PR; idx += PANEL_THREADS) {
         const int c = idx / PR, r = idx - c * PR;
         if (rbase + r < m) A[(long long)(c0 + c) * ld + r0 + rbase + r] = Xs[c * LDX + r];
     }
     // digit planes: a warp per row, lane l holds columns l, l + 32, l + 64, l + 96
-    const int warp = tid >> 5, lane = tid & 31;
     const long long plane = (long long)m * NB;
     for (int rl = warp; rl < PR; rl += PANEL_THREADS / 32) {
         const int row = rbase + rl;
@@ -481,11 +686,12 @@ kfb_status panel(int S, double *A, long long ld, int c0, int r0, int m, const do
 
 namespace {
 
-// The two streams of the look-ahead, per device: the critical path (diagonal
-// blocks, panels, the updates the next panel waits for) at the highest
-// priority, the bulk trailing updates at the lowest.
+// The streams of the look-ahead, per device: the critical path (diagonal
+// blocks, panels, the updates the next block waits for) at the highest
+// priority, the rest of the inner updates below it, the bulk trailing updates
+// at the lowest.
 struct CholStreams {
-    cudaStream_t crit = nullptr, bulk = nullptr;
+    cudaStream_t crit = nullptr, inner = nullptr, bulk = nullptr;
 };
 
 kfb_status chol_streams(CholStreams *&out) {
@@ -498,6 +704,8 @@ kfb_status chol_streams(CholStreams *&out) {
         int least = 0, greatest = 0;
         KFB_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&least, &greatest));
         KFB_CUDA_TRY(cudaStreamCreateWithPriority(&cs.crit, cudaStreamNonBlocking, greatest));
+        KFB_CUDA_TRY(cudaStreamCreateWithPriority(&cs.inner, cudaStreamNonBlocking,
+                                                  std::min(greatest + 1, least)));
         KFB_CUDA_TRY(cudaStreamCreateWithPriority(&cs.bulk, cudaStreamNonBlocking, least));
     }
     out = &cs;
@@ -506,7 +714,7 @@ kfb_status chol_streams(CholStreams *&out) {
 
 // Events of one factorisation, destroyed with it.
 struct CholEvents {
-    cudaEvent_t ev[6] = {};
+    cudaEvent_t ev[8] = {};
     kfb_status init() {
         for (auto &e : ev) KFB_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         return KFB_OK;
@@ -527,23 +735,23 @@ kfb_status chol_dense(double *A, int n, long long ld, int slices, int *info, cud
                          OZ_MAXS);
     static bool attr = false;
     if (!attr) {
-        KFB_CUDA_TRY(cudaFuncSetAttribute(chol_block_kernel<double>,
+        KFB_CUDA_TRY(cudaFuncSetAttribute(chol_block64_kernel,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)blk_smem<double>()));
-        KFB_CUDA_TRY(cudaFuncSetAttribute(chol_block_kernel<float>,
+                                          (int)DBLK_SMEM));
+        KFB_CUDA_TRY(cudaFuncSetAttribute(chol_block_kernel,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)blk_smem<float>()));
+                                          (int)BLK_SMEM));
         attr = true;
     }
     // the diagonal blocks in FP32 for an FP32-class factor (4 or fewer planes)
     const bool f32blk = slices <= 4;
     CholStreams *cs = nullptr;
     KFB_TRY(chol_streams(cs));
-    const cudaStream_t sc = cs->crit, sb = cs->bulk;
+    const cudaStream_t sc = cs->crit, si = cs->inner, sb = cs->bulk;
     CholEvents E;
     KFB_TRY(E.init());
     cudaEvent_t ev_start = E.ev[0], ev_slice = E.ev[1], ev_bulk = E.ev[2], ev_crit_end = E.ev[3],
-                ev_bulk_end = E.ev[4];
+                ev_bulk_end = E.ev[4], ev_panel = E.ev[5], ev_inner = E.ev[6];
     // everything below is ordered after the caller's work on s
     KFB_CUDA_TRY(cudaEventRecord(ev_start, s));
     KFB_CUDA_TRY(cudaStreamWaitEvent(sc, ev_start, 0));
@@ -562,18 +770,19 @@ kfb_status chol_dense(double *A, int n, long long ld, int slices, int *info, cud
             KFB_TRY(osl[b].alloc((size_t)slices * (n - NB2) * NB2, sc));
             KFB_TRY(oex[b].alloc((size_t)(n - NB2) * sizeof(int), sc));
         }
-    // on an early (error) return, let both streams finish before the buffers
+    // on an early (error) return, let the streams finish before the buffers
     // above are released (destroyed after this guard)
     struct Drain {
-        cudaStream_t a, b;
+        cudaStream_t a, b, c;
         bool armed = true;
         ~Drain() {
             if (armed) {
                 cudaStreamSynchronize(a);
                 cudaStreamSynchronize(b);
+                cudaStreamSynchronize(c);
             }
         }
-    } drain{sc, sb};
+    } drain{sc, si, sb};
     // the bulk stream's first work reads buffers allocated on the critical one
     KFB_CUDA_TRY(cudaEventRecord(ev_slice, sc));
     KFB_CUDA_TRY(cudaStreamWaitEvent(sb, ev_slice, 0));
@@ -587,18 +796,24 @@ kfb_status chol_dense(double *A, int n, long long ld, int slices, int *info, cud
     OzEpi epi_bulk = epi;
     epi_bulk.one_tile_per_cta = 1;
     bool bulk_pending = false;   // a bulk update was enqueued and not waited for
+    bool inner_pending = false;  // the rest of an inner update, likewise
     for (int o0 = 0, P = 0; o0 < n; o0 += NB2, ++P) {
         const int ow = std::min(NB2, n - o0);   // outer panel: columns o0 .. o0 + ow - 1
         for (int c0 = o0; c0 < o0 + ow; c0 += NB) {
             const int w = std::min(NB, n - c0);
             const int r0 = c0 + w, m = n - r0;
             if (f32blk)
-                chol_block_kernel<float><<<1, BLK_THREADS, blk_smem<float>(), sc>>>(
+                chol_block_kernel<<<1, BLK_THREADS, BLK_SMEM, sc>>>(
                     A, ld, c0, w, Wd.as<double>(), d_info, d_skip);
             else
-                chol_block_kernel<double><<<1, BLK_THREADS, blk_smem<double>(), sc>>>(
+                chol_block64_kernel<<<1, BLK_THREADS, DBLK_SMEM, sc>>>(
                     A, ld, c0, w, Wd.as<double>(), d_info, d_skip);
             KFB_CUDA_TRY(cudaGetLastError());
+            // (the block itself was updated ahead of the rest of its columns)
+            if (inner_pending) {
+                KFB_CUDA_TRY(cudaStreamWaitEvent(sc, ev_inner, 0));
+                inner_pending = false;
+            }
             if (m == 0) break;
             // L21 = A21 W^T and its digit planes
             KFB_TRY(panel(slices, A, ld, c0, r0, m, Wd.as<double>(), psl.as<int8_t>(),
@@ -618,7 +833,20 @@ kfb_status chol_dense(double *A, int n, long long ld, int slices, int *info, cud
                 g.M = m;
                 g.N = nin;
                 g.c_off = (long long)r0 * ld + r0;
+                // the next diagonal block first (its row of tiles), then the
+                // rest beside that block's factorisation
+                const int all = oz_gen_tiles(g, slices);
+                g.count = std::min(all, (std::min(NB, nin) + oz_bn(slices) - 1) / oz_bn(slices));
+                KFB_CUDA_TRY(cudaEventRecord(ev_panel, sc));
                 KFB_TRY(oz_gemm_gen(Pl, Pl, g, epi, d_err, sc));
+                if (all > g.count) {
+                    KFB_CUDA_TRY(cudaStreamWaitEvent(si, ev_panel, 0));
+                    g.first = g.count;
+                    g.count = all - g.first;
+                    KFB_TRY(oz_gemm_gen(Pl, Pl, g, epi_bulk, d_err, si));
+                    KFB_CUDA_TRY(cudaEventRecord(ev_inner, si));
+                    inner_pending = true;
+                }
             }
         }
         // everything right of the outer panel -= L_panel L_panel^T (K = ow, the

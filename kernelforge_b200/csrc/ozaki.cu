@@ -85,6 +85,7 @@ __host__ __device__ __forceinline__ int lower_tiles(int ti, int ntc, int BN) {
 __host__ __device__ __forceinline__ OzTile gen_tile(const OzGen &g, int BN, long long ldr,
                                                     long long ldc, int t) {
     const int ntc = (g.N + BN - 1) / BN;
+    t += g.first;
     int ti = 0, tj = t;
     if (g.mode == OZ_GEN_LOWER) {
         while (true) {
@@ -679,7 +680,8 @@ kfb_status oz_gemm(const OzSlices &A, const OzSlices &B, const OzTile *tiles, in
 
 kfb_status oz_gemm_gen(const OzSlices &A, const OzSlices &B, const OzGen &g, const OzEpi &epi,
                        int *err, cudaStream_t s) {
-    return oz_gemm_core(A, B, nullptr, g, oz_gen_tiles(g, A.S), epi, err, s);
+    return oz_gemm_core(A, B, nullptr, g, g.count >= 0 ? g.count : oz_gen_tiles(g, A.S), epi, err,
+                        s);
 }
 
 kfb_status oz_gemm_dense(const OzSlices &A, const OzSlices &B, int M, int N, const OzEpi &epi,

@@ -100,7 +100,9 @@ struct OzGen {
     int M = 0, N = 0;
     int a_base = 0, b_base = 0;
     long long c_off = 0;
+    int first = 0, count = -1;   // tiles first .. first + count - 1 of the set (-1: all)
 };
+// tiles of the whole set
 int oz_gen_tiles(const OzGen &g, int S);
 kfb_status oz_gemm_gen(const OzSlices &A, const OzSlices &B, const OzGen &g, const OzEpi &epi,
                        int *err, cudaStream_t s);

@@ -78,6 +78,29 @@ def test_rfp_potrf_potrs_match_lapack(n, uplo, dtype):
     np.testing.assert_allclose(A @ B.cpu().numpy().ravel(), b, rtol=50 * tol, atol=50 * tol)
 
 
+@pytest.mark.parametrize("n", [9, 119, 127, 128, 129, 255, 384, 511, 513, 641, 705])
+def test_potrf_block_edges(n):
+    """Diagonal blocks around the 8-column micro-panels, the 128-column blocks and the 512-column
+    outer panels (partial last blocks, the inner update split after its first row of tiles): the
+    FP64 factor against LAPACK, and the index of a pivot made negative in the first, a middle and
+    the last micro-panel."""
+    import torch
+
+    from kernelforge_b200 import cuda_global_kernels as cgk
+    A = spd(n, n + 5, cond=50.0)
+    arf, _ = lapack.dtrttf(np.asfortranarray(A), transr="N", uplo="L")
+    ref, _ = lapack.dpftrf(n, (arf + 0.0).copy(), transr="N", uplo="L")
+    K = torch.tensor(arf, dtype=torch.float64, device="cuda")
+    assert cgk.rfp_potrf(K, n, 0.0, "L") == 0
+    np.testing.assert_allclose(K.cpu().numpy(), ref, rtol=1e-11, atol=1e-11)
+    for k in sorted({0, 7, 8, n // 2, max(n - 9, 0), n - 1} & set(range(n))):
+        B = A.copy()
+        B[k, k] = -1.0
+        arf, _ = lapack.dtrttf(np.asfortranarray(B), transr="N", uplo="L")
+        K = torch.tensor(arf, dtype=torch.float64, device="cuda")
+        assert cgk.rfp_potrf(K, n, 0.0, "L") == k + 1
+
+
 def test_rfp_potrf_reports_info():
     import torch
 
