@@ -40,7 +40,7 @@ struct kfb_cosmlp {
     kfb::DevBuf grad[4];         // gradients of the last step (one element)
     std::vector<int> steps;      // Adam step count per element
     // batch workspace (2 Bp rows, Bp = max_pairs rounded up to 8)
-    kfb::DevBuf idx, xb, xbt, z1, hb, hbt, z2, dz2, dz2t, dz1t, loss, err;
+    kfb::DevBuf xb, xbt, z1, hb, hbt, z2, factor, dz2, dz2t, dz1t, loss, err;
 };
 
 namespace kfb {
@@ -52,12 +52,16 @@ constexpr float ADAM_B1 = 0.9f, ADAM_B2 = 0.999f, ADAM_EPS = 1e-8f;
 long long ru8(long long v) { return (v + 7) / 8 * 8; }
 unsigned nblk(long long n, int b) { return (unsigned)std::max<long long>(1, (n + b - 1) / b); }
 
-// out[r][c] = bf16(x[idx[r]][c]) (zero row for idx < 0; idx >= nsrc gives a
-// zero row and raises *bad); optionally also the transpose out_t[c * ld_t + r],
+// out[r][c] = bf16(x[a][c]) for a = idx[r], or with idx2 (a pair batch of
+// npairs) idx[r] for r < npairs, idx2[r - nrows / 2] for the first npairs rows
+// of the second half, and no row between; a zero row for a < 0, a zero row and
+// *bad raised for a >= nsrc; optionally also the transpose out_t[c * ld_t + r],
 // through a 32 x 32 shared-memory tile.
 template <class T>
 __global__ void gather_rows_bf16_kernel(const T *__restrict__ x, long long nsrc,
-                                        const int *__restrict__ idx, int nrows, int rep,
+                                        const int *__restrict__ idx,
+                                        const int *__restrict__ idx2, int npairs, int nrows,
+                                        int rep,
                                         bf16 *__restrict__ out, bf16 *__restrict__ out_t,
                                         long long ld_t, int *bad) {
     __shared__ float tile[32][33];
@@ -66,7 +70,13 @@ __global__ void gather_rows_bf16_kernel(const T *__restrict__ x, long long nsrc,
         const int r = r0 + rr, c = c0 + threadIdx.x;
         float v = 0.f;
         if (r < nrows && c < rep) {
-            const int a = idx[r];
+            int a;
+            if (!idx2) {
+                a = idx[r];
+            } else {
+                const int half = nrows / 2, p = r < half ? r : r - half;
+                a = p < npairs ? (r < half ? idx[p] : idx2[p]) : -1;
+            }
             if (a >= nsrc) {
                 if (bad) atomicExch(bad, 1);  // index outside x: zero row, reported
             } else if (a >= 0) {
@@ -235,82 +245,133 @@ __device__ __forceinline__ void sincos_reduced(float x, float &sn, float &cs) {
 // of z2 are the two atoms of pair p.  With s2 = 2 / D:
 //   k_p = s2 sum_d cos z_i[d] cos z_j[d],  r_p = k_p - t_p,  loss += r_p^2
 //   dZ2_i[d] = -(2 r_p / npairs) s2 cos z_j[d] sin z_i[d]   (and i <-> j)
-// Padded pairs (p >= npairs) get zero gradient rows.  One block of 256
-// threads per pair; each thread keeps its float4 slices of both rows in
-// registers between the dot product and the gradient (D <= 256 * 4 * VPT).
-constexpr int PL_THREADS = 256, PL_VPT = 4;
-__global__ void __launch_bounds__(PL_THREADS)
-    pair_loss_kernel(const float *__restrict__ z2, int Bp, int npairs, int D,
-                     const float *__restrict__ target, float s2, float gscale,
-                     bf16 *__restrict__ dz2, double *__restrict__ loss) {
-    const int p = blockIdx.x;
-    const float4 *zi = reinterpret_cast<const float4 *>(z2 + (size_t)p * D);
-    const float4 *zj = reinterpret_cast<const float4 *>(z2 + (size_t)(p + Bp) * D);
-    uint2 *di = reinterpret_cast<uint2 *>(dz2 + (size_t)p * D);
-    uint2 *dj = reinterpret_cast<uint2 *>(dz2 + (size_t)(p + Bp) * D);
-    const int n4 = D / 4;
-    if (p >= npairs) {
-        for (int k = threadIdx.x; k < n4; k += PL_THREADS) {
-            di[k] = make_uint2(0u, 0u);
-            dj[k] = make_uint2(0u, 0u);
-        }
-        return;
-    }
-    // sin / cos of both rows once, kept in registers between the dot product
-    // and the gradient
-    float si[PL_VPT][4], ci[PL_VPT][4], sj[PL_VPT][4], cj[PL_VPT][4];
-    float acc = 0.f;
-#pragma unroll
-    for (int u = 0; u < PL_VPT; ++u) {
-        const int k = threadIdx.x + u * PL_THREADS;
-        if (k < n4) {
+// Padded pairs (p >= npairs) get zero gradient rows.
+//
+// Two passes over z2: the dot products (a warp per pair; factor[p] = (2 r_p /
+// npairs) s2), then the gradients by tiles of 64 pairs x 64 columns, written by
+// rows and, through shared memory, transposed (dz2t, row length 2 Bp), with
+// their column sums (db2, cleared by the caller).  Both are bound by HBM; a
+// transpose pass that reads dZ2 back moves as much and more (50 + 48 us for
+// 8,192 rows of 4,096), and 8- or 16-byte pieces of the transpose written
+// straight from a block of few pairs took 110 us.
+constexpr int PL_MAX_D = 4096;
+__global__ void __launch_bounds__(256)
+    pair_dot_kernel(const float *__restrict__ z2, int Bp, int npairs, int D,
+                    const float *__restrict__ target, float s2, float gscale,
+                    float *__restrict__ factor, double *__restrict__ loss) {
+    const int p = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (p >= Bp) return;
+    float t = 0.f;
+    if (p < npairs) {
+        const float4 *zi = reinterpret_cast<const float4 *>(z2 + (size_t)p * D);
+        const float4 *zj = reinterpret_cast<const float4 *>(z2 + (size_t)(p + Bp) * D);
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+        for (int k = lane; k < D / 4; k += 32) {
             const float4 a = zi[k], b = zj[k];
             const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-                sincos_reduced(av[c], si[u][c], ci[u][c]);
-                sincos_reduced(bv[c], sj[u][c], cj[u][c]);
-                acc = fmaf(ci[u][c], cj[u][c], acc);
+                float sa, ca, sb, cb;
+                sincos_reduced(av[c], sa, ca);
+                sincos_reduced(bv[c], sb, cb);
+                acc[c] = fmaf(ca, cb, acc[c]);
             }
         }
+        t = (acc[0] + acc[1]) + (acc[2] + acc[3]);
     }
-    __shared__ float red[PL_THREADS / 32];
-    for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    float tot = 0.f;
-#pragma unroll
-    for (int w = 0; w < PL_THREADS / 32; ++w) tot += red[w];
-    const float r = s2 * tot - target[p];
-    if (threadIdx.x == 0) atomicAdd(loss, (double)r * (double)r);
-    const float g = gscale * r * s2;
-#pragma unroll
-    for (int u = 0; u < PL_VPT; ++u) {
-        const int k = threadIdx.x + u * PL_THREADS;
-        if (k < n4) {
-            const __nv_bfloat162 x01 = __floats2bfloat162_rn(-g * cj[u][0] * si[u][0],
-                                                             -g * cj[u][1] * si[u][1]);
-            const __nv_bfloat162 x23 = __floats2bfloat162_rn(-g * cj[u][2] * si[u][2],
-                                                             -g * cj[u][3] * si[u][3]);
-            const __nv_bfloat162 y01 = __floats2bfloat162_rn(-g * ci[u][0] * sj[u][0],
-                                                             -g * ci[u][1] * sj[u][1]);
-            const __nv_bfloat162 y23 = __floats2bfloat162_rn(-g * ci[u][2] * sj[u][2],
-                                                             -g * ci[u][3] * sj[u][3]);
-            di[k] = make_uint2(*reinterpret_cast<const uint32_t *>(&x01),
-                               *reinterpret_cast<const uint32_t *>(&x23));
-            dj[k] = make_uint2(*reinterpret_cast<const uint32_t *>(&y01),
-                               *reinterpret_cast<const uint32_t *>(&y23));
+    for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane == 0) {
+        float f = 0.f;
+        if (p < npairs) {
+            const float r = s2 * t - target[p];
+            atomicAdd(loss, (double)r * (double)r);
+            f = gscale * r * s2;
         }
+        factor[p] = f;
     }
 }
 
-// Adam on one parameter tensor (n values), refreshing its BF16 copy (pb)
-// when given.
-__global__ void adam_kernel(float *__restrict__ p, const float *__restrict__ g,
-                            float *__restrict__ m, float *__restrict__ v, long long n, float lr,
-                            float bc1, float bc2, bf16 *__restrict__ pb) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-         i += (long long)gridDim.x * blockDim.x) {
+constexpr int PG_T = 64;   // pairs and columns of a tile
+__global__ void __launch_bounds__(256)
+    pair_grad_kernel(const float *__restrict__ z2, int Bp, int npairs, int D,
+                     const float *__restrict__ factor, bf16 *__restrict__ dz2,
+                     bf16 *__restrict__ dz2t, float *__restrict__ db2) {
+    // [half][column][pair]; rows of 66 (33 words): columns go in and come out
+    // without bank conflicts
+    __shared__ __align__(4) bf16 tile[2][PG_T][PG_T + 2];
+    const int p0 = blockIdx.y * PG_T, c0 = blockIdx.x * PG_T;
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;   // 4 columns, pairs ty, ty + 16, ..
+    const int c = c0 + 4 * tx;
+#pragma unroll
+    for (int h = 0; h < PG_T / 16; ++h) {
+        const int q = ty + 16 * h, p = p0 + q;
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+        float f = 0.f;
+        if (p < npairs && c < D) {   // D is a multiple of 8
+            a = *reinterpret_cast<const float4 *>(z2 + (size_t)p * D + c);
+            b = *reinterpret_cast<const float4 *>(z2 + (size_t)(p + Bp) * D + c);
+            f = factor[p];
+        }
+        const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+        bf16 gi[4], gj[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            float sa, ca, sb, cb;
+            sincos_reduced(av[u], sa, ca);
+            sincos_reduced(bv[u], sb, cb);
+            gi[u] = __float2bfloat16_rn(-f * cb * sa);
+            gj[u] = __float2bfloat16_rn(-f * ca * sb);
+            tile[0][4 * tx + u][q] = gi[u];
+            tile[1][4 * tx + u][q] = gj[u];
+        }
+        if (p < Bp && c < D) {
+            const __nv_bfloat162 w[4] = {{gi[0], gi[1]}, {gi[2], gi[3]}, {gj[0], gj[1]},
+                                         {gj[2], gj[3]}};
+            *reinterpret_cast<uint2 *>(dz2 + (size_t)p * D + c) =
+                *reinterpret_cast<const uint2 *>(w);
+            *reinterpret_cast<uint2 *>(dz2 + (size_t)(p + Bp) * D + c) =
+                *reinterpret_cast<const uint2 *>(w + 2);
+        }
+    }
+    __syncthreads();
+    // a warp per column: 64 pairs of each half, two per lane (Bp is a multiple of 8)
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int cc = warp; cc < PG_T && c0 + cc < D; cc += 8) {
+        float t = 0.f;
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            const __nv_bfloat162 v =
+                *reinterpret_cast<const __nv_bfloat162 *>(&tile[half][cc][2 * lane]);
+            t += __low2float(v) + __high2float(v);
+            if (p0 + 2 * lane < Bp)
+                *reinterpret_cast<__nv_bfloat162 *>(dz2t + (size_t)(c0 + cc) * 2 * Bp +
+                                                    (size_t)half * Bp + p0 + 2 * lane) = v;
+        }
+        for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0) atomicAdd(db2 + c0 + cc, t);
+    }
+}
+
+// Adam on the parameter tensors of an element in one launch, refreshing their
+// BF16 copies (pb) where given; block b works on tensor k with first[k] <= b.
+struct AdamSet {
+    float *p[4], *m[4], *v[4];
+    const float *g[4];
+    bf16 *pb[4];
+    long long n[4];
+    int first[5];
+};
+__global__ void __launch_bounds__(256) adam_kernel(const __grid_constant__ AdamSet a, float lr,
+                                                   float bc1, float bc2) {
+    int k = 0;
+    while (k < 3 && (int)blockIdx.x >= a.first[k + 1]) ++k;
+    float *p = a.p[k], *m = a.m[k], *v = a.v[k];
+    const float *g = a.g[k];
+    bf16 *pb = a.pb[k];
+    const long long n = a.n[k], step = (long long)(a.first[k + 1] - a.first[k]) * blockDim.x;
+    for (long long i = (blockIdx.x - a.first[k]) * (long long)blockDim.x + threadIdx.x; i < n;
+         i += step) {
         const float gi = g[i];
         const float mi = ADAM_B1 * m[i] + (1.f - ADAM_B1) * gi;
         const float vi = ADAM_B2 * v[i] + (1.f - ADAM_B2) * gi * gi;
@@ -758,8 +819,8 @@ kfb_status cosmlp_features_t(kfb_cosmlp *h, const T *x, const int *q, const int 
         for (int r0 = 0; r0 < ne; r0 += chunk) {
             const int nr = std::min(chunk, ne - r0);
             gather_rows_bf16_kernel<T><<<dim3(nblk(rep, 32), nblk(nr, 32)), dim3(32, 8), 0, s>>>(
-                x, (long long)nm * ma, didx.as<int>() + r0, nr, rep, xb.as<bf16>(), nullptr, 0,
-                nullptr);
+                x, (long long)nm * ma, didx.as<int>() + r0, nullptr, 0, nr, rep, xb.as<bf16>(),
+                nullptr, 0, nullptr);
             KFB_CUDA_TRY(cudaGetLastError());
             TcOperand A, B;
             A.hi = xb.ptr;
@@ -813,19 +874,12 @@ kfb_status cosmlp_step_t(kfb_cosmlp *h, int e, const T *x, long long nrows, cons
     const int rep = h->rep, H = h->hidden, D = h->d;
     const int Bp = (int)ru8(npairs);
     const int R = 2 * Bp;  // batch rows: i-atoms then j-atoms
-    int *err = h->err.as<int>();
-    KFB_TRY(zero(err, sizeof(int), s));
+    int *err = h->err.as<int>(), *bad = err + 1;
+    KFB_TRY(zero(err, 2 * sizeof(int), s));
     KFB_TRY(zero(h->loss.ptr, sizeof(double), s));
-    // batch row indices: pi, padding, pj, padding
-    int *idx = h->idx.as<int>();
-    KFB_CUDA_TRY(cudaMemsetAsync(idx, 0xff, (size_t)R * sizeof(int), s));
-    KFB_CUDA_TRY(cudaMemcpyAsync(idx, pi, (size_t)npairs * sizeof(int), cudaMemcpyDeviceToDevice, s));
-    KFB_CUDA_TRY(cudaMemcpyAsync(idx + Bp, pj, (size_t)npairs * sizeof(int),
-                                 cudaMemcpyDeviceToDevice, s));
-    int *bad = h->err.as<int>() + 1;
-    KFB_TRY(zero(bad, sizeof(int), s));
+    // batch rows: pi, padding, pj, padding
     gather_rows_bf16_kernel<T><<<dim3(nblk(rep, 32), nblk(R, 32)), dim3(32, 8), 0, s>>>(
-        x, nrows, idx, R, rep, h->xb.as<bf16>(), h->xbt.as<bf16>(), R, bad);
+        x, nrows, pi, pj, npairs, R, rep, h->xb.as<bf16>(), h->xbt.as<bf16>(), R, bad);
     KFB_CUDA_TRY(cudaGetLastError());
     // forward, layer 1: z1 = X W1^T + b1, h = cos z1 (rows and transposed)
     {
@@ -876,12 +930,14 @@ kfb_status cosmlp_step_t(kfb_cosmlp *h, int e, const T *x, long long nrows, cons
     }
     float *gw1 = h->grad[0].as<float>(), *gb1 = h->grad[1].as<float>();
     float *gw2 = h->grad[2].as<float>(), *gb2 = h->grad[3].as<float>();
-    pair_loss_kernel<<<Bp, PL_THREADS, 0, s>>>(h->z2.as<float>(), Bp, npairs, D, target,
-                                               2.f / (float)D, 2.f / (float)npairs,
-                                               h->dz2.as<bf16>(), h->loss.as<double>());
-    KFB_CUDA_TRY(cudaGetLastError());
     KFB_TRY(zero(gb2, (size_t)D * sizeof(float), s));
-    KFB_TRY(transpose_bf16(h->dz2.as<bf16>(), R, D, h->dz2t.as<bf16>(), R, gb2, s));
+    pair_dot_kernel<<<nblk(Bp, 8), 256, 0, s>>>(h->z2.as<float>(), Bp, npairs, D, target,
+                                                2.f / (float)D, 2.f / (float)npairs,
+                                                h->factor.as<float>(), h->loss.as<double>());
+    pair_grad_kernel<<<dim3(nblk(D, PG_T), nblk(Bp, PG_T)), 256, 0, s>>>(
+        h->z2.as<float>(), Bp, npairs, D, h->factor.as<float>(), h->dz2.as<bf16>(),
+        h->dz2t.as<bf16>(), gb2);
+    KFB_CUDA_TRY(cudaGetLastError());
     // dW2 = dZ2^T H  (D x H, contraction over the batch rows)
     {
         TcOperand A, B;
@@ -974,15 +1030,22 @@ kfb_status cosmlp_step_t(kfb_cosmlp *h, int e, const T *x, long long nrows, cons
              h->w2tb.as<bf16>() + (size_t)e * H * D},
             {&h->b2, 3, 1, D, nullptr, nullptr},
         };
-        for (const P &q : ps) {
+        AdamSet as{};
+        for (int k = 0; k < 4; ++k) {
+            const P &q = ps[k];
             const size_t off = (size_t)e * q.rows * q.cols;
-            const long long n = (long long)q.rows * q.cols;
-            adam_kernel<<<nblk(n, 256 * 4), 256, 0, s>>>(
-                q.p->as<float>() + off, h->grad[q.k].as<float>(), h->mom[q.k].as<float>() + off,
-                h->var[q.k].as<float>() + off, n, lr, bc1, bc2, q.pb);
-            KFB_CUDA_TRY(cudaGetLastError());
-            if (q.pbt) KFB_TRY(transpose_bf16(q.pb, q.rows, q.cols, q.pbt, q.rows, nullptr, s));
+            as.n[k] = (long long)q.rows * q.cols;
+            as.p[k] = q.p->as<float>() + off;
+            as.g[k] = h->grad[q.k].as<float>();
+            as.m[k] = h->mom[q.k].as<float>() + off;
+            as.v[k] = h->var[q.k].as<float>() + off;
+            as.pb[k] = q.pb;
+            as.first[k + 1] = as.first[k] + (int)nblk(as.n[k], 256 * 4);
         }
+        adam_kernel<<<as.first[4], 256, 0, s>>>(as, lr, bc1, bc2);
+        KFB_CUDA_TRY(cudaGetLastError());
+        for (const P &q : ps)
+            if (q.pbt) KFB_TRY(transpose_bf16(q.pb, q.rows, q.cols, q.pbt, q.rows, nullptr, s));
     }
     int herr[2] = {0, 0};
     double lsum = 0.0;
@@ -1099,8 +1162,8 @@ kfb_status kfb_cosmlp_create(int nelem, int rep, int hidden, int d, int max_pair
         if (rep % 16 != 0 || hidden % 16 != 0 || d % 16 != 0)
             return set_error(KFB_ERR_UNSUPPORTED,
                              "cos-MLP: rep, hidden and D must be multiples of 16");
-        if (d > PL_THREADS * 4 * PL_VPT)
-            return set_error(KFB_ERR_UNSUPPORTED, "cos-MLP: D up to %d", PL_THREADS * 4 * PL_VPT);
+        if (d > PL_MAX_D)
+            return set_error(KFB_ERR_UNSUPPORTED, "cos-MLP: D up to %d", PL_MAX_D);
         if (!device_is_sm100())
             return set_error(KFB_ERR_UNSUPPORTED, "cos-MLP needs an sm_100 (B200) device");
         auto *h = new kfb_cosmlp();
@@ -1135,13 +1198,13 @@ kfb_status kfb_cosmlp_create(int nelem, int rep, int hidden, int d, int max_pair
                  KFB_TRY(h->w2b.alloc(n2 * sizeof(bf16), s));
                  KFB_TRY(h->w2tb.alloc(n2 * sizeof(bf16), s));
                  const long long R = 2 * ru8(max_pairs);
-                 KFB_TRY(h->idx.alloc((size_t)R * sizeof(int), s));
                  KFB_TRY(h->xb.alloc((size_t)R * rep * sizeof(bf16), s));
                  KFB_TRY(h->xbt.alloc((size_t)R * rep * sizeof(bf16), s));
                  KFB_TRY(h->z1.alloc((size_t)R * hidden * sizeof(float), s));
                  KFB_TRY(h->hb.alloc((size_t)R * hidden * sizeof(bf16), s));
                  KFB_TRY(h->hbt.alloc((size_t)R * hidden * sizeof(bf16), s));
                  KFB_TRY(h->z2.alloc((size_t)R * d * sizeof(float), s));
+                 KFB_TRY(h->factor.alloc((size_t)R / 2 * sizeof(float), s));
                  KFB_TRY(h->dz2.alloc((size_t)R * d * sizeof(bf16), s));
                  KFB_TRY(h->dz2t.alloc((size_t)R * d * sizeof(bf16), s));
                  KFB_TRY(h->dz1t.alloc((size_t)R * hidden * sizeof(bf16), s));

@@ -100,6 +100,15 @@ __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, int *err
     }
 }
 
+// The problem list of a launch with few problems, passed with the kernel's
+// arguments: two uploads from pageable memory and their buffers cost more than
+// such a launch (the learned map's training step has five of them).
+constexpr int MAXP_ARG = 8;
+struct ArgProbs {
+    TcProb p[MAXP_ARG];
+    int tstart[MAXP_ARG + 1];
+};
+
 // Tile t of the launch: problems own consecutive tile ranges starting at
 // tstart[p] (tstart[nprobs] = all tiles), row blocks outer, column blocks
 // inner.  The largest p with tstart[p] <= t owns t (empty problems share their
@@ -130,8 +139,8 @@ template <int NPROD, int NEPI, int BNT>
 __global__ void __launch_bounds__(Cfg<NPROD, NEPI, BNT>::THREADS, 1)
     tc_gemm_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant__ CUtensorMap ta_lo,
                    const __grid_constant__ CUtensorMap tb_hi, const __grid_constant__ CUtensorMap tb_lo,
-                   const TcProb *__restrict__ probs, const int *__restrict__ tstart, int nprobs, int ntiles,
-                   uint32_t idesc, ElemSink sink, TcEpi epi, int *err) {
+                   const __grid_constant__ ArgProbs arg, const TcProb *__restrict__ probs,
+                   const int *__restrict__ tstart, int nprobs, int ntiles, uint32_t idesc, ElemSink sink, TcEpi epi, int *err) {
     using C = Cfg<NPROD, NEPI, BNT>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>(
@@ -165,14 +174,14 @@ __global__ void __launch_bounds__(Cfg<NPROD, NEPI, BNT>::THREADS, 1)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    const TcProb *P = probs;
-    const int *TS = tstart;
+    const TcProb *P = probs ? probs : arg.p;
+    const int *TS = probs ? tstart : arg.tstart;
     if constexpr (C::MAXP_SMEM > 0) {
         if (nprobs <= C::MAXP_SMEM) {
             TcProb *ps = reinterpret_cast<TcProb *>(smem + C::OFF_PROBS);
             int *ts = reinterpret_cast<int *>(smem + C::OFF_TSTART);
-            for (int i = threadIdx.x; i < nprobs; i += blockDim.x) ps[i] = probs[i];
-            for (int i = threadIdx.x; i <= nprobs; i += blockDim.x) ts[i] = tstart[i];
+            for (int i = threadIdx.x; i < nprobs; i += blockDim.x) ps[i] = P[i];
+            for (int i = threadIdx.x; i <= nprobs; i += blockDim.x) ts[i] = TS[i];
             P = ps;
             TS = ts;
         }
@@ -633,8 +642,8 @@ kfb_status map2d(CUtensorMap *m, const void *ptr, long long rows, long long cols
 
 template <int NPROD, int NEPI, int BNT>
 kfb_status launch_cfg(const CUtensorMap &ma_hi, const CUtensorMap &ma_lo, const CUtensorMap &mb_hi,
-                      const CUtensorMap &mb_lo, const TcProb *probs, const int *tstart,
-                      int nprobs, int ntiles, bool bf16, const ElemSink &sink, const TcEpi &e,
+                      const CUtensorMap &mb_lo, const ArgProbs &arg, const TcProb *probs,
+                      const int *tstart, int nprobs, int ntiles, bool bf16, const ElemSink &sink, const TcEpi &e,
                       int *errp, cudaStream_t s) {
     using C = Cfg<NPROD, NEPI, BNT>;
     static bool done = false;
@@ -646,7 +655,7 @@ kfb_status launch_cfg(const CUtensorMap &ma_hi, const CUtensorMap &ma_lo, const 
     const int grid = std::min(ntiles, device_sm_count());
     const uint32_t idesc = make_idesc(BM, C::BN, bf16 ? 1 : 0);
     tc_gemm_kernel<NPROD, NEPI, BNT><<<grid, C::THREADS, C::SMEM, s>>>(
-        ma_hi, ma_lo, mb_hi, mb_lo, probs, tstart, nprobs, ntiles, idesc, sink, e, errp);
+        ma_hi, ma_lo, mb_hi, mb_lo, arg, probs, tstart, nprobs, ntiles, idesc, sink, e, errp);
     KFB_CUDA_TRY(cudaGetLastError());
     return KFB_OK;
 }
@@ -691,8 +700,14 @@ kfb_status launch(const TcOperand &A, const TcOperand &B, bool bf16,
         mb_lo = mb_hi;
     }
     DevBuf dp, dt, derr;
-    KFB_TRY(upload(dp, probs, s));
-    KFB_TRY(upload(dt, tstart, s));
+    ArgProbs arg{};
+    if (probs.size() <= (size_t)MAXP_ARG) {
+        std::copy(probs.begin(), probs.end(), arg.p);
+        std::copy(tstart.begin(), tstart.end(), arg.tstart);
+    } else {
+        KFB_TRY(upload(dp, probs, s));
+        KFB_TRY(upload(dt, tstart, s));
+    }
     int *errp = err_flag;
     if (!errp) {
         KFB_TRY(derr.alloc(sizeof(int), s));
@@ -700,15 +715,15 @@ kfb_status launch(const TcOperand &A, const TcOperand &B, bool bf16,
         errp = derr.as<int>();
     }
     if (ysplit)
-        KFB_TRY((launch_cfg<NPROD, 16, 128>(ma_hi, ma_lo, mb_hi, mb_lo, dp.as<TcProb>(),
+        KFB_TRY((launch_cfg<NPROD, 16, 128>(ma_hi, ma_lo, mb_hi, mb_lo, arg, dp.as<TcProb>(),
                                             dt.as<int>(), (int)probs.size(), (int)ntiles, bf16,
                                             sink, e, errp, s)));
     else if (narrow)
-        KFB_TRY((launch_cfg<NPROD, 8, 64>(ma_hi, ma_lo, mb_hi, mb_lo, dp.as<TcProb>(),
+        KFB_TRY((launch_cfg<NPROD, 8, 64>(ma_hi, ma_lo, mb_hi, mb_lo, arg, dp.as<TcProb>(),
                                           dt.as<int>(), (int)probs.size(), (int)ntiles, bf16,
                                           sink, e, errp, s)));
     else
-        KFB_TRY((launch_cfg<NPROD, 8, 128>(ma_hi, ma_lo, mb_hi, mb_lo, dp.as<TcProb>(),
+        KFB_TRY((launch_cfg<NPROD, 8, 128>(ma_hi, ma_lo, mb_hi, mb_lo, arg, dp.as<TcProb>(),
                                            dt.as<int>(), (int)probs.size(), (int)ntiles, bf16,
                                            sink, e, errp, s)));
     if (err_flag) return KFB_OK;
