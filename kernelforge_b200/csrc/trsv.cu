@@ -12,11 +12,15 @@
 //  * one persistent cooperative kernel per direction; block I is owned by CTA
 //    I mod grid.  Its CTA accumulates the off-diagonal tiles against the
 //    solution blocks as they are published and then applies the inverted
-//    diagonal block.  Blocks finish in solve order (block I needs block I-1),
-//    so publication is a single counter `done` (st.release / ld.acquire at
-//    gpu scope) and a CTA stages every block published so far in one batch;
-//  * every wait is bounded: after TRSV_WAIT_LIMIT polls the CTA raises *err
-//    and all CTAs leave; the host reads *err once per solve sequence.
+//    diagonal block.  Blocks finish in solve order (block I needs block I-1);
+//    that chain, not the factor's bytes, is what bounds the sweep;
+//  * the solution vector is its own flag: it is filled with a bit pattern that
+//    no result has, and a thread polls the very element that it stages, so a
+//    step of the chain has one store and one load in flight (1.6 and 1.5 us a
+//    block in the two sweeps of n = 10,000; with a counter published behind a
+//    fence and the block read after it 2.4 and 3.1 us);
+//  * every wait is bounded: after TRSV_WAIT_NS a thread raises *err and all
+//    CTAs leave; the host reads *err once per solve sequence.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -29,18 +33,25 @@ namespace kfb {
 namespace {
 
 constexpr int TB = 64;                  // rows per block
-constexpr int TB_BATCH = 8;             // solution blocks staged per wait
 constexpr int TRSV_THREADS = 256;       // 64 rows x 4 column groups
+constexpr int TB_BATCH = TRSV_THREADS / TB;   // solution blocks staged at once
 constexpr unsigned long long TRSV_WAIT_NS = 1000000000ull;   // one second of %globaltimer
 
-__device__ __forceinline__ int ld_acquire(const int *p) {
-    int v;
-    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
+// An element that is not published yet: all bits set (a NaN; a result with
+// these bits is published as another NaN).
+constexpr unsigned long long UNPUBLISHED = ~0ull;
+
+__device__ __forceinline__ bool ld_published(const double *p, double &v) {
+    unsigned long long b;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(b) : "l"(p) : "memory");
+    v = __longlong_as_double((long long)b);
+    return b != UNPUBLISHED;
 }
 
-__device__ __forceinline__ void st_release(int *p, int v) {
-    asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+__device__ __forceinline__ void publish(double *p, double v) {
+    unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    if (b == UNPUBLISHED) b = 0x7ff8000000000000ull;
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(b) : "memory");
 }
 
 __device__ __forceinline__ unsigned long long trsv_clock_ns() {
@@ -49,21 +60,46 @@ __device__ __forceinline__ unsigned long long trsv_clock_ns() {
     return t;
 }
 
-// Thread 0: wait until more than `need` blocks are published; returns the
-// published count, or -1 when the wait gave up (or another CTA gave up).  The
-// limit is elapsed time on %globaltimer (one second), not a poll count:
-// __nanosleep is only a hint, so a count would not bound the wait's length.
-__device__ int wait_published(const int *done, int need, int *err) {
+// Wait for an element; false when the wait gave up (or another CTA gave up).
+// The limit is elapsed time on %globaltimer (one second), not a poll count.
+__device__ bool wait_published(const double *p, double &v, int *err) {
+    for (int i = 0; i < 64; ++i)
+        if (ld_published(p, v)) return true;
     const unsigned long long t0 = trsv_clock_ns();
     while (true) {
-        const int d = ld_acquire(done);
-        if (d > need) return d;
-        if (*reinterpret_cast<volatile int *>(err)) return -1;
+        for (int i = 0; i < 16; ++i)
+            if (ld_published(p, v)) return true;
+        if (*reinterpret_cast<volatile int *>(err)) return false;
         if (trsv_clock_ns() - t0 > TRSV_WAIT_NS) break;
-        __nanosleep(32);
     }
     atomicExch(err, 1);
-    return -1;
+    return false;
+}
+
+// Stage up to TB_BATCH solution blocks, thread (r, g) element r of the g-th: it
+// is at p (valid: it exists and nblk > g; else the element counts as a zero that
+// is there).  The first block is waited for, the others are taken if they are
+// there.  Returns the number of leading blocks in xs, -1 when a wait gave up.
+__device__ __forceinline__ int stage_blocks(const double *p, bool valid, int nblk, double *xs,
+                                            int *state, int *err) {
+    const int t = threadIdx.x, g = t / TB;
+    double v = 0.0;
+    bool ok = true, fail = false;
+    if (valid) {
+        ok = ld_published(p, v);
+        if (!ok && g == 0) {
+            ok = wait_published(p, v, err);
+            fail = !ok;
+        }
+    }
+    xs[t] = v;
+    const bool all = __all_sync(0xffffffffu, ok), bad = __any_sync(0xffffffffu, fail);
+    if ((t & 31) == 0) state[t >> 5] = bad ? -1 : all;
+    __syncthreads();
+    if (state[0] < 0 || state[1] < 0) return -1;
+    int d = 1;
+    while (d < nblk && state[2 * d] > 0 && state[2 * d + 1] > 0) ++d;
+    return d;
 }
 
 // Inverse of each 64 x 64 lower diagonal block: dinv[I] column-major
@@ -102,12 +138,14 @@ __global__ void __launch_bounds__(TB) trsv_dinv_kernel(const double *__restrict_
 // that once block I-1 is published only x_{I-1} is fetched.
 __global__ void __launch_bounds__(TRSV_THREADS) trsv_lower_kernel(
     const double *__restrict__ L, int n, int nb, const double *__restrict__ dinv,
-    const double *__restrict__ b, double *t_out, int *done, int *err) {
-    __shared__ double xs[TB_BATCH * TB];
-    __shared__ double red[4][TB];
+    const double *__restrict__ b, double *t_out, int *err) {
+    __shared__ double xs[2][TB_BATCH * TB];   // (two: a batch is staged while the last is read)
+    __shared__ int state[2][TRSV_THREADS / 32];
+    __shared__ double rhs[TB];
+    __shared__ double red[2][4][TB];
     __shared__ double dsm[TB * TB];
-    __shared__ int avail;
     const int t = threadIdx.x, r = t & (TB - 1), g = t >> 6;
+    int buf = 0;
     for (int I = blockIdx.x; I < nb; I += gridDim.x) {
         const int i0 = I * TB, row = i0 + r;
         const bool rv = row < n;
@@ -117,18 +155,16 @@ __global__ void __launch_bounds__(TRSV_THREADS) trsv_lower_kernel(
 #pragma unroll
         for (int k = 0; k < TB / 4; ++k)
             lvl[k] = (rv && I > 0) ? L[(size_t)row + (size_t)((I - 1) * TB + g + 4 * k) * n] : 0.0;
+        const double bv = t < TB && rv ? b[row] : 0.0;
         double acc = 0.0;
         for (int J = 0; J < I;) {
-            if (t == 0) avail = wait_published(done, J, err);
-            __syncthreads();
-            const int d = avail;
+            // (blocks before I are full)
+            const int nblk = min(TB_BATCH, I - J);
+            const int d = stage_blocks(t_out + (size_t)J * TB + t, g < nblk, nblk, xs[buf],
+                                       state[buf], err);
             if (d < 0) return;
-            const int J1 = min(min(d, I), J + TB_BATCH);
-            for (int e = t; e < (J1 - J) * TB; e += TRSV_THREADS)
-                xs[e] = __ldcg(t_out + (size_t)J * TB + e);   // published blocks: < i0 <= n
-            __syncthreads();
-            for (int jj = J; jj < J1; ++jj) {
-                const double *xv = xs + (jj - J) * TB;
+            for (int jj = J; jj < J + d; ++jj) {
+                const double *xv = xs[buf] + (jj - J) * TB;
                 if (jj == I - 1) {
 #pragma unroll
                     for (int k = 0; k < TB / 4; ++k) acc = fma(lvl[k], xv[g + 4 * k], acc);
@@ -142,25 +178,20 @@ __global__ void __launch_bounds__(TRSV_THREADS) trsv_lower_kernel(
 #pragma unroll
                 for (int k = 0; k < TB / 4; ++k) acc = fma(lv[k], xv[g + 4 * k], acc);
             }
-            __syncthreads();   // xs consumed
-            J = J1;
+            buf ^= 1;
+            J += d;
         }
-        red[g][r] = acc;
+        red[0][g][r] = acc;
         __syncthreads();
-        if (t < TB) xs[t] = rv ? b[row] - (red[0][t] + red[1][t] + red[2][t] + red[3][t]) : 0.0;
+        if (t < TB) rhs[t] = bv - (red[0][0][t] + red[0][1][t] + red[0][2][t] + red[0][3][t]);
         __syncthreads();
         double s = 0.0;
 #pragma unroll
-        for (int k = 0; k < TB / 4; ++k) s = fma(dsm[r + TB * (g + 4 * k)], xs[g + 4 * k], s);
-        __syncthreads();   // red reused
-        red[g][r] = s;
+        for (int k = 0; k < TB / 4; ++k) s = fma(dsm[r + TB * (g + 4 * k)], rhs[g + 4 * k], s);
+        red[1][g][r] = s;
         __syncthreads();
-        if (t < TB && rv) {
-            t_out[row] = red[0][t] + red[1][t] + red[2][t] + red[3][t];
-            __threadfence();
-        }
-        __syncthreads();
-        if (t == 0) st_release(done, I + 1);
+        if (t < TB && rv)
+            publish(t_out + row, red[1][0][t] + red[1][1][t] + red[1][2][t] + red[1][3][t]);
     }
 }
 
@@ -172,13 +203,16 @@ __global__ void __launch_bounds__(TRSV_THREADS) trsv_lower_kernel(
 // I+1, the transposed inverse of the diagonal block).
 __global__ void __launch_bounds__(TRSV_THREADS) trsv_upper_kernel(
     const double *__restrict__ L, int n, int nb, const double *__restrict__ dinvt,
-    const double *__restrict__ tv, double *x, int *done, int *err) {
-    __shared__ double xs[TB_BATCH * TB];
+    const double *__restrict__ tv, double *x, int *err) {
+    __shared__ double xs[2][TB_BATCH * TB];
+    __shared__ int state[2][TRSV_THREADS / 32];
+    __shared__ double rhs[TB];
     __shared__ double red[2][TB];   // [half of the rows][column]
+    __shared__ double sums[4][TB];
     __shared__ double dsm[TB * TB];
-    __shared__ int avail;
     const int t = threadIdx.x, r = t & (TB - 1), g = t >> 6;
     const int lane = t & 31, half = r >> 5;
+    int buf = 0;
     for (int q = blockIdx.x; q < nb; q += gridDim.x) {
         const int I = nb - 1 - q, i0 = I * TB;
         __syncthreads();   // dsm of the previous block consumed
@@ -191,25 +225,18 @@ __global__ void __launch_bounds__(TRSV_THREADS) trsv_upper_kernel(
             for (int k = 0; k < TB / 4; ++k)
                 lvl[k] = jv ? L[(size_t)j + (size_t)(i0 + g + 4 * k) * n] : 0.0;
         }
+        const double bv = t < TB && i0 + t < n ? tv[i0 + t] : 0.0;
         double acc[TB / 4];
 #pragma unroll
         for (int k = 0; k < TB / 4; ++k) acc[k] = 0.0;
         // later blocks J = nb - 1 - p for published ranks p < q
         for (int p = 0; p < q;) {
-            if (t == 0) avail = wait_published(done, p, err);
-            __syncthreads();
-            const int d = avail;
+            const int nblk = min(TB_BATCH, q - p);
+            const int je = (nb - 1 - p - g) * TB + r;   // (the last block may be partial)
+            const int d = stage_blocks(x + je, g < nblk && je < n, nblk, xs[buf], state[buf], err);
             if (d < 0) return;
-            const int p1 = min(min(d, q), p + TB_BATCH);
-            // stage blocks J = nb-1-p .. nb-p1 (rank order)
-            for (int e = t; e < (p1 - p) * TB; e += TRSV_THREADS) {
-                const int pp = p + e / TB, rr = e % TB;
-                const int j = (nb - 1 - pp) * TB + rr;
-                xs[e] = j < n ? __ldcg(x + j) : 0.0;
-            }
-            __syncthreads();
-            for (int pp = p; pp < p1; ++pp) {
-                const double xr = xs[(pp - p) * TB + r];
+            for (int pp = p; pp < p + d; ++pp) {
+                const double xr = xs[buf][(pp - p) * TB + r];
                 if (pp == q - 1) {   // block I+1
 #pragma unroll
                     for (int k = 0; k < TB / 4; ++k) acc[k] = fma(lvl[k], xr, acc[k]);
@@ -224,34 +251,32 @@ __global__ void __launch_bounds__(TRSV_THREADS) trsv_upper_kernel(
 #pragma unroll
                 for (int k = 0; k < TB / 4; ++k) acc[k] = fma(lv[k], xr, acc[k]);
             }
-            __syncthreads();   // xs consumed
-            p = p1;
+            buf ^= 1;
+            p += d;
         }
+        // sum over the lanes, halving the columns that a lane holds: lane l ends
+        // with column 4 (l >> 1) + g
 #pragma unroll
-        for (int k = 0; k < TB / 4; ++k)
-            for (int o = 16; o; o >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
-        if (lane == 0) {
+        for (int o = 16, len = TB / 8; o > 1; o >>= 1, len >>= 1) {
+            const bool up = lane & o;
 #pragma unroll
-            for (int k = 0; k < TB / 4; ++k) red[half][g + 4 * k] = acc[k];
+            for (int k = 0; k < len; ++k) {
+                const double send = up ? acc[k] : acc[k + len];
+                acc[k] = (up ? acc[k + len] : acc[k]) + __shfl_xor_sync(0xffffffffu, send, o);
+            }
         }
+        acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
+        if ((lane & 1) == 0) red[half][g + 4 * (lane >> 1)] = acc[0];
         __syncthreads();
-        if (t < TB) {
-            const int i = i0 + t;
-            xs[t] = i < n ? tv[i] - (red[0][t] + red[1][t]) : 0.0;
-        }
+        if (t < TB) rhs[t] = bv - (red[0][t] + red[1][t]);
         __syncthreads();
         double s = 0.0;
 #pragma unroll
-        for (int k = 0; k < TB / 4; ++k) s = fma(dsm[r + TB * (g + 4 * k)], xs[g + 4 * k], s);
-        // sum the four column groups: reuse xs beyond the first block as scratch
-        xs[TB + g * TB + r] = s;
+        for (int k = 0; k < TB / 4; ++k) s = fma(dsm[r + TB * (g + 4 * k)], rhs[g + 4 * k], s);
+        sums[g][r] = s;
         __syncthreads();
-        if (t < TB && i0 + t < n) {
-            x[i0 + t] = xs[TB + t] + xs[2 * TB + t] + xs[3 * TB + t] + xs[4 * TB + t];
-            __threadfence();
-        }
-        __syncthreads();
-        if (t == 0) st_release(done, q + 1);
+        if (t < TB && i0 + t < n)
+            publish(x + i0 + t, sums[0][t] + sums[1][t] + sums[2][t] + sums[3][t]);
     }
 }
 
@@ -263,8 +288,8 @@ kfb_status TrsvPlan::prepare(const double *L, int n_, cudaStream_t s) {
     if (n <= 0) return KFB_OK;
     KFB_TRY(dinv.alloc((size_t)nb * TB * TB * sizeof(double), s));
     KFB_TRY(dinvt.alloc((size_t)nb * TB * TB * sizeof(double), s));
-    KFB_TRY(sync.alloc(4 * sizeof(int), s));
-    KFB_TRY(zero(sync.ptr, 4 * sizeof(int), s));
+    KFB_TRY(sync.alloc(sizeof(int), s));
+    KFB_TRY(zero(sync.ptr, sizeof(int), s));
     trsv_dinv_kernel<<<nb, TB, 0, s>>>(L, n, dinv.as<double>(), dinvt.as<double>());
     KFB_CUDA_TRY(cudaGetLastError());
     int dev = 0, sms = 0, coop = 0, per_sm_l = 0, per_sm_u = 0;
@@ -284,17 +309,18 @@ kfb_status TrsvPlan::prepare(const double *L, int n_, cudaStream_t s) {
 kfb_status TrsvPlan::solve(const double *L, const double *b, double *tmp, double *x,
                            cudaStream_t s) {
     if (n <= 0) return KFB_OK;
-    int *done = sync.as<int>(), *err = sync.as<int>() + 2;
-    KFB_CUDA_TRY(cudaMemsetAsync(done, 0, 2 * sizeof(int), s));
+    int *err = sync.as<int>();
+    KFB_CUDA_TRY(cudaMemsetAsync(tmp, 0xff, (size_t)n * sizeof(double), s));   // unpublished
     const double *dl = dinv.as<double>(), *du = dinvt.as<double>();
-    int *done_l = done, *done_u = done + 1;
     void *args_l[] = {(void *)&L, (void *)&n, (void *)&nb, (void *)&dl, (void *)&b,
-                      (void *)&tmp, (void *)&done_l, (void *)&err};
+                      (void *)&tmp, (void *)&err};
     KFB_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)trsv_lower_kernel, dim3(grid),
                                              dim3(TRSV_THREADS), args_l, 0, s));
+    // (x may be b, which the forward sweep reads)
+    KFB_CUDA_TRY(cudaMemsetAsync(x, 0xff, (size_t)n * sizeof(double), s));
     const double *tc = tmp;
     void *args_u[] = {(void *)&L, (void *)&n, (void *)&nb, (void *)&du, (void *)&tc,
-                      (void *)&x, (void *)&done_u, (void *)&err};
+                      (void *)&x, (void *)&err};
     KFB_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)trsv_upper_kernel, dim3(grid),
                                              dim3(TRSV_THREADS), args_u, 0, s));
     return KFB_OK;
@@ -303,7 +329,7 @@ kfb_status TrsvPlan::solve(const double *L, const double *b, double *tmp, double
 kfb_status TrsvPlan::check(cudaStream_t s) {
     if (n <= 0) return KFB_OK;
     int e = 0;
-    KFB_CUDA_TRY(cudaMemcpyAsync(&e, sync.as<int>() + 2, sizeof(int), cudaMemcpyDeviceToHost, s));
+    KFB_CUDA_TRY(cudaMemcpyAsync(&e, sync.as<int>(), sizeof(int), cudaMemcpyDeviceToHost, s));
     KFB_CUDA_TRY(cudaStreamSynchronize(s));
     if (e != 0)
         return set_error(KFB_ERR_TIMEOUT, "triangular solve: a block wait gave up");
