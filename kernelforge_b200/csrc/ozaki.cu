@@ -6,15 +6,21 @@
 //               A tile (128 rows) and of the B tile (BN = 128 rows for S <= 4,
 //               else 64), 64-byte swizzle, into a shared-memory ring of 2-4
 //               stages;
-//   warp 1      MMA issuer: per K32 step, for every level L = 2 .. S+1 and every
-//               digit pair p + q = L, tcgen05.mma kind::i8 (M=128, N=BN, K=32,
-//               s32 accumulation) into level L's TMEM accumulator (BN columns
-//               each, S accumulators side by side);
+//   warp 1      MMA issuer: digit pair (p, q) belongs to level L = p + q, whose
+//               s32 accumulator is BN columns of TMEM (S of them side by side).
+//               Per K32 step and digit p of A, the digits q = 1 .. S + 1 - p of
+//               B are one operand (their planes are stacked in shared memory)
+//               and their accumulators one block of columns: tcgen05.mma
+//               kind::i8, M = 128, K = 32, N = BN x up to 256 / BN planes.  With
+//               an instruction per pair (N = 64) each read A from shared memory
+//               again, 70 cycles an instruction where the product takes 32.
 //   warp 2      TMEM allocator (512 columns);
-//   warps 4..11 epilogue, two per TMEM lane quadrant (32-column chunks): load
-//               the S int32 levels, combine them in FP64 (Horner in 2^-7),
-//               release TMEM to the MMA issuer, then scale by 2^(e_a + e_b -
-//               14) alpha and store / accumulate the FP64 outputs.
+//   warp 3      prefetches the old values of a tile that is accumulated into
+//               L2 while its MMAs run;
+//   warps 4..19 epilogue, four per TMEM lane quadrant (16-column chunks): load
+//               the S int32 levels, combine them, release TMEM to the MMA
+//               issuer, then scale by 2^(e_a + e_b - 14) alpha and store /
+//               accumulate the FP64 outputs.
 // Every mbarrier wait is bounded (%globaltimer); a wait that gives up raises
 // the error flag instead of trapping.  No TMA multicast.
 #include <cuda.h>
@@ -36,25 +42,27 @@ using namespace tc;
 
 constexpr int BM = OZ_BM, BK = OZ_BK;
 constexpr int TILE_A = BM * BK;   // bytes per digit plane of an A tile
-constexpr int EPI_WARP0 = 4, NUM_EPI_WARPS = 8;
+constexpr int EPI_WARP0 = 4, NUM_EPI_WARPS = 16;
 constexpr int NUM_THREADS = 32 * (EPI_WARP0 + NUM_EPI_WARPS);
 constexpr int TMEM_COLS = 512;
 
 // S digit planes, BN output columns per tile (S BN <= 512 TMEM columns), as
-// many pipeline stages (up to 4) as fit in 200 KB of shared memory.
+// many pipeline stages (up to 4) as fit in 220 KB of shared memory.
 template <int S>
 struct OzCfg {
     static constexpr int BN = oz_bn(S);
     static constexpr int TILE_B = BN * BK;
     static constexpr int STAGE = S * (TILE_A + TILE_B);
-    static constexpr int NSTAGE = (200 * 1024 / STAGE) < 4 ? (200 * 1024 / STAGE) : 4;
+    static constexpr int NSTAGE = (220 * 1024 / STAGE) < 4 ? (220 * 1024 / STAGE) : 4;
     static constexpr int OFF_BARS = NSTAGE * STAGE;
     static constexpr int NBARS = 2 * NSTAGE + 3;   // full, empty, tmem_full, tmem_empty, done
     static constexpr int OFF_TMEM = OFF_BARS + NBARS * 8;
     static constexpr int SMEM = OFF_TMEM + 16 + 1024;
     // instruction descriptor, kind::i8: signed A and B (K-major), s32 accumulator
-    static constexpr uint32_t IDESC = (2u << 4) | (1u << 7) | (1u << 10) |
-                                      ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+    static constexpr uint32_t idesc(int n) {
+        return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) |
+               ((uint32_t)(BM >> 4) << 24);
+    }
     static_assert(NSTAGE >= 2, "pipeline depth");
     static_assert(S * BN <= TMEM_COLS, "TMEM columns");
     static_assert(SMEM <= 227 * 1024, "shared memory budget");
@@ -65,6 +73,10 @@ struct OzCfg {
 __device__ __forceinline__ uint64_t sdesc64(uint32_t saddr) {
     return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)1 << 16) |
            ((uint64_t)(512 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)4 << 61);
+}
+
+__device__ __forceinline__ void prefetch_l2(const void *p) {
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }
 
 __device__ __forceinline__ void umma_i8(uint32_t dtmem, uint64_t a, uint64_t b, uint32_t idesc,
@@ -88,11 +100,16 @@ __host__ __device__ __forceinline__ OzTile gen_tile(const OzGen &g, int BN, long
     t += g.first;
     int ti = 0, tj = t;
     if (g.mode == OZ_GEN_LOWER) {
-        while (true) {
-            const int cnt = lower_tiles(ti, ntc, BN);
-            if (tj < cnt) break;
-            tj -= cnt;
-            ++ti;
+        // row tiles 0 .. full - 1 have r (ti + 1) column tiles, the others all of them
+        const int r = BM / BN, full = ntc / r, head = r * full * (full + 1) / 2;
+        if (t < head) {
+            ti = (int)((sqrtf(8.0f * (float)(t / r) + 1.0f) - 1.0f) * 0.5f);
+            while (r * ti * (ti + 1) / 2 > t) --ti;
+            while (r * (ti + 1) * (ti + 2) / 2 <= t) ++ti;
+            tj = t - r * ti * (ti + 1) / 2;
+        } else {
+            ti = full + (t - head) / ntc;
+            tj = (t - head) % ntc;
         }
     } else {
         ti = t / ntc;
@@ -119,11 +136,44 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map
         : "memory");
 }
 
-__device__ __forceinline__ void tmem_ld32_i(uint32_t taddr, int (&v)[32]) {
-    float f[32];
-    tmem_ld32(taddr, f);
+// 8 columns of a warp's 32 TMEM lanes, not waited for; tmem_wait8 orders the
+// uses of N such loads behind their arrival.
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, int (&v)[8]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+          "=r"(v[7])
+        : "r"(taddr));
+}
+template <int N>
+__device__ __forceinline__ void tmem_wait8(int (&v)[N][8]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = __float_as_int(f[i]);
+    for (int l = 0; l < N; ++l)
+        asm volatile(""
+                     : "+r"(v[l][0]), "+r"(v[l][1]), "+r"(v[l][2]), "+r"(v[l][3]), "+r"(v[l][4]),
+                       "+r"(v[l][5]), "+r"(v[l][6]), "+r"(v[l][7]));
+}
+
+// r[j] = sum_l v_l[j] 128^(N-1-l) over N (<= 4) levels from TMEM, exactly: the
+// sum is an integer below 2^50 (level l of the first group sums (l + 1) K
+// products below 2^12 in size, K <= 2^16), turned into a double by the bits of
+// 1.5 2^52 + sum.  (A conversion and an FMA per level ran at the conversions'
+// rate, a quarter of the FP64 one.)
+template <int N, int STRIDE>
+__device__ __forceinline__ void tmem_levels(uint32_t taddr, double (&r)[8]) {
+    static_assert(N <= 4, "the sum must stay below 2^51");
+    int v[N][8];
+#pragma unroll
+    for (int l = 0; l < N; ++l) tmem_ld8(taddr + (uint32_t)(l * STRIDE), v[l]);
+    tmem_wait8(v);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        long long t = v[N - 1][j];
+#pragma unroll
+        for (int l = N - 2; l >= 0; --l) t += (long long)v[l][j] * (1 << (7 * (N - 1 - l)));
+        r[j] = __longlong_as_double(t + 0x4338000000000000LL) - 6755399441055744.0;
+    }
 }
 
 template <int S>
@@ -133,7 +183,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
                    const int *__restrict__ eb, const OzTile *__restrict__ tiles, OzGen gen,
                    int ntiles, OzEpi epi, int *err) {
     using C = OzCfg<S>;
-    constexpr int BN = C::BN, TILE_B = C::TILE_B, NSTAGE = C::NSTAGE;
+    constexpr int BN = C::BN, TILE_B = C::TILE_B, NSTAGE = C::NSTAGE, QMAX = 256 / BN;
     if (epi.skip && *(volatile const int *)epi.skip) return;   // block-uniform
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>(
@@ -154,7 +204,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
             mbar_init(empty_bar(s), 1);
         }
         mbar_init(tfull_bar, 1);
-        mbar_init(tempty_bar, NUM_EPI_WARPS);
+        mbar_init(tempty_bar, NUM_EPI_WARPS + 1);   // and the prefetching warp
         mbar_init(done_bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -213,17 +263,16 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
 #pragma unroll
                     for (int ks = 0; ks < BK / 32; ++ks) {
 #pragma unroll
-                        for (int L = 2; L <= S + 1; ++L) {
-                            const uint32_t dtm = tmem_base + (uint32_t)((L - 2) * BN);
+                        for (int p = 1; p <= S; ++p) {
+                            // planes q = 1 .. S + 1 - p of B lie one behind the other
+                            // and so do the accumulators of their levels p + q
+                            const uint64_t da = sdesc64(sa + (p - 1) * TILE_A + ks * 32);
 #pragma unroll
-                            for (int p = 1; p < L; ++p) {
-                                const int q = L - p;
-                                if (p > S || q > S) continue;
-                                const uint64_t da = sdesc64(sa + (p - 1) * TILE_A + ks * 32);
-                                const uint64_t db =
-                                    sdesc64(sa + S * TILE_A + (q - 1) * TILE_B + ks * 32);
-                                const bool first = kb == 0 && ks == 0 && p == 1;
-                                umma_i8(dtm, da, db, C::IDESC, first ? 0u : 1u);
+                            for (int q = 1; q <= S + 1 - p; q += QMAX) {
+                                const int nq = S + 2 - p - q < QMAX ? S + 2 - p - q : QMAX;
+                                umma_i8(tmem_base + (uint32_t)((p + q - 2) * BN), da,
+                                        sdesc64(sa + S * TILE_A + (q - 1) * TILE_B + ks * 32),
+                                        C::idesc(nq * BN), kb == 0 && ks == 0 && p == 1 ? 0u : 1u);
                             }
                         }
                     }
@@ -240,36 +289,58 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
             umma_commit(done_bar);
             mbar_wait(done_bar, 0, err);
         }
+    } else if (warp == 3) {
+        // (the epilogue's loads then cost an L2 latency; from HBM they were half
+        // of a K = 512 tile's time)
+        uint32_t aph = 0;
+        for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+            const OzTile tl = tiles ? tiles[t] : gen_tile(gen, BN, epi.ldr, epi.ldc, t);
+            const double *c = epi.c + tl.c_off;
+            // 32-byte pieces, each by an element that will be read
+            const int di = tl.lower ? tl.a0 + tl.lower_shift - tl.b0 : BN;   // j <= i + di
+            if (epi.mode != OZ_ADD) {
+            } else if (epi.ldr == 1) {
+                const int i = min(lane * 4 + 3, tl.m - 1);
+                const int nj = lane * 4 < tl.m ? min(tl.n, i + di + 1) : 0;
+                for (int j = 0; j < nj; ++j) prefetch_l2(c + (long long)j * epi.ldc + i);
+            } else {
+                for (int i = lane; i < tl.m; i += 32)
+                    for (int j = 0; j < min(tl.n, i + di + 1); j += 4)
+                        prefetch_l2(c + (long long)i * epi.ldr + (long long)j * epi.ldc);
+            }
+            if (!__all_sync(0xffffffffu, mbar_wait(tfull_bar, aph, err))) break;
+            if (lane == 0) mbar_arrive(tempty_bar);
+            aph ^= 1u;
+        }
     } else if (warp >= EPI_WARP0) {
-        // warp (q, h): TMEM lane quadrant q (tile rows 32 q ..), 32-column
-        // chunks h, h + 2, ... of each level
+        // warp (q, h): TMEM lane quadrant q (tile rows 32 q ..), 16-column
+        // chunks h, h + 4, ... of each level
         const int q = warp & 3;
         const int h = (warp - EPI_WARP0) >> 2;
-        constexpr int NCH = BN / 64;
+        constexpr int NCH = BN / 64, HI = (S + 1) / 2, LO = S - HI;
+        constexpr double LO_SCALE = 1.0 / (double)(1LL << (7 * LO));
         uint32_t aph = 0;
         for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
             const OzTile tl = tiles ? tiles[t] : gen_tile(gen, BN, epi.ldr, epi.ldc, t);
             const int i = q * 32 + lane;
+            const int er = i < tl.m ? ea[tl.a0 + i] - 14 - 7 * (HI - 1) : 0;
             const bool got = mbar_wait(tfull_bar, aph, err);
             if (!__all_sync(0xffffffffu, got)) break;
             tc_fence_after();
 #pragma unroll
             for (int ch = 0; ch < NCH; ++ch) {
-                const int col0 = (h + 2 * ch) * 32;
+                const int col0 = (h + 4 * ch) * 16;
                 const uint32_t tb = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)col0;
-                double acc[32];
-                {
-                    int v[32];
-                    tmem_ld32_i(tb + (uint32_t)((S - 1) * BN), v);
+                // the first HI levels and the last LO as one integer each, one
+                // rounding in their sum
+                double acc[16];
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) acc[j] = (double)v[j];
-                }
+                for (int g = 0; g < 16; g += 8) {
+                    double lo[8], hi[8];
+                    tmem_levels<LO, BN>(tb + (uint32_t)(HI * BN + g), lo);
+                    tmem_levels<HI, BN>(tb + (uint32_t)g, hi);
 #pragma unroll
-                for (int l = S - 2; l >= 0; --l) {
-                    int v[32];
-                    tmem_ld32_i(tb + (uint32_t)(l * BN), v);
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) acc[j] = fma(acc[j], 0.0078125, (double)v[j]);
+                    for (int j = 0; j < 8; ++j) acc[g + j] = fma(lo[j], LO_SCALE, hi[j]);
                 }
                 if (ch == NCH - 1) {
                     // every level of this warp's chunks is in registers: hand
@@ -279,35 +350,33 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
                     if (lane == 0) mbar_arrive(tempty_bar);
                 }
                 if (i < tl.m) {
-                    // columns col0 .. col0 + 31 of row i; nv of them are inside
+                    // columns col0 .. col0 + 15 of row i; nv of them are inside
                     // the tile (and on or below the diagonal in lower mode)
-                    const int er = ea[tl.a0 + i] - 14;
                     double *crow = epi.c + tl.c_off + (long long)i * epi.ldr +
                                    (long long)col0 * epi.ldc;
                     const int *ebh = eb + tl.b0 + col0;
-                    int nv = min(tl.n - col0, 32);
+                    int nv = min(tl.n - col0, 16);
                     if (tl.lower) nv = min(nv, tl.a0 + i + tl.lower_shift - tl.b0 - col0 + 1);
-#pragma unroll
-                    for (int j = 0; j < 32; ++j)
-                        if (j < nv) acc[j] = epi.alpha * oz_scale2(acc[j], er + ebh[j]);
                     if (epi.mode == OZ_ADD) {
-                        // the loads of 16 old values first, then their stores: two
-                        // memory latencies per chunk row instead of one per column
 #pragma unroll
-                        for (int hh = 0; hh < 32; hh += 16) {
-                            double old[16];
+                        for (int g = 0; g < 16; g += 8) {
+                            double old[8];   // 8 loads in flight, then their stores
 #pragma unroll
-                            for (int j = 0; j < 16; ++j)
-                                if (hh + j < nv) old[j] = crow[(long long)(hh + j) * epi.ldc];
+                            for (int j = 0; j < 8; ++j)
+                                if (g + j < nv) old[j] = crow[(long long)(g + j) * epi.ldc];
 #pragma unroll
-                            for (int j = 0; j < 16; ++j)
-                                if (hh + j < nv)
-                                    crow[(long long)(hh + j) * epi.ldc] = old[j] + acc[hh + j];
+                            for (int j = 0; j < 8; ++j)
+                                if (g + j < nv)
+                                    crow[(long long)(g + j) * epi.ldc] =
+                                        old[j] +
+                                        epi.alpha * oz_scale2(acc[g + j], er + ebh[g + j]);
                         }
                     } else {
 #pragma unroll
-                        for (int j = 0; j < 32; ++j)
-                            if (j < nv) crow[(long long)j * epi.ldc] = acc[j];
+                        for (int j = 0; j < 16; ++j)
+                            if (j < nv)
+                                crow[(long long)j * epi.ldc] =
+                                    epi.alpha * oz_scale2(acc[j], er + ebh[j]);
                     }
                 }
             }
