@@ -1,30 +1,31 @@
-// Blocked right-looking Cholesky factorisation: the diagonal blocks and panel
-// solves on the FP64 CUDA cores, the trailing updates on the int8 tensor cores
-// (digit-sliced FP64 products, ozaki.h).  Column-major storage, lower triangle.
+// Blocked right-looking Cholesky factorisation: the diagonal blocks, the rows
+// below them and the updates within an outer panel on FP64 mma.sync, the
+// trailing updates on the int8 tensor cores (digit-sliced FP64 products,
+// ozaki.h).  Column-major storage, lower triangle.
 //
-// Two levels of blocking.  Outer panels of 512 columns; inside one, per
-// 128-column block j (c0 = 128 j, rows r0 = c0 + w .. n-1 below it):
-//   1. chol_block64_kernel (FP32-class factor: chol_block_kernel) one CTA
-//                         factors the w x w diagonal block in shared memory and
-//                         forms W = L_jj^{-1}; the first non-positive pivot is
-//                         recorded (LAPACK potrf's info);
-//   2. chol_panel_kernel  L_21 = A_21 W^T in FP64 (64 rows per CTA, W and the
-//                         rows staged in shared memory by cp.async), written
-//                         over A_21, together with the digit planes and row
-//                         exponents of L_21;
-//   3. inner update       the outer panel's remaining columns (all rows below
-//                         them) -= L_21 L_21^T, K = 128 (tensor cores): the next
-//                         diagonal block on the critical stream, the rest on a
-//                         stream of its own beside that block's factorisation;
-// then, once per outer panel, the panel is sliced again (one row scale over
-// its 512 columns) and everything right of it is updated by tensor-core
-// products with K = 512 on the lower triangle only: the next outer panel's
-// columns on a high-priority stream, the rest on a low-priority stream with one
-// CTA per tile, so that the next panel's diagonal blocks, panels and inner
-// updates run while that bulk update proceeds (look-ahead; the digit planes of
-// consecutive outer panels alternate between two buffers).  The FP64 read-modify-write
-// of the trailing matrix, the memory cost of a right-looking factorisation,
-// thereby happens once per 512 columns instead of once per 128.
+// Outer panels of 512 columns.  Per panel (o0, rows R = o0 + 512 .. n - 1 below):
+//   1. its 512 x 512 diagonal block, per 128-column block:
+//      chol_block64_kernel (FP32-class factor: chol_block_kernel): one CTA
+//        factors the w x w diagonal block in shared memory and forms W =
+//        L_jj^{-1}; the first non-positive pivot is recorded (LAPACK potrf's
+//        info);
+//      chol_panel_kernel: L_21 = A_21 W^T for the rows of the outer panel;
+//      chol_update_kernel: the rest of the diagonal block -= L_21 L_21^T, the
+//        next 128 columns on the critical stream, the rest beside that block's
+//        factorisation;
+//   2. chol_far_kernel: the rows below, all 512 columns of a row tile in one
+//      CTA, with their digit planes; the 512 rows of the next diagonal block on
+//      the critical stream, the others on the far stream;
+//   3. trailing products with K = 512 on the tensor cores: the next diagonal
+//      block on the critical stream, the columns below it on the far stream, the
+//      rest on the bulk stream, the columns of the panel after the next first.
+// So the critical path holds what the next diagonal block needs and no more:
+// per panel four diagonal blocks and seven launches of few CTAs.  The other
+// streams' work, which fills the GPU, has a panel's time to finish (look-ahead;
+// digit planes and inverted blocks of consecutive panels alternate between two
+// buffers).  With every row of a 128-column panel on the critical path, and its
+// digit planes sliced per 128 and again per 512 columns, n = 10,000 took 10.6
+// ms; now 5.9 ms.
 // The block order is that of LAPACK's right-looking dpotrf with the panel's
 // triangular solve replaced by a product with the inverted diagonal block
 // (the inverse-based form used by GPU Cholesky codes).  A failed pivot raises
@@ -32,6 +33,7 @@
 // once; the host reads the pivot index once, at the end.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "chol.h"
 #include "kernels_common.cuh"
@@ -49,8 +51,13 @@ constexpr int NWB = 10;           // lower 32 x 32 blocks of a 128 x 128 triangl
 constexpr int BLK_THREADS = 512;
 constexpr int BLK_WARPS = BLK_THREADS / 32;
 constexpr int NB2 = 4 * NB;       // outer panel (two-level blocking)
-constexpr int PR = 64;            // panel rows per CTA
+constexpr int PR = 16;            // panel rows per CTA
+constexpr int UT = 32;            // tile of the near update
 constexpr int PANEL_THREADS = 256;
+constexpr int FAR_THREADS = 256;
+// tiles per CTA of a bulk update: 2 .. 8 are equal within 1%, with persistent CTAs the other
+// streams wait (n = 10,000: 12.2 against 11.1 ms a solve)
+constexpr int BULK_TILES = 4;
 
 static_assert(NB == 4 * SB, "the block kernel assumes four sub-blocks");
 
@@ -59,6 +66,8 @@ __host__ __device__ constexpr int wblk(int i, int j) { return i * (i + 1) / 2 + 
 using F = float;   // arithmetic of the FP32-class diagonal block
 constexpr size_t BLK_SMEM = ((size_t)NB * LDT + (size_t)NWB * SB * LDW + SB) * sizeof(F) + 16;
 constexpr int LDP = NB + 4, LDX = PR + 4;   // panel kernel: strides of W and of the rows (4 mod 16)
+constexpr int LDU = UT + 4;
+constexpr size_t UPD_SMEM = (size_t)2 * NB * LDU * sizeof(double);
 constexpr size_t PANEL_SMEM = (size_t)NB * (LDP + LDX) * sizeof(double);
 
 // Asynchronous global -> shared copies (cp.async): `bytes` of 8 or 16, with
@@ -81,18 +90,6 @@ __device__ __forceinline__ void cp_async_wait_all() {
 
 constexpr unsigned FULL = 0xffffffffu;
 
-// 1 / sqrt(d) for the pivots: the FP32 estimate refined by two Newton steps in
-// FP64 (each squares the relative error: 2^-23 -> 2^-46 -> below FP64
-// rounding), which is shorter on the pivot chain than the FP64 library
-// routine; outside the FP32 range the library routine.
-__device__ __forceinline__ double pivot_rsqrt(double d) {
-    if (!(d > 1e-30 && d < 1e30)) return rsqrt(d);
-    double r = (double)rsqrtf((float)d);
-    const double hd = 0.5 * d;
-    r = r * fma(-hd * r, r, 1.5);
-    r = r * fma(-hd * r, r, 1.5);
-    return r;
-}
 __device__ __forceinline__ float pivot_rsqrt(float d) { return rsqrtf(d); }
 
 // Factor the w x w block at (c0, c0) of the column-major matrix A in place
@@ -331,18 +328,26 @@ __global__ void __launch_bounds__(BLK_THREADS, 1)
 // FP64 diagonal block on mma.sync: the w x w block at (c0, c0) factored in
 // place and W = L^{-1} written to Wout, as chol_block_kernel does in FP32.
 //
-// 16 micro-panels of 8 columns over the whole block, two barriers each:
-//   A  the 8 x 8 diagonal block of panel p, in one thread's registers (every
-//      lane of warp 0 the same: no exchange on the pivot chain);
-//   B  a thread per row below solves its 8 entries; another warp inverts the
-//      8 x 8 block;
-//   C  warp 0 updates the next diagonal block alone and goes on with its A,
-//      while warps 1..15 update the rest of the trailing triangle (8 x 8 tiles,
-//      K = 8) and form row block p of W, -W_pp sum_{k<p} L_pk W_kj, block by
-//      block.
-// What bounds it is the chain A-B over the panels; the rest hides behind A.
+// 16 micro-panels of 8 columns over the whole block, one barrier each:
+//   A  warp 0 factors the 8 x 8 diagonal block of panel p in registers (every
+//      lane the same: no exchange on the pivot chain), and after the barrier
+//      solves the next 8 rows with it, updates the next diagonal block and goes
+//      on with that one's A;
+//   B  four warps solve the other rows below, a thread per row; another one
+//      inverts the 8 x 8 block;
+//   C  when the rows are there, twelve warps update the rest of the trailing
+//      triangle (8 x 8 tiles, K = 8) and form row block p of W, -W_pp sum_{k<p}
+//      L_pk W_kj, block by block.  A tile lives in its warp's registers until
+//      its column is next (its diagonal tile one panel sooner): read and
+//      written in shared memory at every panel, the tiles alone took 2,500
+//      cycles of an early panel.  They are dealt out from the last column
+//      backwards, so that the warps have equal shares at every panel.
+// What bounds it is warp 0's chain over the panels; the rest hides behind it.
+// Warps 4, 8 and 12 only copy: warp 0 has its scheduler's FP64 unit for itself
+// (with their products on it A took 2,450 cycles).
 // (32-column sub-blocks factored by one warp with a lane per row, then
-// inverted and applied in phases of their own, took 75-83 us a block.)
+// inverted and applied in phases of their own, took 75-83 us a block; this one
+// takes 33 us.)
 //
 // Shared memory: T[k * DLT + r] holds the lower triangle in column k, row r;
 // its strict upper triangle takes W's blocks off the diagonal transposed into
@@ -353,42 +358,67 @@ constexpr int DB = 8, DP = NB / DB;      // micro-panel width, their number
 constexpr int DLT = NB + 4;              // shared column stride (4 mod 16)
 constexpr int DLW = DB + 4;              // row stride of an inverted 8 x 8 block
 constexpr size_t DBLK_SMEM =
-    ((size_t)NB * DLT + (size_t)DP * DB * DLW + DB * DB + DB) * sizeof(double) + 16;
+    ((size_t)NB * DLT + (size_t)DP * (DB * DLW + DB * DB + DB)) * sizeof(double) + 16;
+constexpr int BLK_WORK = BLK_WARPS * 3 / 4;   // warps of B and C
 
-// a (lower triangle) -> its Cholesky factor, rinv = 1 / diagonal; returns the
-// first column with a non-positive pivot (DB: none).
-__device__ __forceinline__ int chol8(double (&a)[DB][DB], double (&rinv)[DB]) {
-    int bad = DB;
+// a (lower triangle) -> its Cholesky factor, rinv = 1 / diagonal.  1 /
+// sqrt(pivot) is the approximation instruction (about 2^-20) refined by one
+// step of third order, r (1 + e/2 + 3 e^2/8) with e = 1 - d r^2 (the rest is
+// 5/16 e^3).  False (a, rinv void) unless every pivot is positive and far from
+// the ends of the range: an integer test of the exponents, off the pivot chain.
+__device__ __forceinline__ bool chol8(double (&a)[DB][DB], double (&rinv)[DB]) {
+    bool ok = true;
 #pragma unroll
     for (int c = 0; c < DB; ++c) {
         const double d = a[c][c];
-        if (!(d > 0.0) || !isfinite(d)) bad = min(bad, c);
-        rinv[c] = pivot_rsqrt(d);
-        a[c][c] = d * rinv[c];
+        // exponents -900 .. 900 (a negative number or a NaN is above them)
+        ok &= (unsigned)(__double2hiint(d) - ((1023 - 900) << 20)) <= (1800u << 20);
+        double r;
+        asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+        const double e = fma(-(d * r), r, 1.0);
+        r = fma(r * e, fma(0.375, e, 0.5), r);
+        rinv[c] = r;
+        a[c][c] = d * r;
 #pragma unroll
-        for (int r = c + 1; r < DB; ++r) a[r][c] *= rinv[c];
+        for (int k = c + 1; k < DB; ++k) a[k][c] *= r;
 #pragma unroll
         for (int k = c + 1; k < DB; ++k)
 #pragma unroll
-            for (int r = k; r < DB; ++r) a[r][k] = fma(-a[r][c], a[k][c], a[r][k]);
+            for (int q = k; q < DB; ++q) a[q][k] = fma(-a[q][c], a[k][c], a[q][k]);
+    }
+    return ok;
+}
+
+// The same by one thread in shared memory, for any pivots: t (column stride DLT)
+// -> Ls, rd.  Returns the first column whose pivot is not positive and finite
+// (DB: none).
+__device__ __noinline__ int chol8_any(const double *t, double *Ls, double *rd) {
+    int bad = DB;
+    for (int c = 0; c < DB; ++c) {
+        for (int r = c; r < DB; ++r) {
+            double v = t[c * DLT + r];
+            for (int k = 0; k < c; ++k) v = fma(-Ls[r * DB + k], Ls[c * DB + k], v);
+            if (r == c) {
+                if (!(v > 0.0) || !isfinite(v)) bad = min(bad, c);
+                rd[c] = rsqrt(v);
+            }
+            Ls[r * DB + c] = v * rd[c];
+        }
     }
     return bad;
 }
 
-// Tile (kb, rb) of the trailing triangle -= X_rb X_kb^T for panel columns
-// o .. o + 7: D's rows are the tile's columns k, so that a lane's two values
-// are neighbours in memory.
-__device__ __forceinline__ void chol_tile(double *T, int o, int kb, int rb, int lane) {
+// d (a tile's accumulator lanes) -= X_rb X_kb^T for panel columns o .. o + 7 and
+// the tile (kb, rb): D's rows are the tile's columns, so that a lane's two
+// values are neighbours in T.
+__device__ __forceinline__ void chol_tile(double (&d)[2], const double *T, int o, int kb, int rb,
+                                          int lane) {
     const int i = lane >> 2, j = lane & 3;
-    double2 *c = reinterpret_cast<double2 *>(T + (DB * kb + i) * DLT + DB * rb + 2 * j);
     const double *x0 = T + (o + j) * DLT, *x1 = x0 + 4 * DLT;
     const double a0 = -x0[DB * kb + i], a1 = -x1[DB * kb + i];
     const double b0 = x0[DB * rb + i], b1 = x1[DB * rb + i];
-    const double2 v = *c;
-    double d[2] = {v.x, v.y};
     dmma(d, a0, b0);
     dmma(d, a1, b1);
-    *c = make_double2(d[0], d[1]);
 }
 
 __global__ void __launch_bounds__(BLK_THREADS, 1)
@@ -398,9 +428,9 @@ __global__ void __launch_bounds__(BLK_THREADS, 1)
     extern __shared__ __align__(16) unsigned char sm_raw[];
     double *T = reinterpret_cast<double *>(sm_raw);
     double *Wp = T + NB * DLT;            // [DP][DB][DLW]
-    double *Ls = Wp + DP * DB * DLW;      // [DB][DB] factor of the current 8 x 8 block, by rows
-    double *rd = Ls + DB * DB;            // [DB] 1 / its diagonal
-    int *flag = reinterpret_cast<int *>(rd + DB);
+    // of each panel: [DB][DB] factor of its 8 x 8 block by rows, [DB] 1 / its diagonal
+    double *L8 = Wp + DP * DB * DLW;
+    int *flag = reinterpret_cast<int *>(L8 + DP * (DB * DB + DB));
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const double *blk = A + (long long)c0 * ld + c0;
     if (w == NB && (ld & 1) == 0 && (c0 & 1) == 0) {
@@ -423,121 +453,198 @@ __global__ void __launch_bounds__(BLK_THREADS, 1)
         __syncthreads();
         for (int k = w + tid; k < NB; k += BLK_THREADS) T[k * DLT + k] = 1.0;
     }
-    if (tid == 0) *flag = 0;
+    if (tid == 0) *flag = DP;   // the panel whose factor failed
     __syncthreads();
 
     // phase A of panel p (warp 0)
+    double a[DB][DB], rinv[DB];
     auto factor = [&](int p) {
         const int o = DB * p;
-        double a[DB][DB], rinv[DB];
+        double *Ls = L8 + p * (DB * DB + DB), *rd = Ls + DB * DB;
 #pragma unroll
         for (int c = 0; c < DB; ++c)
 #pragma unroll
-            for (int r = c; r < DB; ++r) a[r][c] = T[(o + c) * DLT + o + r];
-        const int bad = chol8(a, rinv);
-        if (o + bad < w && bad < DB) {
+            for (int r = c & ~1; r < DB; r += 2) {
+                const double2 v = *reinterpret_cast<const double2 *>(T + (o + c) * DLT + o + r);
+                if (r >= c) a[r][c] = v.x;
+                a[r + 1][c] = v.y;
+            }
+        if (chol8(a, rinv)) {   // (the same in every lane)
             if (lane == 0) {
-                *info = c0 + o + bad + 1;
-                atomicExch(skip, 1);
-                *flag = 1;
+#pragma unroll
+                for (int r = 0; r < DB; ++r)
+#pragma unroll
+                    for (int c = 0; c <= r; c += 2)
+                        *reinterpret_cast<double2 *>(Ls + r * DB + c) =
+                            make_double2(a[r][c], c + 1 <= r ? a[r][c + 1] : 0.0);
+#pragma unroll
+                for (int c = 0; c < DB; c += 2)
+                    *reinterpret_cast<double2 *>(rd + c) = make_double2(rinv[c], rinv[c + 1]);
             }
             return;
         }
         if (lane == 0) {
-#pragma unroll
-            for (int c = 0; c < DB; ++c) {
-                rd[c] = rinv[c];
-#pragma unroll
-                for (int r = c; r < DB; ++r) {
-                    Ls[r * DB + c] = a[r][c];
-                    T[(o + c) * DLT + o + r] = a[r][c];
-                }
+            const int bad = chol8_any(T + o * DLT + o, Ls, rd);
+            if (o + bad < w && bad < DB) {
+                *info = c0 + o + bad + 1;
+                atomicExch(skip, 1);
+                *flag = p;
             }
         }
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < DB; ++r) {
+            rinv[r] = rd[r];
+#pragma unroll
+            for (int c = 0; c <= r; ++c) a[r][c] = Ls[r * DB + c];
+        }
     };
-    if (warp == 0) factor(0);
-    for (int p = 0; p < DP; ++p) {
-        const int o = DB * p, below = NB - o - DB;
-        __syncthreads();
-        if (*flag) return;   // block-uniform after the barrier
-        // ---- B: rows below the panel's diagonal block, and its inverse
-        if (tid < below) {
-            double *x = T + o * DLT + o + DB + tid;
-            double v[DB];
+    // the panels' barrier; false, in every thread, when panel p's factor failed
+    // (warp 0 may be at p + 1 already)
+    auto next_panel = [&](int p) {
+        asm volatile("bar.sync 0;" ::: "memory");
+        return *(volatile int *)flag > p;
+    };
+    if (warp == 0) {
+        factor(0);
+        for (int p = 0; p < DP; ++p) {
+            const int o = DB * p;
+            if (!next_panel(p)) return;
+            if (p == DP - 1) {
+                asm volatile("bar.arrive 1, %0;" ::"n"(32 * (BLK_WORK + 1)) : "memory");
+                break;
+            }
+            // the next 8 rows (lanes 8 .. 31 repeat lanes 0 .. 7)
+            double *x = T + o * DLT + o + DB + (lane & 7), v[DB];
 #pragma unroll
             for (int c = 0; c < DB; ++c) v[c] = x[c * DLT];
 #pragma unroll
             for (int c = 0; c < DB; ++c) {
-                v[c] *= rd[c];
+                v[c] *= rinv[c];
 #pragma unroll
-                for (int k = c + 1; k < DB; ++k) v[k] = fma(-v[c], Ls[k * DB + c], v[k]);
+                for (int k = c + 1; k < DB; ++k) v[k] = fma(-v[c], a[k][c], v[k]);
             }
+            __syncwarp();
+            if (lane < DB)
 #pragma unroll
-            for (int c = 0; c < DB; ++c) x[c * DLT] = v[c];
-        } else if (warp == BLK_WARPS - 1 && lane < DB) {
-            // column `lane` of W_pp
-            double s[DB];
-#pragma unroll
-            for (int r = 0; r < DB; ++r) s[r] = r == lane ? 1.0 : 0.0;
-#pragma unroll
-            for (int r = 0; r < DB; ++r) {
-                s[r] *= rd[r];
-#pragma unroll
-                for (int k = r + 1; k < DB; ++k) s[k] = fma(-Ls[k * DB + r], s[r], s[k]);
-            }
-#pragma unroll
-            for (int r = 0; r < DB; ++r) Wp[(p * DB + r) * DLW + lane] = s[r];
+                for (int c = 0; c < DB; ++c) x[c * DLT] = v[c];
+            __syncwarp();
+            asm volatile("bar.arrive 1, %0;" ::"n"(32 * (BLK_WORK + 1)) : "memory");
+            double2 *t = reinterpret_cast<double2 *>(T + (o + DB + (lane >> 2)) * DLT + o + DB +
+                                                     2 * (lane & 3));
+            double d[2] = {t->x, t->y};
+            chol_tile(d, T, o, p + 1, p + 1, lane);
+            *t = make_double2(d[0], d[1]);
+            __syncwarp();
+            factor(p + 1);
         }
-        __syncthreads();
-        // ---- C
-        if (warp == 0) {
-            if (p + 1 < DP) {
-                chol_tile(T, o, p + 1, p + 1, lane);
-                __syncwarp();
-                factor(p + 1);
-            }
-            continue;
-        }
-        // W row block p first (the longer chains): block column j to warp 1 + j
-        if (warp - 1 < p) {
-            const int j = warp - 1, i4 = lane >> 2, k4 = lane & 3;
-            double m0[2] = {0.0, 0.0}, m1[2] = {0.0, 0.0};
-            for (int k = j; k < p; ++k) {
-                // A = L_pk, B = W_kj, K = 8 in two steps
-                const double *l = T + (DB * k + k4) * DLT + o + i4;
-                const double *wk = k == j ? Wp + (DB * j + k4) * DLW + i4
-                                          : T + (DB * k + k4) * DLT + DB * j + i4;
-                const int ws = k == j ? DLW : DLT;
-                dmma(m0, l[0], wk[0]);
-                dmma(m1, l[4 * DLT], wk[4 * ws]);
-            }
-            m0[0] += m1[0];
-            m0[1] += m1[1];
-            // W_pj = -W_pp M: M from its accumulator lanes into B fragments
-            double d[2] = {0.0, 0.0};
+    } else if ((warp & 3) == 0) {
+        for (int p = 0; p < DP; ++p)
+            if (!next_panel(p)) return;
+    } else {
+        const int wk = warp - 1 - (warp >> 2);   // worker 0 .. BLK_WORK - 1
+        // tile number BLK_WORK s + wk from the last column backwards (1 + 2 + ..
+        // tiles of columns DP - 1, DP - 2, ..)
+        constexpr int NS = (DP * (DP + 1) / 2 + BLK_WORK - 1) / BLK_WORK;
+        double acc[NS][2];
+        int kr[NS];   // DP column + row of the tile; -1: none
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int src = (k4 + 4 * h) * 4 + (i4 >> 1);
-                const double e0 = __shfl_sync(FULL, m0[0], src), e1 = __shfl_sync(FULL, m0[1], src);
-                dmma(d, -Wp[(o + i4) * DLW + k4 + 4 * h], (i4 & 1) ? e1 : e0);
+        for (int s = 0; s < NS; ++s) {
+            int u = 0, t = BLK_WORK * s + wk;
+            while (t > u) t -= ++u;
+            kr[s] = u < DP ? (DP - 1 - u) * DP + DP - 1 - u + t : -1;
+            if (kr[s] >= 0) {
+                const double2 v = *reinterpret_cast<const double2 *>(
+                    T + (DB * (kr[s] / DP) + (lane >> 2)) * DLT + DB * (kr[s] % DP) +
+                    2 * (lane & 3));
+                acc[s][0] = v.x;
+                acc[s][1] = v.y;
             }
-            *reinterpret_cast<double2 *>(T + (o + i4) * DLT + DB * j + 2 * k4) =
-                make_double2(d[0], d[1]);
         }
-        // trailing tiles but the next diagonal one, column by column
-        const int m = DP - 1 - p, ntile = m * (m + 1) / 2 - 1;
-        for (int t = BLK_WARPS - 1 - warp; t < ntile; t += BLK_WARPS - 1) {
-            // tile t + 1 of the triangle: columns q = 0 .. m - 1 of m - q tiles
-            int q = 0, left = t + 1;
-            while (left >= m - q) left -= m - q++;
-            chol_tile(T, o, p + 1 + q, p + 1 + q + left, lane);
+        for (int p = 0; p < DP; ++p) {
+            const int o = DB * p, below = NB - o - DB;
+            if (!next_panel(p)) return;
+            const double *Ls = L8 + p * (DB * DB + DB), *rd = Ls + DB * DB;
+            // ---- B: the other rows below, and the inverse of the diagonal block
+            const int row = 32 * wk + lane;
+            if (row < below - DB) {
+                double *x = T + o * DLT + o + DB + DB + row;
+                double v[DB];
+#pragma unroll
+                for (int c = 0; c < DB; ++c) v[c] = x[c * DLT];
+#pragma unroll
+                for (int c = 0; c < DB; ++c) {
+                    v[c] *= rd[c];
+#pragma unroll
+                    for (int k = c + 1; k < DB; ++k) v[k] = fma(-v[c], Ls[k * DB + c], v[k]);
+                }
+#pragma unroll
+                for (int c = 0; c < DB; ++c) x[c * DLT] = v[c];
+            } else if (wk == BLK_WORK - 1 && lane < DB) {
+                // column `lane` of W_pp
+                double s[DB];
+#pragma unroll
+                for (int r = 0; r < DB; ++r) s[r] = r == lane ? 1.0 : 0.0;
+#pragma unroll
+                for (int r = 0; r < DB; ++r) {
+                    s[r] *= rd[r];
+#pragma unroll
+                    for (int k = r + 1; k < DB; ++k) s[k] = fma(-Ls[k * DB + r], s[r], s[k]);
+                }
+#pragma unroll
+                for (int r = 0; r < DB; ++r) Wp[(p * DB + r) * DLW + lane] = s[r];
+            }
+            asm volatile("bar.sync 1, %0;" ::"n"(32 * (BLK_WORK + 1)) : "memory");
+            // ---- C: the tiles of later columns (the next diagonal one is warp 0's)
+#pragma unroll
+            for (int s = 0; s < NS; ++s) {
+                const int kb = kr[s] / DP, rb = kr[s] % DP;
+                if (kr[s] >= 0 && kb > p && (kb > p + 1 || rb > kb)) {
+                    chol_tile(acc[s], T, o, kb, rb, lane);
+                    if (kb == (rb == kb ? p + 2 : p + 1))
+                        *reinterpret_cast<double2 *>(T + (DB * kb + (lane >> 2)) * DLT + DB * rb +
+                                                     2 * (lane & 3)) =
+                            make_double2(acc[s][0], acc[s][1]);
+                }
+            }
+            // W row block p first (the longer chains): block column j to worker j,
+            // those beyond the workers to the ones with the shortest chains
+            for (int j = wk; j < p; j = 2 * BLK_WORK - 1 - j, j = j < BLK_WORK ? p : j) {
+                const int i4 = lane >> 2, k4 = lane & 3;
+                double m0[2] = {0.0, 0.0}, m1[2] = {0.0, 0.0};
+#pragma unroll 4
+                for (int k = j; k < p; ++k) {
+                    // A = L_pk, B = W_kj, K = 8 in two steps
+                    const double *l = T + (DB * k + k4) * DLT + o + i4;
+                    const double *wkj = k == j ? Wp + (DB * j + k4) * DLW + i4
+                                               : T + (DB * k + k4) * DLT + DB * j + i4;
+                    const int ws = k == j ? DLW : DLT;
+                    dmma(m0, l[0], wkj[0]);
+                    dmma(m1, l[4 * DLT], wkj[4 * ws]);
+                }
+                m0[0] += m1[0];
+                m0[1] += m1[1];
+                // W_pj = -W_pp M: M from its accumulator lanes into B fragments
+                double d[2] = {0.0, 0.0};
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int src = (k4 + 4 * h) * 4 + (i4 >> 1);
+                    const double e0 = __shfl_sync(FULL, m0[0], src), e1 = __shfl_sync(FULL, m0[1], src);
+                    dmma(d, -Wp[(o + i4) * DLW + k4 + 4 * h], (i4 & 1) ? e1 : e0);
+                }
+                *reinterpret_cast<double2 *>(T + (o + i4) * DLT + DB * j + 2 * k4) =
+                    make_double2(d[0], d[1]);
+            }
         }
     }
     __syncthreads();
     double *ablk = A + (long long)c0 * ld + c0;
     for (int idx = tid; idx < w * NB; idx += BLK_THREADS) {
         const int k = idx / NB, r = idx - k * NB;
-        if (r < w && r >= k) ablk[(long long)k * ld + r] = T[k * DLT + r];
+        if (r < w && r >= k)
+            ablk[(long long)k * ld + r] =
+                r / DB == k / DB ? L8[(r / DB) * (DB * DB + DB) + (r % DB) * DB + k % DB]
+                                 : T[k * DLT + r];
     }
     // W column-major, two rows per 16-byte store
     for (int idx = tid; idx < NB * NB / 2; idx += BLK_THREADS) {
@@ -554,22 +661,17 @@ __global__ void __launch_bounds__(BLK_THREADS, 1)
     }
 }
 
-// L_21 = A_21 W^T for rows r0 + 64 blockIdx.x ... of the panel (column c0 ..
-// c0 + 127), written over A_21, plus the S digit planes d[s][row][k] (kp =
-// NB) and row exponents of L_21 for the tensor-core trailing update.
-//
-// Products by FP64 mma.sync: warp v holds columns 8 v .. and 8 (15 - v) .. of
-// all 64 rows, so that every warp walks 17 blocks of W's triangle (on the FP64
-// units with 4 x 8 register tiles the kernel took 31 us for 5,000 rows, most of
-// it in shared-memory loads).
+// L_21 = A_21 W^T for rows r0 + 16 blockIdx.x ... of the outer panel (columns
+// c0 .. c0 + 127), written over A_21.  Products by FP64 mma.sync: warp v holds
+// columns 8 v .. and 8 (15 - v) .., so that every warp walks 17 blocks of W's
+// triangle.  At most 384 rows and on the critical path: few rows per CTA, so
+// that loading W is what is left of its time.
 //
 // Shared memory: Ws[k * LDP + c] = W[c][k] (= Wout, column-major W); Xs[k *
 // LDX + r] = A[row r][c0 + k], then the rows of L_21.
-template <int S>
 __global__ void __launch_bounds__(PANEL_THREADS)
     chol_panel_kernel(double *__restrict__ A, long long ld, int c0, int r0, int m,
-                      const double *__restrict__ Wout, int8_t *__restrict__ dpl,
-                      int *__restrict__ dex, const int *skip) {
+                      const double *__restrict__ Wout, const int *skip) {
     if (*(volatile const int *)skip) return;
     extern __shared__ __align__(16) double sm[];
     double *Ws = sm;
@@ -579,10 +681,11 @@ __global__ void __launch_bounds__(PANEL_THREADS)
 #pragma unroll 8
     for (int idx = tid; idx < NB * NB / 2; idx += PANEL_THREADS) {
         const int k = idx / (NB / 2), c = 2 * (idx - k * (NB / 2));
-        cp_async(Ws + k * LDP + c, Wout + 2 * idx, 16, true);
+        if (c + 1 >= k) cp_async(Ws + k * LDP + c, Wout + 2 * idx, 16, true);
+        else Ws[k * LDP + c] = Ws[k * LDP + c + 1] = 0.0;
     }
     const double *arows = A + (long long)c0 * ld + r0 + rbase;
-#pragma unroll 8
+#pragma unroll
     for (int idx = tid; idx < NB * PR; idx += PANEL_THREADS) {
         const int k = idx / PR, r = idx - k * PR;
         const bool v = rbase + r < m;
@@ -590,15 +693,15 @@ __global__ void __launch_bounds__(PANEL_THREADS)
     }
     cp_async_wait_all();
     __syncthreads();
-    static_assert(PANEL_THREADS / 32 == NB / 16 && PR == 64, "two column tiles a warp");
+    static_assert(PANEL_THREADS / 32 == NB / 16, "two column tiles a warp");
     const int t0 = warp, t1 = NB / 8 - 1 - warp;   // column tiles, t0 < t1
+    const int i4 = lane >> 2, k4 = lane & 3;
     double acc[2][PR / 8][2];
 #pragma unroll
     for (int h = 0; h < 2; ++h)
 #pragma unroll
         for (int i = 0; i < PR / 8; ++i) acc[h][i][0] = acc[h][i][1] = 0.0;
     {
-        const int i4 = lane >> 2, k4 = lane & 3;
         const double *xk = Xs + k4 * LDX + i4, *wk = Ws + k4 * LDP + i4;
         // W[c][k] = 0 for k > c
         for (int k = 0; k < 8 * (t1 + 1); k += 4, xk += 4 * LDX, wk += 4 * LDP) {
@@ -614,70 +717,274 @@ __global__ void __launch_bounds__(PANEL_THREADS)
                 for (int i = 0; i < PR / 8; ++i) dmma(acc[0][i], x[i], b0);
             }
         }
-        __syncthreads();   // every warp is past its loads of the rows
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-            for (int i = 0; i < PR / 8; ++i)
-#pragma unroll
-                for (int u = 0; u < 2; ++u)
-                    Xs[(8 * (h ? t1 : t0) + 2 * k4 + u) * LDX + 8 * i + i4] = acc[h][i][u];
     }
+    __syncthreads();   // every warp is past its loads of the rows
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int i = 0; i < PR / 8; ++i)
+#pragma unroll
+            for (int u = 0; u < 2; ++u)
+                Xs[(8 * (h ? t1 : t0) + 2 * k4 + u) * LDX + 8 * i + i4] = acc[h][i][u];
     __syncthreads();
     for (int idx = tid; idx < NB * PR; idx += PANEL_THREADS) {
         const int c = idx / PR, r = idx - c * PR;
         if (rbase + r < m) A[(long long)(c0 + c) * ld + r0 + rbase + r] = Xs[c * LDX + r];
     }
-    // digit planes: a warp per row, lane l holds columns l, l + 32, l + 64, l + 96
-    const long long plane = (long long)m * NB;
-    for (int rl = warp; rl < PR; rl += PANEL_THREADS / 32) {
-        const int row = rbase + rl;
-        if (row >= m) break;
-        double v[4], mx = 0.0;
+}
+
+// The rest of the outer panel's diagonal block -= L_21 L_21^T (rows and columns
+// r0 .. r0 + m - 1, lower triangle, K = 128) by FP64 mma.sync: one 32 x 32 tile
+// per CTA, tile first + blockIdx.x of the triangle by rows (the first ten are
+// the next 128-column block).
+__global__ void __launch_bounds__(PANEL_THREADS)
+    chol_update_kernel(double *__restrict__ A, long long ld, int c0, int r0, int m, int first,
+                       const int *skip) {
+    if (*(volatile const int *)skip) return;
+    extern __shared__ __align__(16) double sm[];
+    double *Xi = sm, *Xj = sm + NB * LDU;   // [k][row] of the tile's rows and columns
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int ti = 0, tj = first + blockIdx.x;
+    while (tj > ti) tj -= ++ti;
+    const int ri = UT * ti, rj = UT * tj;
+    const double *src = A + (long long)c0 * ld + r0;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            v[q] = Xs[(lane + 32 * q) * LDX + rl];
-            mx = fmax(mx, fabs(v[q]));
+    for (int idx = tid; idx < NB * UT; idx += PANEL_THREADS) {
+        const int k = idx / UT, r = idx - k * UT;
+        const bool vi = ri + r < m, vj = rj + r < m;
+        cp_async(Xi + k * LDU + r, vi ? src + (long long)k * ld + ri + r : src, 8, vi);
+        cp_async(Xj + k * LDU + r, vj ? src + (long long)k * ld + rj + r : src, 8, vj);
+    }
+    // D's rows are columns of the tile: a lane's two values are neighbours in memory
+    const int i4 = lane >> 2, k4 = lane & 3;
+    const int col = 8 * (warp & 3) + i4, row = 16 * (warp >> 2) + 2 * k4;
+    double *out = A + (long long)(r0 + rj + col) * ld + r0 + ri + row;
+    double old[2][2];
+    bool ok[2][2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int r = ri + row + 8 * h + u;
+            ok[h][u] = r < m && r >= rj + col;
+            old[h][u] = ok[h][u] ? out[8 * h + u] : 0.0;
         }
+    cp_async_wait_all();
+    __syncthreads();
+    double acc[2][2][2] = {};
+    const double *xj = Xj + k4 * LDU + col, *xi = Xi + k4 * LDU + 16 * (warp >> 2) + i4;
+#pragma unroll 4
+    for (int k = 0; k < NB; k += 8) {
 #pragma unroll
-        for (int o = 16; o; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        for (int v = 0; v < 2; ++v) {
+            const double a = xj[(k + 4 * v) * LDU];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) dmma(acc[v][h], a, xi[(k + 4 * v) * LDU + 8 * h]);
+        }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+            if (ok[h][u]) out[8 * h + u] = old[h][u] - (acc[0][h][u] + acc[1][h][u]);
+}
+
+// Rows below an outer panel's diagonal block: X L_D^T = A for RT rows of all
+// 512 columns per CTA, written over A, with the digit planes and row exponents
+// for the trailing updates.  Block column j: X_j = (A_j - sum_{k<j} X_k
+// L_jk^T) W_j^T, FP64 mma.sync, the rows resident in shared memory and L_jk,
+// W_j streamed through it 16 columns at a time.
+//
+// Bound by the FP64 rate (RT x 147,456 multiply-adds).  One pass replaces four
+// panel solves, three tensor-core updates of the panel's other columns and a
+// slicing pass, which had to run one behind the other beside the bulk update.
+//
+// Xs[k * LDF + r] = A[row r][o0 + k], then X; stage: Bs[k * LDP + c].  Stages
+// of 32 columns and fragments one step ahead: with 16 columns, or every
+// fragment of a stage loaded before its products, shared-memory loads and
+// addressing added 1,000 cycles to the 1,024 of a stage's products (RT = 32).
+template <int RT>
+struct FarCfg {
+    static constexpr int LDF = RT + 4;   // 4 mod 16
+    static constexpr int BKF = 32, NST = RT > 16 ? 2 : 4;
+    static constexpr size_t SMEM =
+        ((size_t)NB2 * LDF + (size_t)NST * BKF * LDP) * sizeof(double);
+};
+
+template <int S, int RT>
+__global__ void __launch_bounds__(FAR_THREADS)
+    chol_far_kernel(double *__restrict__ A, long long ld, int o0, int first, int last, int m,
+                    const double *__restrict__ W, int8_t *__restrict__ dpl,
+                    int *__restrict__ dex, const int *skip) {
+    using C = FarCfg<RT>;
+    constexpr int LDF = C::LDF, BKF = C::BKF, NST = C::NST, NC = NB / BKF;
+    if (*(volatile const int *)skip) return;
+    extern __shared__ __align__(16) double sm[];
+    double *Xs = sm, *Bs = sm + NB2 * LDF;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int rbase = first + blockIdx.x * RT;
+    double *arows = A + (long long)o0 * ld + o0 + NB2 + rbase;
+    for (int idx = tid; idx < NB2 * RT; idx += FAR_THREADS) {
+        const int k = idx / RT, r = idx - k * RT;
+        const bool v = rbase + r < last;
+        cp_async(Xs + k * LDF + r, v ? arows + (long long)k * ld + r : arows, 8, v);
+    }
+    // the stream of chunks: for each j, those of columns 0 .. 128 j - 1 of L's
+    // block row j, then those of W_j
+    const bool vec = (ld & 1) == 0;
+    constexpr int KT = 2 * FAR_THREADS / NB;   // columns a pass of the block's threads (vec)
+    const int lk = tid / (NB / 2), lc = 2 * (tid % (NB / 2));
+    const double *src_l = A + (long long)(o0 + lk) * ld + o0 + lc, *src_w = W + 2 * tid;
+    int lj = 0, lt = 0, ls = 0;
+    auto load = [&] {
+        if (lj < NB2 / NB) {
+            const bool w = lt >= NC * lj;
+            const double *src = w ? src_w : src_l + (long long)(lt * BKF) * ld + NB * lj;
+            const long long sld = w ? NB : ld;
+            double *dst = Bs + ls * BKF * LDP;
+            if (vec || w) {
+#pragma unroll
+                for (int k = 0; k < BKF; k += KT)
+                    cp_async(dst + (lk + k) * LDP + lc, src + k * sld, 16, true);
+            } else {
+                for (int k = 0; k < BKF; k += KT)
+                    for (int u = 0; u < 2; ++u)
+                        cp_async(dst + (lk + k) * LDP + lc + u, src + k * sld + u, 8, true);
+            }
+            if (w) src_w += BKF * NB;
+            if (++lt == NC * (lj + 1)) {
+                lt = 0;
+                ++lj;
+            }
+            ls = ls + 1 == NST ? 0 : ls + 1;
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    for (int q = 0; q < NST - 1; ++q) load();
+    // warp v: all rows, column tiles v and 15 - v (the same share of a triangle)
+    constexpr int RW = RT / 8;
+    static_assert(FAR_THREADS / 32 == NB / 16, "two column tiles a warp");
+    const int t0 = warp, t1 = NB / 8 - 1 - warp;
+    const int i4 = lane >> 2, k4 = lane & 3;
+    double acc[2][RW][2];
+    auto clear = [&] {
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int i = 0; i < RW; ++i) acc[h][i][0] = acc[h][i][1] = 0.0;
+    };
+    // own elements of block column j: Xs = sub ? Xs - acc : acc
+    auto put = [&](int j, bool sub) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int i = 0; i < RW; ++i)
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    double *x = Xs + (NB * j + 8 * (h ? t1 : t0) + 2 * k4 + u) * LDF + 8 * i + i4;
+                    *x = sub ? *x - acc[h][i][u] : acc[h][i][u];
+                }
+    };
+    auto multiply = [&](const double *xk, const double *bk, auto both) {
+        constexpr bool BOTH = decltype(both)::value;
+        double x[2][RW], b[2][2];
+        auto fetch = [&](int k) {
+            b[k & 1][1] = bk[4 * k * LDP + 8 * t1];
+            if constexpr (BOTH) b[k & 1][0] = bk[4 * k * LDP + 8 * t0];
+#pragma unroll
+            for (int i = 0; i < RW; ++i) x[k & 1][i] = xk[4 * k * LDF + 8 * i];
+        };
+        fetch(0);
+#pragma unroll
+        for (int k = 0; k < BKF / 4; ++k) {
+            if (k + 1 < BKF / 4) fetch(k + 1);
+#pragma unroll
+            for (int i = 0; i < RW; ++i) {
+                dmma(acc[1][i], x[k & 1][i], b[k & 1][1]);
+                if constexpr (BOTH) dmma(acc[0][i], x[k & 1][i], b[k & 1][0]);
+            }
+        }
+    };
+    int st = 0;
+    for (int j = 0; j < NB2 / NB; ++j) {
+        clear();
+        for (int t = 0; t < NC * (j + 1); ++t) {
+            const bool w = t >= NC * j;
+            if (t == NC * j && j > 0) {
+                put(j, true);
+                clear();
+            }
+            asm volatile("cp.async.wait_group %0;" ::"n"(NST - 2) : "memory");
+            __syncthreads();   // the chunk has landed, the one before is read, the rows are written
+            load();
+            // k of the chunk within the block column whose rows it multiplies;
+            // W[c][k] = 0 for k > c
+            const int k0 = w ? (t - NC * j) * BKF : 0;
+            const double *xk = Xs + (t * BKF + k4) * LDF + i4;
+            const double *bk = Bs + (st * BKF + k4) * LDP + i4;
+            st = st + 1 == NST ? 0 : st + 1;
+            if (k0 < 8 * (t0 + 1)) multiply(xk, bk, std::true_type{});
+            else if (k0 < 8 * (t1 + 1)) multiply(xk, bk, std::false_type{});
+        }
+        __syncthreads();   // every warp is past its loads of block column j
+        put(j, false);
+    }
+    __syncthreads();
+    for (int idx = tid; idx < NB2 * RT; idx += FAR_THREADS) {
+        const int k = idx / RT, r = idx - k * RT;
+        if (rbase + r < last) arows[(long long)k * ld + r] = Xs[k * LDF + r];
+    }
+    // digit planes: a warp per row, lane l holds columns l, l + 32, ...
+    const long long plane = (long long)m * NB2;
+    for (int rl = warp; rl < RT; rl += FAR_THREADS / 32) {
+        const int row = rbase + rl;
+        if (row >= last) break;
+        double mx = 0.0;
+#pragma unroll
+        for (int c = 0; c < NB2 / 32; ++c) mx = fmax(mx, fabs(Xs[(lane + 32 * c) * LDF + rl]));
+#pragma unroll
+        for (int o = 16; o; o >>= 1) mx = fmax(mx, __shfl_xor_sync(FULL, mx, o));
         const int ex = oz_row_exponent(mx);
         if (lane == 0) dex[row] = ex;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
+        int8_t *d = dpl + (long long)row * NB2 + lane;
+#pragma unroll 4
+        for (int c = 0; c < NB2 / 32; ++c) {
             int8_t dg[S];
-            oz_digits<S>(ldexp(v[q], -ex), dg);
+            oz_digits<S>(oz_scale2(Xs[(lane + 32 * c) * LDF + rl], -ex), dg);
 #pragma unroll
-            for (int s = 0; s < S; ++s) dpl[s * plane + (long long)row * NB + lane + 32 * q] = dg[s];
+            for (int s = 0; s < S; ++s) d[s * plane + 32 * c] = dg[s];
         }
     }
 }
 
-template <int S>
-kfb_status launch_panel(double *A, long long ld, int c0, int r0, int m, const double *W,
-                        int8_t *dpl, int *dex, const int *skip, cudaStream_t s) {
+template <int S, int RT>
+kfb_status launch_far(double *A, long long ld, int o0, int first, int rows, int m, const double *W,
+                      int8_t *dpl, int *dex, const int *skip, cudaStream_t s) {
+    using C = FarCfg<RT>;
     static bool attr = false;
     if (!attr) {
-        KFB_CUDA_TRY(cudaFuncSetAttribute(chol_panel_kernel<S>,
+        KFB_CUDA_TRY(cudaFuncSetAttribute(chol_far_kernel<S, RT>,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)PANEL_SMEM));
+                                          (int)C::SMEM));
         attr = true;
     }
-    chol_panel_kernel<S><<<(m + PR - 1) / PR, PANEL_THREADS, PANEL_SMEM, s>>>(A, ld, c0, r0, m, W,
-                                                                             dpl, dex, skip);
+    chol_far_kernel<S, RT><<<(rows + RT - 1) / RT, FAR_THREADS, C::SMEM, s>>>(
+        A, ld, o0, first, first + rows, m, W, dpl, dex, skip);
     KFB_CUDA_TRY(cudaGetLastError());
     return KFB_OK;
 }
 
-kfb_status panel(int S, double *A, long long ld, int c0, int r0, int m, const double *W,
-                 int8_t *dpl, int *dex, const int *skip, cudaStream_t s) {
+// Rows first .. first + rows - 1 (of the m below the outer panel at o0), RT per CTA.
+template <int RT>
+kfb_status far_rows(int S, double *A, long long ld, int o0, int first, int rows, int m,
+                    const double *W, int8_t *dpl, int *dex, const int *skip, cudaStream_t s) {
     switch (S) {
-        case 2: return launch_panel<2>(A, ld, c0, r0, m, W, dpl, dex, skip, s);
-        case 3: return launch_panel<3>(A, ld, c0, r0, m, W, dpl, dex, skip, s);
-        case 4: return launch_panel<4>(A, ld, c0, r0, m, W, dpl, dex, skip, s);
-        case 5: return launch_panel<5>(A, ld, c0, r0, m, W, dpl, dex, skip, s);
-        case 6: return launch_panel<6>(A, ld, c0, r0, m, W, dpl, dex, skip, s);
-        case 7: return launch_panel<7>(A, ld, c0, r0, m, W, dpl, dex, skip, s);
+        case 2: return launch_far<2, RT>(A, ld, o0, first, rows, m, W, dpl, dex, skip, s);
+        case 3: return launch_far<3, RT>(A, ld, o0, first, rows, m, W, dpl, dex, skip, s);
+        case 4: return launch_far<4, RT>(A, ld, o0, first, rows, m, W, dpl, dex, skip, s);
+        case 5: return launch_far<5, RT>(A, ld, o0, first, rows, m, W, dpl, dex, skip, s);
+        case 6: return launch_far<6, RT>(A, ld, o0, first, rows, m, W, dpl, dex, skip, s);
+        case 7: return launch_far<7, RT>(A, ld, o0, first, rows, m, W, dpl, dex, skip, s);
         default: return set_error(KFB_ERR_INVALID_ARG, "digit planes S=%d", S);
     }
 }
@@ -687,11 +994,11 @@ kfb_status panel(int S, double *A, long long ld, int c0, int r0, int m, const do
 namespace {
 
 // The streams of the look-ahead, per device: the critical path (diagonal
-// blocks, panels, the updates the next block waits for) at the highest
-// priority, the rest of the inner updates below it, the bulk trailing updates
-// at the lowest.
+// blocks, the rows and updates the next ones wait for) at the highest priority,
+// the rest of a diagonal block's updates beside it, the rows below and the next
+// panel's columns after that, the bulk trailing updates at the lowest.
 struct CholStreams {
-    cudaStream_t crit = nullptr, inner = nullptr, bulk = nullptr;
+    cudaStream_t crit = nullptr, near = nullptr, far = nullptr, bulk = nullptr;
 };
 
 kfb_status chol_streams(CholStreams *&out) {
@@ -704,8 +1011,10 @@ kfb_status chol_streams(CholStreams *&out) {
         int least = 0, greatest = 0;
         KFB_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&least, &greatest));
         KFB_CUDA_TRY(cudaStreamCreateWithPriority(&cs.crit, cudaStreamNonBlocking, greatest));
-        KFB_CUDA_TRY(cudaStreamCreateWithPriority(&cs.inner, cudaStreamNonBlocking,
+        KFB_CUDA_TRY(cudaStreamCreateWithPriority(&cs.near, cudaStreamNonBlocking,
                                                   std::min(greatest + 1, least)));
+        KFB_CUDA_TRY(cudaStreamCreateWithPriority(&cs.far, cudaStreamNonBlocking,
+                                                  std::min(greatest + 2, least)));
         KFB_CUDA_TRY(cudaStreamCreateWithPriority(&cs.bulk, cudaStreamNonBlocking, least));
     }
     out = &cs;
@@ -714,7 +1023,7 @@ kfb_status chol_streams(CholStreams *&out) {
 
 // Events of one factorisation, destroyed with it.
 struct CholEvents {
-    cudaEvent_t ev[8] = {};
+    cudaEvent_t ev[12] = {};
     kfb_status init() {
         for (auto &e : ev) KFB_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         return KFB_OK;
@@ -741,30 +1050,35 @@ kfb_status chol_dense(double *A, int n, long long ld, int slices, int *info, cud
         KFB_CUDA_TRY(cudaFuncSetAttribute(chol_block_kernel,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)BLK_SMEM));
+        KFB_CUDA_TRY(cudaFuncSetAttribute(chol_panel_kernel,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)PANEL_SMEM));
+        KFB_CUDA_TRY(cudaFuncSetAttribute(chol_update_kernel,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)UPD_SMEM));
         attr = true;
     }
     // the diagonal blocks in FP32 for an FP32-class factor (4 or fewer planes)
     const bool f32blk = slices <= 4;
     CholStreams *cs = nullptr;
     KFB_TRY(chol_streams(cs));
-    const cudaStream_t sc = cs->crit, si = cs->inner, sb = cs->bulk;
+    const cudaStream_t sc = cs->crit, sn = cs->near, sf = cs->far, sb = cs->bulk;
     CholEvents E;
     KFB_TRY(E.init());
-    cudaEvent_t ev_start = E.ev[0], ev_slice = E.ev[1], ev_bulk = E.ev[2], ev_crit_end = E.ev[3],
-                ev_bulk_end = E.ev[4], ev_panel = E.ev[5], ev_inner = E.ev[6];
+    cudaEvent_t ev_start = E.ev[0], ev_panel = E.ev[1], ev_near = E.ev[2], ev_diag = E.ev[3],
+                ev_rows = E.ev[4], ev_far = E.ev[5], ev_next = E.ev[6], ev_bulk = E.ev[7];
+    cudaEvent_t ev_free[2] = {E.ev[8], E.ev[9]};   // the bulk update has read these digit planes
+    cudaEvent_t ev_end = E.ev[10], ev_bulk_end = E.ev[11];
     // everything below is ordered after the caller's work on s
     KFB_CUDA_TRY(cudaEventRecord(ev_start, s));
     KFB_CUDA_TRY(cudaStreamWaitEvent(sc, ev_start, 0));
-    KFB_CUDA_TRY(cudaStreamWaitEvent(sb, ev_start, 0));
     // flags: [0] info, [1] skip, [2] GEMM pipeline error
-    DevBuf flags, Wd, psl, pex, osl[2], oex[2];
+    DevBuf flags, Wd, osl[2], oex[2];
     KFB_TRY(flags.alloc(4 * sizeof(int), sc));
     KFB_TRY(zero(flags.ptr, 4 * sizeof(int), sc));
     int *d_info = flags.as<int>(), *d_skip = d_info + 1, *d_err = d_info + 2;
-    const long long mmax = std::max(n - NB, 1);
-    KFB_TRY(Wd.alloc((size_t)NB * NB * sizeof(double), sc));
-    KFB_TRY(psl.alloc((size_t)slices * mmax * NB, sc));
-    KFB_TRY(pex.alloc((size_t)mmax * sizeof(int), sc));
+    // inverted diagonal blocks of two outer panels
+    KFB_TRY(Wd.alloc((size_t)2 * NB2 * NB * sizeof(double), sc));
     if (n > NB2)
         for (int b = 0; b < 2; ++b) {
             KFB_TRY(osl[b].alloc((size_t)slices * (n - NB2) * NB2, sc));
@@ -773,19 +1087,13 @@ kfb_status chol_dense(double *A, int n, long long ld, int slices, int *info, cud
     // on an early (error) return, let the streams finish before the buffers
     // above are released (destroyed after this guard)
     struct Drain {
-        cudaStream_t a, b, c;
+        cudaStream_t st[4];
         bool armed = true;
         ~Drain() {
-            if (armed) {
-                cudaStreamSynchronize(a);
-                cudaStreamSynchronize(b);
-                cudaStreamSynchronize(c);
-            }
+            if (armed)
+                for (cudaStream_t t : st) cudaStreamSynchronize(t);
         }
-    } drain{sc, si, sb};
-    // the bulk stream's first work reads buffers allocated on the critical one
-    KFB_CUDA_TRY(cudaEventRecord(ev_slice, sc));
-    KFB_CUDA_TRY(cudaStreamWaitEvent(sb, ev_slice, 0));
+    } drain{{sc, sn, sf, sb}};
     OzEpi epi;
     epi.c = A;
     epi.ldr = 1;
@@ -793,111 +1101,114 @@ kfb_status chol_dense(double *A, int n, long long ld, int slices, int *info, cud
     epi.skip = d_skip;
     epi.mode = OZ_ADD;
     epi.alpha = -1.0;
+    epi.tiles_per_cta = 1;
     OzEpi epi_bulk = epi;
-    epi_bulk.one_tile_per_cta = 1;
-    bool bulk_pending = false;   // a bulk update was enqueued and not waited for
-    bool inner_pending = false;  // the rest of an inner update, likewise
+    epi_bulk.tiles_per_cta = BULK_TILES;
+    bool next_pending = false;   // the columns of this outer panel below its diagonal block
+    bool bulk_pending = false;   // a bulk update of later columns
     for (int o0 = 0, P = 0; o0 < n; o0 += NB2, ++P) {
         const int ow = std::min(NB2, n - o0);   // outer panel: columns o0 .. o0 + ow - 1
+        double *W = Wd.as<double>() + (size_t)(P & 1) * NB2 * NB;
+        // ---- its ow x ow diagonal block
+        bool near_pending = false;   // the rest of an update within it
         for (int c0 = o0; c0 < o0 + ow; c0 += NB) {
             const int w = std::min(NB, n - c0);
-            const int r0 = c0 + w, m = n - r0;
+            const int r0 = c0 + w, m = o0 + ow - r0;
+            double *Wj = W + (size_t)((c0 - o0) / NB) * NB * NB;
             if (f32blk)
-                chol_block_kernel<<<1, BLK_THREADS, BLK_SMEM, sc>>>(
-                    A, ld, c0, w, Wd.as<double>(), d_info, d_skip);
+                chol_block_kernel<<<1, BLK_THREADS, BLK_SMEM, sc>>>(A, ld, c0, w, Wj, d_info,
+                                                                    d_skip);
             else
-                chol_block64_kernel<<<1, BLK_THREADS, DBLK_SMEM, sc>>>(
-                    A, ld, c0, w, Wd.as<double>(), d_info, d_skip);
+                chol_block64_kernel<<<1, BLK_THREADS, DBLK_SMEM, sc>>>(A, ld, c0, w, Wj, d_info,
+                                                                       d_skip);
             KFB_CUDA_TRY(cudaGetLastError());
             // (the block itself was updated ahead of the rest of its columns)
-            if (inner_pending) {
-                KFB_CUDA_TRY(cudaStreamWaitEvent(sc, ev_inner, 0));
-                inner_pending = false;
-            }
+            if (near_pending) KFB_CUDA_TRY(cudaStreamWaitEvent(sc, ev_near, 0));
+            near_pending = false;
             if (m == 0) break;
-            // L21 = A21 W^T and its digit planes
-            KFB_TRY(panel(slices, A, ld, c0, r0, m, Wd.as<double>(), psl.as<int8_t>(),
-                          pex.as<int>(), d_skip, sc));
-            // the rest of the outer panel: columns r0 .. o0 + ow - 1, every row
-            // below them, -= L21 L21^T (a lower trapezoid)
-            const int nin = o0 + ow - r0;
-            if (nin > 0) {
-                OzSlices Pl;
-                Pl.d = psl.as<int8_t>();
-                Pl.e = pex.as<int>();
-                Pl.S = slices;
-                Pl.rows = m;
-                Pl.kp = NB;
-                OzGen g;
-                g.mode = OZ_GEN_LOWER;
-                g.M = m;
-                g.N = nin;
-                g.c_off = (long long)r0 * ld + r0;
-                // the next diagonal block first (its row of tiles), then the
-                // rest beside that block's factorisation
-                const int all = oz_gen_tiles(g, slices);
-                g.count = std::min(all, (std::min(NB, nin) + oz_bn(slices) - 1) / oz_bn(slices));
+            chol_panel_kernel<<<(m + PR - 1) / PR, PANEL_THREADS, PANEL_SMEM, sc>>>(A, ld, c0, r0, m,
+                                                                                   Wj, d_skip);
+            KFB_CUDA_TRY(cudaGetLastError());
+            // the next 128 x 128 block first, the rest beside its factorisation
+            const int nt = (m + UT - 1) / UT, all = nt * (nt + 1) / 2;
+            const int head = std::min(all, (NB / UT) * (NB / UT + 1) / 2);
+            if (all > head) {
                 KFB_CUDA_TRY(cudaEventRecord(ev_panel, sc));
-                KFB_TRY(oz_gemm_gen(Pl, Pl, g, epi, d_err, sc));
-                if (all > g.count) {
-                    KFB_CUDA_TRY(cudaStreamWaitEvent(si, ev_panel, 0));
-                    g.first = g.count;
-                    g.count = all - g.first;
-                    KFB_TRY(oz_gemm_gen(Pl, Pl, g, epi_bulk, d_err, si));
-                    KFB_CUDA_TRY(cudaEventRecord(ev_inner, si));
-                    inner_pending = true;
-                }
+                KFB_CUDA_TRY(cudaStreamWaitEvent(sn, ev_panel, 0));
+                chol_update_kernel<<<all - head, PANEL_THREADS, UPD_SMEM, sn>>>(A, ld, c0, r0, m,
+                                                                               head, d_skip);
+                KFB_CUDA_TRY(cudaGetLastError());
+                KFB_CUDA_TRY(cudaEventRecord(ev_near, sn));
+                near_pending = true;
             }
+            chol_update_kernel<<<head, PANEL_THREADS, UPD_SMEM, sc>>>(A, ld, c0, r0, m, 0, d_skip);
+            KFB_CUDA_TRY(cudaGetLastError());
         }
-        // everything right of the outer panel -= L_panel L_panel^T (K = ow, the
-        // panel sliced once more with one row scale over its columns), in two
-        // parts: the next outer panel's columns on the critical stream (the
-        // next panel's blocks wait for them), the rest on the bulk stream,
-        // where it overlaps the next panel's blocks, panels and inner updates
         const int R = o0 + ow, M = n - R;
-        if (M <= 0) continue;
+        if (M <= 0) break;
+        // ---- the rows below: those of the next diagonal block on the critical
+        // stream, the rest on the far one
         OzSlices O;
         O.d = osl[P & 1].as<int8_t>();
         O.e = oex[P & 1].as<int>();
         O.S = slices;
         O.rows = M;
-        O.kp = oz_kp(ow);
-        KFB_TRY(oz_slice_cols(A + (long long)o0 * ld + R, M, ow, ld, O, sc));
-        KFB_CUDA_TRY(cudaEventRecord(ev_slice, sc));
-        // the previous bulk update wrote these columns too: wait for it
-        if (bulk_pending) KFB_CUDA_TRY(cudaStreamWaitEvent(sc, ev_bulk, 0));
+        O.kp = NB2;
         const int na = std::min(NB2, M);
-        OzGen ga;
-        ga.mode = OZ_GEN_LOWER;
-        ga.M = M;
-        ga.N = na;
-        ga.c_off = (long long)R * ld + R;
-        KFB_TRY(oz_gemm_gen(O, O, ga, epi, d_err, sc));
-        if (M > na) {
-            KFB_CUDA_TRY(cudaStreamWaitEvent(sb, ev_slice, 0));
-            OzGen gb;
-            gb.mode = OZ_GEN_LOWER;
-            gb.M = M - na;
-            gb.N = M - na;
-            gb.a_base = na;
-            gb.b_base = na;
-            gb.c_off = (long long)(R + na) * ld + (R + na);
-            KFB_TRY(oz_gemm_gen(O, O, gb, epi_bulk, d_err, sb));
-            KFB_CUDA_TRY(cudaEventRecord(ev_bulk, sb));
-            bulk_pending = true;
-        } else {
-            bulk_pending = false;
+        if (P >= 2) KFB_CUDA_TRY(cudaStreamWaitEvent(sc, ev_free[P & 1], 0));
+        KFB_CUDA_TRY(cudaEventRecord(ev_diag, sc));
+        if (next_pending) KFB_CUDA_TRY(cudaStreamWaitEvent(sc, ev_next, 0));
+        KFB_TRY(far_rows<8>(slices, A, ld, o0, 0, na, M, W, O.d, O.e, d_skip, sc));
+        KFB_CUDA_TRY(cudaEventRecord(ev_rows, sc));
+        // ---- the next diagonal block -= L L^T (K = 512); the last bulk update
+        // wrote it too
+        OzGen g;
+        g.mode = OZ_GEN_LOWER;
+        g.M = g.N = na;
+        g.c_off = (long long)R * ld + R;
+        if (bulk_pending) KFB_CUDA_TRY(cudaStreamWaitEvent(sc, ev_bulk, 0));
+        KFB_TRY(oz_gemm_gen(O, O, g, epi, d_err, sc));
+        next_pending = M > na;
+        if (M <= na) continue;
+        KFB_CUDA_TRY(cudaStreamWaitEvent(sf, ev_diag, 0));
+        KFB_TRY(far_rows<32>(slices, A, ld, o0, na, M - na, M, W, O.d, O.e, d_skip, sf));
+        KFB_CUDA_TRY(cudaEventRecord(ev_far, sf));
+        // the next outer panel's columns below its diagonal block
+        KFB_CUDA_TRY(cudaStreamWaitEvent(sf, ev_rows, 0));
+        if (bulk_pending) KFB_CUDA_TRY(cudaStreamWaitEvent(sf, ev_bulk, 0));
+        g.mode = OZ_GEN_RECT;
+        g.M = M - na;
+        g.a_base = na;
+        g.c_off += na;
+        KFB_TRY(oz_gemm_gen(O, O, g, epi, d_err, sf));
+        KFB_CUDA_TRY(cudaEventRecord(ev_next, sf));
+        // everything right of them: the columns of the outer panel after the
+        // next one first, which is all that the other streams wait for
+        KFB_CUDA_TRY(cudaStreamWaitEvent(sb, ev_far, 0));
+        g.mode = OZ_GEN_LOWER;
+        for (int c = na; c < M; c = c == na && M > na + NB2 ? na + NB2 : M) {
+            g.M = M - c;
+            g.N = c == na ? std::min(NB2, M - na) : M - c;
+            g.a_base = g.b_base = c;
+            g.c_off = (long long)(R + c) * ld + (R + c);
+            KFB_TRY(oz_gemm_gen(O, O, g, epi_bulk, d_err, sb));
+            if (c == na) KFB_CUDA_TRY(cudaEventRecord(ev_bulk, sb));
         }
+        KFB_CUDA_TRY(cudaEventRecord(ev_free[P & 1], sb));
+        bulk_pending = true;
     }
-    // join both streams back into the caller's
-    KFB_CUDA_TRY(cudaEventRecord(ev_crit_end, sc));
-    KFB_CUDA_TRY(cudaEventRecord(ev_bulk_end, sb));
-    KFB_CUDA_TRY(cudaStreamWaitEvent(s, ev_crit_end, 0));
-    KFB_CUDA_TRY(cudaStreamWaitEvent(s, ev_bulk_end, 0));
+    // join the streams back into the caller's (the near stream has been waited
+    // for; the far one by the critical one)
+    KFB_CUDA_TRY(cudaEventRecord(ev_end, sc));
+    KFB_CUDA_TRY(cudaStreamWaitEvent(s, ev_end, 0));
+    if (bulk_pending) {
+        KFB_CUDA_TRY(cudaEventRecord(ev_bulk_end, sb));
+        KFB_CUDA_TRY(cudaStreamWaitEvent(s, ev_bulk_end, 0));
+    }
     int h[3] = {0, 0, 0};
     KFB_CUDA_TRY(cudaMemcpyAsync(h, d_info, 3 * sizeof(int), cudaMemcpyDeviceToHost, s));
     KFB_CUDA_TRY(cudaStreamSynchronize(s));
-    drain.armed = false;   // both streams joined into s, which is idle now
+    drain.armed = false;   // the streams joined into s, which is idle now
     if (h[2]) return set_error(KFB_ERR_TIMEOUT, "Cholesky: a tensor-core pipeline wait timed out");
     *info = h[0];
     return KFB_OK;

@@ -97,7 +97,6 @@ __host__ __device__ __forceinline__ int lower_tiles(int ti, int ntc, int BN) {
 __host__ __device__ __forceinline__ OzTile gen_tile(const OzGen &g, int BN, long long ldr,
                                                     long long ldc, int t) {
     const int ntc = (g.N + BN - 1) / BN;
-    t += g.first;
     int ti = 0, tj = t;
     if (g.mode == OZ_GEN_LOWER) {
         // row tiles 0 .. full - 1 have r (ti + 1) column tiles, the others all of them
@@ -526,7 +525,8 @@ kfb_status launch(const OzSlices &A, const OzSlices &B, const OzTile *tiles, con
                                           cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
         attr[S] = true;
     }
-    const int grid = epi.one_tile_per_cta ? ntiles : std::min(ntiles, device_sm_count());
+    const int tpc = epi.tiles_per_cta;
+    const int grid = tpc ? (ntiles + tpc - 1) / tpc : std::min(ntiles, device_sm_count());
     oz_gemm_kernel<S><<<grid, NUM_THREADS, C::SMEM, s>>>(ta, tb, A.rows, B.rows, A.kp, A.e, B.e,
                                                          tiles, gen, ntiles, epi, err);
     KFB_CUDA_TRY(cudaGetLastError());
@@ -749,7 +749,7 @@ kfb_status oz_gemm(const OzSlices &A, const OzSlices &B, const OzTile *tiles, in
 
 kfb_status oz_gemm_gen(const OzSlices &A, const OzSlices &B, const OzGen &g, const OzEpi &epi,
                        int *err, cudaStream_t s) {
-    return oz_gemm_core(A, B, nullptr, g, g.count >= 0 ? g.count : oz_gen_tiles(g, A.S), epi, err,
+    return oz_gemm_core(A, B, nullptr, g, oz_gen_tiles(g, A.S), epi, err,
                         s);
 }
 

@@ -76,10 +76,10 @@ struct OzEpi {
     int mode = OZ_STORE;
     double alpha = 1.0;
     const int *skip = nullptr;   // device flag: when non-zero the launch does nothing
-    // one CTA per tile instead of one persistent CTA per SM: the SMs free up
-    // tile by tile, so kernels of a higher-priority stream can start between
-    // tiles (the Cholesky's look-ahead runs its bulk updates this way)
-    int one_tile_per_cta = 0;
+    // so many tiles per CTA instead of one persistent CTA per SM: the SMs free
+    // up as the launch proceeds, so that kernels of a higher-priority stream can
+    // start (the Cholesky's look-ahead); 0: persistent
+    int tiles_per_cta = 0;
 };
 
 // C tiles = alpha * A . B^T (both operands sliced with the same S and kp).
@@ -100,7 +100,6 @@ struct OzGen {
     int M = 0, N = 0;
     int a_base = 0, b_base = 0;
     long long c_off = 0;
-    int first = 0, count = -1;   // tiles first .. first + count - 1 of the set (-1: all)
 };
 // tiles of the whole set
 int oz_gen_tiles(const OzGen &g, int S);

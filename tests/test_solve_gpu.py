@@ -101,6 +101,52 @@ def test_potrf_block_edges(n):
         assert cgk.rfp_potrf(K, n, 0.0, "L") == k + 1
 
 
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+@pytest.mark.parametrize("n", [1023, 1024, 1025, 1058, 1571, 2081])
+def test_potrf_outer_panels(n, dtype):
+    """Several outer panels: rows below a panel that end inside a row tile of either size (8 for the
+    next diagonal block, 32 beyond it), an odd leading dimension, every stream of the look-ahead;
+    the solve with the factor, and a pivot made negative in a later panel.  Tolerances as in
+    test_rfp_potrf_potrs_match_lapack."""
+    import torch
+
+    from kernelforge_b200 import cuda_global_kernels as cgk
+    A = spd(n, n + 3, cond=50.0)
+    arf, _ = lapack.dtrttf(np.asfortranarray(A), transr="N", uplo="L")
+    ref, _ = lapack.dpftrf(n, (arf + 0.0).copy(), transr="N", uplo="L")
+    K = torch.tensor(arf, dtype=getattr(torch, dtype), device="cuda")
+    assert cgk.rfp_potrf(K, n, 0.0, "L") == 0
+    tol = 1e-11 if dtype == "float64" else 2e-4
+    np.testing.assert_allclose(K.cpu().numpy(), ref, rtol=tol, atol=tol)
+    b = np.random.default_rng(n).standard_normal(n)
+    B = torch.tensor(b, dtype=getattr(torch, dtype), device="cuda").reshape(n, 1).contiguous()
+    cgk.rfp_potrs(K, B, "L")
+    np.testing.assert_allclose(A @ B.cpu().numpy().ravel(), b, rtol=50 * tol, atol=50 * tol)
+    k = n - 3
+    A[k, k] = -1.0
+    arf, _ = lapack.dtrttf(np.asfortranarray(A), transr="N", uplo="L")
+    K = torch.tensor(arf, dtype=getattr(torch, dtype), device="cuda")
+    assert cgk.rfp_potrf(K, n, 0.0, "L") == k + 1
+
+
+@pytest.mark.parametrize("p", [-920, 920])
+def test_potrf_pivots_out_of_the_fast_range(p):
+    """Pivots beyond 2^+-900 take the library's reciprocal square root: a power-of-four scale of the
+    matrix scales the factor exactly, up to rounding of the two routes (1e-14 each)."""
+    import torch
+
+    from kernelforge_b200 import cuda_global_kernels as cgk
+    n = 150
+    A = spd(n, 3, cond=50.0)
+    arf, _ = lapack.dtrttf(np.asfortranarray(A), transr="N", uplo="L")
+    K = torch.tensor(arf, dtype=torch.float64, device="cuda")
+    S = torch.tensor(np.ldexp(arf, p), dtype=torch.float64, device="cuda")
+    assert cgk.rfp_potrf(K, n, 0.0, "L") == 0
+    assert cgk.rfp_potrf(S, n, 0.0, "L") == 0
+    np.testing.assert_allclose(np.ldexp(S.cpu().numpy(), -p // 2), K.cpu().numpy(), rtol=1e-12,
+                               atol=1e-13)
+
+
 def test_rfp_potrf_reports_info():
     import torch
 
