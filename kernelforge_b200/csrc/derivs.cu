@@ -907,7 +907,8 @@ __global__ void jmax_per_mol_kernel(const T *__restrict__ dx, int ma, int rep,
 }
 
 // Kernel 1 with t from P: the same outputs as hess_t_kernel (W, Tt, bound;
-// without the rank term in Y (rank_in_y = 0) the bound is max|J_b| sum_j w_ij);
+// without the rank term in Y (rank_in_y = 0) the bound is max|J_b| sum_j w_ij
+// and t is left to hess_rank_kernel, Tt null);
 // weights from the centred dot products G[(a, i)][(b - b0) * ma2 + j] (row
 // length ldg) and the norms; t by a warp per (same-label pair, 32 columns).  P
 // (row length ldp) holds the projections of same-label atoms only: atom (a, i)
@@ -988,7 +989,7 @@ __global__ void __launch_bounds__(256) hess_t_p_kernel(
     const int *prow_a = prow + (size_t)(pr.a - a0) * ma1;
     const int *pcol_b = pcol + (size_t)(pr.b - b0) * ma2;
     const float *PBb = PB + (size_t)pr.b * ma2 * ld2;
-    for (int it = warp; it < npairs * nchunk; it += nwarp) {
+    for (int it = warp; Tt && it < npairs * nchunk; it += nwarp) {
         const int q = it / nchunk, cc = it - q * nchunk;
         int i, j;
         pair_ij(q, i, j);
@@ -1270,22 +1271,35 @@ __global__ void __launch_bounds__(256, 2) hess_y_kernel(
 // projection GEMM problem per label and batch over the label's atoms of the
 // batch's molecules b and the Jacobian rows of its atoms in the batch's
 // molecules a; mu_l the label centre that also centres P).  qrow / qcol map
-// atoms of molecules b0.. / a0.. to their row / first column of Q.  This kernel adds that term to the pair's Hessian block after
-// the contraction wrote it: block per (pair, 64 x 64 tile of (c', c)),
-// 256 threads of 4 x 4 register tiles, the same-label pairs in chunks of HR_Q
-// with their s and t' rows staged in shared memory.  Every output element
-// belongs to one thread of one block and the contraction ran before on the
-// same stream, so the adds need no atomics.  ma1, ma2 <= HR_MAXA.
+// atoms of molecules b0.. / a0.. to their row / first column of Q.  t' is formed
+// here from the weights and the projections, as hess_t_p_kernel does it (written
+// there and read back it moved 3.5 GB more per 45,000 pairs of 21 atoms and the
+// two kernels took 10.1 ms; now 4.8).  This kernel adds that term to the
+// pair's Hessian block after the contraction wrote it: block per (pair, 64 x 64
+// tile of (c', c)), 256 threads of 4 x 4 register tiles, the same-label pairs in
+// chunks of HR_Q with their s and t' rows staged in shared memory, the next
+// chunk's operands in flight meanwhile and their addresses found by one thread
+// per pair (every thread for itself: 6.5 ms instead of 4.5).  Instruction issue
+// and the loads' latency bound it.
+// Every output element belongs to one thread of one block and the contraction
+// ran before on the same stream, so the adds need no atomics.  ma1, ma2 <=
+// HR_MAXA.
 constexpr int HR_Q = 32, HR_T = 64, HR_MAXA = 64;
-__global__ void __launch_bounds__(256) hess_rank_kernel(
+struct HrPair {
+    const float *q, *p, *pb1, *pb;   // rows of Q, P, PB1 and PB from the tile's first column
+    float w;                         // w'_ij
+};
+__global__ void __launch_bounds__(256, 3) hess_rank_kernel(
     const HessPair *__restrict__ pairs, const int *__restrict__ perm1,
     const int *__restrict__ lab1, const int *__restrict__ perm2, const int *__restrict__ lab2,
     int ma1, int ma2, const float *__restrict__ Q, long long ldq, const int *__restrict__ qrow,
-    const int *__restrict__ qcol, int a0, int b0, const float *__restrict__ PB1, const float *__restrict__ Tt, const int *__restrict__ off1,
-    const int *__restrict__ off2, int symmetric, ElemSink sink) {
+    const int *__restrict__ qcol, int a0, int b0, const float *__restrict__ PB1,
+    const float *__restrict__ W, float is2, const float *__restrict__ P, long long ldp,
+    const int *__restrict__ prow, const int *__restrict__ pcol, const float *__restrict__ PB,
+    const int *__restrict__ off1, const int *__restrict__ off2, int symmetric, ElemSink sink) {
     __shared__ int4 groups[HR_MAXA];
     __shared__ int pa[HR_MAXA], pb[HR_MAXA], la[HR_MAXA], lb[HR_MAXA], gstart[HR_MAXA + 1];
-    __shared__ int qi[HR_Q], qj[HR_Q];
+    __shared__ HrPair list[2][HR_Q];   // the pairs of this chunk and the next
     __shared__ int ngroups;
     __shared__ __align__(16) float Ss[HR_Q][HR_T];
     __shared__ __align__(16) float Ts[HR_Q][HR_T];
@@ -1314,42 +1328,67 @@ __global__ void __launch_bounds__(256) hess_rank_kernel(
     }
     __syncthreads();
     const int npairs = gstart[ngroups];
+    const float *Wp = W + (size_t)p * ma1 * ma2;
+    // operand rows of the pairs of a chunk, a thread per pair
+    auto build = [&](int q0) {
+        const int q = q0 + tid;
+        if (tid >= HR_Q || q >= npairs) return;
+        int g = 0;
+        while (gstart[g + 1] <= q) ++g;
+        const int4 gr = groups[g];
+        const int off = q - gstart[g], nbg = gr.w - gr.z;
+        const int i = pa[gr.x + off / nbg], j = pb[gr.z + off % nbg];
+        HrPair e;
+        e.q = Q + (size_t)qrow[(size_t)(pr.b - b0) * ma2 + j] * ldq +
+              qcol[(size_t)(pr.a - a0) * ma1 + i] + r0;
+        e.p = P + (size_t)prow[(size_t)(pr.a - a0) * ma1 + i] * ldp +
+              pcol[(size_t)(pr.b - b0) * ma2 + j] + c0;
+        e.pb1 = PB1 + ((size_t)pr.a * ma1 + i) * ld1 + r0;
+        e.pb = PB + ((size_t)pr.b * ma2 + j) * ld2 + c0;
+        e.w = Wp[i * ma2 + j] * is2;
+        list[(q0 / HR_Q) & 1][tid] = e;
+    };
     const int ty = tid >> 4, tx = tid & 15;
-    const size_t arow = (size_t)pr.a * ma1;
-    const int *qrow_b = qrow + (size_t)(pr.b - b0) * ma2;
-    const int *qcol_a = qcol + (size_t)(pr.a - a0) * ma1;
-    const float *Tp = Tt + (size_t)p * ma1 * ma2 * ld2;
+    // staging: thread (er, eq) column er of rows eq, eq + 4, ... of a chunk
+    const int er = tid & (HR_T - 1), eq = tid / HR_T;
+    constexpr int NE = HR_Q * HR_T / 256;
+    const bool vs = r0 + er < m1, vt = c0 + er < n2;
+    float s1[NE], s2[NE], t1[NE], t2[NE], w[NE];
+    auto fetch = [&](int q0) {
+#pragma unroll
+        for (int k = 0; k < NE; ++k) {
+            const HrPair &e = list[(q0 / HR_Q) & 1][eq + 4 * k];
+            s1[k] = s2[k] = t1[k] = t2[k] = w[k] = 0.f;
+            if (q0 + eq + 4 * k < npairs) {
+                w[k] = e.w;
+                if (vs) {
+                    s1[k] = e.pb1[er];
+                    s2[k] = e.q[er];
+                }
+                if (vt) {
+                    t1[k] = e.p[er];
+                    t2[k] = e.pb[er];
+                }
+            }
+        }
+    };
+    build(0);
+    __syncthreads();
+    fetch(0);
+    build(HR_Q);   // (the other half of the list)
     float acc[4][4] = {};
     for (int q0 = 0; q0 < npairs; q0 += HR_Q) {
-        if (tid < HR_Q) {
-            const int q = q0 + tid;
-            int i = -1, j = -1;
-            if (q < npairs) {
-                int g = 0;
-                while (gstart[g + 1] <= q) ++g;
-                const int4 gr = groups[g];
-                const int off = q - gstart[g], nbg = gr.w - gr.z;
-                i = pa[gr.x + off / nbg];
-                j = pb[gr.z + off % nbg];
-            }
-            qi[tid] = i;
-            qj[tid] = j;
+        if (q0) __syncthreads();   // Ss, Ts read
+#pragma unroll
+        for (int k = 0; k < NE; ++k) {
+            Ss[eq + 4 * k][er] = s1[k] - s2[k];
+            Ts[eq + 4 * k][er] = w[k] * (t1[k] - t2[k]);
         }
         __syncthreads();
-        for (int e = tid; e < HR_Q * HR_T; e += blockDim.x) {
-            const int qq = e / HR_T, r = e - qq * HR_T;
-            const int i = qi[qq], j = qj[qq];
-            float sv = 0.f, tv = 0.f;
-            if (i >= 0) {
-                const size_t col = (arow + i) * ld1;
-                if (r0 + r < m1)
-                    sv = PB1[col + r0 + r] - Q[(size_t)qrow_b[j] * ldq + qcol_a[i] + r0 + r];
-                if (c0 + r < n2) tv = Tp[((size_t)i * ma2 + j) * ld2 + c0 + r];
-            }
-            Ss[qq][r] = sv;
-            Ts[qq][r] = tv;
+        if (q0 + HR_Q < npairs) {
+            fetch(q0 + HR_Q);
+            build(q0 + 2 * HR_Q);   // over the chunk that is in Ss and Ts
         }
-        __syncthreads();
 #pragma unroll 8
         for (int qq = 0; qq < HR_Q; ++qq) {
             const float4 sv = *reinterpret_cast<const float4 *>(&Ss[qq][ty * 4]);
@@ -1360,7 +1399,6 @@ __global__ void __launch_bounds__(256) hess_rank_kernel(
 #pragma unroll
                 for (int v = 0; v < 4; ++v) acc[u][v] = fmaf(sa[u], ta[v], acc[u][v]);
         }
-        __syncthreads();  // Ss, Ts, qi, qj reused
     }
     const int dg = (symmetric && pr.a == pr.b) ? 1 : 0;
 #pragma unroll
@@ -1373,7 +1411,11 @@ __global__ void __launch_bounds__(256) hess_rank_kernel(
             if (C >= n2) continue;
             const double val = -(double)acc[u][v];
             sink_positions(sink, (long long)off1[pr.a] + R, (long long)off2[pr.b] + C, dg,
-                           [&](long long idx) { sink_add(sink, idx, val); });
+                           [&](long long idx) {
+                               // (reductions without a result: no load waits for the store before)
+                               if (sink.f64) atomicAdd(static_cast<double *>(sink.out) + idx, val);
+                               else sink_add(sink, idx, val);
+                           });
         }
     }
 }
@@ -2260,7 +2302,6 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
     batch = std::min(batch, 65535);
     DevBuf W, Tt, Y, dpairs;
     KFB_TRY(W.alloc((size_t)batch * ma1 * ma2 * sizeof(T), s));
-    KFB_TRY(Tt.alloc((size_t)batch * ma1 * ma2 * ld2 * sizeof(T), s));
     if (!tc) KFB_TRY(Y.alloc((size_t)batch * ma1 * rep * ld2 * sizeof(T), s));
     KFB_TRY(dpairs.alloc((size_t)batch * sizeof(HessPair), s));
     std::vector<int> perm1, lab1, perm2, lab2;
@@ -2534,7 +2575,9 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
     } else {
         note_path("hessian:cuda-core-t");
     }
+    if (!hrank) KFB_TRY(Tt.alloc((size_t)batch * ma1 * ma2 * ld2 * sizeof(T), s));
     const size_t smem_p = hess_t_p_smem(ma1, ma2);
+    long long ldp = 0;   // row length of P in this batch
     for (size_t p0 = 0, npz = 0; p0 < pairs.size(); p0 += npz) {
         int np = (int)std::min<size_t>(batch, pairs.size() - p0);
         if (pform)  // the batch's molecules b fit the P buffer
@@ -2566,7 +2609,7 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
                 const int arows = (amax + 1) * ma1 - arow0;
                 std::vector<TcProb> pps;
                 std::vector<int> prow, pcol;
-                const long long ldp = label_problems(
+                ldp = label_problems(
                     lm1, amin, amax, ma1, lm2, bmin, bmax, ma2, ld2, rep,
                     1.0 / ((double)xs_scale * (double)jr_scale), pps, prow, pcol);
                 KFB_CUDA_TRY(cudaMemcpyAsync(d_prow.ptr, prow.data(), prow.size() * sizeof(int),
@@ -2619,7 +2662,8 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
                     d_lab1.as<int>(), d_perm2.as<int>(), d_lab2.as<int>(), ma1, ma2, c2, is2, is4,
                     d_P.as<float>(), ldp, d_prow.as<int>(), d_pcol.as<int>(), amin, bmin,
                     d_pb.as<float>(), d_jbm.as<float>(),
-                    hrank ? 0 : 1, W.as<T>(), Tt.as<T>(), ygemm ? nullptr : yamax.as<float>());
+                    hrank ? 0 : 1, W.as<T>(), hrank ? nullptr : Tt.as<T>(),
+                    ygemm ? nullptr : yamax.as<float>());
                 KFB_CUDA_TRY(cudaGetLastError());
             }
         }
@@ -2750,7 +2794,8 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
                         dpairs.as<HessPair>(), d_perm1.as<int>(), d_lab1.as<int>(),
                         d_perm2.as<int>(), d_lab2.as<int>(), ma1, ma2, d_Q.as<float>(), ldq,
                         d_qrow.as<int>(), d_qcol.as<int>(), amin, bmin,
-                        symmetric ? d_pb.as<float>() : d_pb1.as<float>(), Tt.as<float>(),
+                        symmetric ? d_pb.as<float>() : d_pb1.as<float>(), W.as<float>(), is2,
+                        d_P.as<float>(), ldp, d_prow.as<int>(), d_pcol.as<int>(), d_pb.as<float>(),
                         d_off1.as<int>(), d_off2.as<int>(), symmetric ? 1 : 0, sink);
                     KFB_CUDA_TRY(cudaGetLastError());
                 }
