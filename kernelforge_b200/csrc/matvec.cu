@@ -692,8 +692,10 @@ kfb_status mv_gemm(const OzSlices &A, const OzSlices &B, int M, int N, double *C
 }
 
 // Same-label (query atom, training atom) pairs up to which the direct FP64
-// kernels are used.
-constexpr long long MD_MAX_PAIRS = 6LL << 20;
+// kernels are used: they take 1.1, 1.9, 3.5 and 6.6 ms for 4, 8, 17 and 33
+// million pairs, the label products on the int8 tensor cores (with their
+// launches and host work per label) 1.7, 2.1, 3.1 and 4.6 ms.
+constexpr long long MD_MAX_PAIRS = 10LL << 20;
 constexpr int MD_MAX_REP = 1 << 16;   // (a list of column groups in shared memory)
 
 template <class Tin>
