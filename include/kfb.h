@@ -56,7 +56,7 @@ typedef enum kfb_dtype { KFB_F32 = 0, KFB_F64 = 1 } kfb_dtype;
 
 /* Arithmetic of the distance contraction ||x_i - x_j||^2. */
 typedef enum kfb_precision {
-    KFB_PREC_FP64 = 0,      /* FP64 CUDA cores (the plain FP64 GPU path)           */
+    KFB_PREC_FP64 = 0,      /* FP64 arithmetic (FP64 mma.sync; the plain FP64 path)  */
     KFB_PREC_FP32 = 1,      /* FP32 CUDA cores                                      */
     KFB_PREC_SPLIT_F16 = 2  /* tcgen05 tensor cores: x = hi + lo (fp16 pair),
                                hi*hi + hi*lo + lo*hi with FP32 accumulation in TMEM */
@@ -444,7 +444,7 @@ kfb_status kfb_fchl19_repr(const void *coords, const int32_t *elem, const int32_
  * (held by every GPU that loads the library, until the process exits). */
 #define KFB_NOALLOC_SCRATCH_BYTES (64u << 20)
 
-/* The symmetric scalar kernel of kfb_kernel_gaussian_symm with FP64 CUDA-core
+/* The symmetric scalar kernel of kfb_kernel_gaussian_symm with FP64
  * arithmetic and a double output (layout KFB_DENSE / KFB_RFP_U / KFB_RFP_L),
  * allocating no device memory: for callers that cannot allocate during a call
  * (a host framework that has reserved the device-memory budget up front, or a

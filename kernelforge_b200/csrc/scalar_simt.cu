@@ -1,4 +1,4 @@
-// Scalar FCHL19 local kernel on CUDA cores (FP64 or FP32): the plain GPU
+// Scalar FCHL19 local kernel in FP64 (mma.sync) or FP32 (CUDA cores): the plain
 // path.  Atoms are bucketed by label (one packed, zero-padded row per atom,
 // molecules in order inside a bucket); each CTA computes one 64 x 64 tile of
 // same-label atom pairs, forms e_ij = exp(-(n_i + n_j - 2 x_i.x_j) / 2 sigma^2)

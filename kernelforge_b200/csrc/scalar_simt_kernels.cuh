@@ -1,4 +1,5 @@
-// Device code of the CUDA-core (FP64 / FP32) scalar tile kernel, shared by the
+// Device code of the scalar kernels without a split (FP64 on mma.sync tiles, FP32
+// on CUDA cores), shared by the
 // launchers in scalar_simt.cu and scalar_noalloc.cu.
 #pragma once
 

@@ -8,7 +8,8 @@ names, arguments, shapes and dtypes as src/cuda_local_kernels_bindings.cpp:
   buckets, as the reference does).
 * Scalar kernels run on the tcgen05 tensor cores by default
   (``precision="split_f16"``: two-term fp16 split of the descriptors, FP32
-  accumulation); ``precision="fp32"`` / ``"fp64"`` select CUDA-core paths.
+  accumulation); ``precision="fp32"`` / ``"fp64"`` compute in that precision
+  throughout.
 * RFP outputs use TRANSR='N', Fortran UPLO='L' (unpack with
   ``kernelmath.rfp_to_full(K, n, uplo='U')``) and match ``rfp_potrf``'s default.
 * Work is enqueued on torch's current stream.

@@ -6,7 +6,7 @@ outputs) and exceptions as the pybind11 module (src/local_kernels_bindings.cpp:
 through libkfb: inputs are copied to the device, the kernel runs, the result is
 copied back.  Every function takes one extra keyword-only argument:
 
-``precision``: ``"fp64"`` (default; FP64 CUDA cores, matches the reference's
+``precision``: ``"fp64"`` (default; FP64 throughout, matches the reference's
 FP64 CPU results to rounding), ``"fp32"`` (FP32 CUDA cores) or ``"split_f16"``
 (scalar kernels only: tcgen05 tensor cores with a two-term fp16 split of the
 descriptors and FP32 accumulation; derivative kernels then use FP32).
