@@ -317,7 +317,8 @@ __global__ void __launch_bounds__(JV_THREADS, sizeof(T) == 4 ? 3 : 2) jac_v_kern
 // -------------------------------------------------------- unused columns
 // used[k] = 1 where column k of any real atom (j < nat[m]) is not zero, in x
 // (nm, ma, rep) and, with dx, in its Jacobian's columns c < 3 nat[m] (NaN is
-// not zero); amax (optional): [0] max |x|, [1] max |dx| of the same entries.
+// not zero); amax (optional): [0] max |x|, [1] max |dx| of the same entries,
+// from amax[2 slot] on for an atom with a slot (none for a negative one).
 // Block per atom; the Jacobian is read along its rows, 16 bytes a lane (VEC,
 // rep a multiple of 4), pieces of padding left out: 1.1 GB in 0.2 ms, which is
 // HBM (4 bytes a lane: 0.33 ms).
@@ -326,13 +327,18 @@ __global__ void __launch_bounds__(256) used_columns_kernel(const T *__restrict__
                                                            const T *__restrict__ dx, int ma,
                                                            int rep, const int *__restrict__ nat,
                                                            int *__restrict__ used, int staged,
-                                                           float *__restrict__ amax) {
+                                                           float *__restrict__ amax,
+                                                           const int *__restrict__ slot) {
     // the block's flags; rows too long for 48 KB raise the call's own
     extern __shared__ int uc_s[];   // [rep]
     int *uc = staged ? uc_s : used;
     const int m = blockIdx.x / ma, j = blockIdx.x - m * ma;
     const int na = min(max(nat[m], 0), ma);
     if (j >= na) return;
+    if (slot) {
+        if (slot[blockIdx.x] < 0) return;
+        amax += 2 * slot[blockIdx.x];
+    }
     float mx = 0.f, md = 0.f;
     for (int k = threadIdx.x; k < rep; k += blockDim.x) {
         const T v = x[(size_t)blockIdx.x * rep + k];
@@ -1645,7 +1651,7 @@ size_t budget_bytes() {
 
 template <class T>
 kfb_status scan_columns(const DerivSet &d, int rep, const int *nat, int *used, float *amax,
-                        cudaStream_t s) {
+                        cudaStream_t s, const int *slot) {
     const T *x = static_cast<const T *>(d.x), *dx = static_cast<const T *>(d.dx);
     const long long atoms = (long long)d.v.nm * d.v.ma;
     if (atoms == 0) return KFB_OK;
@@ -1654,14 +1660,14 @@ kfb_status scan_columns(const DerivSet &d, int rep, const int *nat, int *used, f
                      (long long)rep * 3 * d.v.ma < (1LL << 31);
     auto kern = vec ? used_columns_kernel<T, true> : used_columns_kernel<T, false>;
     kern<<<(unsigned)atoms, 256, staged ? rep * sizeof(int) : 0, s>>>(x, dx, d.v.ma, rep, nat, used,
-                                                                      staged ? 1 : 0, amax);
+                                                                      staged ? 1 : 0, amax, slot);
     KFB_CUDA_TRY(cudaGetLastError());
     return KFB_OK;
 }
 template kfb_status scan_columns<float>(const DerivSet &, int, const int *, int *, float *,
-                                        cudaStream_t);
+                                        cudaStream_t, const int *);
 template kfb_status scan_columns<double>(const DerivSet &, int, const int *, int *, float *,
-                                         cudaStream_t);
+                                         cudaStream_t, const int *);
 
 template <class T>
 kfb_status compact_columns(DerivSet &s1, DerivSet &s2, int &rep, CompactSets &keep,

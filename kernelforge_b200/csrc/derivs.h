@@ -109,19 +109,22 @@ __device__ __forceinline__ void sink_positions(const ElemSink &s, long long R, l
 // padded with zero columns to a multiple of 16) and rep by their width.  Either
 // way dx_max of the sets is filled in.  Synchronises the stream (the width is
 // needed on the host).
-// used[k] = 1 (device, rep ints, cleared by the caller) where a real atom of d
-// uses column k in x or dx (null: x alone); amax (optional, device, cleared):
-// [0] max |x|, [1] max |dx| over the real atoms; nat: their counts (device).
-template <class T>
-kfb_status scan_columns(const DerivSet &d, int rep, const int *nat, int *used, float *amax,
-                        cudaStream_t s);
-
 struct CompactSets {
     DevBuf x1, dx1, x2, dx2;
 };
 template <class T>
 kfb_status compact_columns(DerivSet &s1, DerivSet &s2, int &rep, CompactSets &keep,
                            cudaStream_t s);
+
+// The scan that finds them: used[k] = 1 (device, rep ints, cleared by the
+// caller) where a real atom of d uses column k in x or dx (null: x alone); amax
+// (optional, device, cleared): [0] max |x|, [1] max |dx| over the real atoms;
+// nat: their counts (device).  With slot (device, per padded atom) the maxima of
+// an atom go to amax[2 slot], amax[2 slot + 1], and atoms with a negative slot
+// are left out altogether.
+template <class T>
+kfb_status scan_columns(const DerivSet &d, int rep, const int *nat, int *used, float *amax,
+                        cudaStream_t s, const int *slot = nullptr);
 
 // tc: run the contraction GEMMs on the tensor cores (split fp16, three
 // products); needs rep % 16 == 0 and an sm_100 device.

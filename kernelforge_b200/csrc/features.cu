@@ -433,11 +433,13 @@ size_t feature_budget() {
 // Operands of the RFF products (x W_e and dX^T W_e): fp16 pairs with K along
 // the descriptor columns that the atoms use (cols, n of them; W's rows that
 // meet only zeros are left out), K padded with zeros to a multiple of 16, and
-// one power-of-two scale for all of x, of dX and of W.
+// a power-of-two scale for each element's W and for the x and dX of each chunk
+// of an element's atoms: a pair resolves 2^-38 of its scale's largest value, so
+// small elements need scales of their own.
 
-// *amax = max |w|; a column with a value that is not finite counts as used
+// amax[e] = max |w_e|; a column with a value that is not finite counts as used
 // (its products with zeros are not zero).  Rows of d values, row r is column
-// r % rep.
+// r % rep of element r / rep.
 __global__ void __launch_bounds__(256) rff_weight_scan_kernel(const float *__restrict__ w, int rep,
                                                               int d, float *__restrict__ amax,
                                                               int *__restrict__ used) {
@@ -451,7 +453,7 @@ __global__ void __launch_bounds__(256) rff_weight_scan_kernel(const float *__res
     }
     if (bad) used[blockIdx.x % rep] = 1;
     for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<int *>(amax), __float_as_int(m));
+    if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<int *>(amax) + blockIdx.x / rep, __float_as_int(m));
 }
 
 __device__ __forceinline__ void split_fp16(float v, __half &h, __half &l) {
@@ -537,44 +539,62 @@ __global__ void __launch_bounds__(256) rff_jacobian_rows_kernel(
     }
 }
 
-// What both RFF maps prepare: used columns, scales, element rows.
+// What both RFF maps prepare: used columns, scales, element rows.  Chunk r0 /
+// chunk of element e (atoms r0 .. of its list) has the slot first[e] + r0 / chunk.
 struct RffPlan {
     ElemRows er;
     DevBuf cols, err, wh, wl, xh, xl;
-    int n = 0, kpad = 0;
-    float x_scale = 1.f, dx_scale = 1.f, w_scale = 1.f;
+    int n = 0, kpad = 0, chunk = 0;
+    std::vector<int> first;
+    std::vector<float> x_scale, dx_scale, w_scale;   // by slot, by slot, by element
+    int slot(int e, int r0) const { return first[e] + r0 / chunk; }
 };
 
 template <class T>
 kfb_status rff_plan(const T *x, const T *dx, const int *q, const int *n, int nm, int ma, int rep,
-                    const float *w, int nelem, int d, RffPlan &pl, cudaStream_t s) {
+                    const float *w, int nelem, int d, int chunk, RffPlan &pl, cudaStream_t s) {
     KFB_TRY(elem_rows(q, n, nm, ma, nelem, pl.er));
-    // used columns (rep ints), then max |x|, |dx|, |w|
-    DevBuf scan, dn;
-    KFB_TRY(scan.alloc((size_t)rep * sizeof(int) + 3 * sizeof(float), s));
-    KFB_TRY(zero(scan.ptr, (size_t)rep * sizeof(int) + 3 * sizeof(float), s));
+    pl.chunk = chunk;
+    // atom counts, then the slot of every atom (-1: of no element)
+    std::vector<int> atoms((size_t)nm * (ma + 1), -1);
+    std::copy(n, n + nm, atoms.begin());
+    int nslot = 0;
+    for (int e = 0; e < nelem; ++e) {
+        const std::vector<int> &ai = pl.er.idx[e];
+        pl.first.push_back(nslot);
+        for (size_t t = 0; t < ai.size(); ++t)
+            atoms[(size_t)nm + ai[t]] = nslot + (int)(t / (size_t)chunk);
+        nslot += (int)((ai.size() + chunk - 1) / (size_t)chunk);
+    }
+    // used columns (rep ints), then max |w| by element, max |x|, |dx| by slot
+    DevBuf scan, da;
+    const size_t words = (size_t)rep + nelem + 2 * (size_t)nslot;
+    KFB_TRY(scan.alloc(words * sizeof(int), s));
+    KFB_TRY(zero(scan.ptr, words * sizeof(int), s));
     float *amax = reinterpret_cast<float *>(scan.as<int>() + rep);
-    std::vector<int> nat(n, n + nm);
-    KFB_TRY(upload(dn, nat, s));
+    KFB_TRY(upload(da, atoms, s));
     DerivSet ds;
     ds.x = x;
     ds.dx = dx;
-    ds.v.n = nat.data();
+    ds.v.n = atoms.data();
     ds.v.nm = nm;
     ds.v.ma = ma;
-    KFB_TRY(scan_columns<T>(ds, rep, dn.as<int>(), scan.as<int>(), amax, s));
-    rff_weight_scan_kernel<<<(unsigned)(nelem * rep), 256, 0, s>>>(w, rep, d, amax + 2,
+    KFB_TRY(scan_columns<T>(ds, rep, da.as<int>(), scan.as<int>(), amax + nelem, s,
+                            da.as<int>() + nm));
+    rff_weight_scan_kernel<<<(unsigned)(nelem * rep), 256, 0, s>>>(w, rep, d, amax,
                                                                   scan.as<int>());
     KFB_CUDA_TRY(cudaGetLastError());
-    std::vector<int> host(rep + 3), cols;
-    KFB_CUDA_TRY(cudaMemcpyAsync(host.data(), scan.ptr, host.size() * sizeof(int),
+    std::vector<int> host(words), cols;
+    KFB_CUDA_TRY(cudaMemcpyAsync(host.data(), scan.ptr, words * sizeof(int),
                                  cudaMemcpyDeviceToHost, s));
     KFB_CUDA_TRY(cudaStreamSynchronize(s));
-    float mx[3];
-    std::memcpy(mx, host.data() + rep, sizeof(mx));
-    pl.x_scale = pow2_for(mx[0]);
-    pl.dx_scale = pow2_for(mx[1]);
-    pl.w_scale = pow2_for(mx[2]);
+    std::vector<float> mx(words - rep);
+    std::memcpy(mx.data(), host.data() + rep, mx.size() * sizeof(float));
+    for (int e = 0; e < nelem; ++e) pl.w_scale.push_back(pow2_for(mx[e]));
+    for (int k = 0; k < nslot; ++k) {
+        pl.x_scale.push_back(pow2_for(mx[nelem + 2 * k]));
+        pl.dx_scale.push_back(pow2_for(mx[nelem + 2 * k + 1]));
+    }
     for (int k = 0; k < rep; ++k)
         if (host[k]) cols.push_back(k);
     pl.n = (int)cols.size();
@@ -589,10 +609,11 @@ kfb_status rff_plan(const T *x, const T *dx, const int *q, const int *n, int nm,
 }
 
 // W_e as rows of features (B operand of the products)
-kfb_status rff_weights(const RffPlan &pl, const float *w, int d, TcOperand &B, cudaStream_t s) {
+kfb_status rff_weights(const RffPlan &pl, const float *w, int rep, int e, int d, TcOperand &B,
+                       cudaStream_t s) {
     rff_w_rows_kernel<<<dim3(nblk(d, 32), nblk(pl.kpad, 32)), dim3(32, 8), 0, s>>>(
-        w, d, pl.cols.as<int>(), pl.n, pl.kpad, pl.w_scale, pl.wh.as<__half>(),
-        pl.wl.as<__half>());
+        w + (size_t)e * rep * d, d, pl.cols.as<int>(), pl.n, pl.kpad, pl.w_scale[e],
+        pl.wh.as<__half>(), pl.wl.as<__half>());
     KFB_CUDA_TRY(cudaGetLastError());
     B.hi = pl.wh.ptr;
     B.lo = pl.wl.ptr;
@@ -601,13 +622,13 @@ kfb_status rff_weights(const RffPlan &pl, const float *w, int d, TcOperand &B, c
     return KFB_OK;
 }
 
-// Descriptor rows idx[0 .. nr) (device) as the A operand
+// Descriptor rows idx[0 .. nr) (device) of a slot as the A operand
 template <class T>
-kfb_status rff_rows(RffPlan &pl, const T *x, const int *idx, int nr, int rep, TcOperand &A,
-                    cudaStream_t s) {
+kfb_status rff_rows(RffPlan &pl, const T *x, const int *idx, int nr, int rep, int slot,
+                    TcOperand &A, cudaStream_t s) {
     rff_x_rows_kernel<T><<<nblk((long long)nr * pl.kpad, 256 * 8), 256, 0, s>>>(
-        x, idx, nr, rep, pl.cols.as<int>(), pl.n, pl.kpad, pl.x_scale, pl.xh.as<__half>(),
-        pl.xl.as<__half>());
+        x, idx, nr, rep, pl.cols.as<int>(), pl.n, pl.kpad, pl.x_scale[slot],
+        pl.xh.as<__half>(), pl.xl.as<__half>());
     KFB_CUDA_TRY(cudaGetLastError());
     A.hi = pl.xh.ptr;
     A.lo = pl.xl.ptr;
@@ -630,9 +651,10 @@ kfb_status rff_features_t(const T *x, const int *q, const int *n, int nm, int ma
                           cudaStream_t s) {
     KFB_TRY(zero(z, (size_t)nm * d * sizeof(float), s));
     RffPlan pl;
-    KFB_TRY(rff_plan<T>(x, nullptr, q, n, nm, ma, rep, w, nelem, d, pl, s));
-    const size_t row_bytes = (size_t)pl.kpad * 2 * sizeof(__half);
+    // (before the used columns are known: full rows)
+    const size_t row_bytes = (size_t)(rep + 15) / 16 * 16 * 4 * sizeof(__half);
     const int chunk = (int)std::min<size_t>(1 << 30, std::max<size_t>(128, feature_budget() / row_bytes));
+    KFB_TRY(rff_plan<T>(x, nullptr, q, n, nm, ma, rep, w, nelem, d, chunk, pl, s));
     // rows and molecules of every element, one upload
     std::vector<int> rows;
     int most = 1;
@@ -652,15 +674,16 @@ kfb_status rff_features_t(const T *x, const int *q, const int *n, int nm, int ma
         const int ne = (int)pl.er.idx[e].size();
         if (ne == 0) continue;
         TcOperand A, B;
-        KFB_TRY(rff_weights(pl, w + (size_t)e * rep * d, d, B, s));
+        KFB_TRY(rff_weights(pl, w, rep, e, d, B, s));
         for (int r0 = 0; r0 < ne; r0 += chunk) {
             const int nr = std::min(chunk, ne - r0);
-            KFB_TRY(rff_rows<T>(pl, x, idx + r0, nr, rep, A, s));
+            const int slot = pl.slot(e, r0);
+            KFB_TRY(rff_rows<T>(pl, x, idx + r0, nr, rep, slot, A, s));
             TcProb p{};
             p.M = nr;
             p.N = d;
             p.K = pl.kpad;
-            p.alpha = 1.0 / ((double)pl.x_scale * (double)pl.w_scale);
+            p.alpha = 1.0 / ((double)pl.x_scale[slot] * (double)pl.w_scale[e]);
             TcEpi epi;
             epi.mode = EPI_COS_MOLSUM;
             epi.bias = b + (size_t)e * d;
@@ -685,20 +708,21 @@ kfb_status rff_gradient_t(const T *x, const T *dx, const int *q, const int *n, i
     for (int m = 0; m < nm; ++m) offs[m + 1] = offs[m] + 3 * std::min(std::max(n[m], 0), ma);
     KFB_TRY(zero(g, (size_t)std::max(offs[nm], 1) * d * sizeof(float), s));
     RffPlan pl;
-    KFB_TRY(rff_plan<T>(x, dx, q, n, nm, ma, rep, w, nelem, d, pl, s));
-    const int kpad = pl.kpad, ld = 3 * ma;
+    const int ld = 3 * ma;
     // per atom: one row of d sines, one descriptor and up to 3 ma Jacobian rows
+    // (full ones: the used columns are not known yet)
     const size_t atom_bytes = (size_t)d * sizeof(float) +
-                              (size_t)(1 + ld) * kpad * 2 * sizeof(__half) +
-                              (size_t)ld * 2 * sizeof(int);
+                              (size_t)(1 + ld) * ((rep + 15) / 16 * 16) * 4 * sizeof(__half);
     const int chunk = (int)std::min<size_t>((size_t)(1 << 30) / ld,
                                             std::max<size_t>(1, feature_budget() / atom_bytes));
+    KFB_TRY(rff_plan<T>(x, dx, q, n, nm, ma, rep, w, nelem, d, chunk, pl, s));
+    const int kpad = pl.kpad;
     // every element's atoms: descriptor row, then its Jacobian rows, ordered
     // (molecule, c, atom) inside a chunk so that one destination is one run
     std::vector<RffAtom> atoms;
     std::vector<int> idx;
     struct Chunk {
-        int e, a0, na, nr;
+        int e, a0, na, nr, slot;
     };
     std::vector<Chunk> chunks;
     int most_a = 1, most_r = 1;
@@ -706,7 +730,7 @@ kfb_status rff_gradient_t(const T *x, const T *dx, const int *q, const int *n, i
         const std::vector<int> &ai = pl.er.idx[e], &am = pl.er.mol[e];
         for (int a0 = 0; a0 < (int)ai.size(); a0 += chunk) {
             const int na = std::min<int>(chunk, (int)ai.size() - a0);
-            Chunk ck{e, (int)atoms.size(), na, 0};
+            Chunk ck{e, (int)atoms.size(), na, 0, pl.slot(e, a0)};
             int row = 0;
             for (int t = 0; t < na;) {
                 const int m = am[a0 + t];
@@ -741,16 +765,16 @@ kfb_status rff_gradient_t(const T *x, const T *dx, const int *q, const int *n, i
     int elem = -1;
     TcOperand A, B;
     for (const Chunk &ck : chunks) {
-        if (ck.e != elem) KFB_TRY(rff_weights(pl, w + (size_t)ck.e * rep * d, d, B, s));
+        if (ck.e != elem) KFB_TRY(rff_weights(pl, w, rep, ck.e, d, B, s));
         elem = ck.e;
         // sqrt(2/d) sin(x W_e + b_e) of the chunk's atoms: once per atom and
         // feature, not once per Jacobian row (63 of a 21-atom molecule)
-        KFB_TRY(rff_rows<T>(pl, x, didx.as<int>() + ck.a0, ck.na, rep, A, s));
+        KFB_TRY(rff_rows<T>(pl, x, didx.as<int>() + ck.a0, ck.na, rep, ck.slot, A, s));
         TcProb p{};
         p.M = ck.na;
         p.N = d;
         p.K = kpad;
-        p.alpha = 1.0 / ((double)pl.x_scale * (double)pl.w_scale);
+        p.alpha = 1.0 / ((double)pl.x_scale[ck.slot] * (double)pl.w_scale[ck.e]);
         TcEpi epi;
         epi.mode = EPI_DENSE;
         epi.zf32 = sines.as<float>();
@@ -763,7 +787,7 @@ kfb_status rff_gradient_t(const T *x, const T *dx, const int *q, const int *n, i
         // destination row
         rff_jacobian_rows_kernel<T><<<dim3(ck.na, nblk(kpad, 64), nblk(ld, 32)), 256, 0, s>>>(
             dx, datoms.as<RffAtom>() + ck.a0, rep, ld, pl.cols.as<int>(), pl.n, kpad,
-            pl.dx_scale, jh.as<__half>(), jl.as<__half>(), ddst.as<int>(), daux.as<int>());
+            pl.dx_scale[ck.slot], jh.as<__half>(), jl.as<__half>(), ddst.as<int>(), daux.as<int>());
         KFB_CUDA_TRY(cudaGetLastError());
         A.hi = jh.ptr;
         A.lo = jl.ptr;
@@ -773,7 +797,7 @@ kfb_status rff_gradient_t(const T *x, const T *dx, const int *q, const int *n, i
         pj.M = ck.nr;
         pj.N = d;
         pj.K = kpad;
-        pj.alpha = 1.0 / ((double)pl.dx_scale * (double)pl.w_scale);
+        pj.alpha = 1.0 / ((double)pl.dx_scale[ck.slot] * (double)pl.w_scale[ck.e]);
         TcEpi ej;
         ej.mode = EPI_ROW_RUNSUM;
         ej.mol = ddst.as<int>();

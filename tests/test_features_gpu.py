@@ -382,3 +382,36 @@ def test_rff_unused_columns_and_ragged_sizes(rep, used, ma, D):
     Gr = of.rff_gradient_elemental(X.astype(np.float64), dX.astype(np.float64), Q, N, W, b)
     assert rel(Z.cpu().numpy(), Zr) <= 2e-5
     assert np.abs(G.cpu().numpy() - Gr).max() <= 2e-5 * max(1.0, np.abs(Gr).max())
+
+
+@pytest.mark.parametrize("xdtype", ["float32", "float64"])
+def test_rff_elements_of_far_apart_magnitudes(xdtype):
+    """Element 0's descriptors and Jacobians are 2^30 times element 1's and its weights 2^-30 of
+    element 1's, so that both have projections of order one; an atom of no element holds huge
+    values.  An fp16 pair resolves 2^-38 of the largest value that shares its scale: with one
+    scale for both elements element 1 keeps eight bits.  Every molecule holds one element and is
+    compared by itself, with the tolerance of the golden cases."""
+    import torch
+    from kernelforge_b200 import cuda_rff_features as crf
+    rng = np.random.default_rng(41)
+    nm, ma, rep, D = 6, 5, 48, 72
+    N = np.array([5, 5, 4, 3, 5, 4], np.int32)
+    elem = np.array([0, 1, 1, 0, 1, 0])
+    Q = np.repeat(elem[:, None], ma, 1).astype(np.int32)
+    size = np.where(elem == 0, 2.0 ** 15, 2.0 ** -15)
+    X = rng.standard_normal((nm, ma, rep)) * size[:, None, None]
+    dX = rng.standard_normal((nm, ma, rep, 3 * ma)) * size[:, None, None, None]
+    Q[5, 1] = -1
+    X[5, 1] = dX[5, 1] = 2.0 ** 60
+    W = rng.standard_normal((2, rep, D)) / 4 * np.array([2.0 ** -15, 2.0 ** 15])[:, None, None]
+    b = rng.uniform(0, 6.28, (2, D)).astype(np.float32)
+    X, dX, W = X.astype(np.float32), dX.astype(np.float32), W.astype(np.float32)
+    c = lambda a, dt="float32": cuda(a, getattr(torch, dt))
+    Z = crf.rff_features_elemental(c(X, xdtype), Q, N, c(W), c(b)).cpu().numpy()
+    G = crf.rff_gradient_elemental(c(X, xdtype), c(dX, xdtype), Q, N, c(W), c(b)).cpu().numpy()
+    Zr = of.rff_features_elemental(X, Q, N, W, b)
+    Gr = of.rff_gradient_elemental(X, dX, Q, N, W, b)
+    off = np.concatenate([[0], np.cumsum(3 * N)])
+    for m in range(nm):
+        assert rel(Z[m], Zr[m]) <= 2e-5
+        assert rel(G[off[m]:off[m + 1]], Gr[off[m]:off[m + 1]]) <= 2e-5
