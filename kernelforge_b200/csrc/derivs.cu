@@ -2229,7 +2229,7 @@ long long label_problems(const LabelMajor &R, int r0, int r1, int mar, const Lab
 // batch (pairs with that b, in b order, as columns (q, i)), see jk_split_kernel.
 kfb_status hess_y_gemm(const HessPair *pairs, int np, int ma1, int ma2, int rep, int kj,
                        const float *W, const DevBuf &jkh, const DevBuf &jkl, float jk_scale,
-                       float w_scale, float y_scale, DevBuf &wsh, DevBuf &wsl, DevBuf &d_ymap,
+                       float w_scale, const float *y_scale, DevBuf &wsh, DevBuf &wsl, DevBuf &d_ymap,
                        DevBuf &d_border, long long jk_rows, const HessPair *dpairs, __half *yhi,
                        __half *ylo, int *err, cudaStream_t s) {
     const int ld2 = 3 * ma2;
@@ -2248,7 +2248,7 @@ kfb_status hess_y_gemm(const HessPair *pairs, int np, int ma1, int ma2, int rep,
         pb.M = 3 * pr.nb * rep;
         pb.N = (q1 - q) * ma1;
         pb.K = kj;
-        pb.alpha = (double)y_scale / ((double)jk_scale * (double)w_scale);
+        pb.alpha = 1.0 / ((double)jk_scale * (double)w_scale);   // (times *y_scale)
         probs.push_back(pb);
         q = q1;
     }
@@ -2277,6 +2277,7 @@ kfb_status hess_y_gemm(const HessPair *pairs, int np, int ma1, int ma2, int rep,
     epi.y_rep = rep;
     epi.y_ma1 = ma1;
     epi.y_ld2 = ld2;
+    epi.dscale = y_scale;
     return tc_gemm_grouped(A, B, 3, false, probs, ElemSink(), s, epi, err);
 }
 
@@ -2332,7 +2333,7 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
         KFB_TRY(transpose_split_dx<T>(static_cast<const T *>(s1.dx), s1.v.nm, ma1, rep,
                                       d_n1.as<int>(), jth.as<__half>(), jtl.as<__half>(),
                                       &jt_scale, s, s1.dx_max));
-        KFB_TRY(yamax.alloc(sizeof(float), s));
+        KFB_TRY(yamax.alloc(2 * sizeof(float), s));   // the batch's bound of |Y|, its scale
         KFB_TRY(yth.alloc((size_t)batch * ld2 * ma1 * rep * sizeof(__half), s));
         KFB_TRY(ytl.alloc((size_t)batch * ld2 * ma1 * rep * sizeof(__half), s));
     }
@@ -2362,7 +2363,7 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
     // (b, c, k) with kj atom columns, resident for the call
     bool ygemm = false;
     int kj = 0;
-    float w_scale = 1.f, yg_scale = 1.f;
+    float w_scale = 1.f;
     TcErr err;
     if (tc) KFB_TRY(err.init(s));
     DevBuf jkh, jkl, wsh, wsl, d_ymap, d_border;
@@ -2541,13 +2542,12 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
                     ygemm = false;
                 }
             }
-            if (!ygemm) {   // per-molecule max |J| for the bound of |Y|
-                KFB_TRY(d_jbm.alloc((size_t)s2.v.nm * sizeof(float), s));
-                KFB_TRY(zero(d_jbm.ptr, (size_t)s2.v.nm * sizeof(float), s));
-                jmax_per_mol_kernel<float><<<dim3((unsigned)s2.v.nm, 32), 256, 0, s>>>(
-                    dx2f, ma2, rep, d_nat2.as<int>(), d_jbm.as<float>());
-                KFB_CUDA_TRY(cudaGetLastError());
-            }
+            // per-molecule max |J| for the bound of |Y|
+            KFB_TRY(d_jbm.alloc((size_t)s2.v.nm * sizeof(float), s));
+            KFB_TRY(zero(d_jbm.ptr, (size_t)s2.v.nm * sizeof(float), s));
+            jmax_per_mol_kernel<float><<<dim3((unsigned)s2.v.nm, 32), 256, 0, s>>>(
+                dx2f, ma2, rep, d_nat2.as<int>(), d_jbm.as<float>());
+            KFB_CUDA_TRY(cudaGetLastError());
             if (ygemm) {
                 TraceScope tr_j("hessian:jk-split", s);
                 const size_t jsm = (size_t)8 * (ld2 + 1) * sizeof(float);
@@ -2565,16 +2565,6 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
                 KFB_TRY(d_border.alloc((size_t)batch * sizeof(int), s));
                 // 0 < w <= 1 / sigma^2: a fixed power of two brings it under 2^14
                 w_scale = std::exp2(std::floor(std::log2(16384.0 * sigma * sigma)));
-                // |Y| <= max|J| sum_j w_ij <= (2^14 / jr_scale) n / sigma^2 for at most n
-                // atoms of one label in a molecule b: one scale for every batch, so
-                // that no batch waits for its own maximum
-                int ns = 1;
-                for (int m = 0; m < s2.v.nm; ++m)
-                    for (int l = 0; l < L; ++l) ns = std::max(ns, lm2.count(l, m, m));
-                const double yb = 16384.0 / (double)jr_scale * ns / (sigma * sigma);
-                // (a bound, not a maximum: 2^15 still leaves half of fp16's range)
-                yg_scale = (float)std::exp2(15.0 - std::ceil(std::log2(yb)));
-                if (!(yg_scale > 0.f) || !std::isfinite(yg_scale)) yg_scale = 1.f;
             }
             note_path(ygemm ? "hessian:y-gemm" : "hessian:y-cuda-core");
         }
@@ -2604,8 +2594,11 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
         const T *dx2p = static_cast<const T *>(s2.dx);
         auto tr_t = std::make_unique<TraceScope>("hessian:t", s);
         // with tensor cores kernel 1 also bounds |Y| for the power-of-two
-        // scale of the fp16 split that kernel 2 writes
-        if (tc && !ygemm) KFB_TRY(zero(yamax.ptr, sizeof(float), s));
+        // scale of the fp16 split that kernel 2 writes: each batch has its own,
+        // so that one whose weights are all small keeps its bits.  The Y GEMM
+        // and the contraction after it read it on the device (waiting for it on
+        // the host left the GPU idle between batches).
+        if (tc) KFB_TRY(zero(yamax.ptr, sizeof(float), s));
         if constexpr (std::is_same<T, float>::value) {
             if (pform) {
                 // rows of the batch's molecules a only (pairs sorted by a):
@@ -2669,7 +2662,7 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
                     d_P.as<float>(), ldp, d_prow.as<int>(), d_pcol.as<int>(), amin, bmin,
                     d_pb.as<float>(), d_jbm.as<float>(),
                     hrank ? 0 : 1, W.as<T>(), hrank ? nullptr : Tt.as<T>(),
-                    ygemm ? nullptr : yamax.as<float>());
+                    yamax.as<float>());
                 KFB_CUDA_TRY(cudaGetLastError());
             }
         }
@@ -2682,11 +2675,12 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
         auto tr_y = std::make_unique<TraceScope>("hessian:y", s);
         float y_scale = 1.f;
         if (tc) {
-            y_scale = yg_scale;
-            if (!ygemm) KFB_TRY(pow2_from_device(yamax.as<float>(), s, &y_scale));
+            if (ygemm) KFB_TRY(pow2_on_device(yamax.as<float>(), yamax.as<float>() + 1, s));
+            else KFB_TRY(pow2_from_device(yamax.as<float>(), s, &y_scale));
             if (ygemm)
                 KFB_TRY(hess_y_gemm(pairs.data() + p0, np, ma1, ma2, rep, kj, W.as<float>(),
-                                    jkh, jkl, jr_scale, w_scale, y_scale, wsh, wsl, d_ymap,
+                                    jkh, jkl, jr_scale, w_scale, yamax.as<float>() + 1, wsh, wsl,
+                                    d_ymap,
                                     d_border, (long long)s2.v.nm * ld2 * rep,
                                     dpairs.as<HessPair>(), yth.as<__half>(), ytl.as<__half>(),
                                     err.flag(), s));
@@ -2759,6 +2753,7 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
             TcEpi ec;
             ec.tile_n64 = narrow ? 1 : 0;
             ec.sink_t = narrow ? 1 : 0;
+            ec.dscale = ygemm ? yamax.as<float>() + 1 : nullptr;
             KFB_TRY(tc_gemm_grouped(narrow ? Yo : J, narrow ? J : Yo, 3, false, tprobs, sink, s,
                                     ec, err.flag()));
             tr_g.reset();

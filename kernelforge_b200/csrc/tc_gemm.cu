@@ -278,6 +278,7 @@ __global__ void __launch_bounds__(Cfg<NPROD, NEPI, BNT>::THREADS, 1)
         __shared__ float molsum_static[NEPI == 8 ? NEPI : 1][32][33];
         float(*molsum_scr)[32][33] =
             NEPI == 8 ? molsum_static : reinterpret_cast<float(*)[32][33]>(smem + C::OFF_SCR);
+        const float ds = epi.dscale ? *epi.dscale : 1.f;
         int acc = 0;
         uint32_t aph = 0;
         // the tile's problem (and for EPI_YSPLIT the (p, i) offset of this
@@ -365,7 +366,7 @@ __global__ void __launch_bounds__(Cfg<NPROD, NEPI, BNT>::THREADS, 1)
                     const int yc = mo / epi.y_rep;
                     const long long roff =
                         (long long)yc * epi.y_ma1 * epi.y_rep + (mo - yc * epi.y_rep);
-                    const float alpha = (float)pb.alpha;
+                    const float alpha = (float)(pb.alpha * (double)ds);
 #pragma unroll
                     for (int g = 0; g < 4; ++g) {
                         const int j = g * 8 + (lane >> 2);
@@ -401,6 +402,7 @@ __global__ void __launch_bounds__(Cfg<NPROD, NEPI, BNT>::THREADS, 1)
                     continue;
                 }
                 if (epi.mode == EPI_SINK) {
+                    const double alpha = pb.alpha / (double)ds;
                     if (mvalid) {
 #pragma unroll
                         for (int j = 0; j < 32; ++j) {
@@ -408,10 +410,10 @@ __global__ void __launch_bounds__(Cfg<NPROD, NEPI, BNT>::THREADS, 1)
                             if (n < pb.N) {
                                 if (epi.sink_t)
                                     sink_store(sink, pb.col_off + n, pb.row_off + m,
-                                               (double)v[j] * pb.alpha, pb.diag);
+                                               (double)v[j] * alpha, pb.diag);
                                 else
                                     sink_store(sink, pb.row_off + m, pb.col_off + n,
-                                               (double)v[j] * pb.alpha, pb.diag);
+                                               (double)v[j] * alpha, pb.diag);
                             }
                         }
                     }
@@ -917,6 +919,20 @@ kfb_status tc_gemm_grouped(const TcOperand &A, const TcOperand &B, int nprod, bo
 // then carries ~22 significant bits over ~28 binades below the maximum).
 float pow2_for(float m) {
     return (m > 0.f && std::isfinite(m)) ? std::ldexp(1.f, 14 - (int)std::ceil(std::log2(m))) : 1.f;
+}
+
+__global__ void pow2_scale_kernel(const float *__restrict__ dmax, float *__restrict__ scale) {
+    const float m = *dmax;
+    int e = 0;
+    const float f = frexpf(m, &e);   // m = f 2^e, f in [0.5, 1): ceil(log2 m) = e, or e - 1 at 0.5
+    const int p = 14 - (f == 0.5f ? e - 1 : e);
+    *scale = m > 0.f && isfinite(m) ? ldexpf(1.f, min(p, 126)) : 1.f;
+}
+
+kfb_status pow2_on_device(const float *dmax, float *scale, cudaStream_t s) {
+    pow2_scale_kernel<<<1, 1, 0, s>>>(dmax, scale);
+    KFB_CUDA_TRY(cudaGetLastError());
+    return KFB_OK;
 }
 
 kfb_status pow2_from_device(const float *dmax, cudaStream_t s, float *scale) {

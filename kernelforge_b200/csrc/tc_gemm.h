@@ -81,6 +81,10 @@ struct TcEpi {
     const int2 *ymap = nullptr;   // EPI_YSPLIT
     __half *yhi = nullptr, *ylo = nullptr;
     int y_rep = 0, y_ma1 = 0, y_ld2 = 0;
+    // EPI_YSPLIT writes alpha * acc times *dscale, EPI_SINK stores alpha * acc
+    // over *dscale: a power of two that an earlier kernel of the stream found
+    // (null: 1)
+    const float *dscale = nullptr;
 };
 
 // nprod = 3: split operands, hi*hi + hi*lo + lo*hi; nprod = 1: hi only.
@@ -122,6 +126,8 @@ float pow2_for(float m);
 // Host copy of a power of two that brings the device float *dmax to about
 // 2^14 (synchronises the stream).
 kfb_status pow2_from_device(const float *dmax, cudaStream_t s, float *scale);
+// The same left on the device, in *scale.
+kfb_status pow2_on_device(const float *dmax, float *scale, cudaStream_t s);
 template <class T>
 kfb_status transpose_split_y(const T *Y, int np, int ma1, int rep, int ld, const float *amax,
                              __half *hi, __half *lo, float *scale, cudaStream_t s);

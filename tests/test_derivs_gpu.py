@@ -260,3 +260,40 @@ def test_hessian_tensor_core_batches(gb, ycore, path, monkeypatch):
     assert _lib.path_log() == path
     close(lk.kernel_gaussian_full(X1, dX1, X2, dX2, Q1, Q2, N1, N2, s, precision=p),
           o.kernel_gaussian_full(X1, dX1, X2, dX2, Q1, Q2, N1, N2, s), p)
+
+
+@pytest.mark.parametrize("ycore", [None, "cuda-core"])
+def test_hessian_of_far_apart_sets(ycore, monkeypatch):
+    """Set-2 molecules whose weights are all about 2^-4, 2^-13 and 2^-22, 30 atoms of one element
+    each, a batch per molecule b (workspace of 5.7 MB): every block against its own norm.  The
+    distance lies along a column that no Jacobian uses, so that the block is J^T Y alone.  Y's
+    fp16 pair is scaled by the batch's bound; with one scale for weights of up to 1 its absolute
+    floor of 2^-25 leaves 14 bits of the last block (5e-5).  What remains: the weights' pair,
+    2^-25 below 2^-8 (4e-6 on average), and the FP32 exponents of 15 (5e-6): 2e-5."""
+    from kernelforge_b200 import _lib
+    from kernelforge_b200 import local_kernels as lk
+    monkeypatch.setenv("KFB_WORKSPACE_GB", "0.0053")
+    if ycore:
+        monkeypatch.setenv("KFB_HESSIAN_Y", ycore)
+    rng = np.random.default_rng(61)
+    rep, ma, s = 48, 30, 2.0
+    bits = (4, 13, 22)
+
+    def one(nm):
+        X = rng.standard_normal((nm, ma, rep)) * 0.02
+        dX = rng.standard_normal((nm, ma, rep, 3 * ma)) / np.sqrt(rep)
+        dX[:, :, 0] = 0.0
+        return X, dX, np.full((nm, ma), 6, np.int32), np.full(nm, ma, np.int32)
+    X1, dX1, Q1, N1 = one(4)
+    X2, dX2, Q2, N2 = one(len(bits))
+    for b, e in enumerate(bits):
+        X2[b, :, 0] += np.sqrt(2 * s * s * e * np.log(2.0))
+    _lib.path_log_clear()
+    H = lk.kernel_gaussian_hessian(X1, dX1, X2, dX2, Q1, Q2, N1, N2, s, precision="split_f16")
+    assert _lib.path_log() == ["hessian:rank-kernel",
+                               "hessian:y-cuda-core" if ycore else "hessian:y-gemm"]
+    f = lambda a: a.astype(np.float32).astype(np.float64)
+    R = o.kernel_gaussian_hessian(f(X1), f(dX1), f(X2), f(dX2), Q1, Q2, N1, N2, s)
+    for b in range(len(bits)):
+        c = slice(3 * ma * b, 3 * ma * (b + 1))
+        assert np.linalg.norm(H[:, c] - R[:, c]) <= 2e-5 * np.linalg.norm(R[:, c])
