@@ -229,3 +229,44 @@ def test_host_input_more_chunks_than_molecules(monkeypatch):
     rfp = clk.kernel_gaussian_symm_rfp(torch.from_numpy(X).pin_memory(), Q, N, 2.0)
     ref = o.kernel_gaussian_symm(X.astype(np.float64), Q, N, 2.0)
     close32(rfp.cpu().numpy(), o.full_to_rfp(ref, uplo_lower=True))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("labels", [64, 65, 66000])
+def test_many_labels(labels, precision):
+    """Labels are any integers: as many as the column map takes, one more, and more than a grid
+    has slices.  Every label belongs to two atoms, so the kernel is a sum over the labels."""
+    from kernelforge_b200 import local_kernels as lk
+    rng = np.random.default_rng(labels)
+    nm, rep, s = 200, 20, 2.5
+    ma = -(-2 * labels // nm)
+    rows = rng.permutation(nm * ma)[:2 * labels]
+    X, Q = np.zeros((nm, ma, rep)), np.full((nm, ma), -1, np.int32)
+    N = np.zeros(nm, np.int32)
+    label = np.repeat(rng.permutation(4 * labels)[:labels] - labels, 2)
+    place = []
+    for q, r in zip(label, rows):
+        m = r // ma
+        X[m, N[m], ::2] = rng.standard_normal(rep // 2)
+        Q[m, N[m]] = q
+        place.append((m, N[m]))
+        N[m] += 1
+    if precision == "fp32":
+        X = X.astype(np.float32).astype(np.float64)
+    ref = np.zeros((nm, nm))
+    for k in range(0, 2 * labels, 2):
+        (a, i), (b, j) = place[k], place[k + 1]
+        e = np.exp(-np.sum((X[a, i] - X[b, j]) ** 2) / (2 * s * s))
+        ref[a, a] += 1
+        ref[b, b] += 1
+        ref[a, b] += e
+        ref[b, a] += e
+    assert len(np.unique(np.concatenate([Q[m, :N[m]] for m in range(nm)]))) == labels
+    got = lk.kernel_gaussian_symm(X, Q, N, s, precision=precision)
+    half = lk.kernel_gaussian(X, X[:50], Q, Q[:50], N, N[:50], s, precision=precision)
+    if precision == "fp64":
+        np.testing.assert_allclose(np.tril(got), np.tril(ref), rtol=1e-12, atol=1e-12)
+        np.testing.assert_allclose(half, ref[:, :50], rtol=1e-12, atol=1e-12)
+    else:
+        close32(np.tril(got), np.tril(ref))
+        close32(half, ref[:, :50])
