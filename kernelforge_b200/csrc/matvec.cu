@@ -244,7 +244,8 @@ __device__ __forceinline__ void md_piece(T *dst, const T *src, bool ok, int left
     }
 }
 
-// Warp per row.  Query rows r < R1: n1[r] = |x|^2.  Training rows: n2 = |x|^2,
+// Warp per row.  Query rows r < R1: n1[r] = |x|^2 (NaN for a row with a value that
+// is not finite).  Training rows: n2 = |x|^2,
 // sc = x . Ad, and used[g] = 1 for the column groups with a value that is not
 // zero.  Four columns a lane (vec: 16-byte loads, 128 columns of the warp in
 // flight per step), so a group of 8 is two neighbouring lanes.
@@ -261,6 +262,7 @@ __global__ void __launch_bounds__(256) mv_rows_kernel(
     const Tin *x = (train ? x2 : x1) + at;
     const double *a = train && ad ? ad + at : nullptr;
     double n = 0.0, s = 0.0;
+    bool bad = false;
 #pragma unroll 3
     for (int k0 = 0; k0 < rep; k0 += 128) {
         const int k = k0 + 4 * lane;
@@ -291,6 +293,7 @@ __global__ void __launch_bounds__(256) mv_rows_kernel(
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             n = fma(v[u], v[u], n);
+            bad |= !isfinite(v[u]);
             s = fma(v[u], w[u], s);
             on |= !(v[u] == 0.0) || !(w[u] == 0.0);
         }
@@ -300,12 +303,13 @@ __global__ void __launch_bounds__(256) mv_rows_kernel(
         n += __shfl_xor_sync(0xffffffffu, n, o);
         s += __shfl_xor_sync(0xffffffffu, s, o);
     }
+    bad = __any_sync(0xffffffffu, bad);
     if (lane == 0) {
         if (train) {
             n2[r - R1] = n;
             sc[r - R1] = s;
         } else {
-            n1[r] = n;
+            n1[r] = bad ? n - n : n;
         }
     }
 }
@@ -446,7 +450,7 @@ __global__ void __launch_bounds__(256, 2) mv_weights_kernel(
         for (int mi = 0; mi < 2; ++mi) {
             const int i = 16 * wm + 8 * mi + (lane >> 2);
             const double ni = i < na ? n1[lb.sa + i0 + i] : 0.0;
-            const double bad = ni - ni;   // 0, or NaN for a row that is not finite
+            const double bad = ni == ni ? 0.0 : ni;   // NaN for a row that is not finite
             double esum = 0.0, vsum = 0.0;
 #pragma unroll
             for (int nj = 0; nj < 2; ++nj) {

@@ -16,7 +16,7 @@ constexpr int SPAD = 1;
 // column per label, pack_columns_kernel), only the label's used columns are
 // stored; zeros follow up to the next multiple of SK.  The norm is over every
 // column; a row with a value that is not finite has an undefined norm, as its
-// products would have been.
+// products would have been (an infinite norm of finite values stays: e = 0).
 template <class Tin, class T>
 __global__ void pack_rows_kernel(const Tin *__restrict__ x, const int *__restrict__ src, int R,
                                  int rep, int Dp, const int *__restrict__ lab_start, int L,
@@ -32,17 +32,20 @@ __global__ void pack_rows_kernel(const Tin *__restrict__ x, const int *__restric
     const int *pl = pos ? pos + (size_t)l * rep : nullptr;
     T *orow = out + (size_t)warp * Dp;
     double s = 0.0;
+    bool bad = false;
     for (int k = lane; k < rep; k += 32) {
         const double v = (double)xr[k];
         const int p = pl ? pl[k] : k;
         if (p >= 0) orow[p] = (T)v;
+        bad |= !isfinite(v);
         s += v * v;
     }
+    bad = __any_sync(0xffffffffu, bad);
     const int n = pl ? ncols[l] : rep;
     for (int p = n + lane; p < (n + SK - 1) / SK * SK; p += 32) orow[p] = T(0);
     for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (lane == 0) {
-        norm[warp] = (T)(isfinite(s) ? s : s - s);
+        norm[warp] = (T)(bad ? s - s : s);
         mol[warp] = src[warp] / ma;
     }
 }

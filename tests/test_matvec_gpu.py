@@ -237,3 +237,24 @@ def test_fp32_inputs_fp64_arithmetic():
         torch.cuda.current_stream().cuda_stream))
     close(e.cpu().numpy(), Er, 1e-9)
     close(f.cpu().numpy(), Fr, 1e-9)
+
+
+def test_squared_norm_beyond_fp64():
+    """A query atom of finite values whose squared norm is not: its pairs' kernels are zero, and
+    so is all that it adds; one that holds an infinity leaves its molecule's energy undefined and
+    no other."""
+    from kernelforge_b200 import local_kernels as lk
+    X1, dX1, Q1, N1, X2, dX2, Q2, N2, aE, aF = _problem(81)
+    ad = om.alpha_desc(dX2, Q2, N2, aF)
+    a = [m for m in range(len(N1)) if N1[m] and Q1[m, 0] in Q2[:, 0]][:2]
+    X1[a[0], 0, 1] = 1e160
+    with np.errstate(over="ignore"):
+        Er, Fr = om.matvec(X1, dX1, X2, ad, aE, Q1, Q2, N1, N2, 0.9)
+    E, F = lk.kernel_gaussian_local_full_matvec(X1, dX1, X2, ad, aE, Q1, Q2, N1, N2, 0.9)
+    close(E, Er)
+    close(F, Fr)
+    X1[a[1], 0, 1] = np.inf
+    E, F = lk.kernel_gaussian_local_full_matvec(X1, dX1, X2, ad, aE, Q1, Q2, N1, N2, 0.9)
+    assert np.isnan(E[a[1]])
+    keep = np.arange(len(N1)) != a[1]
+    close(E[keep], Er[keep])
