@@ -427,7 +427,10 @@ __global__ void __launch_bounds__(RG_WARPS * 32, 3) fchl19_grad_kernel(
         double *A = atoms + o * RG_ATOM;
         const Vec3 d = sub(position(o), Ri);
         const double r = sqrt(dot(d, d));
-        A[0] = r;
+        // beyond both cutoffs any distance does, and a partner's radial terms, zero times
+        // its pair terms, must be finite (r is not where d's square is no FP64 number)
+        const double rmax = fmax(P.rcut, P.acut);
+        A[0] = r <= rmax ? r : 2.0 * rmax;
         A[1] = d.x / r;
         A[2] = d.y / r;
         A[3] = d.z / r;

@@ -160,3 +160,30 @@ def test_edge_cases_and_errors():
     with pytest.raises(ValueError):
         fr.generate_fchl_acsf_and_gradients(np.eye(3), [1, 1, 1], nFourier=2)
     assert fr.compute_rep_size(5, 24, 20, 2) == 720
+
+
+@pytest.mark.parametrize("far", [50.0, 1e30, 1e200, np.inf, np.nan])
+def test_atoms_beyond_every_cutoff(far):
+    """An atom beyond the cutoffs, also at a distance whose square is no FP64 number: the others'
+    descriptors and Jacobians are those of the molecule without it.  One at no finite place
+    leaves their descriptors (not their Jacobians) as they are."""
+    from kernelforge_b200 import fchl19_repr as fr
+    rng = np.random.default_rng(3)
+    n = 9
+    grid = np.stack(np.meshgrid(*[np.arange(3)] * 3), -1).reshape(-1, 3) * 1.3
+    C = np.zeros((1, n + 1, 3))
+    C[0, :n] = grid[:n] + rng.uniform(-0.2, 0.2, (n, 3))
+    C[0, n, 1] = far
+    Z = rng.choice([1, 6, 8], (1, n + 1)).astype(np.int32)
+    Z[0, n] = 6
+    kw = dict(gradients=True, dtype="float64")
+    X, dX = (t.cpu().numpy() for t in fr.generate_batched(C, Z, np.array([n + 1], np.int32), **kw))
+    X0, dX0 = (t.cpu().numpy() for t in fr.generate_batched(C, Z, np.array([n], np.int32), **kw))
+    # (the atoms of an element are added up in an order that does not depend on the far one)
+    np.testing.assert_allclose(X[0, :n], X0[0, :n], rtol=0, atol=1e-15 * np.abs(X0).max())
+    if np.isfinite(far):
+        np.testing.assert_allclose(dX[0, :n], dX0[0, :n], rtol=0, atol=1e-15 * np.abs(dX0).max())
+    V = fr.generate_batched(C, Z, np.array([n + 1], np.int32), dtype="float64").cpu().numpy()
+    np.testing.assert_allclose(X[0, :n], V[0, :n], rtol=0, atol=1e-13 * np.abs(X0).max())
+    if np.isfinite(far):
+        assert not X[0, n].any() and not dX[0, n].any()
