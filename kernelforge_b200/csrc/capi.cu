@@ -103,29 +103,6 @@ bool use_tc(kfb_precision prec, int rep) {
     return prec == KFB_PREC_SPLIT_F16 && rep % 16 == 0 && device_is_sm100();
 }
 
-// tc: use_tc of the call's own rep (the widths that compact() leaves are
-// multiples of 16 as well).
-kfb_status jac_any(kfb_dtype dt, bool tc, const DerivSet &outer, const DerivSet &inner, int rep,
-                   double sigma, double alpha, const ElemSink &sink, cudaStream_t s) {
-    if (rep <= 0) return KFB_OK;
-    if (dt == KFB_F64) return jacobian_core<double>(outer, inner, rep, sigma, alpha, tc, sink, s);
-    return jacobian_core<float>(outer, inner, rep, sigma, alpha, tc, sink, s);
-}
-
-kfb_status hess_any(kfb_dtype dt, bool tc, const DerivSet &s1, const DerivSet &s2, int rep,
-                    double sigma, bool symmetric, const ElemSink &sink, cudaStream_t s) {
-    if (rep <= 0) return KFB_OK;
-    if (dt == KFB_F64) return hessian_core<double>(s1, s2, rep, sigma, symmetric, tc, sink, s);
-    return hessian_core<float>(s1, s2, rep, sigma, symmetric, tc, sink, s);
-}
-
-// The two sets of a derivative kernel without the columns that neither uses.
-kfb_status compact(kfb_dtype dt, DerivSet &s1, DerivSet &s2, int &rep, CompactSets &keep,
-                   cudaStream_t s) {
-    if (dt == KFB_F64) return compact_columns<double>(s1, s2, rep, keep, s);
-    return compact_columns<float>(s1, s2, rep, keep, s);
-}
-
 DerivSet dset(const void *x, const void *dx, const int32_t *q, const int32_t *n, int nm, int ma) {
     DerivSet d;
     d.x = x;
@@ -133,6 +110,68 @@ DerivSet dset(const void *x, const void *dx, const int32_t *q, const int32_t *n,
     d.v = view(q, n, nm, ma);
     return d;
 }
+
+// A derivative call: the sets as given and as its stages take them, without the
+// columns that neither uses.  The copies that this takes, and the Y GEMM's operand
+// in the Hessian, are made where they can be allocated, without asking how much
+// memory is free (the query has taken up to 6 ms).  A stage that runs out of
+// memory after them gives them back and runs again at the full width and with the
+// Y GEMM only where a workspace stays free beside its operand: the stages store
+// every output before they add to it.
+struct DerivCall {
+    kfb_dtype dt;
+    double sigma;
+    cudaStream_t s;
+    DerivSet d1, d2;       // d1 = d2 for a symmetric call
+    int rep;
+    bool tc, lean = false;
+    CompactSets keep;
+
+    DerivCall(kfb_dtype dt_, kfb_precision prec, double sigma_, cudaStream_t s_,
+              const DerivSet &a, const DerivSet &b, int rep_)
+        : dt(dt_), sigma(sigma_), s(s_), d1(a), d2(b), rep(rep_), tc(use_tc(prec, rep_)),
+          full1(a), full2(b), full_rep(rep_) {}
+
+    kfb_status compact() {
+        const kfb_status st = dt == KFB_F64 ? compact_columns<double>(d1, d2, rep, keep, s)
+                                            : compact_columns<float>(d1, d2, rep, keep, s);
+        full1.dx_max = d1.dx_max;
+        full2.dx_max = d2.dx_max;
+        return st;
+    }
+    // alpha G[o, c], outer set d1 and inner d2 or (transposed) the other way round
+    kfb_status jacobian(bool transposed, double alpha, const ElemSink &sink) {
+        return stage([&] {
+            const DerivSet &o = transposed ? d2 : d1, &i = transposed ? d1 : d2;
+            return dt == KFB_F64 ? jacobian_core<double>(o, i, rep, sigma, alpha, tc, sink, s)
+                                 : jacobian_core<float>(o, i, rep, sigma, alpha, tc, sink, s);
+        });
+    }
+    kfb_status hessian(bool symmetric, const ElemSink &sink) {
+        return stage([&] {
+            return dt == KFB_F64
+                       ? hessian_core<double>(d1, d2, rep, sigma, symmetric, tc, lean, sink, s)
+                       : hessian_core<float>(d1, d2, rep, sigma, symmetric, tc, lean, sink, s);
+        });
+    }
+
+private:
+    DerivSet full1, full2;
+    int full_rep;
+
+    template <class F>
+    kfb_status stage(F run) {
+        const kfb_status st = run();
+        if (st != KFB_ERR_ALLOC || lean) return st;
+        lean = true;
+        for (DevBuf *b : {&keep.x1, &keep.dx1, &keep.x2, &keep.dx2}) b->release();
+        d1 = full1;
+        d2 = full2;
+        rep = full_rep;
+        KFB_TRY(trim_pool(s));
+        return run();
+    }
+};
 
 }  // namespace
 
@@ -286,11 +325,10 @@ kfb_status kfb_kernel_gaussian_jacobian(const void *x1, const void *x2, const vo
     sink.f64 = dt == KFB_F64;
     sink.mode = EM_RECT;
     sink.ld = naq2;
-    DerivSet d1 = dset(x1, nullptr, q1, n1, nm1, ma1), d2 = dset(x2, dx2, q2, n2, nm2, ma2);
-    const bool tc = use_tc(prec, rep);
-    CompactSets keep;
-    KFB_TRY(compact(dt, d1, d2, rep, keep, s));
-    return jac_any(dt, tc, d1, d2, rep, sigma, 1.0, sink, s);
+    DerivCall call(dt, prec, sigma, s, dset(x1, nullptr, q1, n1, nm1, ma1),
+                   dset(x2, dx2, q2, n2, nm2, ma2), rep);
+    KFB_TRY(call.compact());
+    return call.jacobian(false, 1.0, sink);
 }
 
 kfb_status kfb_kernel_gaussian_jacobian_t(const void *x1, const void *dx1, const void *x2,
@@ -319,11 +357,10 @@ kfb_status kfb_kernel_gaussian_jacobian_t(const void *x1, const void *dx1, const
     sink.f64 = dt == KFB_F64;
     sink.mode = EM_RECT_T;
     sink.ld = nm2;
-    DerivSet d1 = dset(x1, dx1, q1, n1, nm1, ma1), d2 = dset(x2, nullptr, q2, n2, nm2, ma2);
-    const bool tc = use_tc(prec, rep);
-    CompactSets keep;
-    KFB_TRY(compact(dt, d1, d2, rep, keep, s));
-    return jac_any(dt, tc, d2, d1, rep, sigma, -1.0, sink, s);
+    DerivCall call(dt, prec, sigma, s, dset(x1, dx1, q1, n1, nm1, ma1),
+                   dset(x2, nullptr, q2, n2, nm2, ma2), rep);
+    KFB_TRY(call.compact());
+    return call.jacobian(true, -1.0, sink);
 }
 
 kfb_status kfb_kernel_gaussian_hessian(const void *x1, const void *dx1, const void *x2,
@@ -351,11 +388,10 @@ kfb_status kfb_kernel_gaussian_hessian(const void *x1, const void *dx1, const vo
     sink.f64 = dt == KFB_F64;
     sink.mode = EM_RECT;
     sink.ld = naq2;
-    DerivSet d1 = dset(x1, dx1, q1, n1, nm1, ma1), d2 = dset(x2, dx2, q2, n2, nm2, ma2);
-    const bool tc = use_tc(prec, rep);
-    CompactSets keep;
-    KFB_TRY(compact(dt, d1, d2, rep, keep, s));
-    return hess_any(dt, tc, d1, d2, rep, sigma, false, sink, s);
+    DerivCall call(dt, prec, sigma, s, dset(x1, dx1, q1, n1, nm1, ma1),
+                   dset(x2, dx2, q2, n2, nm2, ma2), rep);
+    KFB_TRY(call.compact());
+    return call.hessian(false, sink);
 }
 
 kfb_status kfb_kernel_gaussian_hessian_symm(const void *x, const void *dx, const int32_t *q,
@@ -381,11 +417,10 @@ kfb_status kfb_kernel_gaussian_hessian_symm(const void *x, const void *dx, const
     sink.mode = EM_SYM;
     sink.layout = layout == KFB_DENSE ? LAYOUT_DENSE_LOWER : layout;
     sink.ld = naq;
-    DerivSet d1 = dset(x, dx, q, n, nm, ma), d2 = d1;
-    const bool tc = use_tc(prec, rep);
-    CompactSets keep;
-    KFB_TRY(compact(dt, d1, d2, rep, keep, s));
-    return hess_any(dt, tc, d1, d2, rep, sigma, true, sink, s);
+    const DerivSet d = dset(x, dx, q, n, nm, ma);
+    DerivCall call(dt, prec, sigma, s, d, d, rep);
+    KFB_TRY(call.compact());
+    return call.hessian(true, sink);
 }
 
 kfb_status kfb_kernel_gaussian_full(const void *x1, const void *dx1, const void *x2,
@@ -421,10 +456,9 @@ kfb_status kfb_kernel_gaussian_full(const void *x1, const void *dx1, const void 
     ps.mode = OUT_RECT;
     ps.n = C;
     KFB_TRY(scalar_dispatch(p, prec, ps, s));
-    DerivSet d1 = dset(x1, dx1, q1, n1, nm1, ma1), d2 = dset(x2, dx2, q2, n2, nm2, ma2);
-    const bool tc = use_tc(prec, rep);
-    CompactSets keep;
-    KFB_TRY(compact(dt, d1, d2, rep, keep, s));
+    DerivCall call(dt, prec, sigma, s, dset(x1, dx1, q1, n1, nm1, ma1),
+                   dset(x2, dx2, q2, n2, nm2, ma2), rep);
+    KFB_TRY(call.compact());
     // [0:nm1, nm2:] = +jacobian(X1, X2, dX2)
     ElemSink sj;
     sj.out = out;
@@ -432,7 +466,7 @@ kfb_status kfb_kernel_gaussian_full(const void *x1, const void *dx1, const void 
     sj.mode = EM_RECT;
     sj.ld = C;
     sj.col_base = nm2;
-    KFB_TRY(jac_any(dt, tc, d1, d2, rep, sigma, 1.0, sj, s));
+    KFB_TRY(call.jacobian(false, 1.0, sj));
     // [nm1:, 0:nm2] = -jacobian_t(X1, dX1, X2) = G^T with G from (outer 2, inner 1)
     ElemSink st;
     st.out = out;
@@ -440,7 +474,7 @@ kfb_status kfb_kernel_gaussian_full(const void *x1, const void *dx1, const void 
     st.mode = EM_RECT_T;
     st.ld = C;
     st.col_base = nm1;
-    KFB_TRY(jac_any(dt, tc, d2, d1, rep, sigma, 1.0, st, s));
+    KFB_TRY(call.jacobian(true, 1.0, st));
     // [nm1:, nm2:] = hessian
     ElemSink sh;
     sh.out = out;
@@ -449,7 +483,7 @@ kfb_status kfb_kernel_gaussian_full(const void *x1, const void *dx1, const void 
     sh.ld = C;
     sh.row_base = nm1;
     sh.col_base = nm2;
-    return hess_any(dt, tc, d1, d2, rep, sigma, false, sh, s);
+    return call.hessian(false, sh);
 }
 
 kfb_status kfb_kernel_gaussian_full_symm(const void *x, const void *dx, const int32_t *q,
@@ -486,10 +520,9 @@ kfb_status kfb_kernel_gaussian_full_symm(const void *x, const void *dx, const in
         TraceScope tr("full_symm:scalar", s);
         KFB_TRY(scalar_dispatch(p, prec, ps, s));
     }
-    DerivSet d = dset(x, dx, q, n, nm, ma), d2 = d;
-    const bool tc = use_tc(prec, rep);
-    CompactSets keep;
-    KFB_TRY(compact(dt, d, d2, rep, keep, s));
+    const DerivSet d = dset(x, dx, q, n, nm, ma);
+    DerivCall call(dt, prec, sigma, s, d, d, rep);
+    KFB_TRY(call.compact());
     // jacobian block at rows [0, nm), columns [nm, big) and its mirror
     ElemSink sj;
     sj.out = out;
@@ -500,7 +533,7 @@ kfb_status kfb_kernel_gaussian_full_symm(const void *x, const void *dx, const in
     sj.col_base = nm;
     {
         TraceScope tr("full_symm:jacobian", s);
-        KFB_TRY(jac_any(dt, tc, d, d2, rep, sigma, 1.0, sj, s));
+        KFB_TRY(call.jacobian(false, 1.0, sj));
     }
     ElemSink sh;
     sh.out = out;
@@ -511,7 +544,7 @@ kfb_status kfb_kernel_gaussian_full_symm(const void *x, const void *dx, const in
     sh.row_base = nm;
     sh.col_base = nm;
     TraceScope tr("full_symm:hessian", s);
-    return hess_any(dt, tc, d, d2, rep, sigma, true, sh, s);
+    return call.hessian(true, sh);
 }
 
 kfb_status kfb_full_to_rfp(const void *a, int n, kfb_layout uplo, kfb_dtype dt, void *arf,

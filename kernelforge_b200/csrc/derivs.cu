@@ -2283,7 +2283,7 @@ kfb_status hess_y_gemm(const HessPair *pairs, int np, int ma1, int ma2, int rep,
 
 template <class T>
 kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double sigma,
-                        bool symmetric, bool tc, ElemSink sink, cudaStream_t s) {
+                        bool symmetric, bool tc, bool lean, ElemSink sink, cudaStream_t s) {
     std::vector<int> off1, off2;
     deriv_offsets(s1.v, off1);
     deriv_offsets(s2.v, off2);
@@ -2529,8 +2529,9 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
                         jk_rows < INT_MAX &&
                         (long long)batch * ma1 < INT_MAX;
                 // the workspace is allocated by now: up to its size this is simply
-                // tried, more must leave as much free (the query can take milliseconds)
-                if (ygemm && jk_bytes > (long long)budget_bytes()) {
+                // tried, more (or any in a lean call) must leave as much free (the query
+                // can take milliseconds)
+                if (ygemm && (lean || jk_bytes > (long long)budget_bytes())) {
                     size_t free_b = 0, total_b = 0;
                     KFB_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
                     ygemm = jk_bytes + (long long)budget_bytes() <= (long long)free_b;
@@ -2836,8 +2837,8 @@ template kfb_status jacobian_core<double>(const DerivSet &, const DerivSet &, in
 template kfb_status jacobian_core<float>(const DerivSet &, const DerivSet &, int, double, double,
                                          bool, ElemSink, cudaStream_t);
 template kfb_status hessian_core<double>(const DerivSet &, const DerivSet &, int, double, bool,
-                                         bool, ElemSink, cudaStream_t);
+                                         bool, bool, ElemSink, cudaStream_t);
 template kfb_status hessian_core<float>(const DerivSet &, const DerivSet &, int, double, bool,
-                                        bool, ElemSink, cudaStream_t);
+                                        bool, bool, ElemSink, cudaStream_t);
 
 }  // namespace kfb

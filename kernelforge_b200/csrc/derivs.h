@@ -104,11 +104,12 @@ __device__ __forceinline__ void sink_positions(const ElemSink &s, long long R, l
 
 // Columns of the descriptors that no real atom of either set uses (x and dx
 // zero everywhere) contribute nothing to any derivative kernel.  When they are
-// at least an eighth of the columns and the copies fit in a quarter of the
-// free memory, s1 and s2 are replaced by copies without them (held by `keep`,
-// padded with zero columns to a multiple of 16) and rep by their width.  Either
-// way dx_max of the sets is filled in.  Synchronises the stream (the width is
-// needed on the host).
+// at least an eighth of the columns, s1 and s2 are replaced by copies without
+// them (held by `keep`, padded with zero columns to a multiple of 16) and rep by
+// their width; not where the copies cannot be allocated, nor where they exceed
+// both the workspace budget and a quarter of the free memory.  Either way dx_max
+// of the sets is filled in.  Synchronises the stream (the width is needed on the
+// host).
 struct CompactSets {
     DevBuf x1, dx1, x2, dx2;
 };
@@ -127,13 +128,14 @@ kfb_status scan_columns(const DerivSet &d, int rep, const int *nat, int *used, f
                         cudaStream_t s, const int *slot = nullptr);
 
 // tc: run the contraction GEMMs on the tensor cores (split fp16, three
-// products); needs rep % 16 == 0 and an sm_100 device.
+// products); needs rep % 16 == 0 and an sm_100 device.  lean: the Y GEMM, whose
+// operand is held for the call, only where a whole workspace stays free beside it.
 template <class T>
 kfb_status jacobian_core(const DerivSet &outer, const DerivSet &inner, int rep, double sigma,
                          double alpha, bool tc, ElemSink sink, cudaStream_t s);
 
 template <class T>
 kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double sigma,
-                        bool symmetric, bool tc, ElemSink sink, cudaStream_t s);
+                        bool symmetric, bool tc, bool lean, ElemSink sink, cudaStream_t s);
 
 }  // namespace kfb

@@ -72,6 +72,16 @@ void DevBuf::release() {
     bytes = 0;
 }
 
+kfb_status trim_pool(cudaStream_t s) {
+    KFB_CUDA_TRY(cudaStreamSynchronize(s));
+    int dev = 0;
+    cudaMemPool_t pool;
+    KFB_CUDA_TRY(cudaGetDevice(&dev));
+    KFB_CUDA_TRY(cudaDeviceGetDefaultMemPool(&pool, dev));
+    KFB_CUDA_TRY(cudaMemPoolTrimTo(pool, 0));
+    return KFB_OK;
+}
+
 // Labels are nuclear charges or element indices: small non-negative integers
 // take a direct table, anything else a map.  Labels are numbered in the order
 // they are met and sorted at the end.

@@ -49,6 +49,9 @@ struct DevBuf {
     template <class T> T *as() const { return static_cast<T *>(ptr); }
 };
 
+// Waits for the stream and returns the pool's unused memory to the driver.
+kfb_status trim_pool(cudaStream_t s);
+
 // Copy a host vector to a fresh device buffer on `s` (the host vector must stay
 // alive until the stream reaches the copy; callers keep it in scope and the
 // copy is issued from pageable memory, which the runtime stages synchronously).

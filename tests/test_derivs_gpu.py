@@ -297,3 +297,84 @@ def test_hessian_of_far_apart_sets(ycore, monkeypatch):
     for b in range(len(bits)):
         c = slice(3 * ma * b, 3 * ma * (b + 1))
         assert np.linalg.norm(H[:, c] - R[:, c]) <= 2e-5 * np.linalg.norm(R[:, c])
+
+
+_FULL_GPU = r"""
+import sys
+import numpy as np
+import torch
+from kernelforge_b200 import cuda_local_kernels as clk, _lib
+kind = sys.argv[1]
+nm, ma, rep, used = 150, 24, 720, 480
+g = torch.Generator(device="cuda")
+g.manual_seed(5)
+X = torch.randn((nm, ma, rep), generator=g, device="cuda") * 0.1
+dX = torch.randn((nm, ma, rep, 3 * ma), generator=g, device="cuda") * 0.1
+off = torch.arange(rep, device="cuda") % 3 == 2
+Q = np.random.default_rng(5).choice([1, 6, 8], (nm, ma)).astype(np.int32)
+N = np.full(nm, ma, np.int32)
+N[::3] -= 3
+naq = 3 * int(N.sum())
+J = torch.empty((nm, naq), device="cuda")
+
+def call():
+    if kind == "ef":
+        return clk.kernel_gaussian_full_symm_rfp(X, dX, Q, N, 2.0)
+    J.fill_(float("nan"))
+    _lib.check(_lib.lib().kfb_kernel_gaussian_jacobian(
+        X.data_ptr(), X.data_ptr(), dX.data_ptr(), Q.ctypes.data, Q.ctypes.data, N.ctypes.data,
+        N.ctypes.data, nm, nm, ma, ma, rep, naq, 2.0, _lib.KFB_F32, _lib.PREC["split_f16"],
+        J.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    return J
+
+def needs(limit_mb, step_mb):
+    # the smallest free memory, in steps, at which the call still runs; the results agree
+    K, good = None, None
+    for mb in range(limit_mb, 0, -step_mb):
+        torch.cuda.synchronize()      # (the pool keeps nothing: KFB_POOL_KEEP_GB=0)
+        free = torch.cuda.mem_get_info()[0]
+        fill = torch.empty(free - (mb << 20), dtype=torch.uint8, device="cuda")
+        try:
+            out = call()
+            torch.cuda.synchronize()
+        except _lib.KfbError as e:
+            assert "cudaMallocAsync" in str(e), e
+            out = None
+        del fill
+        torch.cuda.empty_cache()
+        if out is None:
+            return good
+        good = mb
+        if K is None:
+            K = out.clone()
+        # (two widths: FP32 sums of 17,280 terms in two orders, each 1e-5 from 64 bits)
+        assert torch.linalg.norm(out - K) <= 5e-5 * torch.linalg.norm(K)
+        del out
+    return good
+
+call(), torch.cuda.synchronize()
+limit = 3072 if kind == "jacobian" else 6144
+dense = needs(limit, 128)
+X[:, :, off] = 0
+dX[:, :, off] = 0
+sparse = needs(limit, 128)
+print("full width", dense, "MB, unused columns", sparse, "MB")
+assert dense < limit and sparse <= dense
+"""
+
+
+@pytest.mark.parametrize("kind", ["jacobian", "ef"])
+def test_derivative_kernels_on_a_nearly_full_gpu(kind):
+    """A third of the columns unused: the copies without them, and the Y GEMM's operand, are
+    taken where they can be allocated.  The call runs wherever one of the same size that uses
+    every column does, with the same result at every amount of free memory (an ordinary
+    allocation holds the rest).  In a process of its own: the memory pool's settings are read
+    once."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    env = dict(os.environ, KFB_POOL_KEEP_GB="0", KFB_WORKSPACE_GB="1", PYTHONPATH=root)
+    r = subprocess.run([sys.executable, "-c", _FULL_GPU, kind], env=env, cwd=root,
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
