@@ -774,13 +774,20 @@ kfb_status matvec_direct(const Tin *x1, const Tin *dx1, const Tin *x2, const dou
     const double c = -1.0 / (2.0 * sigma * sigma), is2 = 1.0 / (sigma * sigma), is4 = is2 * is2;
     const int nlab = (int)labs.size();
     const MvLabel *dl = reinterpret_cast<const MvLabel *>(dp);
+    // the kernels' limit is that of the longest list, the same in every call: another
+    // thread's call may come between this one's setting and its launch
+    constexpr size_t st_w = (size_t)MvW<Tin>::NST * MvW<Tin>::STAGE;
+    constexpr size_t st_g = (size_t)MvG<Tin>::NST * MvG<Tin>::STAGE;
+    constexpr size_t lmax = (size_t)(MD_MAX_REP / 8 + 1) * sizeof(int);
+    static_assert(st_w + lmax <= 227 * 1024 && st_g + lmax <= 227 * 1024, "shared memory");
     const size_t lbytes = (size_t)(ng + 1) * sizeof(int);
-    const size_t sm_w = (size_t)MvW<Tin>::NST * MvW<Tin>::STAGE + lbytes;
-    const size_t sm_g = (size_t)MvG<Tin>::NST * MvG<Tin>::STAGE + lbytes;
+    const size_t sm_w = st_w + lbytes, sm_g = st_g + lbytes;
     KFB_CUDA_TRY(cudaFuncSetAttribute(mv_weights_kernel<Tin>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_w));
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)(st_w + lmax)));
     KFB_CUDA_TRY(cudaFuncSetAttribute(mv_grad_kernel<Tin>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_g));
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)(st_g + lmax)));
     mv_rows_kernel<Tin><<<nblk((long long)R1 + R2, 8), 256, 0, s>>>(
         x1, dp + o_src1, R1, x2, dp + o_src2, R2, ad, rep, vec, n1, n2, sc, used);
     mv_weights_kernel<Tin><<<tiles1, 256, sm_w, s>>>(

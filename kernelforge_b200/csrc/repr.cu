@@ -667,7 +667,8 @@ kfb_status kfb_fchl19_repr(const void *coords, const int32_t *elem, const int32_
     const bool g = grad != nullptr;
     const size_t smem = (size_t)(3 * ma + P.rep + (g ? 3 * P.rep : 0)) * sizeof(double) +
                         (size_t)REPR_WARPS * 32 * sizeof(TripleSlot) + (size_t)ma * sizeof(int);
-    if (smem > 200 * 1024)
+    constexpr size_t SMEM_MAX = 200 * 1024;
+    if (smem > SMEM_MAX)
         return set_error(KFB_ERR_INVALID_ARG, "descriptor too large for one block (%zu bytes)", smem);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     std::vector<int> ev(elem, elem + (size_t)nm * ma), nv(natoms, natoms + nm);
@@ -676,19 +677,21 @@ kfb_status kfb_fchl19_repr(const void *coords, const int32_t *elem, const int32_
     KFB_TRY(upload(d_n, nv, s));
     const int *de = d_elem.as<int>(), *dn = d_n.as<int>();
     const dim3 grid((unsigned)ma, (unsigned)nm);
+    // (the kernels' limit is the same in every call: another thread's call may come
+    // between this one's setting and its launch)
     auto launch = [&](auto kern) -> kfb_status {
         if (smem > 48 * 1024)
             KFB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)smem));
+                                              (int)SMEM_MAX));
         return KFB_OK;
     };
     // the row-wise gradient kernel holds a centre's pairs in shared memory (40
     // atoms); larger molecules take the kernel that forms them as it goes
     const size_t rg = rg_smem(ma);
-    if (g && rg <= 200 * 1024) {
+    if (g && rg <= SMEM_MAX) {
         auto run = [&](auto kern, auto *c, auto *r, auto *d) -> kfb_status {
             KFB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)rg));
+                                              (int)SMEM_MAX));
             kern<<<grid, RG_WARPS * 32, rg, s>>>(c, de, dn, ma, P, r, d);
             KFB_CUDA_TRY(cudaGetLastError());
             return KFB_OK;

@@ -258,3 +258,46 @@ def test_squared_norm_beyond_fp64():
     assert np.isnan(E[a[1]])
     keep = np.arange(len(N1)) != a[1]
     close(E[keep], Er[keep])
+
+
+@pytest.mark.parametrize("kind", ["matvec", "descriptors"])
+def test_calls_of_different_sizes_in_threads(kind):
+    """Calls that take more and less shared memory (long and short descriptors, large and small
+    molecules), each from its own thread and stream: all run, with one thread's results."""
+    import threading
+    import torch
+    from kernelforge_b200 import cuda_local_kernels as clk
+    from kernelforge_b200 import fchl19_repr as fr
+    f32 = lambda a: torch.tensor(np.asarray(a, np.float32), device="cuda")
+    i32 = lambda a: torch.tensor(np.asarray(a, np.int32), device="cuda")
+    calls = []
+    for size in (0, 1):
+        if kind == "matvec":
+            X1, dX1, Q1, N1, X2, dX2, Q2, N2, aE, aF = _problem(91, nm1=2, nm2=3,
+                                                                rep=(16, 24576)[size])
+            ad = om.alpha_desc(dX2, Q2, N2, aF)
+            args = (f32(X1), f32(dX1), i32(Q1), i32(N1), f32(X2), i32(Q2), i32(N2), f32(aE),
+                    f32(ad), 50.0)
+            calls.append(lambda args=args: clk.kernel_gaussian_full_matvec(*args)[1])
+        else:
+            ma = (3, 40)[size]
+            grid = np.stack(np.meshgrid(*[np.arange(4.0)] * 3), -1).reshape(-1, 3)[:ma]
+            args = (f32(grid[None]), np.full((1, ma), 6, np.int32), np.array([ma], np.int32))
+            calls.append(lambda args=args: fr.generate_batched(*args, gradients=True)[1])
+    refs = [c().double().cpu().numpy() for c in calls]
+    failed = []
+
+    def work(k):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(300):
+                try:
+                    close(calls[k]().double().cpu().numpy(), refs[k], 1e-6)
+                except Exception as e:
+                    failed.append(repr(e)[:300])
+                    return
+    threads = [threading.Thread(target=work, args=(k % 2,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed
