@@ -119,30 +119,30 @@ def test_against_restatement_and_finite_differences():
                                    atol=1e-6 * np.abs(J).max())
 
 
-@pytest.mark.parametrize("n", [1, 2, 9, 20, 33, 40])
+@pytest.mark.parametrize("n", [1, 2, 9, 20, 33, 41])
 @pytest.mark.parametrize("hyper", [{}, dict(nRs2=7, nRs3=5, rcut=3.0, acut=2.5)])
 def test_row_wise_gradients_match_large_molecule_kernel(n, hyper):
-    """Up to 40 padded atoms the Jacobian rows come from shared-memory pair terms, above from the
-    kernel that forms them as it goes: the same molecules padded to 40 and to 41 atoms.  Both sum
+    """Up to 41 padded atoms the Jacobian rows come from shared-memory pair terms, above from the
+    kernel that forms them as it goes: the same molecules padded to 41 and to 42 atoms.  Both sum
     the same FP64 terms in another order (1e-13 of the largest entry); atoms beyond the cutoffs,
     elements that one or no atom has, partial row groups."""
     import torch
     from kernelforge_b200 import fchl19_repr as fr
     rng = np.random.default_rng(n)
     nm = 3
-    C = np.zeros((nm, 41, 3))
-    Z = np.zeros((nm, 41), np.int32)
+    C = np.zeros((nm, 42, 3))
+    Z = np.zeros((nm, 42), np.int32)
     grid = np.stack(np.meshgrid(*[np.arange(4)] * 3), -1).reshape(-1, 3) * 1.3
     for m in range(nm):
         C[m, :n] = grid[rng.permutation(64)[:n]] + rng.uniform(-0.2, 0.2, (n, 3))
         Z[m, :n] = rng.choice([[1], [1, 6], [1, 6, 8, 16]][m], n)
     N = np.array([n, n, max(n - 1, 0)], np.int32)
     out = []
-    for ma in (40, 41):
+    for ma in (41, 42):
         X, dX = fr.generate_batched(C[:, :ma], Z[:, :ma], N, gradients=True, dtype="float64",
                                     **hyper)
         assert not dX[:, :, :, 3 * n:].any() and not X[2, N[2]:].any()
-        out.append((X[:, :40].cpu().numpy(), dX[:, :40, :, :120].cpu().numpy()))
+        out.append((X[:, :41].cpu().numpy(), dX[:, :41, :, :123].cpu().numpy()))
     for a, b in zip(*out):
         np.testing.assert_allclose(a, b, rtol=0, atol=1e-13 * max(1e-3, np.abs(b).max()))
 
@@ -187,3 +187,27 @@ def test_atoms_beyond_every_cutoff(far):
     np.testing.assert_allclose(X[0, :n], V[0, :n], rtol=0, atol=1e-13 * np.abs(X0).max())
     if np.isfinite(far):
         assert not X[0, n].any() and not dX[0, n].any()
+
+
+@pytest.mark.parametrize("n", [42, 57])
+def test_large_molecules(n):
+    """More atoms than the row-wise kernel takes: descriptors as the kernel without gradients
+    gives them, Jacobians against central finite differences of those (h = 1e-5: 1e-10 of the
+    values' rounding over h, and h^2 times third derivatives), rows that sum to zero."""
+    from kernelforge_b200 import fchl19_repr as fr
+    rng = np.random.default_rng(n)
+    grid = np.stack(np.meshgrid(*[np.arange(4)] * 3), -1).reshape(-1, 3) * 1.4
+    R = grid[rng.permutation(64)[:n]] + rng.uniform(-0.2, 0.2, (n, 3))
+    Z = rng.choice([1, 6, 7, 8, 16], n).astype(np.int32)
+    X, J = fr.generate_fchl_acsf_and_gradients(R, Z)
+    X0 = fr.generate_fchl_acsf(R, Z)
+    np.testing.assert_allclose(X, X0, rtol=0, atol=1e-13 * np.abs(X0).max())
+    J = J.reshape(n, -1, n, 3)
+    assert np.abs(J.sum(2)).max() <= 1e-12 * np.abs(J).max()
+    h = 1e-5
+    for a, t in [(0, 0), (n // 2, 1), (n - 1, 2)]:
+        Rp, Rm = R.copy(), R.copy()
+        Rp[a, t] += h
+        Rm[a, t] -= h
+        fd = (fr.generate_fchl_acsf(Rp, Z) - fr.generate_fchl_acsf(Rm, Z)) / (2 * h)
+        np.testing.assert_allclose(J[:, :, a, t], fd, rtol=1e-5, atol=1e-6 * np.abs(J).max())
