@@ -69,6 +69,25 @@ def test_seven_planes_are_fp64_class():
     assert (np.abs(f32 - want) / scale).max() > 1e-9
 
 
+def test_level_sums_at_the_largest_k():
+    """K = 65,536 with every digit of every entry 63 (all of one sign, then random signs): the
+    level sums are as large as they get, 2^30.8 in a level and 2^49 in the integer that four
+    levels of seven planes are combined in."""
+    rng = np.random.default_rng(65536)
+    m, n, k = 130, 65, 65536
+    v = 63.0 / 127.0
+    A, B = np.full((m, k), v), np.full((n, k), -v)
+    A[1:] *= np.exp2(rng.integers(-3, 4, m - 1))[:, None]
+    sign = rng.choice([-1.0, 1.0], (2, k))
+    A[100:] *= sign[0]
+    B[40:] *= sign[1]
+    want = A @ B.T
+    for S in (2, 4, 6, 7):
+        err = np.abs(gemm(A, B, S) - want)
+        # (and the FP64 rounding of the reference's own sums)
+        assert np.all(err <= bound(A, B, S) + 1e-13 * np.abs(want).max())
+
+
 def test_accumulate_and_alpha():
     rng = np.random.default_rng(3)
     A = rng.standard_normal((200, 96))

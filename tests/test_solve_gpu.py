@@ -261,3 +261,27 @@ def test_mixed_solve_fp64_factor_small_orders(n):
     ref = np.linalg.solve(A32.astype(np.float64) + 1e-3 * np.eye(n), y)
     np.testing.assert_allclose(alpha.cpu().numpy(), ref, rtol=1e-8,
                                atol=1e-8 * np.abs(ref).max())
+
+
+@pytest.mark.parametrize("n", [3, 64, 200])
+@pytest.mark.parametrize("bits", [0xFFFFFFFFFFFFFFFF, 0x7FF8000000000000, 0x7FF0000000000000])
+def test_triangular_solves_of_undefined_right_hand_sides(n, bits):
+    """The sweeps mark elements that are not there yet by a bit pattern (all ones, a NaN): a
+    right-hand side that holds that pattern, another NaN or an infinity ends without a timeout
+    and with no finite number; the right-hand sides before and after it are unaffected."""
+    import torch
+
+    from kernelforge_b200 import cuda_global_kernels as cgk
+    rng = np.random.default_rng(n)
+    G = rng.normal(size=(n, n))
+    A = G @ G.T / n + np.eye(n)
+    K = torch.tensor(o.full_to_rfp(A, uplo_lower=True), device="cuda")
+    assert cgk.rfp_potrf(K, n) == 0
+    b = rng.normal(size=(3, n))
+    b[1, n // 2] = np.array([bits], np.uint64).view(np.float64)[0]
+    B = torch.tensor(b.reshape(n, 3), device="cuda")   # (column-major: three columns of n)
+    cgk.rfp_potrs(K, B, "L")
+    x = B.cpu().numpy().reshape(3, n)
+    assert not np.isfinite(x[1]).any()
+    for k in (0, 2):
+        np.testing.assert_allclose(x[k], np.linalg.solve(A, b[k]), rtol=1e-9, atol=1e-9)
