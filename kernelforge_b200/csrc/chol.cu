@@ -362,9 +362,11 @@ constexpr size_t DBLK_SMEM =
 constexpr int BLK_WORK = BLK_WARPS * 3 / 4;   // warps of B and C
 
 // a (lower triangle) -> its Cholesky factor, rinv = 1 / diagonal.  1 /
-// sqrt(pivot) is the approximation instruction (about 2^-20) refined by one
-// step of third order, r (1 + e/2 + 3 e^2/8) with e = 1 - d r^2 (the rest is
-// 5/16 e^3).  False (a, rinv void) unless every pivot is positive and far from
+// sqrt(pivot) is PTX's approximation instruction (about 2^-20) refined by one step
+// of Chebyshev's third-order iteration (Traub, Iterative Methods for the Solution
+// of Equations, 1964) for f(r) = r^-2 - d: with e = 1 - d r^2, the
+// first terms of the binomial series (1 - e)^(-1/2) = 1 + e/2 + 3 e^2/8 + ...; the
+// rest is 5/16 e^3.  False (a, rinv void) unless every pivot is positive and far from
 // the ends of the range: an integer test of the exponents, off the pivot chain.
 __device__ __forceinline__ bool chol8(double (&a)[DB][DB], double (&rinv)[DB]) {
     bool ok = true;

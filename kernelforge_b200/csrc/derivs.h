@@ -38,7 +38,7 @@ struct DerivSet {
     const void *x = nullptr;   // device (nm, ma, rep)
     const void *dx = nullptr;  // device (nm, ma, rep, 3 ma) or null
     SetView v;
-    float dx_max = -1.f;       // max |dx| over the real atoms (< 0: not known)
+    float dx_max = 0.f;        // max |dx| over the real atoms (compact_columns)
 };
 
 __device__ __forceinline__ void sink_put(const ElemSink &s, long long idx, double v) {

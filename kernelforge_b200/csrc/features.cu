@@ -107,13 +107,11 @@ __global__ void gather_rows_f32_kernel(const T *__restrict__ x, const int *__res
     }
 }
 
-// dst[c * ld_dst + r] = src[r][c] for a BF16 (rows, cols) array, and
-// colsum[c] += sum_r src[r][c] (FP32, optional).  64 x 64 tiles through shared
-// memory; bf16x2 loads along c and bf16x2 stores along r when cols, ld_dst and
+// dst[c * ld_dst + r] = src[r][c] for a BF16 (rows, cols) array.  64 x 64 tiles
+// through shared memory; bf16x2 loads along c and bf16x2 stores along r when cols, ld_dst and
 // the pointers allow it (128-byte accesses per warp), element-wise otherwise.
 __global__ void transpose_bf16_kernel(const bf16 *__restrict__ src, int rows, int cols,
-                                      bf16 *__restrict__ dst, long long ld_dst,
-                                      float *__restrict__ colsum, int pairs) {
+                                      bf16 *__restrict__ dst, long long ld_dst, int pairs) {
     __shared__ float tile[64][65];
     const int r0 = blockIdx.y * 64, c0 = blockIdx.x * 64;
     const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
@@ -147,21 +145,16 @@ __global__ void transpose_bf16_kernel(const bf16 *__restrict__ src, int rows, in
                 if (r + 1 < rows) d[1] = __float2bfloat16_rn(v1);
             }
         }
-        if (colsum) {
-            float t = v0 + v1;
-            for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-            if (tx == 0 && c < cols) atomicAdd(colsum + c, t);
-        }
     }
 }
 
 kfb_status transpose_bf16(const bf16 *src, int rows, int cols, bf16 *dst, long long ld_dst,
-                          float *colsum, cudaStream_t s) {
+                          cudaStream_t s) {
     const bool pairs = cols % 2 == 0 && ld_dst % 2 == 0 &&
                        (reinterpret_cast<uintptr_t>(src) & 3u) == 0 &&
                        (reinterpret_cast<uintptr_t>(dst) & 3u) == 0;
     transpose_bf16_kernel<<<dim3(nblk(cols, 64), nblk(rows, 64)), dim3(32, 8), 0, s>>>(
-        src, rows, cols, dst, ld_dst, colsum, pairs ? 1 : 0);
+        src, rows, cols, dst, ld_dst, pairs ? 1 : 0);
     KFB_CUDA_TRY(cudaGetLastError());
     return KFB_OK;
 }
@@ -254,7 +247,7 @@ __device__ __forceinline__ void sincos_reduced(float x, float &sn, float &cs) {
 // transpose pass that reads dZ2 back moves as much and more (50 + 48 us for
 // 8,192 rows of 4,096), and 8- or 16-byte pieces of the transpose written
 // straight from a block of few pairs took 110 us.
-constexpr int PL_MAX_D = 4096;
+constexpr int PL_MAX_D = 4096;   // largest D a map is created with (what the tests cover)
 __global__ void __launch_bounds__(256)
     pair_dot_kernel(const float *__restrict__ z2, int Bp, int npairs, int D,
                     const float *__restrict__ target, float s2, float gscale,
@@ -1069,7 +1062,7 @@ kfb_status cosmlp_step_t(kfb_cosmlp *h, int e, const T *x, long long nrows, cons
         adam_kernel<<<as.first[4], 256, 0, s>>>(as, lr, bc1, bc2);
         KFB_CUDA_TRY(cudaGetLastError());
         for (const P &q : ps)
-            if (q.pbt) KFB_TRY(transpose_bf16(q.pb, q.rows, q.cols, q.pbt, q.rows, nullptr, s));
+            if (q.pbt) KFB_TRY(transpose_bf16(q.pb, q.rows, q.cols, q.pbt, q.rows, s));
     }
     int herr[2] = {0, 0};
     double lsum = 0.0;
@@ -1280,7 +1273,7 @@ kfb_status kfb_cosmlp_sync(kfb_cosmlp *h, int reset_optimizer, void *stream) {
             nullptr);
         KFB_CUDA_TRY(cudaGetLastError());
         KFB_TRY(transpose_bf16(h->w2b.as<bf16>() + (size_t)e * D * H, D, H,
-                               h->w2tb.as<bf16>() + (size_t)e * H * D, D, nullptr, s));
+                               h->w2tb.as<bf16>() + (size_t)e * H * D, D, s));
     }
     if (reset_optimizer) {
         const size_t sizes[4] = {(size_t)h->nelem * H * rep, (size_t)h->nelem * H,

@@ -1,7 +1,7 @@
 // FP64-class products on the int8 tensor cores: slicing kernels and the
 // tcgen05 kind::i8 GEMM (see ozaki.h for the scheme).
 //
-// Kernel roles (one persistent CTA per SM over a tile list, 384 threads):
+// Kernel roles (a CTA per SM or per few tiles over a tile set, 640 threads):
 //   warp 0      TMA producer: per 64-byte K slice, the S digit planes of the
 //               A tile (128 rows) and of the B tile (BN = 128 rows for S <= 4,
 //               else 64), 64-byte swizzle, into a shared-memory ring of 2-4
@@ -89,8 +89,8 @@ __device__ __forceinline__ void umma_i8(uint32_t dtmem, uint64_t a, uint64_t b, 
 }
 
 // Column tiles of row tile ti in lower mode: the ones holding some j <= i.
-__host__ __device__ __forceinline__ int lower_tiles(int ti, int ntc, int BN) {
-    return min(ntc, ((ti + 1) * BM + BN - 1) / BN);
+inline int lower_tiles(int ti, int ntc, int BN) {
+    return std::min(ntc, ((ti + 1) * BM + BN - 1) / BN);
 }
 
 // Tile t of a generated tile set (see OzGen), BN columns per tile.
@@ -425,59 +425,6 @@ __global__ void slice_rows_kernel(const T *__restrict__ src, long long rows, int
     }
 }
 
-// Column-major source: a block takes 32 rows, stages their K columns
-// (coalesced along the rows) in shared memory, then one warp per row.
-template <int S>
-__global__ void slice_cols_kernel(const double *__restrict__ src, long long rows, int K,
-                                  long long ld, int kp, int8_t *__restrict__ d,
-                                  int *__restrict__ e) {
-    extern __shared__ double tile[];   // [K][33]
-    const long long r0 = (long long)blockIdx.x * 32;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    {
-        // every load of the tile in flight at once (cp.async, 8 bytes each;
-        // rows beyond the source are zero-filled)
-        const long long r = r0 + lane;
-        const bool ok = r < rows;
-        const double *col0 = src + (ok ? r : 0);
-        for (int k = warp; k < K; k += nw) {
-            const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(tile + k * 33 + lane));
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d),
-                         "l"(col0 + (long long)k * ld), "r"(ok ? 8 : 0)
-                         : "memory");
-        }
-        asm volatile("cp.async.wait_all;" ::: "memory");
-    }
-    __syncthreads();
-    const long long plane = rows * (long long)kp;
-    for (int rl = warp; rl < 32; rl += nw) {
-        const long long r = r0 + rl;
-        if (r >= rows) break;
-        double m = 0.0;
-        for (int k = lane; k < K; k += 32) m = fmax(m, fabs(tile[k * 33 + rl]));
-        for (int o = 16; o; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-        const int ex = oz_row_exponent(m);
-        if (lane == 0) e[r] = ex;
-        for (int k0 = lane * 4; k0 < kp; k0 += 128) {
-            int8_t dg[4][S];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int k = k0 + c;
-                const double v = k < K ? ldexp(tile[k * 33 + rl], -ex) : 0.0;
-                oz_digits<S>(v, dg[c]);
-            }
-#pragma unroll
-            for (int s = 0; s < S; ++s) {
-                const uint32_t w = (uint32_t)(uint8_t)dg[0][s] |
-                                   ((uint32_t)(uint8_t)dg[1][s] << 8) |
-                                   ((uint32_t)(uint8_t)dg[2][s] << 16) |
-                                   ((uint32_t)(uint8_t)dg[3][s] << 24);
-                *reinterpret_cast<uint32_t *>(d + s * plane + r * kp + k0) = w;
-            }
-        }
-    }
-}
-
 PFN_cuTensorMapEncodeTiled_v12000 oz_encoder() {
     static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
     static std::once_flag once;
@@ -573,40 +520,6 @@ template kfb_status oz_slice_rows<double>(const double *, long long, int, long l
                                           const OzSlices &, cudaStream_t);
 template kfb_status oz_slice_rows<float>(const float *, long long, int, long long,
                                          const OzSlices &, cudaStream_t);
-
-kfb_status oz_slice_cols(const double *src, long long rows, int K, long long ld,
-                         const OzSlices &o, cudaStream_t s) {
-    KFB_TRY(oz_check(o, K));
-    if (rows <= 0) return KFB_OK;
-    if (K > 512) return set_error(KFB_ERR_INVALID_ARG, "column-major slicing takes K <= 512");
-    const unsigned g = (unsigned)((rows + 31) / 32);
-    const size_t sm = (size_t)std::max(K, 1) * 33 * sizeof(double);
-    switch (o.S) {
-#define KFB_OZ_COLS(SS)                                                                       \
-    case SS: {                                                                                \
-        static bool a = false;                                                                \
-        if (!a) {                                                                             \
-            KFB_CUDA_TRY(cudaFuncSetAttribute(slice_cols_kernel<SS>,                           \
-                                              cudaFuncAttributeMaxDynamicSharedMemorySize,    \
-                                              512 * 33 * (int)sizeof(double)));               \
-            a = true;                                                                         \
-        }                                                                                     \
-        slice_cols_kernel<SS><<<g, 256, sm, s>>>(src, rows, K, ld, o.kp, o.d, o.e);           \
-        break;                                                                                \
-    }
-        KFB_OZ_COLS(2)
-        KFB_OZ_COLS(3)
-        KFB_OZ_COLS(4)
-        KFB_OZ_COLS(5)
-        KFB_OZ_COLS(6)
-        KFB_OZ_COLS(7)
-#undef KFB_OZ_COLS
-        default:
-            return set_error(KFB_ERR_INVALID_ARG, "digit planes S=%d outside 2..%d", o.S, OZ_MAXS);
-    }
-    KFB_CUDA_TRY(cudaGetLastError());
-    return KFB_OK;
-}
 
 namespace {
 
@@ -749,8 +662,7 @@ kfb_status oz_gemm(const OzSlices &A, const OzSlices &B, const OzTile *tiles, in
 
 kfb_status oz_gemm_gen(const OzSlices &A, const OzSlices &B, const OzGen &g, const OzEpi &epi,
                        int *err, cudaStream_t s) {
-    return oz_gemm_core(A, B, nullptr, g, oz_gen_tiles(g, A.S), epi, err,
-                        s);
+    return oz_gemm_core(A, B, nullptr, g, oz_gen_tiles(g, A.S), epi, err, s);
 }
 
 kfb_status oz_gemm_dense(const OzSlices &A, const OzSlices &B, int M, int N, const OzEpi &epi,

@@ -9,8 +9,9 @@
 //     C_L = sum_{p + q = L} sum_k d_p[r][k] d'_q[c][k]      (L = 2 .. S + 1)
 // where every C_L is an exact int32 sum of int8 x int8 products (|C_L| <=
 // S K 4096 < 2^31 for K <= 65536).  The S level sums of one output tile live
-// in TMEM side by side; the epilogue combines them in FP64 (Horner in 2^-7),
-// so the only rounding is the slicing remainder and the final FP64 additions:
+// in TMEM side by side; the epilogue combines the first half of them and the
+// second half as one exact integer each and adds the two in FP64, so the only
+// rounding is the slicing remainder, that addition and the final scaling:
 // about 7 S - 1 significant bits per operand (S = 7: ~48 bits, S = 4: ~27).
 //
 // S(S+1)/2 int8 MMAs per K step replace one FP64 product; the int8 tensor
@@ -48,11 +49,9 @@ inline int oz_kp(int k) { return (k + OZ_BK - 1) / OZ_BK * OZ_BK; }
 template <class T>
 kfb_status oz_slice_rows(const T *src, long long rows, int K, long long ld, const OzSlices &out,
                          cudaStream_t s);
-// Slice rows of a column-major source: a[r][k] = src[k * ld + r] (K <= 512).
-kfb_status oz_slice_cols(const double *src, long long rows, int K, long long ld,
-                         const OzSlices &out, cudaStream_t s);
-// The same for any K (<= 65536): row maxima in a first pass (scratch_max, one
-// 64-bit word per row), then the digits through shared-memory tiles.
+// Slice rows of a column-major source: a[r][k] = src[k * ld + r], row maxima in a
+// first pass (scratch_max, one 64-bit word per row), then the digits through
+// shared-memory tiles.
 kfb_status oz_slice_colmajor(const double *src, long long rows, int K, long long ld,
                              const OzSlices &out, unsigned long long *scratch_max,
                              cudaStream_t s);

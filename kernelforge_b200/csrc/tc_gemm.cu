@@ -737,51 +737,6 @@ kfb_status launch(const TcOperand &A, const TcOperand &B, bool bf16,
 }
 
 // ---------------------------------------------------------------- packing
-template <class T>
-__global__ void absmax_kernel(const T *__restrict__ src, long long n, float *out) {
-    float m = 0.f;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-         i += (long long)gridDim.x * blockDim.x)
-        m = fmaxf(m, fabsf((float)src[i]));
-    for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    // non-negative floats order like their bit patterns
-    if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<int *>(out), __float_as_int(m));
-}
-
-// max |dX[m][j][k][c]| over the real atoms of each molecule (j < nat[m],
-// c < 3 nat[m]); padding entries are never read by the GEMMs and may hold
-// anything
-template <class T>
-__global__ void absmax_dx_kernel(const T *__restrict__ dx, int ma, int rep,
-                                 const int *__restrict__ nat, float *out) {
-    const int m = blockIdx.y;
-    const int na = min(max(nat[m], 0), ma);
-    const int ld = 3 * ma, nc = 3 * na;
-    const long long n = (long long)na * rep * nc;
-    const T *base = dx + (size_t)m * ma * rep * ld;
-    // warp per row (j, k), lanes over its 3 na columns
-    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    const long long nrow = n / (nc > 0 ? nc : 1);
-    float v = 0.f;
-    for (long long row = (long long)blockIdx.x * nw + (threadIdx.x >> 5); row < nrow;
-         row += (long long)gridDim.x * nw)
-        for (int c = lane; c < nc; c += 32) v = fmaxf(v, fabsf((float)base[row * ld + c]));
-    for (int o = 16; o; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<int *>(out), __float_as_int(v));
-}
-
-template <class T>
-__global__ void split_rows_kernel(const T *__restrict__ src, long long n, float scale,
-                                  __half *__restrict__ hi, __half *__restrict__ lo) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-         i += (long long)gridDim.x * blockDim.x) {
-        const float v = (float)src[i] * scale;
-        const __half h = __float2half_rn(v);
-        hi[i] = h;
-        lo[i] = __float2half_rn(v - __half2float(h));
-    }
-}
-
 // Jt[(m, c)][(j, k)] = dX[m][j][k][c].  Tiles of 64 (j,k) x 32 c through
 // shared memory (rows of dX read 128 bytes per warp, rows of Jt written as
 // fp16 pairs, 128 bytes per warp); tiles wholly beyond the molecule's atoms
@@ -872,37 +827,6 @@ __global__ void __launch_bounds__(256) transpose_split_dx_rows_kernel(
     }
 }
 
-// Yt[(p, c)][(i, k)] = Y[p][i][k][c], Y with row stride ld (the Hessian's
-// per-pair Y blocks, ma1 x rep x ld each).
-template <class T>
-__global__ void transpose_split_y_kernel(const T *__restrict__ Y, int ma1, int rep, int ld,
-                                         float scale, __half *__restrict__ hi,
-                                         __half *__restrict__ lo) {
-    __shared__ float tile[32][33];
-    const int p = blockIdx.z;
-    const long long kk_total = (long long)ma1 * rep;
-    const long long kk0 = (long long)blockIdx.x * 32;
-    const int c0 = blockIdx.y * 32;
-    const T *base = Y + (size_t)p * kk_total * ld;
-    for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-        const long long kk = kk0 + r;
-        const int c = c0 + threadIdx.x;
-        tile[r][threadIdx.x] = (kk < kk_total && c < ld) ? (float)base[kk * ld + c] : 0.f;
-    }
-    __syncthreads();
-    for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-        const int c = c0 + r;
-        const long long kk = kk0 + threadIdx.x;
-        if (c < ld && kk < kk_total) {
-            const float v = tile[threadIdx.x][r] * scale;
-            const __half h = __float2half_rn(v);
-            const size_t o = ((size_t)p * ld + c) * kk_total + kk;
-            hi[o] = h;
-            lo[o] = __float2half_rn(v - __half2float(h));
-        }
-    }
-}
-
 }  // namespace
 
 kfb_status tc_gemm_grouped(const TcOperand &A, const TcOperand &B, int nprod, bool bf16,
@@ -944,47 +868,12 @@ kfb_status pow2_from_device(const float *dmax, cudaStream_t s, float *scale) {
 }
 
 template <class T>
-kfb_status pow2_scale(const T *src, long long n, cudaStream_t s, float *scale) {
-    *scale = 1.f;
-    if (n <= 0) return KFB_OK;
-    DevBuf d;
-    KFB_TRY(d.alloc(sizeof(float), s));
-    KFB_TRY(zero(d.ptr, sizeof(float), s));
-    const unsigned blocks = (unsigned)std::min<long long>((n + 255) / 256, 148LL * 16);
-    absmax_kernel<T><<<blocks, 256, 0, s>>>(src, n, d.as<float>());
-    KFB_CUDA_TRY(cudaGetLastError());
-    return pow2_from_device(d.as<float>(), s, scale);
-}
-
-template <class T>
-kfb_status split_rows(const T *src, long long n, __half *hi, __half *lo, float *scale,
-                      cudaStream_t s) {
-    KFB_TRY(pow2_scale(src, n, s, scale));
-    if (n <= 0) return KFB_OK;
-    const unsigned blocks = (unsigned)std::min<long long>((n + 255) / 256, 148LL * 64);
-    split_rows_kernel<T><<<blocks, 256, 0, s>>>(src, n, *scale, hi, lo);
-    KFB_CUDA_TRY(cudaGetLastError());
-    return KFB_OK;
-}
-
-template <class T>
 kfb_status transpose_split_dx(const T *dx, int nm, int ma, int rep, const int *nat, __half *hi,
                               __half *lo, float *scale, cudaStream_t s, float dx_max) {
     const long long kk = (long long)ma * rep;
     *scale = 1.f;
     if (nm <= 0) return KFB_OK;
-    if (dx_max >= 0.f) {
-        *scale = pow2_for(dx_max);
-    } else {
-        DevBuf d;
-        KFB_TRY(d.alloc(sizeof(float), s));
-        KFB_TRY(zero(d.ptr, sizeof(float), s));
-        const long long per = kk * 3 * ma;
-        const unsigned bx = (unsigned)std::min<long long>((per + 255) / 256, 64);
-        absmax_dx_kernel<T><<<dim3(bx, (unsigned)nm), 256, 0, s>>>(dx, ma, rep, nat, d.as<float>());
-        KFB_CUDA_TRY(cudaGetLastError());
-        KFB_TRY(pow2_from_device(d.as<float>(), s, scale));
-    }
+    *scale = pow2_for(dx_max);
     dim3 grid((unsigned)((kk + 64 * TDX_TILES - 1) / (64 * TDX_TILES)),
               (unsigned)((3 * ma + 31) / 32), (unsigned)nm);
     transpose_split_dx_kernel<T><<<grid, 256, 0, s>>>(dx, ma, rep, nat, *scale, hi, lo);
@@ -998,18 +887,7 @@ kfb_status transpose_split_dx_rows(const T *dx, int nm, int ma, int rep, const i
                                    const int *blockmap, float dx_max) {
     *scale = 1.f;
     if (nm <= 0) return KFB_OK;
-    if (dx_max >= 0.f) {
-        *scale = pow2_for(dx_max);
-    } else {
-        DevBuf d;
-        KFB_TRY(d.alloc(sizeof(float), s));
-        KFB_TRY(zero(d.ptr, sizeof(float), s));
-        const long long per = (long long)ma * rep * 3 * ma;
-        const unsigned bx = (unsigned)std::min<long long>((per + 255) / 256, 64);
-        absmax_dx_kernel<T><<<dim3(bx, (unsigned)nm), 256, 0, s>>>(dx, ma, rep, nat, d.as<float>());
-        KFB_CUDA_TRY(cudaGetLastError());
-        KFB_TRY(pow2_from_device(d.as<float>(), s, scale));
-    }
+    *scale = pow2_for(dx_max);
     dim3 grid((unsigned)(nm * ma), (unsigned)((rep + 31) / 32), (unsigned)((3 * ma + 31) / 32));
     transpose_split_dx_rows_kernel<T><<<grid, 256, 0, s>>>(dx, ma, rep, nat, blockmap, *scale,
                                                            hi, lo);
@@ -1017,22 +895,6 @@ kfb_status transpose_split_dx_rows(const T *dx, int nm, int ma, int rep, const i
     return KFB_OK;
 }
 
-template <class T>
-kfb_status transpose_split_y(const T *Y, int np, int ma1, int rep, int ld, const float *amax,
-                             __half *hi, __half *lo, float *scale, cudaStream_t s) {
-    const long long kk = (long long)ma1 * rep;
-    KFB_TRY(pow2_from_device(amax, s, scale));
-    if (np <= 0) return KFB_OK;
-    dim3 grid((unsigned)((kk + 31) / 32), (unsigned)((ld + 31) / 32), (unsigned)np);
-    transpose_split_y_kernel<T><<<grid, dim3(32, 8), 0, s>>>(Y, ma1, rep, ld, *scale, hi, lo);
-    KFB_CUDA_TRY(cudaGetLastError());
-    return KFB_OK;
-}
-
-template kfb_status split_rows<float>(const float *, long long, __half *, __half *, float *,
-                                      cudaStream_t);
-template kfb_status split_rows<double>(const double *, long long, __half *, __half *, float *,
-                                       cudaStream_t);
 template kfb_status transpose_split_dx_rows<float>(const float *, int, int, int, const int *,
                                                    __half *, __half *, float *, cudaStream_t,
                                                    const int *, float);
@@ -1040,9 +902,4 @@ template kfb_status transpose_split_dx<float>(const float *, int, int, int, cons
                                               __half *, float *, cudaStream_t, float);
 template kfb_status transpose_split_dx<double>(const double *, int, int, int, const int *,
                                                __half *, __half *, float *, cudaStream_t, float);
-template kfb_status transpose_split_y<float>(const float *, int, int, int, int, const float *,
-                                             __half *, __half *, float *, cudaStream_t);
-template kfb_status transpose_split_y<double>(const double *, int, int, int, int, const float *,
-                                              __half *, __half *, float *, cudaStream_t);
-
 }  // namespace kfb

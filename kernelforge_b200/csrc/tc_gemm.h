@@ -95,32 +95,25 @@ kfb_status tc_gemm_grouped(const TcOperand &A, const TcOperand &B, int nprod, bo
                            const std::vector<TcProb> &probs, const ElemSink &sink,
                            cudaStream_t s, const TcEpi &epi = TcEpi(), int *err_flag = nullptr);
 
-// Split packers: multiply by a power-of-two scale (returned in *scale; the
-// largest magnitude of the entries the GEMMs read lands near 2^14) and write
-// the fp16 pair hi = fp16(v), lo = fp16(v - hi).  GEMM results are divided by
-// the two operands' scales.
-//   split_rows:         every entry of src is read;
-//   transpose_split_dx: nat (device int32, per molecule) limits the scale to
-//                       the real atoms, padding may hold anything; 32 x 32
-//                       tiles wholly beyond the real atoms stay unwritten;
-//                       dx_max >= 0 is that largest magnitude when the caller
-//                       knows it (else a pass and a synchronisation find it);
-//   transpose_split_y:  amax (device float) is the largest |entry| the
-//                       producer wrote (the rest of Y is never read).
+// Split packers: multiply by a power-of-two scale (returned in *scale: the
+// largest magnitude of the entries the GEMMs read, dx_max, lands near 2^14) and
+// write the fp16 pair hi = fp16(v), lo = fp16(v - hi).  GEMM results are divided
+// by the two operands' scales.
+//
+// Jt[(m, c)][(j, k)] = dX[m][j][k][c]: padding may hold anything; tiles of 64
+// (j, k) x 32 c wholly beyond the real atoms (nat, device, per molecule) stay
+// unwritten.
 template <class T>
-kfb_status split_rows(const T *src, long long n, __half *hi, __half *lo, float *scale,
-                      cudaStream_t s);
+kfb_status transpose_split_dx(const T *dx, int nm, int ma, int rep, const int *nat, __half *hi,
+                              __half *lo, float *scale, cudaStream_t s, float dx_max);
 // Jr[(m, j, c)][k] = dX[m][j][k][c] as scaled fp16 pairs: a K-major row of rep
 // per (atom, coordinate column); rows of padding atoms and columns are not
-// written.  blockmap (device, per atom m * ma + j, optional) moves atom (m, j)'s
+// written.  blockmap (device, per atom m * ma + j, or null) moves atom (m, j)'s
 // 3 ma rows to block blockmap[m * ma + j] (< 0: not written).
 template <class T>
 kfb_status transpose_split_dx_rows(const T *dx, int nm, int ma, int rep, const int *nat,
                                    __half *hi, __half *lo, float *scale, cudaStream_t s,
-                                   const int *blockmap = nullptr, float dx_max = -1.f);
-template <class T>
-kfb_status transpose_split_dx(const T *dx, int nm, int ma, int rep, const int *nat, __half *hi,
-                              __half *lo, float *scale, cudaStream_t s, float dx_max = -1.f);
+                                   const int *blockmap, float dx_max);
 // Power of two that brings m to about 2^14 (1 for 0 and what is not finite).
 float pow2_for(float m);
 // Host copy of a power of two that brings the device float *dmax to about
@@ -128,8 +121,5 @@ float pow2_for(float m);
 kfb_status pow2_from_device(const float *dmax, cudaStream_t s, float *scale);
 // The same left on the device, in *scale.
 kfb_status pow2_on_device(const float *dmax, float *scale, cudaStream_t s);
-template <class T>
-kfb_status transpose_split_y(const T *Y, int np, int ma1, int rep, int ld, const float *amax,
-                             __half *hi, __half *lo, float *scale, cudaStream_t s);
 
 }  // namespace kfb
