@@ -181,6 +181,20 @@ def p_sym(Q, N):
                                                                           counts.tolist()))
 
 
+def scalar_columns(X, Q, N):
+    """Columns that the tensor-core scalar kernel multiplies, by label: those that one of the
+    label's atoms uses, up to whole MMA steps of 16."""
+    act = np.arange(Q.shape[1])[None, :] < np.clip(N, 0, Q.shape[1])[:, None]
+    out = {}
+    for l in np.unique(Q[act]).tolist():
+        used = np.zeros(X.shape[2], bool)
+        rows = np.flatnonzero(act & (Q == l))
+        for r in range(0, rows.size, 8192):
+            used |= (X.reshape(-1, X.shape[2])[rows[r:r + 8192]] != 0).any(axis=0)
+        out[l] = max(16, -(-int(used.sum()) // 16) * 16)
+    return out
+
+
 def load_peaks():
     try:
         with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
@@ -389,8 +403,10 @@ def run_ours(args, rank, world, local):
         return
     peaks, peak_kind = load_peaks()
     psym, per_label = p_sym(Q, N)
-    # the three compensated fp16 products over the unique same-label pairs
-    flops = 3 * 2.0 * REP * psym
+    # the three compensated fp16 products over the unique same-label pairs and the
+    # columns that are multiplied (not those that no atom of the label uses)
+    cols = scalar_columns(X, Q, N)
+    flops = sum(3 * 2.0 * cols[l] * (c * (c + 1) // 2) for l, c in per_label.items())
     kms = statistics.median(kernel_ms)
     achieved = flops / (kms * 1e-3) / 1e12
     peak = peaks.get("bf16_tflops")
@@ -427,7 +443,8 @@ def run_ours(args, rank, world, local):
         "roofline": {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                      "frac": achieved / peak if peak else None, "traffic": traffic_per_launch(),
                      "peak_kind": f"{peak_kind} bf16 dense (f16 MMAs run at the same rate)",
-                     "flops_per_launch": flops, "unique_pairs": psym},
+                     "flops_per_launch": flops, "unique_pairs": psym,
+                     "columns_by_label": {str(l): c for l, c in cols.items()}},
         "cpu_baseline": cpu,
         "clocks": clk_info,
         "e2e": {"value": entries * world / (e2e_ms * 1e-3), "unit": "entries/s",
@@ -440,7 +457,7 @@ def run_ours(args, rank, world, local):
 
 def fp64_and_accuracy(X, Q, N, y, dev, nsub=2000, ntrain=1600):
     """Outside the timed region: (1) the plain FP64 GPU fit of the same workload
-    (FP64 CUDA-core kernel + FP64 RFP Cholesky), timed once; (2) on a
+    (FP64 kernel + FP64 RFP Cholesky), timed once; (2) on a
     2,000-molecule subset, the tensor-core kernel's error against the FP64
     kernel (which matches the CPU oracle to 1e-12 in the tests) and the KRR test
     MAE of the FP32-TC + FP64-refinement fit against the FP64 fit (1600/400)."""
@@ -1251,7 +1268,10 @@ def run_rff_force(args):
     # GEMM rows of the force features: every atom contributes the 3 n columns of
     # its molecule's Jacobian (three fp16 products per multiply-add)
     gemm_rows = int((3 * N.astype(np.int64) * N).sum())
-    g_flops = 3 * 2 * gemm_rows * 720 * D
+    # (the columns that X or dX uses, up to whole MMA steps of 16)
+    used = (X != 0).flatten(0, 1).any(0) | (dX != 0).flatten(0, 1).flatten(2).any(2).any(0)
+    kcols = -(-int(used.sum()) // 16) * 16
+    g_flops = 3 * 2 * gemm_rows * kcols * D
     for l2 in (1e-6, 1e-4, 1e-2):
         w, info = fit(l2)
         Ep = (crf.rff_features_elemental(Xt, Qt, Nt, W, b).double() @ w).cpu().numpy() + em
@@ -1267,6 +1287,7 @@ def run_rff_force(args):
           "ridge solve on [Z; G]", "f16x3 / f32 features + f64 refinement",
           {"higher_is_better": False, "lambda_scan": out, "lambda_best": float(best),
            "force_features_ms": g_ms, "force_feature_gemm_rows": gemm_rows,
+           "force_feature_columns": kcols,
            "roofline": {"bound": "tensor", "achieved": g_flops / (g_ms * 1e-3) / 1e12,
                         "peak": peaks["bf16_tflops"], "unit": "TFLOP/s",
                         "frac": g_flops / (g_ms * 1e-3) / 1e12 / peaks["bf16_tflops"],
