@@ -893,20 +893,40 @@ __global__ void __launch_bounds__(256) pb_kernel(const T *__restrict__ x2,
 }
 
 // max |J_b| over the real atoms and columns of each molecule b (out zeroed
-// first; blockIdx.y splits a molecule's rows, warps per row)
-template <class T>
-__global__ void jmax_per_mol_kernel(const T *__restrict__ dx, int ma, int rep,
-                                    const int *__restrict__ nat, float *__restrict__ out) {
+// first; blockIdx.y splits a molecule's rows).  VEC (16-byte aligned, rep a
+// multiple of 4): the real atoms' rows are one run of memory, read 16 bytes a
+// lane, padding columns left out of the maximum; bound by HBM.  Else a warp per
+// row.
+template <bool VEC>
+__global__ void __launch_bounds__(256) jmax_per_mol_kernel(const float *__restrict__ dx, int ma,
+                                                           int rep, const int *__restrict__ nat,
+                                                           float *__restrict__ out) {
     const int m = blockIdx.x;
     const int na = min(max(nat[m], 0), ma), ld = 3 * ma, nc = 3 * na;
-    const T *base = dx + (size_t)m * ma * rep * ld;
+    const float *base = dx + (size_t)m * ma * rep * ld;
     float v = 0.f;
     const long long nrow = (long long)na * rep;
-    const int nw = blockDim.x >> 5;
-    for (long long row = (long long)blockIdx.y * nw + (threadIdx.x >> 5); row < nrow;
-         row += (long long)gridDim.y * nw)
-        for (int c = threadIdx.x & 31; c < nc; c += 32)
-            v = fmaxf(v, fabsf((float)base[row * ld + c]));
+    if constexpr (VEC) {
+        const float4 *p = reinterpret_cast<const float4 *>(base);
+        const unsigned n = (unsigned)(nrow * ld / 4), step = gridDim.y * 256;
+#pragma unroll 4
+        for (unsigned e = blockIdx.y * 256 + threadIdx.x; e < n; e += step) {
+            const float4 w = p[e];
+            const float a[4] = {w.x, w.y, w.z, w.w};
+            unsigned c = 4 * e % (unsigned)ld;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (c < (unsigned)nc) v = fmaxf(v, fabsf(a[u]));
+                if (++c == (unsigned)ld) c = 0;
+            }
+        }
+    } else {
+        const int nw = blockDim.x >> 5;
+        for (long long row = (long long)blockIdx.y * nw + (threadIdx.x >> 5); row < nrow;
+             row += (long long)gridDim.y * nw)
+            for (int c = threadIdx.x & 31; c < nc; c += 32)
+                v = fmaxf(v, fabsf(base[row * ld + c]));
+    }
     for (int o = 16; o; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
     // non-negative floats order like their bit patterns
     if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<int *>(out + m), __float_as_int(v));
@@ -2229,7 +2249,7 @@ long long label_problems(const LabelMajor &R, int r0, int r1, int mar, const Lab
 // batch (pairs with that b, in b order, as columns (q, i)), see jk_split_kernel.
 kfb_status hess_y_gemm(const HessPair *pairs, int np, int ma1, int ma2, int rep, int kj,
                        const float *W, const DevBuf &jkh, const DevBuf &jkl, float jk_scale,
-                       float w_scale, const float *y_scale, DevBuf &wsh, DevBuf &wsl, DevBuf &d_ymap,
+                       float w_scale, const float *y_max, DevBuf &wsh, DevBuf &wsl, DevBuf &d_ymap,
                        DevBuf &d_border, long long jk_rows, const HessPair *dpairs, __half *yhi,
                        __half *ylo, int *err, cudaStream_t s) {
     const int ld2 = 3 * ma2;
@@ -2248,7 +2268,7 @@ kfb_status hess_y_gemm(const HessPair *pairs, int np, int ma1, int ma2, int rep,
         pb.M = 3 * pr.nb * rep;
         pb.N = (q1 - q) * ma1;
         pb.K = kj;
-        pb.alpha = 1.0 / ((double)jk_scale * (double)w_scale);   // (times *y_scale)
+        pb.alpha = 1.0 / ((double)jk_scale * (double)w_scale);   // (and Y's own scale)
         probs.push_back(pb);
         q = q1;
     }
@@ -2277,7 +2297,7 @@ kfb_status hess_y_gemm(const HessPair *pairs, int np, int ma1, int ma2, int rep,
     epi.y_rep = rep;
     epi.y_ma1 = ma1;
     epi.y_ld2 = ld2;
-    epi.dscale = y_scale;
+    epi.dmax = y_max;
     return tc_gemm_grouped(A, B, 3, false, probs, ElemSink(), s, epi, err);
 }
 
@@ -2333,7 +2353,7 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
         KFB_TRY(transpose_split_dx<T>(static_cast<const T *>(s1.dx), s1.v.nm, ma1, rep,
                                       d_n1.as<int>(), jth.as<__half>(), jtl.as<__half>(),
                                       &jt_scale, s, s1.dx_max));
-        KFB_TRY(yamax.alloc(2 * sizeof(float), s));   // the batch's bound of |Y|, its scale
+        KFB_TRY(yamax.alloc(sizeof(float), s));
         KFB_TRY(yth.alloc((size_t)batch * ld2 * ma1 * rep * sizeof(__half), s));
         KFB_TRY(ytl.alloc((size_t)batch * ld2 * ma1 * rep * sizeof(__half), s));
     }
@@ -2546,8 +2566,11 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
             // per-molecule max |J| for the bound of |Y|
             KFB_TRY(d_jbm.alloc((size_t)s2.v.nm * sizeof(float), s));
             KFB_TRY(zero(d_jbm.ptr, (size_t)s2.v.nm * sizeof(float), s));
-            jmax_per_mol_kernel<float><<<dim3((unsigned)s2.v.nm, 32), 256, 0, s>>>(
-                dx2f, ma2, rep, d_nat2.as<int>(), d_jbm.as<float>());
+            const bool jvec = rep % 4 == 0 && (reinterpret_cast<size_t>(dx2f) & 15) == 0 &&
+                              (long long)ma2 * rep * ld2 < (1LL << 30);
+            auto jmax = jvec ? jmax_per_mol_kernel<true> : jmax_per_mol_kernel<false>;
+            jmax<<<dim3((unsigned)s2.v.nm, 32), 256, 0, s>>>(dx2f, ma2, rep, d_nat2.as<int>(),
+                                                             d_jbm.as<float>());
             KFB_CUDA_TRY(cudaGetLastError());
             if (ygemm) {
                 TraceScope tr_j("hessian:jk-split", s);
@@ -2676,11 +2699,10 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
         auto tr_y = std::make_unique<TraceScope>("hessian:y", s);
         float y_scale = 1.f;
         if (tc) {
-            if (ygemm) KFB_TRY(pow2_on_device(yamax.as<float>(), yamax.as<float>() + 1, s));
-            else KFB_TRY(pow2_from_device(yamax.as<float>(), s, &y_scale));
+            if (!ygemm) KFB_TRY(pow2_from_device(yamax.as<float>(), s, &y_scale));
             if (ygemm)
                 KFB_TRY(hess_y_gemm(pairs.data() + p0, np, ma1, ma2, rep, kj, W.as<float>(),
-                                    jkh, jkl, jr_scale, w_scale, yamax.as<float>() + 1, wsh, wsl,
+                                    jkh, jkl, jr_scale, w_scale, yamax.as<float>(), wsh, wsl,
                                     d_ymap,
                                     d_border, (long long)s2.v.nm * ld2 * rep,
                                     dpairs.as<HessPair>(), yth.as<__half>(), ytl.as<__half>(),
@@ -2754,7 +2776,7 @@ kfb_status hessian_core(const DerivSet &s1, const DerivSet &s2, int rep, double 
             TcEpi ec;
             ec.tile_n64 = narrow ? 1 : 0;
             ec.sink_t = narrow ? 1 : 0;
-            ec.dscale = ygemm ? yamax.as<float>() + 1 : nullptr;
+            ec.dmax = ygemm ? yamax.as<float>() : nullptr;
             KFB_TRY(tc_gemm_grouped(narrow ? Yo : J, narrow ? J : Yo, 3, false, tprobs, sink, s,
                                     ec, err.flag()));
             tr_g.reset();

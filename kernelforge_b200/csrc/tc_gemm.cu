@@ -135,6 +135,14 @@ __device__ __forceinline__ TcTile tile_at(const TcProb *__restrict__ probs,
     return TcTile{lo, mt * BM, (loc - mt * ntn) * bn, 0};
 }
 
+// pow2_for on the device
+__device__ __forceinline__ float pow2_near(float m) {
+    int e = 0;
+    const float f = frexpf(m, &e);   // m = f 2^e, f in [0.5, 1): ceil(log2 m) = e, or e - 1 at 0.5
+    const int p = 14 - (f == 0.5f ? e - 1 : e);
+    return m > 0.f && isfinite(m) ? ldexpf(1.f, min(p, 126)) : 1.f;
+}
+
 template <int NPROD, int NEPI, int BNT>
 __global__ void __launch_bounds__(Cfg<NPROD, NEPI, BNT>::THREADS, 1)
     tc_gemm_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant__ CUtensorMap ta_lo,
@@ -278,7 +286,7 @@ __global__ void __launch_bounds__(Cfg<NPROD, NEPI, BNT>::THREADS, 1)
         __shared__ float molsum_static[NEPI == 8 ? NEPI : 1][32][33];
         float(*molsum_scr)[32][33] =
             NEPI == 8 ? molsum_static : reinterpret_cast<float(*)[32][33]>(smem + C::OFF_SCR);
-        const float ds = epi.dscale ? *epi.dscale : 1.f;
+        const float ds = epi.dmax ? pow2_near(*epi.dmax) : 1.f;
         int acc = 0;
         uint32_t aph = 0;
         // the tile's problem (and for EPI_YSPLIT the (p, i) offset of this
@@ -843,20 +851,6 @@ kfb_status tc_gemm_grouped(const TcOperand &A, const TcOperand &B, int nprod, bo
 // then carries ~22 significant bits over ~28 binades below the maximum).
 float pow2_for(float m) {
     return (m > 0.f && std::isfinite(m)) ? std::ldexp(1.f, 14 - (int)std::ceil(std::log2(m))) : 1.f;
-}
-
-__global__ void pow2_scale_kernel(const float *__restrict__ dmax, float *__restrict__ scale) {
-    const float m = *dmax;
-    int e = 0;
-    const float f = frexpf(m, &e);   // m = f 2^e, f in [0.5, 1): ceil(log2 m) = e, or e - 1 at 0.5
-    const int p = 14 - (f == 0.5f ? e - 1 : e);
-    *scale = m > 0.f && isfinite(m) ? ldexpf(1.f, min(p, 126)) : 1.f;
-}
-
-kfb_status pow2_on_device(const float *dmax, float *scale, cudaStream_t s) {
-    pow2_scale_kernel<<<1, 1, 0, s>>>(dmax, scale);
-    KFB_CUDA_TRY(cudaGetLastError());
-    return KFB_OK;
 }
 
 kfb_status pow2_from_device(const float *dmax, cudaStream_t s, float *scale) {

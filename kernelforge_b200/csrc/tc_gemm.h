@@ -81,10 +81,10 @@ struct TcEpi {
     const int2 *ymap = nullptr;   // EPI_YSPLIT
     __half *yhi = nullptr, *ylo = nullptr;
     int y_rep = 0, y_ma1 = 0, y_ld2 = 0;
-    // EPI_YSPLIT writes alpha * acc times *dscale, EPI_SINK stores alpha * acc
-    // over *dscale: a power of two that an earlier kernel of the stream found
-    // (null: 1)
-    const float *dscale = nullptr;
+    // with dmax (device), a bound that an earlier kernel of the stream left:
+    // EPI_YSPLIT writes alpha * acc times the power of two that brings it to about
+    // 2^14, EPI_SINK stores alpha * acc over it
+    const float *dmax = nullptr;
 };
 
 // nprod = 3: split operands, hi*hi + hi*lo + lo*hi; nprod = 1: hi only.
@@ -119,7 +119,5 @@ float pow2_for(float m);
 // Host copy of a power of two that brings the device float *dmax to about
 // 2^14 (synchronises the stream).
 kfb_status pow2_from_device(const float *dmax, cudaStream_t s, float *scale);
-// The same left on the device, in *scale.
-kfb_status pow2_on_device(const float *dmax, float *scale, cudaStream_t s);
 
 }  // namespace kfb
