@@ -244,8 +244,8 @@ __device__ __forceinline__ void md_piece(T *dst, const T *src, bool ok, int left
     }
 }
 
-// Warp per row.  Query rows r < R1: n1[r] = |x|^2 (NaN for a row with a value that
-// is not finite).  Training rows: n2 = |x|^2,
+// Warp per row.  Query rows r < R1: n1[r] = |x|^2 (-infinity for a row that holds an
+// infinity, unlike one whose finite values have too large a sum).  Training rows: n2 = |x|^2,
 // sc = x . Ad, and used[g] = 1 for the column groups with a value that is not
 // zero.  Four columns a lane (vec: 16-byte loads, 128 columns of the warp in
 // flight per step), so a group of 8 is two neighbouring lanes.
@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(256) mv_rows_kernel(
     const Tin *x = (train ? x2 : x1) + at;
     const double *a = train && ad ? ad + at : nullptr;
     double n = 0.0, s = 0.0;
-    bool bad = false;
+    bool inf = false;
 #pragma unroll 3
     for (int k0 = 0; k0 < rep; k0 += 128) {
         const int k = k0 + 4 * lane;
@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(256) mv_rows_kernel(
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             n = fma(v[u], v[u], n);
-            bad |= !isfinite(v[u]);
+            inf |= isinf(v[u]);
             s = fma(v[u], w[u], s);
             on |= !(v[u] == 0.0) || !(w[u] == 0.0);
         }
@@ -303,13 +303,13 @@ __global__ void __launch_bounds__(256) mv_rows_kernel(
         n += __shfl_xor_sync(0xffffffffu, n, o);
         s += __shfl_xor_sync(0xffffffffu, s, o);
     }
-    bad = __any_sync(0xffffffffu, bad);
+    inf = __any_sync(0xffffffffu, inf);
     if (lane == 0) {
         if (train) {
             n2[r - R1] = n;
             sc[r - R1] = s;
         } else {
-            n1[r] = bad ? n - n : n;
+            n1[r] = inf ? -n : n;
         }
     }
 }
@@ -450,7 +450,7 @@ __global__ void __launch_bounds__(256, 2) mv_weights_kernel(
         for (int mi = 0; mi < 2; ++mi) {
             const int i = 16 * wm + 8 * mi + (lane >> 2);
             const double ni = i < na ? n1[lb.sa + i0 + i] : 0.0;
-            const double bad = ni == ni ? 0.0 : ni;   // NaN for a row that is not finite
+            const double bad = ni >= 0.0 ? 0.0 : ni - ni;   // NaN for a row that is not finite
             double esum = 0.0, vsum = 0.0;
 #pragma unroll
             for (int nj = 0; nj < 2; ++nj) {
@@ -460,8 +460,10 @@ __global__ void __launch_bounds__(256, 2) mv_weights_kernel(
                 for (int u = 0; u < 2; ++u) {
                     if (i >= na || j + u >= nb) continue;
                     const int jr = lb.sb + j0 + j + u;
-                    const double d2 = fmax(ni + n2[jr] - 2.0 * g[mi][nj][u], 0.0);
-                    const double e = exp(c * d2);
+                    // (with a norm that is not finite the product need not be either)
+                    const double nn = fabs(ni) + n2[jr];
+                    const double e =
+                        exp(c * (isfinite(nn) ? fmax(nn - 2.0 * g[mi][nj][u], 0.0) : nn));
                     const double dad = ad ? p[mi][nj][u] - sc[jr] + bad : 0.0;
                     const double ae = alpha_e ? alpha_e[idx2[jr] / ma2] : 0.0;
                     w[u] = e * is2;

@@ -15,8 +15,8 @@ constexpr int SPAD = 1;
 // Packed rows, their squared norms and molecules.  With `pos` (packed place of every
 // column per label, pack_columns_kernel), only the label's used columns are
 // stored; zeros follow up to the next multiple of SK.  The norm is over every
-// column; a row with a value that is not finite has an undefined norm, as its
-// products would have been (an infinite norm of finite values stays: e = 0).
+// column; a row with a value that is not finite in a column that is not stored
+// has an undefined norm, as its products with that column's zeros would have been.
 template <class Tin, class T>
 __global__ void pack_rows_kernel(const Tin *__restrict__ x, const int *__restrict__ src, int R,
                                  int rep, int Dp, const int *__restrict__ lab_start, int L,
@@ -37,7 +37,7 @@ __global__ void pack_rows_kernel(const Tin *__restrict__ x, const int *__restric
         const double v = (double)xr[k];
         const int p = pl ? pl[k] : k;
         if (p >= 0) orow[p] = (T)v;
-        bad |= !isfinite(v);
+        bad |= p < 0 && !isfinite(v);
         s += v * v;
     }
     bad = __any_sync(0xffffffffu, bad);

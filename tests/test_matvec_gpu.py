@@ -258,6 +258,21 @@ def test_squared_norm_beyond_fp64():
     assert np.isnan(E[a[1]])
     keep = np.arange(len(N1)) != a[1]
     close(E[keep], Er[keep])
+    # energies alone (no Ad) of an energy-trained model: an infinite distance is a zero
+    import ctypes
+    import torch
+    from kernelforge_b200 import _lib
+    with np.errstate(invalid="ignore"):
+        Er, _ = om.matvec(X1, None, X2, None, aE, Q1, Q2, N1, N2, 0.9)
+    x1, x2, ae = (torch.tensor(v, device="cuda") for v in (X1, X2, aE))
+    e = torch.empty(len(N1), dtype=torch.float64, device="cuda")
+    i = [np.ascontiguousarray(v, np.int32) for v in (Q1, Q2, N1, N2)]
+    _lib.check(_lib.lib().kfb_local_matvec(
+        x1.data_ptr(), None, x2.data_ptr(), None, ae.data_ptr(), *(v.ctypes.data for v in i),
+        len(N1), len(N2), X1.shape[1], X2.shape[1], X1.shape[2], ctypes.c_double(0.9),
+        _lib.KFB_F64, e.data_ptr(), None, torch.cuda.current_stream().cuda_stream))
+    assert np.isfinite(Er).all()
+    close(e.cpu().numpy(), Er)
 
 
 @pytest.mark.parametrize("kind", ["matvec", "descriptors"])

@@ -274,19 +274,22 @@ def test_many_labels(labels, precision):
 
 def test_squared_norm_beyond_fp64():
     """Finite values whose square is not: the norm is infinite and the pair's kernel zero, in a
-    column that the other set uses and in one that it does not; a value that is not finite
-    leaves its molecule undefined and no other."""
+    column that the other set uses and in one that it does not; an infinity leaves the entries
+    undefined whose products it makes so (all, in a column of zeros) and no other."""
     from kernelforge_b200 import local_kernels as lk
     X1, _, Q1, N1 = make_set(6, 6, 20, 3, 71)
-    X2, _, Q2, N2 = make_set(5, 6, 20, 3, 72)
+    X2, _, Q2, N2 = make_set(6, 6, 20, 3, 72)
     X1[:, :, 15:] = 0.0
     X2[1, 0, 3] = 1e160
     X2[3, 1, 17] = -1e200
     X2[4, 0, 2] = np.inf
+    X2[5, 0, 18] = np.inf
     with np.errstate(over="ignore", invalid="ignore"):
         ref = o.kernel_gaussian(X1, X2[:4], Q1, Q2[:4], N1, N2[:4], 2.5)
     assert np.isfinite(ref).all()
     got = lk.kernel_gaussian(X1, X2, Q1, Q2, N1, N2, 2.5)
     np.testing.assert_allclose(got[:, :4], ref, rtol=1e-12, atol=1e-13)
-    same = [np.isin(Q2[4, 0], Q1[a, :N1[a]]) for a in range(6)]
-    np.testing.assert_array_equal(np.isnan(got[:, 4]), same)
+    for b, k in ((4, 2), (5, 18)):
+        undefined = [np.any((Q1[a, :N1[a]] == Q2[b, 0]) & (X1[a, :N1[a], k] >= 0)) for a in range(6)]
+        np.testing.assert_array_equal(np.isnan(got[:, b]), undefined)
+        assert np.any(undefined)
