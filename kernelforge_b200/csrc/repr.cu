@@ -431,9 +431,12 @@ __global__ void __launch_bounds__(RG_WARPS * 32, 3) fchl19_grad_kernel(
         // its pair terms, must be finite (r is not where d's square is no FP64 number)
         const double rmax = fmax(P.rcut, P.acut);
         A[0] = r <= rmax ? r : 2.0 * rmax;
-        A[1] = d.x / r;
-        A[2] = d.y / r;
-        A[3] = d.z / r;
+        // (an atom at the centre has no direction: its own terms are undefined, the
+        // zeros of channels without a partner stay zeros)
+        const double rd = r == 0.0 ? 1.0 : r;
+        A[1] = d.x / rd;
+        A[2] = d.y / rd;
+        A[3] = d.z / rd;
         A[4] = half_cos_decay(r, P.acut);
         A[5] = -0.5 * M_PI / P.acut * sin(M_PI * r / P.acut);
         const TwoBody tb = two_body_terms(P, r);

@@ -211,3 +211,15 @@ def test_large_molecules(n):
         Rm[a, t] -= h
         fd = (fr.generate_fchl_acsf(Rp, Z) - fr.generate_fchl_acsf(Rm, Z)) / (2 * h)
         np.testing.assert_allclose(J[:, :, a, t], fd, rtol=1e-5, atol=1e-6 * np.abs(J).max())
+
+
+def test_coincident_atoms_without_a_triple():
+    """Two atoms at one place, the others beyond the cutoff of both: their pair terms are
+    undefined, the three-body rows, which hold no triple, are zero."""
+    from kernelforge_b200 import fchl19_repr as fr
+    R = np.array([[[0, 0, 0], [2, 0, 0], [2, 0, 0], [0, 1, 0]]], float)
+    Z = np.array([[1, 6, 6, 8]], np.int32)
+    X, dX = fr.generate_batched(R, Z, np.array([4], np.int32), gradients=True, dtype="float64",
+                                rcut=1.0, acut=1.0)
+    assert not X[..., 120:].any() and not dX[:, :, 120:].any()
+    assert not np.isfinite(X[0, 1, 24:48].cpu().numpy()).any()
