@@ -262,7 +262,6 @@ __global__ void __launch_bounds__(256) mv_rows_kernel(
     const Tin *x = (train ? x2 : x1) + at;
     const double *a = train && ad ? ad + at : nullptr;
     double n = 0.0, s = 0.0;
-    bool inf = false;
 #pragma unroll 3
     for (int k0 = 0; k0 < rep; k0 += 128) {
         const int k = k0 + 4 * lane;
@@ -293,7 +292,6 @@ __global__ void __launch_bounds__(256) mv_rows_kernel(
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             n = fma(v[u], v[u], n);
-            inf |= isinf(v[u]);
             s = fma(v[u], w[u], s);
             on |= !(v[u] == 0.0) || !(w[u] == 0.0);
         }
@@ -303,7 +301,11 @@ __global__ void __launch_bounds__(256) mv_rows_kernel(
         n += __shfl_xor_sync(0xffffffffu, n, o);
         s += __shfl_xor_sync(0xffffffffu, s, o);
     }
-    inf = __any_sync(0xffffffffu, inf);
+    bool inf = false;
+    if (!train && isinf(n)) {   // (warp-uniform; its values' sum or one of them)
+        for (int k = lane; k < rep; k += 32) inf |= isinf((double)x[k]);
+        inf = __any_sync(0xffffffffu, inf);
+    }
     if (lane == 0) {
         if (train) {
             n2[r - R1] = n;
